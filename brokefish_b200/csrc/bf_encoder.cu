@@ -1777,9 +1777,9 @@ __global__ void __launch_bounds__(kThreads, 1) encoder_kernel(const Params p) {
             }
         }
     } else if (warp == kProducerWarp) {
-        if (lane == 0) producer_loop<kAr>(smem, abort_flag, p, blockIdx.x, gridDim.x, n_tiles);
+        if (elect_one()) producer_loop<kAr>(smem, abort_flag, p, blockIdx.x, gridDim.x, n_tiles);
     } else {
-        if (lane == 0) mma_loop<kAr>(smem, tmem, abort_flag, p, blockIdx.x, gridDim.x, n_tiles, warp - kMmaWarp);
+        if (elect_one()) mma_loop<kAr>(smem, tmem, abort_flag, p, blockIdx.x, gridDim.x, n_tiles, warp - kMmaWarp);
     }
     __syncwarp();
     tc_fence_before();
