@@ -1,6 +1,7 @@
 // Legal-move generation and move application for the 32-slot piece-list board, in two forms:
 // `legal_word`, one warp per board with lane = slot (what the evaluator's expansion warp calls),
-// and the stand-alone kernels further down, one thread per board.
+// and the stand-alone kernels further down, eight lanes per board (launches that do not fill the
+// GPU) or one thread per board (the large ones).
 //
 // The contract of the reference's engine (brokefish/env/torch_impl.py:254-291, csrc/movegen.cuh):
 // `mask [n,32]` 64-bit words, bit s of word p set when the piece in slot p may legally move to
@@ -720,6 +721,435 @@ __global__ void __launch_bounds__(kTpbThreads) engine_board_kernel(
     if (mask != nullptr)
         for (int j = tid; j < here * 32; j += kTpbThreads)
             mask[first * 32 + j] = s_out[(j >> 5) * kTpbOutStride + (j & 31)];
+}
+
+// ------------------------------------------------------------------------------------------
+// EIGHT LANES per board, four boards per warp: the form of a launch that does not fill the GPU.
+// Lane j of a board holds slots j, 8 + j, 16 + j and 24 + j -- a white pawn, a white piece, a black
+// pawn and a black piece on almost every board -- and direction j of the eight a slider moves along.
+//
+// A small launch is bound by the length of one thread's chain.  A thread per board walks 32 slots
+// and then the mover's sixteen one after the other: 5,400 instructions from the first load to the
+// last store, 18 us for any number of boards up to 16,000 (39 us with a move before and a key
+// after).  With eight lanes a lane decodes four words, the bitboards are completed by three
+// xor-shuffles, the sliders' attacks are one fill with a different direction on every lane, so are
+// the king's rays, and the mover's sixteen slots are two passes (pawns together, pieces together):
+// 6 us (8 us) for 4096 boards.  It costs half as many instructions again as the thread form, so the
+// large launches, bound by the integer pipe, keep that one.  Boards and legal words need no staging:
+// a board's lanes read 16 contiguous bytes and write 64 at a time.
+// ------------------------------------------------------------------------------------------
+constexpr int kEngineThreads = 128;
+constexpr int kEngineBoards = kEngineThreads / 8;       // boards per block
+
+// ---- reductions over the eight lanes of a board (all 32 lanes of the warp take part) ----
+__device__ __forceinline__ unsigned group_or(unsigned v) {
+#pragma unroll
+    for (int off = 1; off < 8; off <<= 1) v |= __shfl_xor_sync(kFull, v, off);
+    return v;
+}
+__device__ __forceinline__ unsigned long long group_or(unsigned long long v) {
+    const unsigned lo = group_or(static_cast<unsigned>(v)), hi = group_or(static_cast<unsigned>(v >> 32));
+    return (static_cast<unsigned long long>(hi) << 32) | lo;
+}
+__device__ __forceinline__ int group_min(int v) {
+#pragma unroll
+    for (int off = 1; off < 8; off <<= 1) v = min(v, __shfl_xor_sync(kFull, v, off));
+    return v;
+}
+__device__ __forceinline__ unsigned pick_word(const unsigned (&w)[4], int i) {
+    const unsigned lo = (i & 1) ? w[1] : w[0], hi = (i & 1) ? w[3] : w[2];
+    return (i & 2) ? hi : lo;
+}
+__device__ __forceinline__ void put_word(unsigned (&w)[4], int i, unsigned v) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) w[k] = i == k ? v : w[k];
+}
+
+// A board as six bit planes over the squares: occupied, black, the three type bits, "special".
+struct Board {
+    unsigned long long occ, own;                 // own: the side to move's pieces
+    unsigned long long e_pawns, e_knights, e_diag, e_line, e_king, ep_pawns;   // the opponent's; its
+                                                 // pawns that have just made a double step
+    unsigned long long my_king, my_pawns, fresh_rooks;
+};
+__device__ __forceinline__ Board board_planes(const unsigned (&w)[4], bool black) {
+    unsigned long long occ = 0, blk = 0, t0 = 0, t1 = 0, t2 = 0, sp = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const unsigned word = w[i];
+        const unsigned long long bb = static_cast<unsigned long long>((word >> 11 & 1u) ^ 1u) << (word & 63u);
+        occ |= bb;
+        if (word & 0x400u) blk |= bb;
+        if (word & 0x040u) t0 |= bb;
+        if (word & 0x080u) t1 |= bb;
+        if (word & 0x100u) t2 |= bb;
+        if (word & 0x200u) sp |= bb;
+    }
+    occ = group_or(occ); blk = group_or(blk); t0 = group_or(t0); t1 = group_or(t1); t2 = group_or(t2); sp = group_or(sp);
+    Board b;
+    b.occ = occ;
+    b.own = black ? blk : occ & ~blk;
+    const unsigned long long opp = occ & ~b.own;
+    const unsigned long long pawns = occ & ~(t0 | t1 | t2), queens = t2 & ~(t1 | t0);
+    b.e_pawns = opp & pawns;
+    b.my_pawns = b.own & pawns;
+    b.ep_pawns = b.e_pawns & sp;
+    b.e_knights = opp & t0 & ~(t1 | t2);
+    b.e_diag = opp & ((t1 & ~(t0 | t2)) | queens);
+    b.e_line = opp & ((t1 & t0 & ~t2) | queens);
+    const unsigned long long kings = t2 & t0 & ~t1;
+    b.e_king = opp & kings;
+    b.my_king = b.own & kings;
+    b.fresh_rooks = b.own & t1 & t0 & ~(t2 | sp);
+    return b;
+}
+// Is the mover's king attacked when the occupancy is `after` and the pawn `gone` has left?  (What
+// an en passant capture, which takes two pieces off one rank at once, has to be tested with.)
+__device__ __forceinline__ bool king_hit(const Board& b, bool black, unsigned long long after, unsigned long long gone) {
+    if (b.my_king == 0ull) return false;
+    const int sq = __ffsll(static_cast<long long>(b.my_king)) - 1;
+    return (knight_pattern(b.my_king) & b.e_knights) != 0ull ||
+           (pawn_attacks(b.my_king, black) & (b.e_pawns & ~gone)) != 0ull ||
+           (king_pattern(b.my_king) & b.e_king) != 0ull ||
+           ((line_attacks(b.my_king, after, diag_ex(sq)) | line_attacks(b.my_king, after, anti_ex(sq))) & b.e_diag) != 0ull ||
+           ((line_attacks(b.my_king, after, rank_ex(sq)) | line_attacks(b.my_king, after, file_ex(sq))) & b.e_line) != 0ull;
+}
+// The set's bits spread over empty squares by `s` squares a step (doubling steps 1, 2, 4), then one
+// more step lands on the first occupied square; `wrap` clears the file a step must not arrive on.
+__device__ __forceinline__ unsigned long long fill_up(unsigned long long gen, unsigned long long occ, int s,
+                                                      unsigned long long wrap) {
+    unsigned long long pro = ~occ & wrap;
+    gen |= pro & (gen << s);
+    pro &= pro << s;
+    gen |= pro & (gen << (2 * s));
+    pro &= pro << (2 * s);
+    gen |= pro & (gen << (4 * s));
+    return (gen << s) & wrap;
+}
+
+// Legal words of the board into `mask` (the board's 32 words); returns whether the side to move is
+// in check.  `store`: this board is to be written.
+__device__ __forceinline__ bool group_moves(const unsigned (&w)[4], const Board& b, bool black, int lane, bool store,
+                                            unsigned long long* mask) {
+    const int j = lane & 7;
+    const unsigned long long occ = b.occ, own = b.own, opp = occ & ~own, my_king = b.my_king;
+    const int king_sq = my_king ? __ffsll(static_cast<long long>(my_king)) - 1 : 0;
+    // ---- this lane's direction: up the board for lanes 0-3 (file, rank, the two diagonals), the
+    //      same on the reversed board for lanes 4-7.  What the opponent's sliders attack along it
+    //      with the mover's king lifted off the board; whether the first piece from the king is a
+    //      checker; whether it is an own piece that shields the king from a slider behind it ----
+    unsigned long long danger, answers, pinned;
+    bool checks;
+    {
+        const int k = j & 3;
+        const bool down = (j & 4) != 0;
+        const int s = (0x7918 >> (4 * k)) & 15;
+        const unsigned long long wrap = k == 0 ? ~0ull : (k == 3 ? ~kFileH : ~kFileA);
+        auto flip = [&](unsigned long long v) { return down ? __brevll(v) : v; };
+        const unsigned long long O = flip(occ), E = flip(k < 2 ? b.e_line : b.e_diag), K = flip(my_king), W = flip(own);
+        danger = flip(fill_up(E, O & ~K, s, wrap));
+        // the king's ray, and the ray from the first piece on it: on the whole line through the
+        // king, subtracting a piece's bit from the occupancy flips the squares up to and including
+        // the next occupied one
+        const int ks = down ? 63 - king_sq : king_sq, kr = ks >> 3, kf = ks & 7;
+        const int sh = k == 0 ? kf : 8 * (k == 1 ? kr : (k == 2 ? kr - kf : kr + kf - 7));
+        const unsigned long long base = k == 0 ? kFileA : (k == 1 ? 0xFFull : (k == 2 ? 0x8040201008040201ull : 0x0102040810204080ull));
+        const unsigned long long line = sh >= 0 ? base << sh : base >> -sh;
+        const unsigned long long o1 = O & line & ~K, ray = (o1 ^ (o1 - K)) & line & ~K;
+        checks = (ray & E) != 0ull;
+        answers = checks ? flip(ray) : 0ull;
+        const unsigned long long shield = ray & W, o2 = o1 & ~shield;
+        pinned = ((o2 ^ (o2 - shield)) & line & ~shield & E) ? flip(shield) : 0ull;
+    }
+    danger = group_or(danger) | pawn_attacks(b.e_pawns, !black) | knight_pattern(b.e_knights) | king_pattern(b.e_king);
+    answers = group_or(answers);
+    pinned = group_or(pinned);
+    const unsigned long long leapers = (knight_pattern(my_king) & b.e_knights) | (pawn_attacks(my_king, black) & b.e_pawns);
+    const int checkers = __popc((__ballot_sync(kFull, checks) >> (lane & 24)) & 0xFFu) + __popcll(leapers);
+    const bool chk = checkers != 0;
+    // one checker: the other pieces may only capture it or step between; two: only the king moves
+    const unsigned long long target_mask = checkers == 0 ? ~0ull : (checkers == 1 ? answers | leapers : 0ull);
+
+    // ---- the mover's pieces: its pawn slots, then its piece slots; the other colour's slots only
+    //      when some board of the warp does not keep the colours apart by slot ----
+    bool mine[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) mine[i] = (w[i] & 0x800u) == 0u && ((w[i] & 0x400u) != 0u) == black;
+    const bool stray = black ? (mine[0] || mine[1]) : (mine[2] || mine[3]);
+    const int passes = __any_sync(kFull, stray) ? 4 : 2;
+#pragma unroll 1
+    for (int pass = 0; pass < passes; ++pass) {
+        const int i = black ? pass ^ 2 : pass;
+        const unsigned word = pick_word(w, i);
+        unsigned long long legal = 0ull;
+        if ((word & 0x800u) == 0u && ((word & 0x400u) != 0u) == black) {
+            const bool special = (word & 0x200u) != 0u;
+            const int type = (word >> 6) & 7, sq = word & 63;
+            const unsigned long long bb = 1ull << sq;
+            if (type == KING) {
+                legal = king_pattern(bb) & ~danger;
+                // castling: neither the king's square nor the one it crosses nor the one it lands on
+                // may be attacked
+                if (!special && !chk) {
+                    const int row = black ? 56 : 0;
+                    if ((b.fresh_rooks >> (row + 7)) & 1ull)
+                        if (((occ >> (row + 5)) & 3ull) == 0ull && ((danger >> (row + 5)) & 3ull) == 0ull)
+                            legal |= 1ull << (row + 6);
+                    if ((b.fresh_rooks >> row) & 1ull)
+                        if (((occ >> (row + 1)) & 7ull) == 0ull && ((danger >> (row + 2)) & 3ull) == 0ull)
+                            legal |= 1ull << (row + 2);
+                }
+                legal &= ~own;
+            } else {
+                unsigned long long cand = 0ull, ep = 0ull;
+                if (type == PAWN) {
+                    const int rank = sq >> 3;
+                    unsigned long long one, two;
+                    if (black) {
+                        one = (bb >> 8) & ~occ;
+                        two = rank == 6 ? (one >> 8) & ~occ : 0ull;
+                    } else {
+                        one = (bb << 8) & ~occ;
+                        two = rank == 1 ? (one << 8) & ~occ : 0ull;
+                    }
+                    const unsigned long long att = pawn_attacks(bb, black);
+                    cand = one | two | (att & opp);
+                    // en passant: an enemy pawn that has just made its double step stands beside us
+                    if (b.ep_pawns != 0ull && rank == (black ? 3 : 4))
+                        ep = att & (black ? b.ep_pawns >> 8 : b.ep_pawns << 8) & ~own;
+                } else if (type == KNIGHT) {
+                    cand = knight_pattern(bb);
+                } else {
+                    if (type == BISHOP || type == QUEEN)
+                        cand |= line_attacks(bb, occ, diag_ex(sq)) | line_attacks(bb, occ, anti_ex(sq));
+                    if (type == ROOK || type == QUEEN)
+                        cand |= line_attacks(bb, occ, rank_ex(sq)) | line_attacks(bb, occ, file_ex(sq));
+                }
+                legal = cand & ~own & target_mask;
+                if (bb & pinned) legal &= line_through(king_sq, sq);
+                for (; ep != 0ull; ep &= ep - 1ull) {
+                    const unsigned long long tb = ep & (0ull - ep);
+                    const unsigned long long gone = black ? tb << 8 : tb >> 8;
+                    if (!king_hit(b, black, ((occ & ~bb) & ~gone) | tb, gone)) legal |= tb;
+                }
+            }
+        }
+        if (store) mask[8 * i + j] = legal;
+    }
+    if (passes == 2 && store) {
+        mask[(black ? 0 : 16) + j] = 0ull;
+        mask[(black ? 8 : 24) + j] = 0ull;
+    }
+    return chk;
+}
+
+// Castling rights KQkq as four bits (torch_impl.py:294-318).
+__device__ __forceinline__ unsigned group_rights(const unsigned (&w)[4]) {
+    unsigned f = 0u;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const unsigned word = w[i];
+        if (word & 0xA00u) continue;                                // captured, or has moved
+        const bool is_black = (word & 0x400u) != 0u;
+        const int type = (word >> 6) & 7, sq = word & 63;
+        if (type == KING) f |= is_black ? 32u : 16u;
+        if (type == ROOK) {
+            if (!is_black) f |= (sq == 7 ? 1u : 0u) | (sq == 0 ? 2u : 0u);
+            else           f |= (sq == 63 ? 4u : 0u) | (sq == 56 ? 8u : 0u);
+        }
+    }
+    f = group_or(f);
+    return ((f & 16u) ? f & 3u : 0u) | ((f & 32u) ? f & 12u : 0u);
+}
+// Apply one move (`move` = slot * 64 + target, -1 = no move; `promo` 0..3 = N B R Q, negative =
+// queen): the reference's `step` without its hash (brokefish/env/torch_impl.py:412-548).  Capture:
+// the first live piece on the target square, or for a pawn the en passant victim, which carries the
+// double-step flag and stands beside the target's file neighbour, not on it.  `irreversible`:
+// capture, pawn move or a change of castling rights.
+__device__ __forceinline__ void group_step(unsigned (&w)[4], int lane, int control, int move, int promo, int& new_control,
+                                           bool& irreversible) {
+    const int j = lane & 7;
+    const bool moves = move >= 0;
+    const int source = moves ? (move >> 6) & 31 : 0, target = move & 63;
+    const bool white = control > 0;
+    const unsigned mover = __shfl_sync(kFull, pick_word(w, source >> 3), source & 7, 8);
+    const int mtype = (mover >> 6) & 7, from = mover & 63;
+    const bool is_pawn = mtype == PAWN;
+    const unsigned rights_before = group_rights(w);
+    const unsigned victim_word = ((white ? 3u : 1u) << 9) + static_cast<unsigned>(target + (white ? -8 : 8));
+    const int dx = target - from;
+    const bool castling = moves && mtype == KING && (dx == 2 || dx == -2);
+    int captured = 32;
+#pragma unroll
+    for (int i = 3; i >= 0; --i)
+        if (((w[i] & 0x800u) == 0u && static_cast<int>(w[i] & 63u) == target) || (is_pawn && w[i] == victim_word))
+            captured = 8 * i + j;
+    captured = group_min(captured);
+    // the corner rook is looked for by its square before anything moved, by its type after the capture
+    int rook = 32;
+    if (__any_sync(kFull, castling)) {
+        const int corner = (white ? 0 : 56) + (dx > 0 ? 7 : 0);
+#pragma unroll
+        for (int i = 3; i >= 0; --i)
+            if (castling && 8 * i + j != captured && ((w[i] >> 6) & 7u) == ROOK && static_cast<int>(w[i] & 63u) == corner)
+                rook = 8 * i + j;
+        rook = group_min(rook);
+    }
+    if (moves) {
+        if ((captured & 7) == j && captured < 32) put_word(w, captured >> 3, 1u << 11);
+        if ((source & 7) == j) {
+            unsigned v = (pick_word(w, source >> 3) & ~63u & 0xFFFu) + static_cast<unsigned>(target);
+            if (is_pawn && (target >> 3) == (white ? 7 : 0))
+                v += static_cast<unsigned>(promo < 0 ? QUEEN : promo + KNIGHT) << 6;
+            if (mtype == KING || mtype == ROOK) v |= 1u << 9;
+            put_word(w, source >> 3, v);
+        }
+        if ((rook & 7) == j && rook < 32)
+            put_word(w, rook >> 3,
+                     (pick_word(w, rook >> 3) & ~63u & 0xFFFu) + static_cast<unsigned>((white ? 0 : 56) + (dx > 0 ? 5 : 3)));
+        // the en passant flag lives for one ply: clear every pawn's, set the double-stepper's
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if ((w[i] & 0x3C0u) == 0x200u) w[i] = w[i] & ~(1u << 9) & 0xFFFu;
+        if (is_pawn && (dx == 16 || dx == -16) && (source & 7) == j)
+            put_word(w, source >> 3, pick_word(w, source >> 3) | (1u << 9));
+    }
+    const unsigned rights_after = group_rights(w);
+    const bool reset = captured < 32 || is_pawn;
+    const int mag = reset ? 1 : (control < 0 ? -control : control) + 1;
+    new_control = moves ? (white ? -mag : mag) : control;
+    irreversible = moves && (reset || rights_after != rights_before);
+}
+
+// Key of a board.  The en passant file counts only when a capture is really available: a pawn of the
+// mover stands beside the pawn that has just made its double step, and taking it does not leave the
+// mover's king attacked.
+__device__ __forceinline__ unsigned long long group_hash(const unsigned (&w)[4], const Board& b, bool black, int lane) {
+    unsigned long long h = 0ull;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const unsigned word = w[i];
+        const int type = (word >> 6) & 7, sq = word & 63;
+        if ((word & 0x800u) == 0u) h ^= zobrist_key((((word & 0x400u) ? 6 : 0) + type) * 64 + sq);
+    }
+    // side to move and rights: one key each on lanes of their own
+    const unsigned rights = group_rights(w);
+    const int j = lane & 7;
+    const bool own_key = j < 4 ? ((rights >> j) & 1u) != 0u : (j == 4 && black);
+    if (own_key) h ^= zobrist_key(j < 4 ? ZOBRIST_CASTLE + j : ZOBRIST_SIDE);
+    unsigned lo = static_cast<unsigned>(h), hi = static_cast<unsigned>(h >> 32);
+#pragma unroll
+    for (int off = 1; off < 8; off <<= 1) {
+        lo ^= __shfl_xor_sync(kFull, lo, off);
+        hi ^= __shfl_xor_sync(kFull, hi, off);
+    }
+    h = (static_cast<unsigned long long>(hi) << 32) | lo;
+    if (b.ep_pawns != 0ull) {
+        const unsigned long long victim = b.ep_pawns & (0ull - b.ep_pawns);
+        const unsigned long long target = black ? victim >> 8 : victim << 8;
+        bool legal = false;
+#pragma unroll 1
+        for (int side = 0; side < 2; ++side) {
+            const unsigned long long capturer = side ? ((victim << 1) & ~kFileA) : ((victim >> 1) & ~kFileH);
+            if ((capturer & b.my_pawns) != 0ull)
+                legal |= !king_hit(b, black, ((b.occ & ~capturer) & ~victim) | target, victim);
+        }
+        if (legal) h ^= zobrist_key(ZOBRIST_EP + ((__ffsll(static_cast<long long>(victim)) - 1) & 7));
+    }
+    return h;
+}
+
+// kStep: play `move` first (or, with kPick, the floor(r * count)-th legal move of the incoming
+// `mask` in (slot, square) order; a board without legal moves stays as it is) and write the new
+// board, control word and irreversible flag; `mask` non-null: the legal words of the resulting
+// board follow; `hash_out` non-null: its key.  In place (boards_out == boards) is safe: a board's
+// lanes read all of it first.
+template <bool kStep, bool kPick>
+__global__ void __launch_bounds__(kEngineThreads) engine_group_kernel(
+        const uint16_t* boards, const int16_t* control, const int* __restrict__ move,
+        const signed char* __restrict__ promo, const float* __restrict__ r, int n, uint16_t* boards_out,
+        int16_t* control_out, unsigned char* __restrict__ irreversible, unsigned long long* mask,
+        unsigned char* __restrict__ in_check, int* __restrict__ move_out, unsigned long long* __restrict__ hash_out) {
+    const int lane = threadIdx.x & 31, j = lane & 7;
+    const long board = static_cast<long>(blockIdx.x) * kEngineBoards + (threadIdx.x >> 3);
+    const bool valid = board < n;
+    unsigned w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = valid ? boards[board * 32 + 8 * i + j] : 0x800u;
+    int ctl = valid ? control[board] : 1;
+    unsigned long long* words = mask + board * 32;
+    const bool generate = mask != nullptr;
+    bool moved = true;
+    if (kStep) {
+        int mv;
+        if (kPick) {
+            // this lane's legal words and, packed two counts to a register, their running totals
+            // over the lanes: the order is slot-major, that is lane by lane within each i
+            unsigned long long m[4];
+            unsigned cnt[4], run[2];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                m[i] = valid ? words[8 * i + j] : 0ull;
+                cnt[i] = __popcll(m[i]);
+            }
+            run[0] = cnt[0] | (cnt[1] << 16);
+            run[1] = cnt[2] | (cnt[3] << 16);
+#pragma unroll
+            for (int off = 1; off < 8; off <<= 1) {
+                const unsigned a = __shfl_up_sync(kFull, run[0], off, 8), c = __shfl_up_sync(kFull, run[1], off, 8);
+                if (j >= off) { run[0] += a; run[1] += c; }
+            }
+            const unsigned all0 = __shfl_sync(kFull, run[0], 7, 8), all1 = __shfl_sync(kFull, run[1], 7, 8);
+            const int sum[4] = {static_cast<int>(all0 & 0xFFFFu), static_cast<int>(all0 >> 16),
+                                static_cast<int>(all1 & 0xFFFFu), static_cast<int>(all1 >> 16)};
+            const int total = sum[0] + sum[1] + sum[2] + sum[3];
+            int pick = valid ? static_cast<int>(__fmul_rn(r[board], static_cast<float>(total))) : 0;
+            pick = pick < total - 1 ? pick : total - 1;
+            mv = 0x7fffffff;
+            int before = 0;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int upto = before + static_cast<int>((i & 1) ? run[i >> 1] >> 16 : run[i >> 1] & 0xFFFFu);
+                int rest = pick - (upto - static_cast<int>(cnt[i]));
+                if (total > 0 && rest >= 0 && pick < upto) {
+                    unsigned long long v = m[i];
+                    for (; rest > 0; --rest) v &= v - 1ull;
+                    mv = (8 * i + j) * 64 + __ffsll(static_cast<long long>(v)) - 1;
+                }
+                before += sum[i];
+            }
+            mv = group_min(mv);
+            if (mv == 0x7fffffff) mv = -1;
+            moved = mv >= 0;
+            if (move_out != nullptr && valid && j == 0) move_out[board] = mv;
+        } else {
+            mv = valid ? move[board] : -1;
+        }
+        int nc;
+        bool irr;
+        group_step(w, lane, ctl, mv, promo != nullptr && valid ? promo[board] : -1, nc, irr);
+        if (valid && moved) {
+            if (j == 0) {
+                control_out[board] = static_cast<int16_t>(nc);
+                if (irreversible != nullptr) irreversible[board] = irr ? 1 : 0;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) boards_out[board * 32 + 8 * i + j] = static_cast<uint16_t>(w[i]);
+        }
+        ctl = nc;
+    }
+    if (!generate && hash_out == nullptr) return;
+    const bool black = ctl < 0;
+    const Board b = board_planes(w, black);
+    if (generate) {
+        // a finished game of a playout keeps its (empty) legal words
+        const bool chk = group_moves(w, b, black, lane, valid && moved, words);
+        if (in_check != nullptr && valid && j == 0) in_check[board] = chk ? 1 : 0;
+    }
+    if (hash_out != nullptr) {
+        const unsigned long long h = group_hash(w, b, black, lane);
+        if (valid && j == 0) hash_out[board] = h;
+    }
 }
 
 // Why a game is over, one thread per board (brokefish/env/torch_impl.py:632-676): 1 checkmate,

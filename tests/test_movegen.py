@@ -269,3 +269,27 @@ def test_position_keys_repetition_ring_and_threefold_rule():
     packed = np.concatenate([p["boards"].view(np.uint16).astype(np.int64), p["control"][:, None].astype(np.int64)], axis=1)
     assert len(np.unique(keys)) <= len(np.unique(packed, axis=0))
     assert len(np.unique(keys)) >= 0.9 * len(np.unique(packed, axis=0))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 3, 4097, 49152, 49153, 98304, 98305])
+def test_both_forms_of_the_engine_kernels_agree_at_every_size(n, pos4096):
+    """The launches pick eight lanes or one thread per board by their size: on either side of the
+    line, and with a ragged last block, every board gets the answer it gets in a batch of 4096."""
+    from brokefish_b200 import env
+    cu = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    boards, control = cu(pos4096["boards"]), cu(pos4096["control"])
+    place = torch.arange(n, device="cuda") % 4096
+    mask, chk = env.movegen(boards, control)
+    moves = mask.ne(0).float().argmax(dim=1)
+    word = mask.gather(1, moves[:, None])
+    square = ((word >> torch.arange(64, device="cuda")) & 1).argmax(dim=1)
+    move = torch.where(mask.ne(0).any(dim=1), moves * 64 + square, torch.full_like(moves, -1))
+    promo = torch.arange(4096, device="cuda") % 4
+    key = env.hash_position(boards, control)
+    want = (mask, chk, key) + env.step(boards, control, move, promo, with_moves=True, hash=key)
+    b, c = boards[place], control[place]
+    got = env.movegen(b, c) + (env.hash_position(b, c),) + \
+        env.step(b, c, move[place], promo[place], with_moves=True, hash=key[place])
+    for g, w in zip(got, want):
+        assert torch.equal(g, w[place])
