@@ -1,16 +1,20 @@
-"""Build and load the C-ABI shared library (``libbrokefish_b200.so``).
+"""Build and load the C-ABI shared library (``libbrokefish_b200.so``) and the PyTorch binding
+of its short calls (``_torch_ops.so``).
 
-The library is built in-tree with one ``nvcc`` line for sm_100a; there is no JIT cache
-and no fallback: if the library is missing or does not load, every entry point of the
-package that needs the GPU raises.
+The library is built in-tree with one ``nvcc`` line for sm_100a, the binding with one ``g++``
+line against the torch headers; there is no JIT cache
+and no fallback: if either is missing or does not load, every entry point of the
+package that needs it raises.
 """
 
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
 import shutil
 import subprocess
+import sysconfig
 from typing import List, Optional
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
@@ -24,6 +28,11 @@ DEPS = SOURCES + [os.path.join(PKG_DIR, "csrc", name) for name in
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
               "-Xcompiler", "-fPIC", "-shared", "-diag-suppress", "177,550"]
 
+#: The binding, its source and what it depends on.
+OPS_PATH = os.path.join(PKG_DIR, "_torch_ops.so")
+OPS_SOURCE = os.path.join(PKG_DIR, "csrc", "bf_torch.cpp")
+OPS_DEPS = [OPS_SOURCE, os.path.join(ROOT, "include", "brokefish_b200.h")]
+
 #: Every symbol ``include/brokefish_b200.h`` declares.
 EXPORTS = ["bf_version", "bf_last_error", "bf_create", "bf_destroy", "bf_info", "bf_forward",
            "bf_forward_stage", "bf_forward_stage_at", "bf_forward_capture", "bf_forward_host", "bf_status",
@@ -32,7 +41,7 @@ EXPORTS = ["bf_version", "bf_last_error", "bf_create", "bf_destroy", "bf_info", 
            "bf_forward_priors_host", "bf_selftest_timeout", "bf_movegen", "bf_step", "bf_random_ply",
            "bf_forward_leaves", "bf_measure_elementwise", "bf_forward_backbone", "bf_int8_q_max",
            "bf_fp8_q_max", "bf_terminal", "bf_hash", "bf_history_push",
-           "bf_repetition_count"]
+           "bf_repetition_count", "bf_history_push_to", "bf_terminal_history"]
 
 
 def nvcc_path() -> str:
@@ -42,25 +51,45 @@ def nvcc_path() -> str:
     return cand
 
 
-def is_stale() -> bool:
-    if not os.path.exists(LIB_PATH):
+def is_stale(path: str = LIB_PATH, deps: Optional[List[str]] = None) -> bool:
+    if not os.path.exists(path):
         return True
-    built = os.path.getmtime(LIB_PATH)
-    return any(os.path.getmtime(p) > built for p in DEPS)
+    built = os.path.getmtime(path)
+    return any(os.path.getmtime(p) > built for p in (DEPS if deps is None else deps))
 
 
-def build(force: bool = False, verbose: bool = False, extra: Optional[List[str]] = None) -> str:
-    """Compile the library if it is missing or older than its sources."""
-    if not force and not is_stale():
-        return LIB_PATH
-    cmd = [nvcc_path()] + NVCC_FLAGS + (extra or []) + ["-o", LIB_PATH] + SOURCES
+def _compile(cmd: List[str], verbose: bool) -> None:
     res = subprocess.run(cmd, capture_output=True, text=True)
     if verbose or res.returncode != 0:
         print(" ".join(cmd))
         print(res.stdout)
         print(res.stderr)
     if res.returncode != 0:
-        raise RuntimeError(f"nvcc failed with code {res.returncode}:\n{res.stderr[-4000:]}")
+        raise RuntimeError(f"{cmd[0]} failed with code {res.returncode}:\n{res.stderr[-4000:]}")
+
+
+def build_ops(force: bool = False, verbose: bool = False) -> str:
+    """Compile the PyTorch binding if it is missing or older than its sources."""
+    if not force and not is_stale(OPS_PATH, OPS_DEPS):
+        return OPS_PATH
+    import torch
+    from torch.utils.cpp_extension import CUDA_HOME, include_paths
+    inc = include_paths() + [sysconfig.get_paths()["include"],
+                             os.path.join(CUDA_HOME or os.path.dirname(os.path.dirname(nvcc_path())), "include")]
+    libs = os.path.join(os.path.dirname(torch.__file__), "lib")
+    _compile(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=_torch_ops",
+              f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+             + [a for i in inc for a in ("-isystem", i)]
+             + [OPS_SOURCE, "-o", OPS_PATH, f"-L{libs}", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda",
+                "-ltorch_python", "-ldl"], verbose)
+    return OPS_PATH
+
+
+def build(force: bool = False, verbose: bool = False, extra: Optional[List[str]] = None) -> str:
+    """Compile the library and the binding if they are missing or older than their sources."""
+    if force or is_stale():
+        _compile([nvcc_path()] + NVCC_FLAGS + (extra or []) + ["-o", LIB_PATH] + SOURCES, verbose)
+    build_ops(force, verbose)
     return LIB_PATH
 
 
@@ -104,6 +133,8 @@ def lib() -> ctypes.CDLL:
     L.bf_hash.argtypes = [i32, vp, vp, i32, vp, vp]
     L.bf_history_push.argtypes = [i32, vp, vp, vp, vp, i32, vp]
     L.bf_repetition_count.argtypes = [i32, vp, vp, vp, i32, vp, vp]
+    L.bf_history_push_to.argtypes = [i32, vp, vp, vp, vp, i32, vp, vp, vp]
+    L.bf_terminal_history.argtypes = [i32, vp, vp, vp, vp, vp, vp, vp, i32, vp, vp, vp]
     L.bf_random_ply.argtypes = [i32, vp, vp, vp, vp, vp, i32, vp, vp]
     L.bf_step.argtypes = [i32, vp, vp, vp, vp, i32, vp, vp, vp, vp, vp, vp, vp]
     L.bf_forward_priors_host.argtypes = [vp, vp, vp, vp, vp, i32, i32, vp, vp, vp, vp]
@@ -143,3 +174,22 @@ def check(rc: int, what: str) -> None:
     if rc == -3:
         raise NotImplementedError(f"{what}: {msg}")
     raise NativeError(f"{what} failed ({rc}): {msg}")
+
+
+_OPS = None
+
+
+def torch_ops():
+    """The PyTorch binding, bound to the library.  Raises if either is not built."""
+    global _OPS
+    if _OPS is None:
+        lib()
+        if not os.path.exists(OPS_PATH):
+            raise RuntimeError(f"{OPS_PATH} is not built; run `python -c 'import __graft_entry__ as g; g.build()'`")
+        import torch  # noqa: F401  (its libraries have to be loaded first)
+        spec = importlib.util.spec_from_file_location("_torch_ops", OPS_PATH)
+        ops = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(ops)
+        ops.bind(os.path.abspath(LIB_PATH), check)
+        _OPS = ops
+    return _OPS

@@ -2536,6 +2536,28 @@ int bf_history_push(int device, uint64_t* ring, long long* length, const uint64_
     return BF_OK;
 }
 
+int bf_history_push_to(int device, const uint64_t* ring, const long long* length, const uint64_t* hash,
+                       const unsigned char* irreversible, int n, uint64_t* new_ring, long long* new_length,
+                       void* stream) {
+    if (n < 0) return fail(BF_EINVAL, "n must be >= 0");
+    if (n == 0) return BF_OK;
+    if (ring == nullptr || length == nullptr || hash == nullptr || irreversible == nullptr || new_ring == nullptr ||
+        new_length == nullptr)
+        return fail(BF_EINVAL, "ring, length, hash, irreversible and both outputs must be non-null");
+    BF_ON_DEVICE(device);
+    const auto* src = reinterpret_cast<const unsigned long long*>(ring);
+    const auto* key = reinterpret_cast<const unsigned long long*>(hash);
+    auto* dst = reinterpret_cast<unsigned long long*>(new_ring);
+    const bool wide = ((reinterpret_cast<uintptr_t>(ring) | reinterpret_cast<uintptr_t>(new_ring)) & 15u) == 0;
+    const long pieces = static_cast<long>(n) * (wide ? bfmg::kMaxHistory / 2 : bfmg::kMaxHistory);
+    const unsigned blocks = static_cast<unsigned>((pieces + 255) / 256);
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (wide) bfmg::history_push_to_kernel<2><<<blocks, 256, 0, s>>>(src, length, key, irreversible, n, dst, new_length);
+    else      bfmg::history_push_to_kernel<1><<<blocks, 256, 0, s>>>(src, length, key, irreversible, n, dst, new_length);
+    BF_CUDA(cudaGetLastError());
+    return BF_OK;
+}
+
 int bf_repetition_count(int device, const uint64_t* hash, const uint64_t* ring, const long long* length, int n,
                         int* count, void* stream) {
     if (n < 0) return fail(BF_EINVAL, "n must be >= 0");
@@ -2543,7 +2565,7 @@ int bf_repetition_count(int device, const uint64_t* hash, const uint64_t* ring, 
     if (ring == nullptr || length == nullptr || hash == nullptr || count == nullptr)
         return fail(BF_EINVAL, "hash, ring, length and count must be non-null");
     BF_ON_DEVICE(device);
-    bfmg::repetition_kernel<<<(n + 127) / 128, 128, 0, static_cast<cudaStream_t>(stream)>>>(
+    bfmg::repetition_kernel<<<(n + 3) / 4, 128, 0, static_cast<cudaStream_t>(stream)>>>(
         reinterpret_cast<const unsigned long long*>(hash), reinterpret_cast<const unsigned long long*>(ring), length,
         n, count);
     BF_CUDA(cudaGetLastError());
@@ -2565,18 +2587,38 @@ int bf_step(int device, const uint16_t* boards, const int16_t* control, const in
     return BF_OK;
 }
 
+namespace {
+int launch_terminal(int device, const uint64_t* mask, const unsigned char* in_check, const int16_t* control,
+                    const uint16_t* boards, const int* rep_count, const uint64_t* hash, const uint64_t* ring,
+                    const long long* length, int n, unsigned char* code, signed char* result, void* stream) {
+    if (mask == nullptr || in_check == nullptr || control == nullptr || boards == nullptr || code == nullptr)
+        return fail(BF_EINVAL, "mask, in_check, control, boards and code must be non-null");
+    BF_ON_DEVICE(device);
+    bfmg::terminal_kernel<<<(n + 3) / 4, 128, 0, static_cast<cudaStream_t>(stream)>>>(
+        reinterpret_cast<const unsigned long long*>(mask), in_check, control, boards, rep_count,
+        reinterpret_cast<const unsigned long long*>(hash), reinterpret_cast<const unsigned long long*>(ring), length, n,
+        code, result);
+    BF_CUDA(cudaGetLastError());
+    return BF_OK;
+}
+}  // namespace
+
 int bf_terminal(int device, const uint64_t* mask, const unsigned char* in_check, const int16_t* control,
                 const uint16_t* boards, const int* rep_count, int n, unsigned char* code, signed char* result,
                 void* stream) {
     if (n < 0) return fail(BF_EINVAL, "n must be >= 0");
     if (n == 0) return BF_OK;
-    if (mask == nullptr || in_check == nullptr || control == nullptr || boards == nullptr || code == nullptr)
-        return fail(BF_EINVAL, "mask, in_check, control, boards and code must be non-null");
-    BF_ON_DEVICE(device);
-    bfmg::terminal_kernel<<<(n + 127) / 128, 128, 0, static_cast<cudaStream_t>(stream)>>>(
-        reinterpret_cast<const unsigned long long*>(mask), in_check, control, boards, rep_count, n, code, result);
-    BF_CUDA(cudaGetLastError());
-    return BF_OK;
+    return launch_terminal(device, mask, in_check, control, boards, rep_count, nullptr, nullptr, nullptr, n, code, result, stream);
+}
+
+int bf_terminal_history(int device, const uint64_t* mask, const unsigned char* in_check, const int16_t* control,
+                        const uint16_t* boards, const uint64_t* hash, const uint64_t* ring, const long long* length,
+                        int n, unsigned char* code, signed char* result, void* stream) {
+    if (n < 0) return fail(BF_EINVAL, "n must be >= 0");
+    if (n == 0) return BF_OK;
+    if (hash == nullptr || ring == nullptr || length == nullptr)
+        return fail(BF_EINVAL, "hash, ring and length must be non-null");
+    return launch_terminal(device, mask, in_check, control, boards, nullptr, hash, ring, length, n, code, result, stream);
 }
 
 int bf_random_ply(int device, uint16_t* boards, int16_t* control, uint64_t* mask, const float* r,

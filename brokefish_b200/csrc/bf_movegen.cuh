@@ -1152,51 +1152,61 @@ __global__ void __launch_bounds__(kEngineThreads) engine_group_kernel(
     }
 }
 
-// Why a game is over, one thread per board (brokefish/env/torch_impl.py:632-676): 1 checkmate,
+// How many of the first `length` entries of a game's ring equal `hash`: warp-collective.
+constexpr int kMaxHistory = 100;
+__device__ __forceinline__ int ring_matches(const unsigned long long* __restrict__ ring, long long length,
+                                            unsigned long long hash, int lane) {
+    const int len = static_cast<int>(length < kMaxHistory ? length : kMaxHistory);
+    int c = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int i = 32 * k + lane;
+        if (i < len) c += ring[i] == hash;
+    }
+    return static_cast<int>(__reduce_add_sync(kFull, static_cast<unsigned>(c)));
+}
+
+// Why a game is over (brokefish/env/torch_impl.py:632-676): 1 checkmate,
 // 2 stalemate (no legal move, with or without check), else 3 when the control word's magnitude
 // has reached 101 (fifty moves without capture or pawn move), else 4 when the position has
-// occurred three times (`rep_count`, from `repetition_kernel`; skipped when null), else 5 when
-// neither side can mate -- no pawn, rook or queen and
+// occurred three times (`rep_count` when it is given, else counted in the game's `ring`; skipped
+// without either), else 5 when neither side can mate -- no pawn, rook or queen and
 // either no knight and every bishop on one colour of squares, or one knight and no bishop
 // (torch_impl.py:604-629) -- else 0.  `result` is -1 for checkmate (the side to move lost), else 0.
+//
+// One WARP per game, lane = slot: a game's words, board and ring are contiguous runs that a warp
+// reads whole, where a thread per game walked 1.1 KB of its own (4096 games with rings of up to
+// forty entries: 4 us instead of 12 us for the two launches this one replaces).
 __global__ void __launch_bounds__(128) terminal_kernel(const unsigned long long* __restrict__ mask,
                                                        const unsigned char* __restrict__ in_check,
                                                        const int16_t* __restrict__ control,
                                                        const uint16_t* __restrict__ boards,
-                                                       const int* __restrict__ rep_count, int n,
+                                                       const int* __restrict__ rep_count,
+                                                       const unsigned long long* __restrict__ hash,
+                                                       const unsigned long long* __restrict__ ring,
+                                                       const long long* __restrict__ length, int n,
                                                        unsigned char* __restrict__ code, signed char* __restrict__ result) {
-    const long board = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31;
+    const long board = static_cast<long>(blockIdx.x) * 4 + (threadIdx.x >> 5);
     if (board >= n) return;
-    unsigned long long any = 0ull;
-    const ulonglong2* m2 = reinterpret_cast<const ulonglong2*>(mask + board * 32);
-#pragma unroll 4
-    for (int p = 0; p < 16; ++p) {
-        const ulonglong2 v = __ldg(m2 + p);
-        any |= v.x | v.y;
-    }
-    int heavy = 0, knights = 0, bishops = 0, dark = 0;
-    const uint4* b4 = reinterpret_cast<const uint4*>(boards + board * 32);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const uint4 v = __ldg(b4 + q);
-        const unsigned w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const unsigned word = (w[k >> 1] >> (16 * (k & 1))) & 0xFFFFu;
-            if ((word >> 11) & 1u) continue;
-            const int type = (word >> 6) & 7, sq = word & 63;
-            heavy += type == PAWN || type == ROOK || type == QUEEN;
-            knights += type == KNIGHT;
-            bishops += type == BISHOP;
-            dark += type == BISHOP && (((sq & 7) + (sq >> 3)) & 1) == 0;
-        }
-    }
+    const unsigned word = boards[board * 32 + lane];
+    const bool moves = __any_sync(kFull, mask[board * 32 + lane] != 0ull);
+    int seen = rep_count != nullptr ? rep_count[board] : 1;
+    if (ring != nullptr) seen += ring_matches(ring + board * kMaxHistory, length[board], hash[board], lane);
+    const bool live = (word & 0x800u) == 0u;
+    const int type = (word >> 6) & 7, sq = word & 63;
+    const bool heavy = __any_sync(kFull, live && (type == PAWN || type == ROOK || type == QUEEN));
+    const int knights = __popc(__ballot_sync(kFull, live && type == KNIGHT));
+    const bool bishop = live && type == BISHOP;
+    const int bishops = __popc(__ballot_sync(kFull, bishop));
+    const int dark = __popc(__ballot_sync(kFull, bishop && (((sq & 7) + (sq >> 3)) & 1) == 0));
+    if (lane != 0) return;
     const int c = control[board];
     int out = 0;
-    if (any == 0ull) out = in_check[board] ? 1 : 2;
+    if (!moves) out = in_check[board] ? 1 : 2;
     else if ((c < 0 ? -c : c) >= 101) out = 3;
-    else if (rep_count != nullptr && rep_count[board] >= 3) out = 4;
-    else if (heavy == 0 && ((knights == 0 && (dark == 0 || dark == bishops)) || (knights == 1 && bishops == 0))) out = 5;
+    else if (seen >= 3) out = 4;
+    else if (!heavy && ((knights == 0 && (dark == 0 || dark == bishops)) || (knights == 1 && bishops == 0))) out = 5;
     code[board] = static_cast<unsigned char>(out);
     if (result != nullptr) result[board] = out == 1 ? -1 : 0;
 }
@@ -1205,7 +1215,6 @@ __global__ void __launch_bounds__(128) terminal_kernel(const unsigned long long*
 // since the last irreversible move, `length` [n].  Push: record the position being left (`hash`
 // is the key BEFORE the move, `irreversible` describes the move); an irreversible move empties
 // the ring, because nothing at or before it can recur.
-constexpr int kMaxHistory = 100;
 __global__ void __launch_bounds__(128) history_push_kernel(unsigned long long* __restrict__ ring,
                                                            long long* __restrict__ length,
                                                            const unsigned long long* __restrict__ hash,
@@ -1217,19 +1226,48 @@ __global__ void __launch_bounds__(128) history_push_kernel(unsigned long long* _
     ring[g * kMaxHistory + (len < kMaxHistory - 1 ? len : kMaxHistory - 1)] = hash[g];
     length[g] = len + 1 < kMaxHistory ? len + 1 : kMaxHistory;
 }
-// How many times the position has occurred, counting the present one.
+// The same into new arrays: one pass copies the ring and puts the key in its place.  Bound by memory
+// (1,632 bytes per game); a thread copies 16 bytes (a ring is fifty of them), or 8 where an array
+// does not start on a 16-byte boundary.
+template <int kWords>
+__global__ void __launch_bounds__(256) history_push_to_kernel(const unsigned long long* __restrict__ ring,
+                                                              const long long* __restrict__ length,
+                                                              const unsigned long long* __restrict__ hash,
+                                                              const unsigned char* __restrict__ irreversible, int n,
+                                                              unsigned long long* __restrict__ new_ring,
+                                                              long long* __restrict__ new_length) {
+    constexpr unsigned kPieces = kMaxHistory / kWords;
+    const long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const long g = i / kPieces;
+    const int piece = static_cast<int>(i - g * kPieces);
+    if (g >= n) return;
+    unsigned long long v[kWords];
+    if constexpr (kWords == 2) {
+        const ulonglong2 t = reinterpret_cast<const ulonglong2*>(ring)[i];
+        v[0] = t.x; v[1] = t.y;
+    } else {
+        v[0] = ring[i];
+    }
+    const bool empties = irreversible[g] != 0;
+    const long long len = length[g];
+    const int at = empties ? -1 : static_cast<int>(len < kMaxHistory - 1 ? len : kMaxHistory - 1);
+#pragma unroll
+    for (int k = 0; k < kWords; ++k)
+        if (piece * kWords + k == at) v[k] = hash[g];
+    if constexpr (kWords == 2) reinterpret_cast<ulonglong2*>(new_ring)[i] = make_ulonglong2(v[0], v[1]);
+    else new_ring[i] = v[0];
+    if (piece == 0) new_length[g] = empties ? 0 : (len + 1 < kMaxHistory ? len + 1 : kMaxHistory);
+}
+// How many times the position has occurred, counting the present one: one warp per game.
 __global__ void __launch_bounds__(128) repetition_kernel(const unsigned long long* __restrict__ hash,
                                                          const unsigned long long* __restrict__ ring,
                                                          const long long* __restrict__ length, int n,
                                                          int* __restrict__ count) {
-    const long g = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31;
+    const long g = static_cast<long>(blockIdx.x) * 4 + (threadIdx.x >> 5);
     if (g >= n) return;
-    const unsigned long long h = hash[g];
-    long long len = length[g];
-    len = len < kMaxHistory ? len : kMaxHistory;
-    int c = 1;
-    for (long long i = 0; i < len; ++i) c += ring[g * kMaxHistory + i] == h;
-    count[g] = c;
+    const int c = 1 + ring_matches(ring + g * kMaxHistory, length[g], hash[g], lane);
+    if (lane == 0) count[g] = c;
 }
 
 }  // namespace bfmg

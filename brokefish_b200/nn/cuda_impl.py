@@ -284,6 +284,14 @@ class FusedEncoder:
             self.value_out = torch.empty(n, device=dev, dtype=torch.float)
             self._buffered_full = n
 
+    def _ensure_prior_buffers(self, n: int, e_cap: int) -> None:
+        if getattr(self, "_prior_shape", None) != (n, e_cap):
+            dev = torch.device("cuda", self.device)
+            self.prior_out = torch.zeros(n, e_cap, device=dev, dtype=torch.half)
+            self.move_out = torch.zeros(n, e_cap, device=dev, dtype=torch.int16)
+            self.nedges_out = torch.zeros(n, device=dev, dtype=torch.int32)
+            self._prior_shape = (n, e_cap)
+
     @staticmethod
     def _check_inputs(boards, control, rep):
         n = boards.shape[0]
@@ -311,17 +319,9 @@ class FusedEncoder:
         Returns views on internal buffers, which the next call overwrites.
         """
         self._require_net("forward_full")
-        n = self._check_inputs(boards, control, rep)
-        self._check_device(boards, control, rep, legal)
-        if legal is not None and (tuple(legal.shape) != (n, self.T) or legal.dtype is not torch.int64):
-            raise ValueError(f"legal must be [{n}, 32] int64, got {tuple(legal.shape)} {legal.dtype}")
-        self._ensure_full_buffers(n)
-        b, c, r = boards.contiguous(), control.contiguous(), rep.contiguous()
-        lg = legal.contiguous() if legal is not None else None
-        stream = ctypes.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
-        _native.check(_native.lib().bf_forward(
-            self._handle, _ptr(b), _ptr(c), _ptr(r), _ptr(lg), n, _ptr(self.policy_out),
-            _ptr(self.promo_out), _ptr(self.value_out), stream), "bf_forward")
+        ops = _native.torch_ops()
+        self._ensure_full_buffers(ops.check_evaluation(self.device, boards, control, rep, legal))
+        ops.forward(self._handle.value, boards, control, rep, legal, self.policy_out, self.promo_out, self.value_out)
         return self.policy_out, self.promo_out, self.value_out
 
     def forward_priors(self, boards, control, rep, legal, e_cap: int = 96, logits: bool = False):
@@ -334,29 +334,18 @@ class FusedEncoder:
         promotion logits are written as well (``self.policy_out``, ``self.promo_out``).
         Returns views on internal buffers, which the next call overwrites."""
         self._require_net("forward_priors")
-        n = self._check_inputs(boards, control, rep)
-        self._check_device(boards, control, rep, legal)
-        if legal is not None and (tuple(legal.shape) != (n, self.T) or legal.dtype is not torch.int64):
-            raise ValueError(f"legal must be [{n}, 32] int64 or None")
+        ops = _native.torch_ops()
+        n = ops.check_evaluation(self.device, boards, control, rep, legal)
         if legal is None and logits:
             raise ValueError("the masked policy needs the legality words; pass them or leave logits off")
-        if not 1 <= int(e_cap) <= 255:
+        e_cap = int(e_cap)
+        if not 1 <= e_cap <= 255:
             raise ValueError(f"e_cap must be in 1..255, got {e_cap}")
         self._ensure_full_buffers(n)
-        dev = torch.device("cuda", self.device)
-        if getattr(self, "_prior_shape", None) != (n, int(e_cap)):
-            self.prior_out = torch.zeros(n, int(e_cap), device=dev, dtype=torch.half)
-            self.move_out = torch.zeros(n, int(e_cap), device=dev, dtype=torch.int16)
-            self.nedges_out = torch.zeros(n, device=dev, dtype=torch.int32)
-            self._prior_shape = (n, int(e_cap))
-        b, c, r = boards.contiguous(), control.contiguous(), rep.contiguous()
-        lg = legal.contiguous() if legal is not None else None
-        stream = ctypes.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
-        _native.check(_native.lib().bf_forward_priors(
-            self._handle, _ptr(b), _ptr(c), _ptr(r), _ptr(lg), n, int(e_cap), _ptr(self.prior_out),
-            _ptr(self.move_out), _ptr(self.nedges_out), _ptr(self.value_out),
-            _ptr(self.policy_out) if logits else None, _ptr(self.promo_out) if logits else None, stream),
-            "bf_forward_priors")
+        self._ensure_prior_buffers(n, e_cap)
+        ops.forward_priors(self._handle.value, boards, control, rep, legal, e_cap, self.prior_out, self.move_out,
+                           self.nedges_out, self.value_out, self.policy_out if logits else None,
+                           self.promo_out if logits else None)
         return self.prior_out, self.move_out, self.nedges_out, self.value_out
 
     def forward_leaves(self, boards, control, rep, leaf_index, leaf_count, legal=None, e_cap: int = 0):
@@ -371,38 +360,25 @@ class FusedEncoder:
         optional as in :meth:`forward_priors`, and the masked policy is written when they are
         given).  Views on internal buffers."""
         self._require_net("forward_leaves")
-        n = self._check_inputs(boards, control, rep)
-        self._check_device(boards, control, rep, legal, leaf_index, leaf_count)
+        ops = _native.torch_ops()
+        n = ops.check_evaluation(self.device, boards, control, rep, legal)
+        self._check_device(leaf_index, leaf_count)
         if leaf_index.dim() != 1 or leaf_index.dtype is not torch.int32 or leaf_index.shape[0] > n:
             raise ValueError(f"leaf_index must be int32 [k], k <= {n}")
         if leaf_count.dtype is not torch.int32 or leaf_count.numel() != 1:
             raise ValueError("leaf_count must be a one-element int32 tensor")
-        if legal is not None and (tuple(legal.shape) != (n, self.T) or legal.dtype is not torch.int64):
-            raise ValueError(f"legal must be [{n}, 32] int64 or None")
         e_cap = int(e_cap)
         if not 0 <= e_cap <= 255:
             raise ValueError(f"e_cap must be in 0..255, got {e_cap}")
         self._ensure_full_buffers(n)
-        dev = torch.device("cuda", self.device)
-        if e_cap and getattr(self, "_prior_shape", None) != (n, e_cap):
-            self.prior_out = torch.zeros(n, e_cap, device=dev, dtype=torch.half)
-            self.move_out = torch.zeros(n, e_cap, device=dev, dtype=torch.int16)
-            self.nedges_out = torch.zeros(n, device=dev, dtype=torch.int32)
-            self._prior_shape = (n, e_cap)
-        capacity = int(leaf_index.shape[0])
-        if capacity == 0:
-            return ((self.prior_out, self.move_out, self.nedges_out, self.value_out) if e_cap
-                    else (self.policy_out, self.promo_out, self.value_out))
-        b, c, r, li = boards.contiguous(), control.contiguous(), rep.contiguous(), leaf_index.contiguous()
-        lg = legal.contiguous() if legal is not None else None
-        want_policy = not e_cap or lg is not None
-        stream = ctypes.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
-        _native.check(_native.lib().bf_forward_leaves(
-            self._handle, _ptr(b), _ptr(c), _ptr(r), _ptr(lg), _ptr(li), _ptr(leaf_count), capacity,
-            _ptr(self.policy_out) if want_policy else None, _ptr(self.promo_out) if want_policy else None,
-            _ptr(self.value_out), e_cap, _ptr(self.prior_out) if e_cap else None,
-            _ptr(self.move_out) if e_cap else None, _ptr(self.nedges_out) if e_cap else None, stream),
-            "bf_forward_leaves")
+        if e_cap:
+            self._ensure_prior_buffers(n, e_cap)
+        want_policy = not e_cap or legal is not None
+        if leaf_index.shape[0]:
+            ops.forward_leaves(self._handle.value, boards, control, rep, leaf_index, leaf_count, legal,
+                               self.policy_out if want_policy else None, self.promo_out if want_policy else None,
+                               self.value_out, e_cap, self.prior_out if e_cap else None,
+                               self.move_out if e_cap else None, self.nedges_out if e_cap else None)
         if e_cap:
             return self.prior_out, self.move_out, self.nedges_out, self.value_out
         return self.policy_out, self.promo_out, self.value_out

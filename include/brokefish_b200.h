@@ -157,6 +157,13 @@ int bf_history_push(int device, uint64_t* ring, long long* length, const uint64_
 int bf_repetition_count(int device, const uint64_t* hash, const uint64_t* ring, const long long* length, int n,
                         int* count, void* stream);
 
+/* bf_history_push into new arrays: the old ring and length are read, `new_ring` [n,100] and
+ * `new_length` [n] receive what bf_history_push would have made of them (the whole ring, its
+ * entries beyond the length included), in one pass.  The outputs must not overlap the inputs. */
+int bf_history_push_to(int device, const uint64_t* ring, const long long* length, const uint64_t* hash,
+                       const unsigned char* irreversible, int n, uint64_t* new_ring, long long* new_length,
+                       void* stream);
+
 /* Why each of `n` games is over, from a position's legal words, check flag, control word and
  * board (device pointers): `code` [n] uint8 = 1 checkmate, 2 stalemate, 3 fifty-move rule
  * (control magnitude >= 101), 4 threefold repetition (`rep_count` [n] from bf_repetition_count;
@@ -166,6 +173,12 @@ int bf_repetition_count(int device, const uint64_t* hash, const uint64_t* ring, 
 int bf_terminal(int device, const uint64_t* mask, const unsigned char* in_check, const int16_t* control,
                 const uint16_t* boards, const int* rep_count, int n, unsigned char* code, signed char* result,
                 void* stream);
+
+/* bf_terminal with the repetition count taken from the game's ring in the same launch: `hash` [n],
+ * `ring` [n,100] and `length` [n] as bf_repetition_count reads them. */
+int bf_terminal_history(int device, const uint64_t* mask, const unsigned char* in_check, const int16_t* control,
+                        const uint16_t* boards, const uint64_t* hash, const uint64_t* ring, const long long* length,
+                        int n, unsigned char* code, signed char* result, void* stream);
 
 /* One ply of a uniform-random playout, in place (device pointers): from `mask` (the legal moves
  * of `boards`, bf_movegen's output) the floor(r[i] * count)-th legal move in (slot, square) order
