@@ -23,7 +23,7 @@ ROOT = os.path.dirname(PKG_DIR)
 LIB_PATH = os.environ.get("BROKEFISH_B200_LIB") or os.path.join(PKG_DIR, "libbrokefish_b200.so")
 SOURCES = [os.path.join(PKG_DIR, "csrc", "bf_encoder.cu")]
 DEPS = SOURCES + [os.path.join(PKG_DIR, "csrc", name) for name in
-                  ("bf_ptx.cuh", "bf_movegen.cuh", "bf_encoder_one.cuh")] + [
+                  ("bf_ptx.cuh", "bf_movegen.cuh", "bf_encoder_ws.cuh")] + [
                       os.path.join(ROOT, "include", "brokefish_b200.h")]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
               "-Xcompiler", "-fPIC", "-shared", "-diag-suppress", "177,550"]
@@ -41,7 +41,8 @@ EXPORTS = ["bf_version", "bf_last_error", "bf_create", "bf_destroy", "bf_info", 
            "bf_forward_priors_host", "bf_selftest_timeout", "bf_movegen", "bf_step", "bf_random_ply",
            "bf_forward_leaves", "bf_measure_elementwise", "bf_forward_backbone", "bf_int8_q_max",
            "bf_fp8_q_max", "bf_terminal", "bf_hash", "bf_history_push",
-           "bf_repetition_count", "bf_history_push_to", "bf_terminal_history"]
+           "bf_repetition_count", "bf_history_push_to", "bf_terminal_history",
+           "bf_selftest_scales"]
 
 
 def nvcc_path() -> str:
@@ -150,6 +151,7 @@ def lib() -> ctypes.CDLL:
     L.bf_host_link_gbps.argtypes = [vp]
     L.bf_host_link_gbps.restype = ctypes.c_double
     L.bf_host_plan.argtypes = [i32, i32, i32, ctypes.c_double, ctypes.POINTER(i32)]
+    L.bf_selftest_scales.argtypes = [i32, ctypes.POINTER(ctypes.c_ulonglong)]
     L.bf_selftest_umma.argtypes = [i32, i32, vp, vp, vp]
     for name in EXPORTS:
         fn = getattr(L, name)

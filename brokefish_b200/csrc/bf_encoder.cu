@@ -12,7 +12,9 @@
 // integers; fp16 x fp16 with fp16 accumulators, which carries the bits of the reference's
 // fp16-accumulate mma.sync); the 32 x 32 attention products run as mma.sync on the row warps.
 //
-// Shape of the kernel
+// Plain evaluations run on one- and two-board tiles (bf_encoder_ws.cuh).  The kernel below, on
+// four-board tiles, is the large-batch form of the arithmetics with fp16 products, carries re-injection
+// and is the instrumented arm.  Its shape
 //   * persistent grid, one CTA per SM, each CTA loops over tiles of 128 token rows
 //     (4 boards);
 //   * 19 warps: 16 "row" warps, one weight-stream producer, two MMA issuers;
@@ -62,6 +64,7 @@ constexpr int kNClock = 101, kNRep = 3, kNTypeSpecial = 12;
 //   kArI8Qkv FFN and QKV s8 x s8, out-projection fp16 x fp16 (the reference's "ffn+qkv" int8
 //            scheme, quant 4)
 enum { kArInt8 = 0, kArE4M3 = 1, kArF16 = 2, kArI8Ffn = 3, kArI8Qkv = 4 };
+enum { kKindI8 = 0, kKindF16 = 1, kKindF8 = 2 };           // tcgen05.mma kinds
 // The front of the map depends on the arithmetic.  int8: the A operand is 32 KB of bytes and
 // the weight ring has 112 KB.  With fp16 attention GEMMs (e4m3, fp16 arms) the A operand is 64 KB
 // (4 K-slabs of 64 halves) and the ring gives up two slots.
@@ -120,6 +123,7 @@ struct Params {
                                 // 0: the hardware approximation, as the reference's rsqrtf (encoder.cu:597)
     float eps;
     float one;                  // 1.0f (see quant16)
+    int one_most;               // at most so many boards per CTA run as one-board tiles (bf_encoder_ws.cuh)
     const uint8_t* wstream;
     const uint8_t* lparams;
     const __half* emb;
@@ -1409,7 +1413,7 @@ __device__ __forceinline__ void row_warps_tile(RowCtx& c, const Params& p, int t
 }
 
 }  // namespace bf
-#include "bf_encoder_one.cuh"
+#include "bf_encoder_ws.cuh"
 namespace bf {
 
 // ------------------------------------------------------------------------------------------
@@ -1479,7 +1483,6 @@ struct MmaState {
     uint32_t accn[2];         // units issued into each accumulator slot
     uint32_t aready, a2n[2];  // operand-ready phases consumed
 };
-enum { kKindI8 = 0, kKindF16 = 1, kKindF8 = 2 };
 
 // One GEMM unit: `n_stages` K-slabs of 128 bytes, 4 MMAs each.
 template <int kAr>
@@ -1713,12 +1716,7 @@ __device__ __forceinline__ void mma_loop(uint32_t smem, uint32_t tmem, volatile 
 }
 
 // ------------------------------------------------------------------------------------------
-// `kForm`: 0 = four boards per tile; 1 = the small-batch form, one board per tile with its rows
-// replicated in the four lane quadrants (bf_encoder_one.cuh; plain int8 evaluation only); 2 = chosen
-// when the kernel starts, by the number of positions it finds (a leaf list's length is only known
-// on the device): one board per tile if every board gets a CTA of its own, else four.
-enum { kFormFour = 0, kFormOne = 1, kFormByCount = 2 };
-template <bool kDbg, bool kRJ, int kAr, int kForm = kFormFour>
+template <bool kDbg, bool kRJ, int kAr>
 __global__ void __launch_bounds__(kThreads, 1) encoder_kernel(const Params p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -1751,8 +1749,7 @@ __global__ void __launch_bounds__(kThreads, 1) encoder_kernel(const Params p) {
     // (clamped to the capacity the grid was sized for); every role reads the same word
     int n_eval = p.n;
     if (p.leaf_count != nullptr) n_eval = min(max(__ldg(p.leaf_count), 0), p.n);
-    const bool one = kForm == kFormOne || (kForm == kFormByCount && n_eval <= static_cast<int>(gridDim.x));
-    const int n_tiles = one ? n_eval : (n_eval + 3) / 4;
+    const int n_tiles = (n_eval + 3) / 4;
     if (warp < kRowWarps) {
         RowCtx c;
         c.n = n_eval;
@@ -1764,18 +1761,7 @@ __global__ void __launch_bounds__(kThreads, 1) encoder_kernel(const Params p) {
         c.one2 = pk2(p.one, p.one);
         c.prof_on = kDbg && p.prof != nullptr && threadIdx.x == 0;
         c.t_last = c.prof_on ? clock64() : 0;
-        for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-            if constexpr (kForm == kFormFour) {
-                row_warps_tile<kDbg, kRJ, kAr>(c, p, tile);
-            } else {
-                if (one)
-                    one::row_warps_tile(c, p, tile, [&](RowCtx& cc, int board, uint32_t word, int ctl, uint32_t alive) {
-                        head_epilogue<false>(cc, p, board, word, ctl, alive);
-                    });
-                else
-                    row_warps_tile<kDbg, kRJ, kAr>(c, p, tile);
-            }
-        }
+        for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) row_warps_tile<kDbg, kRJ, kAr>(c, p, tile);
     } else if (warp == kProducerWarp) {
         if (elect_one()) producer_loop<kAr>(smem, abort_flag, p, blockIdx.x, gridDim.x, n_tiles);
     } else {
@@ -2032,6 +2018,30 @@ __global__ void __launch_bounds__(64, 1) timeout_kernel(int code, int* status, l
 }
 
 // ------------------------------------------------------------------------------------------
+// Scale self test: the row scales and reciprocals of bf_encoder_ws.cuh against IEEE division over
+// every value they can be given: all positive fp16 maxima with the three operand ranges (counts 0-2:
+// scale or reciprocal differs), and every fp32 softmax sum from 1 to 32 (count 3).
+// ------------------------------------------------------------------------------------------
+__global__ void scales_kernel(unsigned long long* differ) {
+    const unsigned first = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+    for (unsigned i = first; i <= 0x7bffu; i += step) {
+        const float amax = __half2float(__ushort_as_half(static_cast<unsigned short>(i)));
+        const float range[3] = {kQMaxS8, kQMaxU8, kQMaxE4M3};
+        const ws::Scale got[3] = {ws::scale_s8(amax), ws::scale_u8(amax), ws::scale_e4m3(amax)};
+        for (int k = 0; k < 3; ++k) {
+            const float scale = amax > 0.f ? __fdiv_rn(amax, range[k]) : 1.0f;
+            if (__float_as_uint(got[k].scale) != __float_as_uint(scale) ||
+                __float_as_uint(got[k].inverse) != __float_as_uint(__fdiv_rn(1.0f, scale)))
+                atomicAdd(differ + k, 1ull);
+        }
+    }
+    for (unsigned i = first; i <= 5u << 23; i += step) {
+        const float x = __uint_as_float(0x3f800000u + i);
+        if (__float_as_uint(ws::reciprocal(x)) != __float_as_uint(__fdiv_rn(1.0f, x))) atomicAdd(differ + 3, 1ull);
+    }
+}
+
+// ------------------------------------------------------------------------------------------
 // Tensor-core self test: one tile, one GEMM, no network.
 // ------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(128, 1) selftest_kernel(int mode, const uint8_t* a, const uint8_t* w,
@@ -2269,6 +2279,22 @@ struct LeafList {
     const int* count;           // device: how many of them (read by the kernel when it starts)
 };
 
+// Which form a plain evaluation runs in: one- and two-board tiles (bf_encoder_ws.cuh) or four-board tiles.
+// A tile takes the same time whatever the batch, so the tiles of the busiest SM decide.  Measured, us
+// per one-, two- and four-board tile of an SM (B200):
+//   int8 96 / 141 / 280    int8 FFN+QKV 104 / 143 / 276    int8 FFN 115 / 146 / 277
+//   e4m3 115 / 143 / 270   fp16 143 / 166 / 252
+// The first two never gain from the four-board form.  The others' fp16 products, 32 bytes of K at half
+// the rate, weigh more on fewer rows.
+bool small_tiles(int quant, int n, int sm_count) {
+    static const int us[5][3] = {{143, 166, 252}, {115, 143, 270}, {115, 146, 277}, {1, 1, 1000}, {1, 1, 1000}};
+    const int* t = us[quant];
+    const long full = n / (2 * sm_count), rest = n - full * 2 * sm_count;
+    const long small = full * t[1] + (rest == 0 ? 0 : rest <= sm_count ? t[0] : t[1]);
+    const long four = static_cast<long>((n + 4L * sm_count - 1) / (4L * sm_count)) * t[2];
+    return small <= four;
+}
+
 int launch(bf_handle* h, const uint16_t* boards, const int16_t* control, const uint8_t* rep,
            const uint64_t* legal, int n, void* policy, void* promo, float* value, void* y, int stage,
            int stage_layer, int cap_layer, int cap_op, uint8_t* cap_a, int32_t* cap_acc, cudaStream_t stream,
@@ -2307,42 +2333,27 @@ int launch(bf_handle* h, const uint16_t* boards, const int16_t* control, const u
     const int grid = n_tiles < h->sm_count ? n_tiles : h->sm_count;
     // the instrumented instantiation only when a dump, a capture or the phase clock is asked for
     const bool dbg = stage != 0 || cap_layer >= 0 || p.prof != nullptr;
-    if (p.quant == 0) {
-        if (cap_layer >= 0) return fail(BF_ENOTSUP, "operand capture is for the int8 arithmetic");
-        if (p.rj_mode != 0) {
-            if (dbg) bf::encoder_kernel<true, true, bf::kArF16><<<grid, bf::kThreads, bf::kSmemRequest, stream>>>(p);
-            else     bf::encoder_kernel<false, true, bf::kArF16><<<grid, bf::kThreads, bf::kSmemRequest, stream>>>(p);
-        } else if (dbg) bf::encoder_kernel<true, false, bf::kArF16><<<grid, bf::kThreads, bf::kSmemRequest, stream>>>(p);
-        else     bf::encoder_kernel<false, false, bf::kArF16><<<grid, bf::kThreads, bf::kSmemRequest, stream>>>(p);
-    } else if (p.quant == 4) {
-        if (cap_layer >= 0) return fail(BF_ENOTSUP, "operand capture is for the int8 arithmetic");
-        if (dbg) bf::encoder_kernel<true, false, bf::kArI8Qkv><<<grid, bf::kThreads, bf::kSmemRequest, stream>>>(p);
-        else     bf::encoder_kernel<false, false, bf::kArI8Qkv><<<grid, bf::kThreads, bf::kSmemRequest, stream>>>(p);
-    } else if (p.quant == 2) {
-        if (cap_layer >= 0) return fail(BF_ENOTSUP, "operand capture is for the int8 arithmetic");
-        if (dbg) bf::encoder_kernel<true, false, bf::kArI8Ffn><<<grid, bf::kThreads, bf::kSmemRequest, stream>>>(p);
-        else     bf::encoder_kernel<false, false, bf::kArI8Ffn><<<grid, bf::kThreads, bf::kSmemRequest, stream>>>(p);
-    } else if (p.quant == 1) {
-        if (cap_layer >= 0) return fail(BF_ENOTSUP, "operand capture is for the int8 arithmetic");
-        if (dbg) bf::encoder_kernel<true, false, bf::kArE4M3><<<grid, bf::kThreads, bf::kSmemRequest, stream>>>(p);
-        else     bf::encoder_kernel<false, false, bf::kArE4M3><<<grid, bf::kThreads, bf::kSmemRequest, stream>>>(p);
-    } else if (p.rj_mode != 0) {
-        if (dbg) bf::encoder_kernel<true, true, bf::kArInt8><<<grid, bf::kThreads, bf::kSmemRequest, stream>>>(p);
-        else     bf::encoder_kernel<false, true, bf::kArInt8><<<grid, bf::kThreads, bf::kSmemRequest, stream>>>(p);
+    if (cap_layer >= 0 && p.quant != 3) return fail(BF_ENOTSUP, "operand capture is for the int8 arithmetic");
+    if (!dbg && p.rj_mode == 0 && small_tiles(p.quant, n, h->sm_count)) {
+        p.one_most = h->one_board_factor;
+        const int ctas = n < h->sm_count ? n : h->sm_count;
+        const auto kernel = p.quant == 0 ? bf::ws::encoder_ws_kernel<bf::kArF16> : p.quant == 1 ? bf::ws::encoder_ws_kernel<bf::kArE4M3>
+                          : p.quant == 2 ? bf::ws::encoder_ws_kernel<bf::kArI8Ffn> : p.quant == 4 ? bf::ws::encoder_ws_kernel<bf::kArI8Qkv>
+                                                                                                : bf::ws::encoder_ws_kernel<bf::kArInt8>;
+        kernel<<<ctas, bf::ws::kThreads, bf::ws::kSmemRequest, stream>>>(p);
     } else {
-        // a batch that leaves SMs idle (at most one board per SM) runs in the one-board-per-tile
-        // form: sixteen row warps per board instead of four, about half the latency, same bits
-        const bool small_form = !dbg && bb == nullptr && p.vmode != 2 && h->one_board_factor > 0;
-        const bool one = small_form && n <= h->sm_count * h->one_board_factor;
-        const int grid_one = n < h->sm_count ? n : h->sm_count;
-        if (dbg) bf::encoder_kernel<true, false, bf::kArInt8><<<grid, bf::kThreads, bf::kSmemRequest, stream>>>(p);
-        else if (one)
-            bf::encoder_kernel<false, false, bf::kArInt8, bf::kFormOne><<<grid_one, bf::kThreads, bf::kSmemRequest, stream>>>(p);
-        else if (small_form && leaves != nullptr)
-            // a leaf list may turn out short: one CTA per SM, and the kernel picks the form by the
-            // count it reads
-            bf::encoder_kernel<false, false, bf::kArInt8, bf::kFormByCount><<<grid_one, bf::kThreads, bf::kSmemRequest, stream>>>(p);
-        else     bf::encoder_kernel<false, false, bf::kArInt8><<<grid, bf::kThreads, bf::kSmemRequest, stream>>>(p);
+        // four-board tiles: large batches of the arithmetics with fp16 products, re-injection, and the
+        // instrumented arms (dumps, captures, the phase clock, the backbone entry)
+        const auto kernel =
+            p.quant == 0 ? (p.rj_mode == 0 ? (dbg ? bf::encoder_kernel<true, false, bf::kArF16> : bf::encoder_kernel<false, false, bf::kArF16>)
+                                           : (dbg ? bf::encoder_kernel<true, true, bf::kArF16> : bf::encoder_kernel<false, true, bf::kArF16>))
+            : p.quant == 4 ? bf::encoder_kernel<true, false, bf::kArI8Qkv>
+            : p.quant == 2 ? (dbg ? bf::encoder_kernel<true, false, bf::kArI8Ffn> : bf::encoder_kernel<false, false, bf::kArI8Ffn>)
+            : p.quant == 1 ? (dbg ? bf::encoder_kernel<true, false, bf::kArE4M3> : bf::encoder_kernel<false, false, bf::kArE4M3>)
+            : p.rj_mode == 0 ? bf::encoder_kernel<true, false, bf::kArInt8>
+            : dbg            ? bf::encoder_kernel<true, true, bf::kArInt8>
+                             : bf::encoder_kernel<false, true, bf::kArInt8>;
+        kernel<<<grid, bf::kThreads, bf::kSmemRequest, stream>>>(p);
     }
     BF_CUDA(cudaGetLastError());
     h->launches++;
@@ -2406,29 +2417,25 @@ int bf_create(const void* blob, size_t blob_bytes, int device, bf_handle** out) 
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->chunk_done, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreate(&h->copy_t0);
     if (e == cudaSuccess) e = cudaEventCreate(&h->copy_t1);
-    const void* kernels[14] = {
-        reinterpret_cast<const void*>(&bf::encoder_kernel<false, false, bf::kArI8Qkv>),
-        reinterpret_cast<const void*>(&bf::encoder_kernel<true, false, bf::kArI8Qkv>),
-        reinterpret_cast<const void*>(&bf::encoder_kernel<false, false, bf::kArI8Ffn>),
-        reinterpret_cast<const void*>(&bf::encoder_kernel<true, false, bf::kArI8Ffn>),
-        reinterpret_cast<const void*>(&bf::encoder_kernel<false, true, bf::kArF16>),
-        reinterpret_cast<const void*>(&bf::encoder_kernel<true, true, bf::kArF16>),
-        reinterpret_cast<const void*>(&bf::encoder_kernel<false, false, bf::kArInt8>),
-        reinterpret_cast<const void*>(&bf::encoder_kernel<true, false, bf::kArInt8>),
-        reinterpret_cast<const void*>(&bf::encoder_kernel<false, true, bf::kArInt8>),
-        reinterpret_cast<const void*>(&bf::encoder_kernel<true, true, bf::kArInt8>),
-        reinterpret_cast<const void*>(&bf::encoder_kernel<false, false, bf::kArE4M3>),
-        reinterpret_cast<const void*>(&bf::encoder_kernel<true, false, bf::kArE4M3>),
-        reinterpret_cast<const void*>(&bf::encoder_kernel<false, false, bf::kArF16>),
-        reinterpret_cast<const void*>(&bf::encoder_kernel<true, false, bf::kArF16>)};
-    for (int i = 0; i < 14 && e == cudaSuccess; ++i)
-        e = cudaFuncSetAttribute(kernels[i], cudaFuncAttributeMaxDynamicSharedMemorySize, bf::kSmemRequest);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(bf::encoder_kernel<false, false, bf::kArInt8, bf::kFormOne>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, bf::kSmemRequest);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(bf::encoder_kernel<false, false, bf::kArInt8, bf::kFormByCount>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, bf::kSmemRequest);
+    for (const void* k : {reinterpret_cast<const void*>(&bf::encoder_kernel<false, false, bf::kArI8Ffn>),
+                          reinterpret_cast<const void*>(&bf::encoder_kernel<false, false, bf::kArE4M3>),
+                          reinterpret_cast<const void*>(&bf::encoder_kernel<false, false, bf::kArF16>),
+                          reinterpret_cast<const void*>(&bf::encoder_kernel<true, false, bf::kArI8Qkv>),
+                          reinterpret_cast<const void*>(&bf::encoder_kernel<true, false, bf::kArI8Ffn>),
+                          reinterpret_cast<const void*>(&bf::encoder_kernel<true, false, bf::kArE4M3>),
+                          reinterpret_cast<const void*>(&bf::encoder_kernel<true, false, bf::kArF16>),
+                          reinterpret_cast<const void*>(&bf::encoder_kernel<false, true, bf::kArF16>),
+                          reinterpret_cast<const void*>(&bf::encoder_kernel<true, true, bf::kArF16>),
+                          reinterpret_cast<const void*>(&bf::encoder_kernel<true, false, bf::kArInt8>),
+                          reinterpret_cast<const void*>(&bf::encoder_kernel<false, true, bf::kArInt8>),
+                          reinterpret_cast<const void*>(&bf::encoder_kernel<true, true, bf::kArInt8>)})
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bf::kSmemRequest);
+    for (const void* k : {reinterpret_cast<const void*>(&bf::ws::encoder_ws_kernel<bf::kArInt8>),
+                          reinterpret_cast<const void*>(&bf::ws::encoder_ws_kernel<bf::kArI8Ffn>),
+                          reinterpret_cast<const void*>(&bf::ws::encoder_ws_kernel<bf::kArI8Qkv>),
+                          reinterpret_cast<const void*>(&bf::ws::encoder_ws_kernel<bf::kArE4M3>),
+                          reinterpret_cast<const void*>(&bf::ws::encoder_ws_kernel<bf::kArF16>)})
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bf::ws::kSmemRequest);
     if (e != cudaSuccess) {
         bf_destroy(h);
         return fail(BF_ECUDA, std::string("bf_create: ") + cudaGetErrorString(e));
@@ -3015,6 +3022,21 @@ int bf_selftest_timeout(int device, int code, int* status, long long* waited_cyc
     return BF_OK;
 }
 
+int bf_selftest_scales(int device, unsigned long long* differ) {
+    if (differ == nullptr) return fail(BF_EINVAL, "differ is null");
+    BF_ON_DEVICE(device);
+    unsigned long long* d = nullptr;
+    BF_CUDA(cudaMalloc(&d, 4 * sizeof(*d)));
+    cudaError_t e = cudaMemset(d, 0, 4 * sizeof(*d));
+    if (e == cudaSuccess) {
+        bf::scales_kernel<<<592, 256>>>(d);
+        e = cudaMemcpy(differ, d, 4 * sizeof(*d), cudaMemcpyDeviceToHost);
+    }
+    cudaFree(d);
+    if (e != cudaSuccess) return fail(BF_ECUDA, cudaGetErrorString(e));
+    return BF_OK;
+}
+
 int bf_selftest_umma(int device, int mode, const void* a, const void* w_image, void* out) {
     if (mode < 0 || mode > 4 || a == nullptr || w_image == nullptr || out == nullptr)
         return fail(BF_EINVAL, "bad self-test argument");
@@ -3087,8 +3109,8 @@ int noalloc_setup(int device, NoAllocDevice** out) {
         void* ptr = nullptr;
         BF_CUDA(cudaGetSymbolAddress(&ptr, bf::g_noalloc_scratch));
         BF_CUDA(cudaMemset(ptr, 0, bf::kNoAllocScratchBytes));
-        BF_CUDA(cudaFuncSetAttribute(bf::encoder_kernel<false, false, bf::kArInt8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     bf::kSmemRequest));
+        BF_CUDA(cudaFuncSetAttribute(bf::ws::encoder_ws_kernel<bf::kArInt8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     bf::ws::kSmemRequest));
         d.scratch = ptr;
         d.sm_count = prop.multiProcessorCount;
         d.ready = true;
@@ -3175,9 +3197,9 @@ int bf_forward_noalloc(int device, const void* blob_dev, size_t blob_bytes, cons
     p.cap_layer = -1; p.cap_op = -1; p.cap_a = nullptr; p.cap_acc = nullptr;
     p.status = static_cast<int*>(scratch);         // the device address, not the symbol
     p.prof = nullptr;
-    const int n_tiles = (n + 3) / 4;
-    const int grid = n_tiles < sm_count ? n_tiles : sm_count;
-    bf::encoder_kernel<false, false, bf::kArInt8><<<grid, bf::kThreads, bf::kSmemRequest, static_cast<cudaStream_t>(stream)>>>(p);
+    p.one_most = 1;
+    bf::ws::encoder_ws_kernel<bf::kArInt8><<<n < sm_count ? n : sm_count, bf::ws::kThreads, bf::ws::kSmemRequest,
+                                             static_cast<cudaStream_t>(stream)>>>(p);
     BF_CUDA(cudaGetLastError());
     return BF_OK;
 }

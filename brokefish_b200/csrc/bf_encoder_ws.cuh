@@ -1,0 +1,1053 @@
+// The evaluator kernel on weight-stationary tensor-core tiles of one or two boards (included by
+// bf_encoder.cu): the form every plain evaluation runs in.
+//
+// Why one or two boards.  `tcgen05.mma.ws` takes an M of 32 or 64 and lays the product out over all
+// 128 lanes of tensor memory: lane quadrant q holds, for M = 32, all 32 rows and output columns
+// 64 q .. 64 q + 63 of an N = 256 product; for M = 64, the 32 rows of board q & 1 and output columns
+// 128 (q >> 1) .. + 127.  So sixteen row warps (four per quadrant, thread = row x 16 or 32 columns)
+// share the element-wise work of one or two boards, where a 128-row tile gives a board four warps,
+// and an N = 256 product of 32 / 64 / 128 rows costs 84 / 92 / 166 cycles per 32 bytes of K (measured;
+// the weights' way out of shared memory alone is 64).  A board then takes as long as its own chain
+// of phases, and that chain is a quarter as long.
+//
+// What follows from a thread's columns being the same in every product:
+//   * the residual stream x stays in the owning thread's registers from the embedding to the heads;
+//   * all of tensor memory is accumulators: four slots of one N = 256 product.  Q, K, V, out-projection
+//     take slots 0-3, the four hidden chunks of ff1 slots 0-3, their ff2 products the slot of the
+//     chunk they come from, so every product of a phase is issued as soon as its operand is there
+//     and no slot needs an "empty" barrier: the operand that starts a product is published by warps
+//     that have read what was in its slot;
+//   * with two boards a thread holds a whole head's row (32 columns) of Q, K and V: attention needs
+//     no other warp, only a 2 KB scratch block per warp.
+//
+// The arithmetic is the four-board kernel's, bit for bit (the order of every sum included).
+//
+// Measured on one B200, int8, against the forms before it (four boards per tile; one board per tile
+// with its rows written four times into a 128-row operand): batch 1-148 94-97 us (167), 149-296 141 us
+// (281), 333 233 us (281), 4096 1.92 ms (1.95).  What bounds it: the element-wise work of the row warps,
+// four to a scheduler and all in the same phase; of a two-board tile's 35,000 cycles per layer 22,000
+// are that work at the rate the CUDA cores sustain on it, 6,000 waits for a product whose operand has
+// only just been written (of a one-board tile's 23,000: 11,000 and 5,000).
+#pragma once
+
+namespace bf {
+namespace ws {
+
+constexpr int kProducerWarp = 16, kMmaWarp = 17, kThreads = 576;
+constexpr uint32_t kStage = 32768;                 // one 128-byte K-slab of 256 weight rows
+// ---- shared memory map ------------------------------------------------------------------
+// A operand: K-slabs of [rows][128 B], two of bytes or (where QKV or the out-projection runs in fp16)
+// four of halves.  H: the ff2 operand's chunks; before and after that the attention scratch, the norms'
+// partial sums, the head operand.
+template <int kAr>
+struct Map {
+    static constexpr int kStages = Cfg<kAr>::kHalfA ? 3 : 4;
+    static constexpr uint32_t SM_H = Cfg<kAr>::kHalfA ? 32768 : 16384;
+    static constexpr uint32_t SM_RING = SM_H + 65536;
+};
+constexpr uint32_t SM_A = 0;
+constexpr uint32_t kHeadA = 32768;                 // the head operand's place in H, clear of the other board's partial sums
+constexpr uint32_t SM_STAT = 16384 + 65536 + 4 * kStage;
+constexpr uint32_t SM_MAX = SM_STAT + 1024;        // row maxima: attention output, four hidden chunks
+constexpr uint32_t SM_LIST = SM_MAX + 5 * 256;     // fused expansion: 1 KB per board
+constexpr uint32_t SM_BAR = SM_LIST + 2048;
+constexpr uint32_t SM_MISC = SM_BAR + 128;
+constexpr uint32_t SM_BYTES = SM_MISC + 64, kSmemRequest = SM_BYTES + 1024;
+static_assert(Map<kArF16>::SM_RING + 3 * kStage <= SM_STAT && Map<kArInt8>::SM_RING + 4 * kStage <= SM_STAT, "shared memory map");
+enum { B_FULL = 0, B_EMPTY = 4, B_ACC = 8, B_A = 12, B_H = 13, B_COUNT = 15 };
+__device__ __forceinline__ uint32_t bar(uint32_t smem, int i) { return smem + SM_BAR + 8u * i; }
+
+// Which boards a CTA evaluates, tile by tile.  At most `one_most` boards per CTA: one-board tiles alone.
+// More: as many whole waves of two-board tiles as there are, then what is left, one board per CTA where
+// that is enough (and allowed), else two.  A one-board tile takes about two thirds of a two-board
+// tile's time.
+struct Tiles {
+    int n, grid, cta, full, rest, per;
+    bool singles;
+    __device__ Tiles(int n_, int grid_, int cta_, int one_most) : n(n_), grid(grid_), cta(cta_) {
+        singles = n <= one_most * grid;
+        full = n / (2 * grid);
+        rest = n - full * 2 * grid;
+        per = rest <= grid && one_most > 0 ? 1 : 2;
+    }
+    // number of tiles of this CTA; tile k starts at board `first` and holds `boards` (1 or 2)
+    __device__ int count() const {
+        if (singles) return cta < n ? (n - cta + grid - 1) / grid : 0;
+        return full + (cta * per < rest ? 1 : 0);
+    }
+    __device__ void at(int k, int& first, int& boards) const {
+        if (singles) { boards = 1; first = k * grid + cta; return; }
+        boards = k < full ? 2 : per;
+        first = k < full ? 2 * (k * grid + cta) : 2 * full * grid + per * cta;
+    }
+};
+
+struct Row {
+    int lane, q, s;             // lane quadrant, warp within the quadrant
+    uint32_t smem, tm;          // tm: tensor memory with this warp's lane offset
+    uint8_t* smem_gen;
+    volatile int* abort_flag;
+    uint64_t one2;
+    uint32_t layers, tiles;     // layers and tiles finished so far: three products per layer go through
+                                // each slot, and one per tile (the heads') through slot 0
+    int n;
+    uint32_t h;                 // shared address of H
+    __device__ uint32_t a() const { return smem + SM_A; }
+};
+
+// A tile of NB boards as its thread sees it.
+template <int NB>
+struct Own {
+    static constexpr int kW = 16 * NB;                       // columns per thread of a 256-wide row
+    static constexpr int kRowsT = 32 * NB;
+    static constexpr uint32_t kSlab = kRowsT * 128;          // bytes of a K-slab of an operand
+    static constexpr uint32_t kSlot = NB == 1 ? 64 : 128;    // tensor-memory columns of a slot
+    static constexpr int kGroup = 16 / NB;                   // threads that share a row
+    static __device__ int board(const Row& c) { return NB == 1 ? 0 : c.q & 1; }
+    static __device__ int col(const Row& c) { return NB == 1 ? 64 * c.q + 16 * c.s : 128 * (c.q >> 1) + 32 * c.s; }
+    static __device__ int member(const Row& c) { return NB == 1 ? 4 * c.q + c.s : 4 * (c.q >> 1) + c.s; }
+    static __device__ int row(const Row& c) { return 32 * board(c) + c.lane; }
+    static __device__ uint32_t slot(const Row& c, int k) { return c.tm + kSlot * k + kW * c.s; }
+};
+// The warps of a board meet here (barriers of their own for one- and two-board tiles: a warp may be a
+// tile ahead).
+template <int NB>
+__device__ __forceinline__ void board_sync(const Row& c) { __syncwarp(); named_bar_sync(NB == 1 ? 11 : 1 + Own<NB>::board(c), 512 / NB); }
+
+// The two warps of a head (one-board tiles).
+__device__ __forceinline__ void pair_sync(int head) { __syncwarp(); named_bar_sync(3 + head, 64); }
+
+// The `use`-th product of the layer in slot `slot` (0: Q, K, V, out-projection, or the heads; 1: ff1;
+// 2: ff2).
+__device__ __forceinline__ void wait_acc(const Row& c, int slot, int use) {
+    const uint32_t n = 3u * c.layers + use + (slot == 0 ? c.tiles : 0u);
+    mbar_wait(bar(c.smem, B_ACC + slot), n & 1u, c.abort_flag, kErrRowAcc);
+    __syncwarp();                                            // what follows is for a converged warp
+    tc_fence_after();
+}
+// This warp's operand rows are written and what it read of tensor memory has arrived: publish.
+__device__ __forceinline__ void publish(const Row& c, int b) {
+    tc_fence_before();
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (c.lane == 0) mbar_arrive(bar(c.smem, b));
+    __syncwarp();
+}
+__device__ __forceinline__ float lds_f(uint32_t addr) {
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint32_t lds_u(uint32_t addr) {
+    uint32_t v;
+    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint64_t lds_u64(uint32_t addr) {
+    uint64_t v;
+    asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(addr) : "memory");
+    return v;
+}
+// Row maxima of non-negative values meet in shared memory by an integer maximum of their bits.
+__device__ __forceinline__ void max_to(uint32_t addr, float v) {
+    asm volatile("red.shared.max.u32 [%0], %1;" ::"r"(addr), "r"(__float_as_uint(v)) : "memory");
+}
+// A row's scale amax / Q and its reciprocal, both correctly rounded, amax being a positive fp16 value: a
+// quotient corrected by its own remainder, and one Newton step on the hardware's reciprocal with the
+// residual taken by fma (Markstein 1990).  Neither leaves the normal range here, and every one of the
+// 31,743 values of amax gives the bits of `__fdiv_rn` for each of the three ranges, as does the
+// reciprocal of every fp32 value from 1 to 32, a softmax row's sum (`scales_kernel`).  Two divisions one after the other
+// took 300 cycles, this takes 45.
+struct Scale { float scale, inverse; };
+__device__ __forceinline__ float reciprocal(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return __fmaf_rn(__fmaf_rn(-x, y, 1.0f), y, y);
+}
+__device__ __forceinline__ Scale row_scale(float amax, float q_max, float q_inv) {
+    const float q = __fmul_rn(amax, q_inv);
+    const float sc = amax > 0.f ? __fmaf_rn(__fmaf_rn(-q, q_max, amax), q_inv, q) : 1.0f;
+    return {sc, reciprocal(sc)};
+}
+__device__ __forceinline__ Scale scale_s8(float amax) { return row_scale(amax, kQMaxS8, 1.0f / kQMaxS8); }
+__device__ __forceinline__ Scale scale_u8(float amax) { return row_scale(amax, kQMaxU8, 1.0f / kQMaxU8); }
+__device__ __forceinline__ Scale scale_e4m3(float amax) { return row_scale(amax, kQMaxE4M3, 1.0f / kQMaxE4M3); }
+// This thread's columns of a slot, 16 at a time: `use(piece, words)`.  No load is left in flight while
+// another piece is worked on: the registers that one lands in are then free of pressure from the code
+// around them, and the scheduler's other warps cover its latency.
+template <int NB, class F>
+__device__ __forceinline__ void each_piece(uint32_t t, F&& use) {
+#pragma unroll
+    for (int k = 0; k < NB; ++k) {
+        uint32_t acc[16];
+        tmem_ld16(t + 16 * k, acc);
+        tmem_wait_ld();
+        use(k, acc);
+    }
+}
+// Piece k (16 columns) of this thread's columns into an operand: quantised to bytes (two K-slabs), or as
+// fp16 (four).
+template <int NB, bool kE4M3 = false>
+__device__ __forceinline__ void store_operand8(const Row& c, uint32_t base, int k, const uint32_t* v, float inv) {
+    using O = Own<NB>;
+    const int col = O::col(c);
+    sts128(base + (col >> 7) * O::kSlab + sw_off(O::row(c), ((col & 127) >> 4) + k), quant16_any<kE4M3>(v, inv, c.one2));
+}
+template <int NB>
+__device__ __forceinline__ void store_operand16(const Row& c, uint32_t base, int k, const uint32_t* v) {
+    using O = Own<NB>;
+    const int col = O::col(c), row = O::row(c), group = ((col & 63) >> 3) + 2 * k;
+    const uint32_t slab = base + (col >> 6) * O::kSlab;
+    sts128(slab + sw_off(row, group), make_uint4(v[0], v[1], v[2], v[3]));
+    sts128(slab + sw_off(row, group + 1), make_uint4(v[4], v[5], v[6], v[7]));
+}
+
+// ---- LayerNorm ----
+// Partial sums of eight columns each, then the butterfly 16, 8, 4, 2, 1 over the row's 32 partials,
+// in the reference's order (see `ln_stage`).  A row's partials meet in shared memory; a few of the
+// board's warps, eight rows each, then finish them -- four lanes to a row: sums and squares, each
+// with half of what the member threads' order leaves after the butterfly's outer levels, which are plain
+// additions in the lane -- and leave mean, 1/sqrt, 1/scale and scale for everybody.  (Every thread reading
+// all of its row's partials instead is 1,500 cycles of shared-memory bandwidth per norm; all sixteen
+// warps finishing two to four rows each put the same chain of 90 instructions into every scheduler
+// four times over, 780 cycles.)
+template <int NB, int kAr>
+__device__ __forceinline__ float4 row_statistics(const Row& c, const Params& p, const uint32_t (&x)[8 * NB]) {
+    using O = Own<NB>;
+    constexpr uint32_t kSquares = 8 * 512 + 64;                 // NB == 2: the squares' offset (other banks)
+    constexpr uint32_t kMinMax = 12288;
+    const uint32_t base = c.h + 16384u * O::board(c);
+    const int t = O::member(c);
+    {
+        uint64_t s2[NB], q2[NB];
+#pragma unroll
+        for (int pr = 0; pr < NB; ++pr) {
+            s2[pr] = pk2(0.f, 0.f);
+            q2[pr] = pk2(0.f, 0.f);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const uint32_t wa = x[8 * pr + k], wb = x[8 * pr + 4 + k];
+                uint64_t f = h2_to_f2(__byte_perm(wa, wb, 0x5410));
+                s2[pr] = add2(s2[pr], f);
+                q2[pr] = fma2(f, f, q2[pr]);
+                f = h2_to_f2(__byte_perm(wa, wb, 0x7632));
+                s2[pr] = add2(s2[pr], f);
+                q2[pr] = fma2(f, f, q2[pr]);
+            }
+        }
+        __half2 mn = as_h2(x[0]), mx = as_h2(x[0]);
+#pragma unroll
+        for (int i = 1; i < 8 * NB; ++i) {
+            mn = __hmin2(mn, as_h2(x[i]));
+            mx = __hmax2(mx, as_h2(x[i]));
+        }
+        const uint32_t at = base + 512u * t + 16u * c.lane;
+        float a0, a1, b0, b1;
+        upk2(s2[0], a0, a1);
+        if constexpr (NB == 1) {
+            upk2(q2[0], b0, b1);
+            sts_f4(at, make_float4(a0, a1, b0, b1));
+        } else {
+            upk2(s2[1], b0, b1);
+            sts_f4(at, make_float4(a0, a1, b0, b1));
+            upk2(q2[0], a0, a1);
+            upk2(q2[1], b0, b1);
+            sts_f4(at + kSquares, make_float4(a0, a1, b0, b1));
+        }
+        // (minimum, -maximum): one packed minimum reduces both
+        const __half2 lo = __lows2half2(mn, __hneg2(mx)), hi = __highs2half2(mn, __hneg2(mx));
+        sts32(base + kMinMax + 128u * t + 4u * c.lane, as_u32(__hmin2(lo, hi)));
+    }
+    board_sync<NB>(c);
+    if (c.s < NB) {
+        const int lane = c.lane, j = lane & 3;                           // j: bit 1 squares, bit 0 which half
+        const int r = 8 * (NB == 1 ? c.q : 2 * (c.q >> 1) + c.s) + (lane >> 2);
+        float v;
+        if constexpr (NB == 1) {
+            // levels 16 and 8 over the quadrants, 4 and 2 over s, 1 over the thread's two partials
+            const uint32_t at = base + 16u * r + 4u * j;
+            float m[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                m[k] = __fadd_rn(__fadd_rn(lds_f(at + 512u * k), lds_f(at + 512u * (k + 8))),
+                                 __fadd_rn(lds_f(at + 512u * (k + 4)), lds_f(at + 512u * (k + 12))));
+            v = __fadd_rn(__fadd_rn(m[0], m[2]), __fadd_rn(m[1], m[3]));
+            v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 1));
+        } else {
+            // levels 16, 8 and 4 over the members, 2 over the halves of their four partials, 1 in the lane
+            const uint32_t at = base + (j >> 1) * kSquares + 16u * r + 8u * (j & 1);
+            uint64_t m[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) m[k] = lds_u64(at + 512u * k);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) m[k] = add2(m[k], m[k + 4]);
+            float a, b;
+            upk2(add2(add2(m[0], m[2]), add2(m[1], m[3])), a, b);
+            a = __fadd_rn(a, __shfl_xor_sync(0xffffffffu, a, 1));
+            b = __fadd_rn(b, __shfl_xor_sync(0xffffffffu, b, 1));
+            v = __fadd_rn(a, b);
+        }
+        __half2 mm = as_h2(lds_u(base + kMinMax + 128u * j + 4u * r));
+#pragma unroll
+        for (int k = 4; k < O::kGroup; k += 4) mm = __hmin2(mm, as_h2(lds_u(base + kMinMax + 128u * (j + k) + 4u * r)));
+        mm = __hmin2(mm, as_h2(__shfl_xor_sync(0xffffffffu, as_u32(mm), 1)));
+        mm = __hmin2(mm, as_h2(__shfl_xor_sync(0xffffffffu, as_u32(mm), 2)));
+        const float other = __shfl_xor_sync(0xffffffffu, v, 2);
+        const float tot = (j & 2) ? other : v, totq = (j & 2) ? v : other;
+        const float xmin = __low2float(mm), xmax = -__high2float(mm);
+        const float mean = __fmul_rn(tot, 1.0f / 256.0f);
+        const float var = fmaxf(__fsub_rn(__fmul_rn(totq, 1.0f / 256.0f), __fmul_rn(mean, mean)), 0.f);
+        const float rstd = p.rsqrt_rn ? __frsqrt_rn(__fadd_rn(var, p.eps)) : rsqrtf(__fadd_rn(var, p.eps));
+        const float e_lo = __half2float(__float2half_rn(__fmul_rn(__fsub_rn(xmin, mean), rstd)));
+        const float e_hi = __half2float(__float2half_rn(__fmul_rn(__fsub_rn(xmax, mean), rstd)));
+        const float amax = fmaxf(fabsf(e_lo), fabsf(e_hi));
+        const Scale sc = kAr == kArE4M3 ? scale_e4m3(amax) : scale_s8(amax);
+        if (j == 0) sts_f4(c.smem + SM_STAT + 16u * (32 * O::board(c) + r), make_float4(-mean, rstd, sc.inverse, sc.scale));
+    }
+    board_sync<NB>(c);
+    return lds_f4(c.smem + SM_STAT + 16u * O::row(c));
+}
+
+// An attention or FFN norm: x_hat = fp16((x - mean) * rstd) into the A operand, quantised (returns the
+// row's scale) or as it is.
+template <int NB, int kAr>
+__device__ __forceinline__ float norm_to_operand(const Row& c, const Params& p, const uint32_t (&x)[8 * NB], bool as_f16) {
+    const float4 st = row_statistics<NB, kAr>(c, p, x);
+    const uint64_t nmean2 = pk2(st.x, st.x), rstd2 = pk2(st.y, st.y);
+#pragma unroll
+    for (int k = 0; k < NB; ++k) {
+        uint32_t v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = f2_to_h2(mul2(add2(h2_to_f2(x[8 * k + i]), nmean2), rstd2));
+        if (kAr != kArInt8 && kAr != kArI8Qkv && as_f16) store_operand16<NB>(c, c.a(), k, v);
+        else store_operand8<NB, kAr == kArE4M3>(c, c.a(), k, v, st.z);
+    }
+    publish(c, B_A);
+    return st.w;
+}
+
+// ---- attention ----
+// A head's 32 rows of 32 halves in a 2 KB block: 64-byte rows, 16-byte groups moved by the row pair so
+// that eight rows of one group (what ldmatrix and a warp's stores touch at a time) hit all banks.
+__device__ __forceinline__ uint32_t head_off(int row, int group) {
+    return static_cast<uint32_t>(row) * 64u + (static_cast<uint32_t>(group ^ ((row >> 1) & 3)) << 4);
+}
+// Scores of 16 query rows (fragments qa) against the head's 32 keys, softmax, probabilities as A
+// fragments: `attention_unit`'s arithmetic.
+__device__ __forceinline__ void scores(const uint32_t (&qa)[2][4], uint32_t ks, int lane, uint32_t (&s)[4][2]) {
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) {
+        s[nt][0] = s[nt][1] = 0u;
+        uint32_t kb[4];
+        ldmatrix_x4(kb, ks + head_off(8 * nt + (lane & 7), lane >> 3));
+        mma_f16_f16(s[nt], qa[0], kb[0], kb[1]);      // dims 0-15, then 16-31
+        mma_f16_f16(s[nt], qa[1], kb[2], kb[3]);
+    }
+}
+// e^x as 2^(x log2 e) on the hardware's 2^x.  `__expf` is the same but for results below 2^-126, which it
+// keeps as denormals: beside a row sum of at least 1 they change neither the sum nor a probability.
+__device__ __forceinline__ float exp_fast(float x) { return ex2_approx(__fmul_rn(x, 1.44269504088896340736f)); }
+__device__ __forceinline__ void softmax(uint32_t (&s)[4][2], const uint32_t (&dead)[4]) {
+#pragma unroll
+    for (int hi = 0; hi < 2; ++hi) {
+        float pv[4][2];
+        float mx = -INFINITY;
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) {
+            const __half2 val = __hadd2(as_h2(s[nt][hi]), as_h2(dead[nt]));
+            pv[nt][0] = __low2float(val);
+            pv[nt][1] = __high2float(val);
+            mx = fmaxf(mx, fmaxf(pv[nt][0], pv[nt][1]));
+        }
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+        float sum = 0.f;
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) {
+            pv[nt][0] = exp_fast(pv[nt][0] - mx);     // an all-dead row keeps the reference's NaN
+            pv[nt][1] = exp_fast(pv[nt][1] - mx);
+            sum += pv[nt][0] + pv[nt][1];
+        }
+        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+        const float inv = reciprocal(sum);
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) s[nt][hi] = pack_h2(pv[nt][0] * inv, pv[nt][1] * inv);
+    }
+}
+__device__ __forceinline__ void load_query(uint32_t (&qa)[2][4], uint32_t qs, int first, int lane) {
+#pragma unroll
+    for (int kk = 0; kk < 2; ++kk) ldmatrix_x4(qa[kk], qs + head_off(first + (lane & 15), 2 * kk + (lane >> 4)));
+}
+__device__ __forceinline__ void weighted_values(const uint32_t (&s)[4][2], uint32_t vs, int lane, uint32_t (&o)[4][2]) {
+    uint32_t pa[2][4];
+#pragma unroll
+    for (int kk = 0; kk < 2; ++kk) {
+        pa[kk][0] = s[2 * kk][0];     pa[kk][1] = s[2 * kk][1];
+        pa[kk][2] = s[2 * kk + 1][0]; pa[kk][3] = s[2 * kk + 1][1];
+    }
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) {
+        o[nt][0] = o[nt][1] = 0u;
+        uint32_t vb[4];
+        ldmatrix_x4_trans(vb, vs + head_off(lane, nt));
+        mma_f16_f16(o[nt], pa[0], vb[0], vb[1]);      // keys 0-15, then 16-31
+        mma_f16_f16(o[nt], pa[1], vb[2], vb[3]);
+    }
+}
+__device__ __forceinline__ void store_outputs(const uint32_t (&o)[4][2], uint32_t os, int first, int lane) {
+    const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) {
+        sts32(os + head_off(first + g, nt) + 4 * t, o[nt][0]);
+        sts32(os + head_off(first + g + 8, nt) + 4 * t, o[nt][1]);
+    }
+}
+
+// This thread's columns of product `m` (0 Q, 1 K, 2 V) as fp16 into its head's block.
+template <int NB, int kAr>
+__device__ __forceinline__ void stage_qkv(const Row& c, const LayerParams& lp, float sa, int m, uint32_t block) {
+    using O = Own<NB>;
+    const int col = O::col(c);
+    wait_acc(c, m, 0);
+    const float sw = __ldg(lp.sw_qkv + m * 2 + (col >> 7));
+    const __half* bias = lp.b_qkv + (col >> 6) * 192 + m * 64 + (col & 63);
+    each_piece<NB>(O::slot(c, m), [&](int k, const uint32_t (&acc)[16]) {
+        uint32_t h[8];
+        descale<16, false, Cfg<kAr>::kQkvF16 ? kAccPlain : kAccInt>(acc, sa, sw, bias + 16 * k, h);
+        if (k == 0) __syncwarp();
+        const int group = ((col & 31) >> 3) + 2 * k;
+        sts128(block + head_off(c.lane, group), make_uint4(h[0], h[1], h[2], h[3]));
+        sts128(block + head_off(c.lane, group + 1), make_uint4(h[4], h[5], h[6], h[7]));
+    });
+}
+
+template <int NB, int kAr>
+__device__ __forceinline__ void attention_block(const Row& c, const LayerParams& lp, float sa, uint32_t alive, uint32_t (&x)[8 * NB]) {
+    using O = Own<NB>;
+    const int lane = c.lane, col = O::col(c);
+    uint32_t dead[4];
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) {
+        const uint32_t two = (alive >> (8 * nt + 2 * (lane & 3))) & 3u;
+        dead[nt] = ((two & 1u) ? 0u : 0xfc00u) | ((two & 2u) ? 0u : 0xfc000000u);
+    }
+    uint32_t oh[8 * NB];
+    // Q, K and V one after the other.  Two boards: one warp per head, whose block serves Q, K, V and the
+    // outputs in turn.  One board: two warps per head, each with half the query rows; Q, K and V have
+    // blocks of their own and the outputs go over Q.
+    const int head = NB == 1 ? 2 * c.q + (c.s >> 1) : 4 * c.q + c.s;
+    const int first = NB == 1 ? 16 * (c.s & 1) : 0;
+    const uint32_t block = c.h + 2048u * head;
+    uint32_t qa[NB][2][4], s[NB][4][2];
+#pragma unroll
+    for (int u = 0; u < NB; ++u) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) { qa[u][i >> 2][i & 3] = 0u; s[u][i >> 1][i & 1] = 0u; }
+    }
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+        const uint32_t at = NB == 1 ? block + 16384u * m : block;
+        stage_qkv<NB, kAr>(c, lp, sa, m, at);
+        if (NB == 1) { if (m > 0) pair_sync(head); } else __syncwarp();
+        if (m == 0) {
+            if (NB == 2) {
+                load_query(qa[0], at, 0, lane);
+                load_query(qa[NB - 1], at, 16, lane);
+            }
+        } else if (m == 1) {
+            if (NB == 1) load_query(qa[0], block, first, lane);
+#pragma unroll
+            for (int u = 0; u < NB; ++u) scores(qa[u], at, lane, s[u]);
+#pragma unroll
+            for (int u = 0; u < NB; ++u) softmax(s[u], dead);
+        } else {
+            uint32_t o[NB][4][2];
+#pragma unroll
+            for (int u = 0; u < NB; ++u) weighted_values(s[u], at, lane, o[u]);
+            __syncwarp();
+#pragma unroll
+            for (int u = 0; u < NB; ++u) store_outputs(o[u], block, first + 16 * u, lane);
+        }
+    }
+    if (NB == 1) pair_sync(head); else __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 2 * NB; ++k) {
+        const uint4 v = lds128(block + head_off(lane, ((col & 31) >> 3) + k));
+        oh[4 * k] = v.x; oh[4 * k + 1] = v.y; oh[4 * k + 2] = v.z; oh[4 * k + 3] = v.w;
+    }
+    // the attention output is the out-projection's operand: quantised by its row maximum, or as it is
+    Scale so = {1.f, 1.f};
+    if constexpr (Cfg<kAr>::kOutF16) {
+#pragma unroll
+        for (int k = 0; k < NB; ++k) store_operand16<NB>(c, c.a(), k, &oh[8 * k]);
+    } else {
+        const uint32_t m = c.smem + SM_MAX + 4u * O::row(c);
+        max_to(m, amax_h2<8 * NB>(oh, true));
+        board_sync<NB>(c);
+        so = scale_s8(lds_f(m));
+#pragma unroll
+        for (int k = 0; k < NB; ++k) store_operand8<NB>(c, c.a(), k, &oh[8 * k], so.inverse);
+    }
+    publish(c, B_A);
+    // x = fp16(x + fp16(fp16(descale) + b_o))
+    wait_acc(c, 3, 0);
+    const float sw = __ldg(lp.sw_o + (col >> 7));
+    each_piece<NB>(O::slot(c, 3), [&](int k, const uint32_t (&acc)[16]) {
+        uint32_t y[8];
+        descale<16, false, Cfg<kAr>::kOutF16 ? kAccPlain : kAccInt>(acc, so.scale, sw, lp.b_o + col + 16 * k, y);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[8 * k + i] = as_u32(__hadd2(as_h2(x[8 * k + i]), as_h2(y[i])));
+    });
+}
+
+// ---- FFN ----
+// Two hidden chunks at a time: ff1's epilogue (descale, bias, ReLU, row maximum), one meeting of the
+// board for both maxima, quantisation into the ff2 operand.  ff2's products of the first pair run
+// under the second pair's epilogue; their four sums are added to the fp16 running total in order.
+template <int NB, int kAr>
+__device__ __forceinline__ void ffn_block(const Row& c, const LayerParams& lp, float sa, uint32_t (&x)[8 * NB]) {
+    using O = Own<NB>;
+    const int col = O::col(c), row = O::row(c);
+    float s1[4] = {1.f, 1.f, 1.f, 1.f};
+#pragma unroll 1
+    for (int pair = 0; pair < 2; ++pair) {
+        uint32_t hid[2][8 * NB];
+        const uint32_t m = c.smem + SM_MAX + 256u * (1 + 2 * pair) + 4u * row;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int ch = 2 * pair + k;
+            wait_acc(c, ch, 1);
+            const float sw = __ldg(lp.sw_ff1 + 2 * ch + (col >> 7));
+            each_piece<NB>(O::slot(c, ch), [&](int i, const uint32_t (&acc)[16]) {
+                descale<16, true, kAr == kArE4M3 ? kAccFloat : kAccInt>(acc, sa, sw, lp.b_ff1 + 256 * ch + col + 16 * i, &hid[k][8 * i]);
+            });
+            max_to(m + 256u * k, amax_h2<8 * NB>(hid[k], false));
+        }
+        board_sync<NB>(c);
+        s1[0] = s1[2]; s1[1] = s1[3];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const float amax = lds_f(m + 256u * k);
+            const Scale sc = kAr == kArE4M3 ? scale_e4m3(amax) : scale_u8(amax);
+            s1[2 + k] = sc.scale;
+#pragma unroll
+            for (int i = 0; i < NB; ++i)
+                store_operand8<NB, kAr == kArE4M3>(c, c.h + (2 * pair + k) * 2 * O::kSlab, i, &hid[k][8 * i], sc.inverse);
+        }
+        publish(c, B_H + pair);
+    }
+    uint32_t run[8 * NB];
+#pragma unroll
+    for (int i = 0; i < 8 * NB; ++i) run[i] = 0u;
+    const float s2 = __ldg(lp.sw_ff2 + (col >> 7));
+    const uint64_t s2_2 = pk2(s2, s2);
+#pragma unroll 1
+    for (int ch = 0; ch < 4; ++ch) {
+        wait_acc(c, ch, 2);
+        const uint64_t s1_2 = pk2(s1[0], s1[0]);
+        s1[0] = s1[1]; s1[1] = s1[2]; s1[2] = s1[3];
+        each_piece<NB>(O::slot(c, ch), [&](int k, const uint32_t (&acc)[16]) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                // `float(acc) * sa * sw + float(run)`: the second product and the sum are one fma (and
+                // with the zero that the total starts from, a plain product)
+                const uint64_t f = mul2(kAr == kArE4M3 ? pk2(__uint_as_float(acc[2 * i]), __uint_as_float(acc[2 * i + 1]))
+                                                       : pk2(static_cast<float>(static_cast<int>(acc[2 * i])),
+                                                             static_cast<float>(static_cast<int>(acc[2 * i + 1]))), s1_2);
+                run[8 * k + i] = f2_to_h2(fma2(f, s2_2, h2_to_f2(run[8 * k + i])));
+            }
+        });
+    }
+    // + b_ff2, residual: x = fp16(x + fp16(run + b))
+    const uint4* b4 = reinterpret_cast<const uint4*>(lp.b_ff2 + col);
+#pragma unroll
+    for (int v = 0; v < 2 * NB; ++v) {
+        const uint4 bv = __ldg(b4 + v);
+        const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int i = 4 * v + k;
+            x[i] = as_u32(__hadd2(as_h2(x[i]), __hadd2(as_h2(run[i]), as_h2(bw[k]))));
+        }
+    }
+}
+
+// The fp16 arithmetic's FFN: ff1's epilogue is bias and ReLU, a chunk goes out as ff2's fp16 operand, and
+// ff2's fp16 accumulators (slot 0) run on through the four chunks.  H holds two chunks, so the second
+// pair is written when the first pair's ff2 products are done (a completion of slot 0 that says no more
+// than that); the last completion, on every slot, says that the sums are there.
+template <int NB>
+__device__ __forceinline__ void ffn_block_f16(const Row& c, const LayerParams& lp, uint32_t (&x)[8 * NB]) {
+    using O = Own<NB>;
+    const int col = O::col(c);
+#pragma unroll 1
+    for (int pair = 0; pair < 2; ++pair) {
+#pragma unroll 1
+        for (int k = 0; k < 2; ++k) {
+            const int ch = 2 * pair + k;
+            wait_acc(c, ch, 1);
+            if (ch == 2) wait_acc(c, 0, 2);
+            each_piece<NB>(O::slot(c, ch), [&](int i, const uint32_t (&acc)[16]) {
+                uint32_t h[8];
+                descale<16, true, kAccPlain>(acc, 1.f, 1.f, lp.b_ff1 + 256 * ch + col + 16 * i, h);
+                store_operand16<NB>(c, c.h + k * 4 * O::kSlab, i, h);
+            });
+        }
+        publish(c, B_H + pair);
+    }
+    wait_acc(c, 1, 2);
+    each_piece<NB>(O::slot(c, 0), [&](int k, const uint32_t (&acc)[16]) {
+        uint32_t y[8];
+        descale<16, false, kAccPlain>(acc, 1.f, 1.f, lp.b_ff2 + col + 16 * k, y);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[8 * k + i] = as_u32(__hadd2(as_h2(x[8 * k + i]), as_h2(y[i])));
+    });
+}
+
+// ---- heads ----
+// The "prenorm" value head (see `prenorm_value`): column means over the board's live tokens, one
+// LayerNorm with affine of that vector, dotted with the value rows; every thread returns the logits.
+template <int NB>
+__device__ __forceinline__ void prenorm_logits(const Row& c, const Params& p, uint32_t alive, const uint32_t (&x)[8 * NB], float (&logit)[3]) {
+    using O = Own<NB>;
+    const bool live = (alive >> c.lane) & 1u;
+    const int nlive = __popc(alive);
+    const float inv_live = 1.0f / static_cast<float>(nlive > 0 ? nlive : 1);
+    const uint32_t xch = c.h + 16384u * O::board(c);
+    float v[11];
+#pragma unroll
+    for (int piece = 0; piece < NB; ++piece) {               // sixteen columns at a time, whatever NB: one order of sums
+        const int col = O::col(c) + 16 * piece;
+#pragma unroll
+        for (int i = 0; i < 11; ++i) v[i] = 0.f;             // s, q, s1[3], s2[3], s3[3]
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float2 f = __half22float2(as_h2(x[8 * piece + i]));
+            float a0 = live ? f.x : 0.f, a1 = live ? f.y : 0.f;
+#pragma unroll
+            for (int off = 16; off; off >>= 1) {
+                a0 += __shfl_xor_sync(0xffffffffu, a0, off);
+                a1 += __shfl_xor_sync(0xffffffffu, a1, off);
+            }
+            a0 *= inv_live; a1 *= inv_live;
+            v[0] += a0 + a1;
+            v[1] += a0 * a0 + a1 * a1;
+            const float2 g = __half22float2(as_h2(__ldg(reinterpret_cast<const uint32_t*>(p.tail + col) + i)));
+            const float2 b = __half22float2(as_h2(__ldg(reinterpret_cast<const uint32_t*>(p.tail + kD + col) + i)));
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const float2 w = __half22float2(as_h2(__ldg(reinterpret_cast<const uint32_t*>(p.tail + 2 * kD + k * kD + col) + i)));
+                v[2 + k] += a0 * g.x * w.x + a1 * g.y * w.y;
+                v[5 + k] += g.x * w.x + g.y * w.y;
+                v[8 + k] += b.x * w.x + b.y * w.y;
+            }
+        }
+        if (c.lane == 0)
+#pragma unroll
+            for (int i = 0; i < 11; ++i) sts32(xch + 4u * col + 4u * i, __float_as_uint(v[i]));    // 64 bytes per piece
+    }
+    board_sync<NB>(c);
+#pragma unroll
+    for (int i = 0; i < 11; ++i) v[i] = 0.f;
+#pragma unroll 1
+    for (int t = 0; t < 16; ++t)
+#pragma unroll
+        for (int i = 0; i < 11; ++i) v[i] += lds_f(xch + 64u * t + 4u * i);
+    board_sync<NB>(c);
+    const float mean = v[0] * (1.0f / 256.0f);
+    const float rstd = rsqrtf(fmaxf(__fsub_rn(v[1] * (1.0f / 256.0f), __fmul_rn(mean, mean)), 0.f) + p.eps);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) logit[k] = rstd * (v[2 + k] - mean * v[5 + k]) + v[8 + k];
+}
+
+// Final norm into the head product's fp16 operand, then the epilogue: the product's 128 output columns
+// (64 policy, 4 promotion, value, padding) lie 8 NB to a thread.  Policy columns are masked and stored
+// by the threads that hold them; with a fused expansion the board's logits are staged in its own rows
+// of the A operand (which the next tile writes only after a meeting of the board) for one warp.
+template <int NB, int kAr>
+__device__ __forceinline__ void heads(const Row& c, const Params& p, int board, bool valid, uint32_t word, int ctl, uint32_t alive,
+                                      const uint32_t (&x)[8 * NB]) {
+    using O = Own<NB>;
+    const int col = O::col(c), row = O::row(c), lane = c.lane;
+    const long grow = static_cast<long>(board) * kT + lane;
+    float pre[3] = {0.f, 0.f, 0.f};
+    if (p.vmode == 2) prenorm_logits<NB>(c, p, alive, x, pre);
+    {
+        const float4 st = row_statistics<NB, kAr>(c, p, x);
+        const uint64_t nmean2 = pk2(st.x, st.x), rstd2 = pk2(st.y, st.y);
+        const uint4* g4 = reinterpret_cast<const uint4*>(p.tail + col);
+        const uint4* b4 = reinterpret_cast<const uint4*>(p.tail + kD + col);
+#pragma unroll
+        for (int v = 0; v < 2 * NB; ++v) {
+            const uint4 gv = __ldg(g4 + v), bv = __ldg(b4 + v);
+            const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w}, bw[4] = {bv.x, bv.y, bv.z, bv.w};
+            uint32_t y[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                y[j] = f2_to_h2(fma2(mul2(add2(h2_to_f2(x[4 * v + j]), nmean2), rstd2), h2_to_f2(gw[j]), h2_to_f2(bw[j])));
+            sts128(c.h + kHeadA + (col >> 6) * O::kSlab + sw_off(row, ((col & 63) >> 3) + v), make_uint4(y[0], y[1], y[2], y[3]));
+        }
+        publish(c, B_A);
+    }
+    // output columns of this thread: hc .. hc + 8 NB - 1
+    const int hc = NB == 1 ? 32 * c.q + 8 * c.s : 64 * (c.q >> 1) + 16 * c.s;
+    // while the product runs: the legality words, given or (for the expansion warp, lane = slot) made here
+    const bool expander = p.prior != nullptr && hc == 72 + 8 * (NB - 1);     // a warp whose columns are padding
+    unsigned long long lw = ~0ull, moves = 0ull;
+    if (p.legal != nullptr && valid && (hc < 64 || expander)) lw = p.legal[grow];
+    if (expander && valid) {
+        bool in_check;
+        moves = p.legal != nullptr ? lw : bfmg::legal_word(word, ctl, in_check);
+    }
+    wait_acc(c, 0, 0);
+    uint32_t v[4 * NB];
+    {
+        uint32_t acc[8 * NB];
+        const uint32_t t = c.tm + 8 * NB * c.s;
+        if constexpr (NB == 1) tmem_ld8(t, acc); else tmem_ld16(t, acc);
+        tmem_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 4 * NB; ++i) v[i] = __byte_perm(acc[2 * i], acc[2 * i + 1], 0x5410);
+    }
+    const uint32_t stage_pol = c.a(), stage_aux = c.a() + O::kSlab;
+    if (p.prior != nullptr && hc <= 64) {
+#pragma unroll
+        for (int k = 0; k < NB; ++k)
+            sts128((hc < 64 ? stage_pol : stage_aux) + sw_off(row, ((hc & 63) >> 3) + k),
+                   make_uint4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]));
+    }
+    if (hc < 64) {
+        if (valid && p.policy != nullptr) {
+            const uint32_t bits = static_cast<uint32_t>(lw >> hc);
+#pragma unroll
+            for (int i = 0; i < 4 * NB; ++i) {
+                if (!((bits >> (2 * i)) & 1u)) v[i] = (v[i] & 0xffff0000u) | 0xfc00u;
+                if (!((bits >> (2 * i + 1)) & 1u)) v[i] = (v[i] & 0x0000ffffu) | 0xfc000000u;
+            }
+            store_words<4 * NB>(p.policy + grow * 64 + hc, v);
+        }
+    } else if (hc == 64) {
+        if (valid && p.promo != nullptr) *reinterpret_cast<uint2*>(p.promo + grow * 4) = make_uint2(v[0], v[1]);
+        // value logits: columns 68, 69, 70
+        float a = __low2float(as_h2(v[2])), b = __high2float(as_h2(v[2])), d = __low2float(as_h2(v[3]));
+        if (p.vmode == 1) {
+            // live tokens in slot order, one after the other
+            float ta = 0.f, tb = 0.f, td = 0.f;
+#pragma unroll 1
+            for (int tt = 0; tt < kT; ++tt) {
+                const float at = __shfl_sync(0xffffffffu, a, tt), bt = __shfl_sync(0xffffffffu, b, tt);
+                const float dt = __shfl_sync(0xffffffffu, d, tt);
+                if ((alive >> tt) & 1u) { ta += at; tb += bt; td += dt; }
+            }
+            const int nlive = __popc(alive);
+            const float inv = 1.0f / static_cast<float>(nlive > 0 ? nlive : 1);
+            a = ta * inv; b = tb * inv; d = td * inv;
+        }
+        if (p.vmode == 2) { a = pre[0]; b = pre[1]; d = pre[2]; }
+        const bool writer = p.vmode != 0 ? lane == 0 : lane == (ctl < 0 ? 31 : 15);
+        if (writer && valid && p.value != nullptr) {
+            float o;
+            if (p.n_value == 1) {
+                o = tanhf(a);
+            } else {
+                const float m = fmaxf(a, fmaxf(b, d));
+                const float ea = expf(a - m), eb = expf(b - m), ec = expf(d - m);
+                o = (ec - ea) / (ea + eb + ec);
+            }
+            if (p.vmode != 0 && ctl < 0) o = -o;
+            p.value[board] = o;
+        }
+    }
+    if (p.prior != nullptr) {
+        board_sync<NB>(c);                                   // the board's logits are staged
+        if (expander)
+            expand_board(p, board, lane, valid, word, ctl, moves, stage_pol, stage_aux, row,
+                         c.smem_gen + SM_LIST + 1024u * O::board(c));
+    }
+}
+
+// One tile of NB boards, from the piece words to the outputs.
+template <int NB, int kAr>
+__device__ __forceinline__ void row_tile(Row& c, const Params& p, int first) {
+    using O = Own<NB>;
+    const int item = first + O::board(c), lane = c.lane, col = O::col(c);
+    const bool valid = item < c.n;
+    const int board = (valid && p.leaf_index != nullptr) ? __ldg(p.leaf_index + item) : item;
+    const uint32_t word = valid ? p.boards[static_cast<long>(board) * kT + lane] : 0u;
+    uint32_t alive = __ballot_sync(0xffffffffu, ((word >> 11) & 1u) == 0u);
+    const int ctl = valid ? static_cast<int>(p.control[board]) : 1;
+    if (!valid) alive = 0xffffffffu;
+    uint32_t x[8 * NB];
+    // ---- embedding: ((square + type_special) + color_turn) + (clock + rep), fp16 ----
+    {
+        const int stm = ctl < 0;
+        const int clk = min(max((ctl < 0 ? -ctl : ctl) - 1, 0), kNClock - 1);
+        const int rp = min(valid ? static_cast<int>(p.rep[board]) : 0, kNRep - 1);
+        const int sq = word & 63;
+        const int ts = min(static_cast<int>(((word >> 6) & 7) * 2 + ((word >> 9) & 1)), kNTypeSpecial - 1);
+        const int ct = ((word >> 10) & 1) * 2 + stm;
+        const uint4* e_sq = reinterpret_cast<const uint4*>(p.emb + (EMB_SQUARE + sq) * kD + col);
+        const uint4* e_ts = reinterpret_cast<const uint4*>(p.emb + (EMB_TS + ts) * kD + col);
+        const uint4* e_ct = reinterpret_cast<const uint4*>(p.emb + (EMB_CT + ct) * kD + col);
+        const uint4* e_ck = reinterpret_cast<const uint4*>(p.emb + (EMB_CLOCK + clk) * kD + col);
+        const uint4* e_rp = reinterpret_cast<const uint4*>(p.emb + (EMB_REP + rp) * kD + col);
+#pragma unroll
+        for (int k = 0; k < 2 * NB; ++k) {
+            const uint4 a = __ldg(e_sq + k), b = __ldg(e_ts + k), d = __ldg(e_ct + k);
+            const uint4 e = __ldg(e_ck + k), f = __ldg(e_rp + k);
+            const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
+            const uint32_t dw[4] = {d.x, d.y, d.z, d.w}, ew[4] = {e.x, e.y, e.z, e.w};
+            const uint32_t fw[4] = {f.x, f.y, f.z, f.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                __half2 v = __hadd2(as_h2(aw[j]), as_h2(bw[j]));
+                v = __hadd2(v, as_h2(dw[j]));
+                x[4 * k + j] = as_u32(__hadd2(v, __hadd2(as_h2(ew[j]), as_h2(fw[j]))));
+            }
+        }
+    }
+    const int id = 128 * c.q + 32 * c.s + lane;              // 0 .. 511
+    // half-layers, so that the norm's code is there once
+    const int n_half = 2 * p.n_layers;
+    const uint8_t* lpb = p.lparams;
+#pragma unroll 1
+    for (int half = 0; half < n_half; ++half) {
+        // the layer's scales and biases are asked into L1 a norm ahead of their first use
+        if (id < kLparamStride / 128) prefetch_l1(lpb + 128 * id);
+        LayerParams lp;
+        lp.sw_qkv = reinterpret_cast<const float*>(lpb + LP_SW_QKV);
+        lp.sw_o = reinterpret_cast<const float*>(lpb + LP_SW_O);
+        lp.sw_ff1 = reinterpret_cast<const float*>(lpb + LP_SW_FF1);
+        lp.sw_ff2 = reinterpret_cast<const float*>(lpb + LP_SW_FF2);
+        lp.b_qkv = reinterpret_cast<const __half*>(lpb + LP_B_QKV);
+        lp.b_o = reinterpret_cast<const __half*>(lpb + LP_B_O);
+        lp.b_ff1 = reinterpret_cast<const __half*>(lpb + LP_B_FF1);
+        lp.b_ff2 = reinterpret_cast<const __half*>(lpb + LP_B_FF2);
+        // the row maxima start at zero: the hidden chunks' are cleared before the attention norm's
+        // meetings, the attention output's before the FFN norm's (and at the start), ahead of their use
+        const uint32_t mx = c.smem + SM_MAX + 4u * O::row(c);
+        if ((half & 1) == 0 && O::member(c) < 4) sts32(mx + 256u * (1 + O::member(c)), 0u);
+        if (((half & 1) || half == 0) && O::member(c) == 4) sts32(mx, 0u);
+        const float sa = norm_to_operand<NB, kAr>(c, p, x, kAr == kArF16 || (half & 1) == 0);
+        if ((half & 1) == 0) {
+            attention_block<NB, kAr>(c, lp, sa, alive, x);
+        } else {
+            if constexpr (kAr == kArF16) ffn_block_f16<NB>(c, lp, x);
+            else ffn_block<NB, kAr>(c, lp, sa, x);
+            c.layers++;
+            lpb += kLparamStride;
+        }
+    }
+    if (id < static_cast<int>(kTailBytes / 128)) prefetch_l1(reinterpret_cast<const uint8_t*>(p.tail) + 128 * id);
+    heads<NB, kAr>(c, p, board, valid, word, ctl, alive, x);
+    c.tiles++;
+}
+
+// ---- weight stream ----
+// The blob's stages are the four-board kernel's: per head pair [Q 64 | K 64 | V 64 rows], then 128-row
+// units, two to each 256-row product.  A stage here is 256 rows of one K-slab, put together from four
+// or two of their pieces.
+template <int kAr>
+__device__ __forceinline__ void producer(uint32_t smem, volatile int* abort_flag, const Params& p, int n_tiles) {
+    using C = Cfg<kAr>;
+    constexpr uint32_t kStages = Map<kAr>::kStages, kRing = Map<kAr>::SM_RING;
+    uint32_t i = 0;
+    auto begin = [&](uint32_t bytes) -> uint32_t {
+        const uint32_t k = i % kStages;
+        mbar_wait(bar(smem, B_EMPTY + k), (i / kStages - 1u) & 1u, abort_flag, kErrProducer);
+        mbar_arrive_expect_tx(bar(smem, B_FULL + k), bytes);
+        ++i;
+        return k;
+    };
+    // K-slab s of the product whose two 128-row units start at `u0` and `u1`
+    auto two_units = [&](const uint8_t* u0, const uint8_t* u1, int s) {
+        const uint32_t k = begin(kStage), dst = smem + kRing + k * kStage;
+        bulk_g2s(dst, u0 + s * kRStage, kRStage, bar(smem, B_FULL + k));
+        bulk_g2s(dst + kRStage, u1 + s * kRStage, kRStage, bar(smem, B_FULL + k));
+    };
+    for (int tile = 0; tile < n_tiles; ++tile) {
+        const uint8_t* src = p.wstream;
+        for (int layer = 0; layer < p.n_layers; ++layer, src += C::kLayerStream) {
+            for (int m = 0; m < 3; ++m)                                     // Q, K, V
+                for (int s = 0; s < C::kQkvSlabs; ++s) {
+                    const uint32_t k = begin(kStage), dst = smem + kRing + k * kStage;
+                    const uint8_t* from = src + s * kQStage + m * 8192;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        bulk_g2s(dst + 8192 * j, from + C::kQkvSlabs * j * kQStage, 8192, bar(smem, B_FULL + k));
+                }
+            const uint8_t* out = src + 4 * C::kQkvSlabs * kQStage;
+            for (int s = 0; s < C::kOutSlabs; ++s) two_units(out, out + C::kOutSlabs * kRStage, s);
+            // ff1 chunks 0-3, then ff2 chunks 0-3; where their two units lie in the packed order
+            const uint8_t* ffn = out + 2 * C::kOutSlabs * kRStage;
+            for (int u = 0; u < 8; ++u) {
+                int u0, u1;
+                if (kAr == kArF16) {
+                    const int ch = u & 3;
+                    u0 = u < 4 ? (ch == 0 ? 0 : 4 * ch - 2) : (ch < 3 ? 4 * ch + 3 : 14);
+                    u1 = u < 4 ? 4 * ch + 1 : (ch < 3 ? 4 * ch + 4 : 15);
+                } else {
+                    u0 = (0xEC84A620u >> (4 * u)) & 15u;
+                    u1 = u0 + 1;
+                }
+                for (int s = 0; s < C::kFfnSlabs; ++s)
+                    two_units(ffn + u0 * C::kFfnSlabs * kRStage, ffn + u1 * C::kFfnSlabs * kRStage, s);
+            }
+        }
+        for (uint32_t st = 0; st < kHeadStages; ++st, src += kHeadStage) {
+            const uint32_t k = begin(kHeadStage);
+            bulk_g2s(smem + kRing + k * kStage, src, kHeadStage, bar(smem, B_FULL + k));
+        }
+    }
+    // after a time-out copies may still be in flight: a bounded while for them to land
+    if (*abort_flag != 0) {
+        const long long t0 = clock64();
+        while (clock64() - t0 < 2000000LL) { }
+    }
+}
+
+// ---- MMA issue ----
+struct Issue {
+    uint32_t smem, tmem;
+    volatile int* abort_flag;
+    uint32_t i, a, h;           // weight stages, A operands, hidden pairs consumed
+};
+// One product: `slabs` K-slabs of 128 bytes; `more`: on top of what the slot holds.
+template <int kAr, int kKind>
+__device__ __forceinline__ void issue_unit(Issue& st, uint32_t d, uint32_t a_base, uint32_t slab, int slabs, uint32_t idesc,
+                                           bool more = false) {
+    constexpr uint32_t kStages = Map<kAr>::kStages;
+    for (int s = 0; s < slabs; ++s) {
+        const uint32_t k = st.i % kStages;
+        mbar_wait(bar(st.smem, B_FULL + k), (st.i / kStages) & 1u, st.abort_flag, kErrMmaWeights);
+        tc_fence_after();
+        const uint64_t ad = umma_desc_k128(a_base + s * slab), bd = umma_desc_k128(st.smem + Map<kAr>::SM_RING + k * kStage);
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+            const uint32_t accumulate = (more || (s | kk) != 0) ? 1u : 0u;
+            if (kKind == kKindF16)     umma_ws_f16(d, ad + 2 * kk, bd + 2 * kk, idesc, accumulate);
+            else if (kKind == kKindF8) umma_ws_f8(d, ad + 2 * kk, bd + 2 * kk, idesc, accumulate);
+            else                       umma_ws_i8(d, ad + 2 * kk, bd + 2 * kk, idesc, accumulate);
+        }
+        tc_commit(bar(st.smem, B_EMPTY + k));
+        st.i++;
+    }
+}
+__device__ __forceinline__ void issue_done(const Issue& st, int slot) { tc_commit(bar(st.smem, B_ACC + slot)); }
+__device__ __forceinline__ void issue_wait(const Issue& st, int b, uint32_t n) {
+    mbar_wait(bar(st.smem, b), n & 1u, st.abort_flag, kErrMmaOperand);
+    tc_fence_after();
+}
+template <int NB, int kAr>
+__device__ __forceinline__ void issue_tile(Issue& st, int n_layers) {
+    using O = Own<NB>;
+    using C = Cfg<kAr>;
+    constexpr uint32_t kI_S8 = umma_idesc(kAccS32, kFmtS8, kFmtS8, 32 * NB, 256);
+    constexpr uint32_t kI_F16 = umma_idesc(kAccF16, kFmtF16, kFmtF16, 32 * NB, 256);
+    constexpr uint32_t kI_E4M3 = umma_idesc(kAccF32, kFmtE4M3, kFmtE4M3, 32 * NB, 256);
+    constexpr uint32_t kI_QKV = C::kQkvF16 ? kI_F16 : kI_S8, kI_OUT = C::kOutF16 ? kI_F16 : kI_S8;
+    constexpr uint32_t kI_FF1 = kAr == kArF16 ? kI_F16 : kAr == kArE4M3 ? kI_E4M3 : kI_S8;
+    constexpr uint32_t kI_FF2 = kAr == kArF16 ? kI_F16 : kAr == kArE4M3 ? kI_E4M3
+                                              : umma_idesc(kAccS32, kFmtU8, kFmtS8, 32 * NB, 256);
+    constexpr uint32_t kI_HEAD = umma_idesc(kAccF16, kFmtF16, kFmtF16, 32 * NB, 128);
+    constexpr int kQkvKind = C::kQkvF16 ? kKindF16 : kKindI8, kOutKind = C::kOutF16 ? kKindF16 : kKindI8;
+    constexpr int kFfnKind = kAr == kArE4M3 ? kKindF8 : (kAr == kArF16 ? kKindF16 : kKindI8);
+    const uint32_t a = st.smem + SM_A, h = st.smem + Map<kAr>::SM_H;
+    for (int layer = 0; layer < n_layers; ++layer) {
+        issue_wait(st, B_A, st.a++);
+        for (int m = 0; m < 3; ++m) {
+            issue_unit<kAr, kQkvKind>(st, st.tmem + O::kSlot * m, a, O::kSlab, C::kQkvSlabs, kI_QKV);
+            issue_done(st, m);
+        }
+        issue_wait(st, B_A, st.a++);
+        issue_unit<kAr, kOutKind>(st, st.tmem + O::kSlot * 3, a, O::kSlab, C::kOutSlabs, kI_OUT);
+        issue_done(st, 3);
+        issue_wait(st, B_A, st.a++);
+        for (int ch = 0; ch < 4; ++ch) {
+            issue_unit<kAr, kFfnKind>(st, st.tmem + O::kSlot * ch, a, O::kSlab, C::kFfnSlabs, kI_FF1);
+            issue_done(st, ch);
+        }
+        for (int ch = 0; ch < 4; ++ch) {
+            if ((ch & 1) == 0) issue_wait(st, B_H + (ch >> 1), st.h);
+            if (kAr == kArF16) {
+                issue_unit<kAr, kFfnKind>(st, st.tmem, h + (ch & 1) * 4 * O::kSlab, O::kSlab, C::kFfnSlabs, kI_FF2, ch > 0);
+                if (ch == 1) issue_done(st, 0);
+            } else {
+                issue_unit<kAr, kFfnKind>(st, st.tmem + O::kSlot * ch, h + ch * 2 * O::kSlab, O::kSlab, C::kFfnSlabs, kI_FF2);
+                issue_done(st, ch);
+            }
+        }
+        if (kAr == kArF16)
+            for (int slot = 1; slot < 4; ++slot) issue_done(st, slot);
+        st.h++;
+    }
+    issue_wait(st, B_A, st.a++);
+    issue_unit<kAr, kKindF16>(st, st.tmem, h + kHeadA, O::kSlab, kHeadStages, kI_HEAD);
+    issue_done(st, 0);
+}
+
+// launch bounds: 640 threads, so that a scheduler's five warps fit its registers (96 each)
+template <int kAr>
+__global__ void __launch_bounds__(640, 1) encoder_ws_kernel(const Params p) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    const uint32_t smem = smem_u32(sm);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + SM_MISC + 4);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + SM_MISC);
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < B_COUNT; ++i) mbar_init(bar(smem, i), i >= B_A ? kRowWarps : 1);
+        *abort_flag = 0;
+        fence_barrier_init();
+    }
+    if (warp == kMmaWarp) {
+        tmem_alloc(smem + SM_MISC, TM_COLS);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    int n_eval = p.n;
+    if (p.leaf_count != nullptr) n_eval = min(max(__ldg(p.leaf_count), 0), p.n);
+    const Tiles tiles(n_eval, gridDim.x, blockIdx.x, p.one_most);
+    const int n_tiles = tiles.count();
+    if (warp < kRowWarps) {
+        Row c;
+        c.lane = lane; c.q = warp & 3; c.s = warp >> 2;
+        c.smem = smem; c.smem_gen = sm; c.h = smem + Map<kAr>::SM_H;
+        c.tm = tmem + (static_cast<uint32_t>(32 * c.q) << 16);
+        c.abort_flag = abort_flag;
+        c.one2 = pk2(p.one, p.one);
+        c.layers = c.tiles = 0;
+        c.n = n_eval;
+        for (int k = 0; k < n_tiles; ++k) {
+            int first, boards;
+            tiles.at(k, first, boards);
+            if (boards == 1) row_tile<1, kAr>(c, p, first);
+            else             row_tile<2, kAr>(c, p, first);
+        }
+    } else if (warp == kProducerWarp) {
+        if (elect_one()) producer<kAr>(smem, abort_flag, p, n_tiles);
+    } else {
+        if (elect_one()) {
+            Issue st = {smem, tmem, abort_flag, 0, 0, 0};
+            for (int k = 0; k < n_tiles; ++k) {
+                int first, boards;
+                tiles.at(k, first, boards);
+                if (boards == 1) issue_tile<1, kAr>(st, p.n_layers);
+                else             issue_tile<2, kAr>(st, p.n_layers);
+            }
+        }
+    }
+    __syncwarp();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == kMmaWarp) tmem_dealloc(tmem, TM_COLS);
+    if (threadIdx.x == 0 && *abort_flag != 0) atomicCAS(p.status, 0, *abort_flag);
+}
+
+}  // namespace ws
+}  // namespace bf

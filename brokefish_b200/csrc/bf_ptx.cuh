@@ -57,23 +57,29 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity)
 // Bounded wait.  `abort_flag` is a CTA-shared word: once any wait in the CTA has run
 // out of time it is set, and every later wait returns at once, so a lost arrival ends
 // the kernel with an error status instead of a hang.  Returns false on time-out.
-constexpr long long kWaitCycles = 400000000LL;   // ~0.2 s at 2 GHz
-__device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, volatile int* abort_flag,
-                                            int code) {
-    const long long t0 = clock64();
-    while (true) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if (*abort_flag != 0) return false;
-        if (clock64() - t0 > kWaitCycles) {
-            atomicCAS(const_cast<int*>(abort_flag), 0, code);
-            return false;
-        }
-    }
-}
+//
+// All of it inline: the single-thread regions of the weight stream and the MMA issuers keep addresses
+// and descriptors in uniform registers, and a function call in the middle of such a region is not
+// something to build on.
+constexpr unsigned kWaitCycles = 400000000u;     // ~0.2 s at 2 GHz
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity,
                                           volatile int* abort_flag, int code) {
     if (mbar_try_wait(bar, parity)) return true;
-    return mbar_wait_slow(bar, parity, abort_flag, code);
+    const uint32_t flag = smem_u32(const_cast<int*>(abort_flag));
+    uint32_t t0, t;
+    asm volatile("mov.u32 %0, %%clock;" : "=r"(t0) :: "memory");
+#pragma unroll 1
+    while (!mbar_try_wait(bar, parity)) {
+        int aborted;
+        asm volatile("ld.volatile.shared.b32 %0, [%1];" : "=r"(aborted) : "r"(flag) : "memory");
+        if (aborted != 0) return false;
+        asm volatile("mov.u32 %0, %%clock;" : "=r"(t) :: "memory");
+        if (t - t0 > kWaitCycles) {
+            asm volatile("{\n\t.reg .b32 o;\n\tatom.shared.cas.b32 o, [%0], 0, %1;\n\t}" ::"r"(flag), "r"(code) : "memory");
+            return false;
+        }
+    }
+    return true;
 }
 
 // Ask a 128-byte line of global memory into L1 (no register, no wait).
@@ -262,6 +268,36 @@ __device__ __forceinline__ void umma_f8(uint32_t d_tmem, uint64_t adesc, uint64_
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// The weight-stationary forms: M = 32 or 64 rows, N = 64, 128 or 256, the product laid out over all
+// 128 lanes (M = 32: quadrant q has columns q N / 4 .. ; M = 64: rows 32 (q & 1) .., columns
+// (q >> 1) N / 2 ..).  Operands, descriptors and accumulators as above.
+__device__ __forceinline__ void umma_ws_i8(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                           uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.ws.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void umma_ws_f16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                            uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.ws.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void umma_ws_f8(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                           uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.ws.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }

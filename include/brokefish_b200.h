@@ -101,8 +101,8 @@ int bf_forward_priors(bf_handle* h, const uint16_t* boards, const int16_t* contr
  * (`boards`, `control`, `rep`, `legal` indexed by place), the count read ON THE DEVICE when the
  * kernel starts, so the caller needs no host synchronisation to know it.  `capacity` is the most
  * the list can hold (the grid is sized for it; a larger count is clamped, a negative one is 0);
- * CTAs beyond the count's tiles leave at once, so a short list runs short, and an int8 list of at
- * most one position per SM runs in the small-batch form (BF_OPT_ONE_BOARD).  Every output is
+ * CTAs beyond the count's tiles leave at once, so a short list runs short, and a list of at
+ * most one position per SM runs on one-board tiles (BF_OPT_ONE_BOARD).  Every output is
  * written at the position's own place in the staged arrays (policy [place,32,64], value [place],
  * prior [place,e_cap] ...); places not in the list are not touched.  Any of policy / promo /
  * value may be NULL; pass prior, move and nedges (all three, else all NULL) for the fused
@@ -260,10 +260,10 @@ int bf_forward_priors_host(bf_handle* h, const uint16_t* boards, const int16_t* 
  *                    written straight into the caller's buffers (if pinned and device-mapped).
  *                    1: always the fast-link sizes; 2: always the equal launches.  Same outputs. */
 #define BF_OPT_HOST_PLAN 4
-/*   BF_OPT_ONE_BOARD k (default 1): an int8 evaluation of at most k boards per SM runs in the
- *                    small-batch form of the kernel -- one board per tile, its rows replicated in
- *                    the four lane quadrants, sixteen row warps per board instead of four, about
- *                    half the latency of a tile; 0 switches the form off.  Same outputs. */
+/*   BF_OPT_ONE_BOARD k (default 1): an evaluation of at most k boards per SM runs on tiles of one board,
+ *                    sixteen warps per board, and so does what is left of a larger one after whole
+ *                    waves of two-board tiles when it is at most one board per SM; 0 switches one-board
+ *                    tiles off.  Same outputs. */
 #define BF_OPT_ONE_BOARD 5
 int bf_set_option(bf_handle* h, int option, int value);
 
@@ -371,6 +371,12 @@ int bf_measure_elementwise(int device, int block, int iters, double* elements_pe
  * bf_status().  `waited_cycles` (may be NULL): [0] cycles the first waiter spent, [1] cycles a
  * second waiter spent after the flag was set (it returns at once).  Nothing faults or hangs. */
 int bf_selftest_timeout(int device, int code, int* status, long long* waited_cycles);
+
+/* Scale self test; no counterpart in the reference.  The evaluator's row scales and reciprocals are
+ * corrected approximations instead of divisions; this compares them with IEEE division over every
+ * value they can be given and counts the differences: `differ[0..2]` over all positive fp16 row maxima
+ * for the s8, u8 and e4m3 ranges, `differ[3]` over every fp32 softmax sum from 1 to 32. */
+int bf_selftest_scales(int device, unsigned long long* differ);
 
 /* Tensor-core self test (no network): one 128-row tile times a packed weight tile.
  *   mode 0: s8 x s8, N=128, K=256     mode 1: u8 x s8, N=128, K=256

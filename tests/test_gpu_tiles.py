@@ -1,0 +1,50 @@
+"""The evaluator on one- and two-board tiles: at every size where the tiling changes, a position's
+outputs are those it gets in any other batch, in every arithmetic; and the arithmetic helpers the tiles
+use instead of divisions equal division on everything they can be given."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+ARITHMETICS = {"int8": dict(int8=True), "f16": {}, "e4m3": dict(fp8=True), "ffn": dict(int8=True, int8_scheme="ffn"),
+               "ffn+qkv": dict(int8=True, int8_scheme="ffn+qkv")}
+
+
+def cu(a):
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+@pytest.mark.parametrize("arithmetic", ARITHMETICS)
+def test_every_tiling_gives_a_position_the_same_outputs(arithmetic, nets, pos4096):
+    from brokefish_b200.nn.cuda_impl import FusedEncoder
+    enc = FusedEncoder(nets["B"], **ARITHMETICS[arithmetic])
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    b, c, r = (cu(pos4096[k]) for k in ("boards", "control", "rep"))
+    legal = cu(pos4096["legal"].view(np.int64))
+    want = [t.clone() for t in enc.forward_full(b, c, r, legal)]
+    priors = [t.clone() for t in enc.forward_priors(b, c, r, legal, 96)]
+    for n in (1, 2, sms - 1, sms, sms + 1, 2 * sms - 1, 2 * sms, 2 * sms + 1, 3 * sms, 3 * sms + 1, 4 * sms, 4 * sms + 1,
+              6 * sms + 1):
+        lo = 4096 - n
+        part = [t[lo:] for t in (b, c, r, legal)]
+        for got, w in zip(enc.forward_full(*part), want):
+            assert torch.equal(got, w[lo:]), n
+        for got, w in zip(enc.forward_priors(*part, 96), priors):
+            assert torch.equal(got, w[lo:]), n
+    # one-board tiles off, and up to two rounds of them
+    for one in (0, 2):
+        enc.set_one_board(one)
+        for n in (1, sms + 1, 2 * sms - 1, 2 * sms + 5):
+            for got, w in zip(enc.forward_full(*(t[:n] for t in (b, c, r, legal))), want):
+                assert torch.equal(got, w[:n]), (one, n)
+    enc.check_status()
+
+
+def test_scales_and_reciprocals_equal_division():
+    from brokefish_b200 import _native
+    differ = (ctypes.c_ulonglong * 4)()
+    _native.check(_native.lib().bf_selftest_scales(0, differ), "bf_selftest_scales")
+    assert list(differ) == [0, 0, 0, 0]
