@@ -1439,8 +1439,10 @@ __device__ __forceinline__ void producer_loop(uint32_t smem, volatile int* abort
                 for (int st = 0; st < 4 * C::kQkvSlabs; ++st, ++qi) {
                     const uint32_t s = qi % kQS;
                     mbar_wait(bar_addr(smem, B_WQ_EMPTY + s), (qi / kQS - 1u) & 1u, abort_flag, kErrProducer);
-                    mbar_arrive_expect_tx(bar_addr(smem, B_WQ_FULL + s), kQStage);
-                    bulk_g2s(smem + C::SM_RING + s * kQStage, src, kQStage, bar_addr(smem, B_WQ_FULL + s));
+                    if (elect_one()) {
+                        mbar_arrive_expect_tx(bar_addr(smem, B_WQ_FULL + s), kQStage);
+                        bulk_g2s(smem + C::SM_RING + s * kQStage, src, kQStage, bar_addr(smem, B_WQ_FULL + s));
+                    }
                     src += kQStage;
                 }
                 for (uint32_t s = 0; s < kQS; ++s)
@@ -1452,8 +1454,10 @@ __device__ __forceinline__ void producer_loop(uint32_t smem, volatile int* abort
             for (int st = 0; st < n_st; ++st, ++ri) {
                 const uint32_t s = ri % kRS;
                 mbar_wait(bar_addr(smem, B_WR_EMPTY + s), (ri / kRS - 1u) & 1u, abort_flag, kErrProducer);
-                mbar_arrive_expect_tx(bar_addr(smem, B_WR_FULL + s), bytes);
-                bulk_g2s(smem + C::SM_RING + s * kRStage, src, bytes, bar_addr(smem, B_WR_FULL + s));
+                if (elect_one()) {
+                    mbar_arrive_expect_tx(bar_addr(smem, B_WR_FULL + s), bytes);
+                    bulk_g2s(smem + C::SM_RING + s * kRStage, src, bytes, bar_addr(smem, B_WR_FULL + s));
+                }
                 src += bytes;
             }
         }
@@ -1461,8 +1465,10 @@ __device__ __forceinline__ void producer_loop(uint32_t smem, volatile int* abort
         for (uint32_t st = 0; st < kHeadStages; ++st, ++ri) {
             const uint32_t s = ri % kRS;
             mbar_wait(bar_addr(smem, B_WR_EMPTY + s), (ri / kRS - 1u) & 1u, abort_flag, kErrProducer);
-            mbar_arrive_expect_tx(bar_addr(smem, B_WR_FULL + s), kHeadStage);
-            bulk_g2s(smem + C::SM_RING + s * kRStage, src, kHeadStage, bar_addr(smem, B_WR_FULL + s));
+            if (elect_one()) {
+                mbar_arrive_expect_tx(bar_addr(smem, B_WR_FULL + s), kHeadStage);
+                bulk_g2s(smem + C::SM_RING + s * kRStage, src, kHeadStage, bar_addr(smem, B_WR_FULL + s));
+            }
             src += kHeadStage;
         }
     }
@@ -1476,7 +1482,7 @@ __device__ __forceinline__ void producer_loop(uint32_t smem, volatile int* abort
 }
 
 // ------------------------------------------------------------------------------------------
-// MMA issuer: one thread walks the static GEMM schedule.
+// MMA issuer: one warp walks the static GEMM schedule and waits, one elected lane of it issues.
 // ------------------------------------------------------------------------------------------
 struct MmaState {
     uint32_t qc, rc;          // weight stages consumed from each ring
@@ -1512,17 +1518,19 @@ __device__ __forceinline__ void mma_unit(uint32_t smem, volatile int* abort_flag
             st.rc++;
         }
         if (!seen) tc_fence_after();
-        const uint64_t ad = umma_desc_k128(a_base + s * 16384), bd = umma_desc_k128(w_addr);
+        if (elect_one()) {
+            const uint64_t ad = umma_desc_k128(a_base + s * 16384), bd = umma_desc_k128(w_addr);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const uint32_t accumulate = (s > 0 || k > 0) ? 1u : 0u;
-            if (kind == kKindF16)     umma_f16(tmem_d, ad + 2 * k, bd + 2 * k, idesc, accumulate);
-            else if (kind == kKindF8) umma_f8(tmem_d, ad + 2 * k, bd + 2 * k, idesc, accumulate);
-            else                      umma_i8(tmem_d, ad + 2 * k, bd + 2 * k, idesc, accumulate);
+            for (int k = 0; k < 4; ++k) {
+                const uint32_t accumulate = (s > 0 || k > 0) ? 1u : 0u;
+                if (kind == kKindF16)     umma_f16(tmem_d, ad + 2 * k, bd + 2 * k, idesc, accumulate);
+                else if (kind == kKindF8) umma_f8(tmem_d, ad + 2 * k, bd + 2 * k, idesc, accumulate);
+                else                      umma_i8(tmem_d, ad + 2 * k, bd + 2 * k, idesc, accumulate);
+            }
+            tc_commit(w_empty);
+            if (s == n_stages - 1) tc_commit(bar_addr(smem, B_ACC_FULL + slot));
         }
-        tc_commit(w_empty);
     }
-    tc_commit(bar_addr(smem, B_ACC_FULL + slot));
     st.accn[slot]++;
 }
 
@@ -1563,12 +1571,12 @@ __device__ __forceinline__ void mma_pass_over(uint32_t smem, volatile int* abort
     for (int i = 0; i < n_stages; ++i) {
         const uint32_t k = st.rc % C::kRSlots;
         mbar_wait(bar_addr(smem, B_WR_FULL + k), (st.rc / C::kRSlots) & 1u, abort_flag, kErrMmaWeights);
-        mbar_arrive(bar_addr(smem, B_WR_EMPTY + k));
+        if (elect_one()) mbar_arrive(bar_addr(smem, B_WR_EMPTY + k));
         st.rc++;
     }
 }
 
-// Two threads (lane 0 of two warps) share the schedule: issuing one unit costs a thread well
+// Two warps share the schedule: issuing one unit costs a thread well
 // over twice the unit's time on the tensor pipe (barrier waits, descriptors, a full MMA queue),
 // and the units of a step come in pairs -- the two 128-wide halves of an out-projection, of a
 // hidden chunk, of an ff2 chunk -- that are independent of one another.  Issuer `who` takes the
@@ -1665,15 +1673,17 @@ __device__ __forceinline__ void mma_loop(uint32_t smem, uint32_t tmem, volatile 
                             mbar_wait(bar_addr(smem, B_WR_FULL + k), (st.rc / C::kRSlots) & 1u, abort_flag, kErrMmaWeights);
                             st.rc++;
                             tc_fence_after();
-                            const uint64_t ad = umma_desc_k128(sm_r + sl * 16384);
-                            const uint64_t bd = umma_desc_k128(smem + C::SM_RING + k * kRStage);
+                            if (elect_one()) {
+                                const uint64_t ad = umma_desc_k128(sm_r + sl * 16384);
+                                const uint64_t bd = umma_desc_k128(smem + C::SM_RING + k * kRStage);
 #pragma unroll
-                            for (int kk = 0; kk < 4; ++kk)
-                                umma_f16(dst, ad + 2 * kk, bd + 2 * kk, kI_FF2, (ch > 0 || sl > 0 || kk > 0) ? 1u : 0u);
-                            tc_commit(bar_addr(smem, B_WR_EMPTY + k));
+                                for (int kk = 0; kk < 4; ++kk)
+                                    umma_f16(dst, ad + 2 * kk, bd + 2 * kk, kI_FF2, (ch > 0 || sl > 0 || kk > 0) ? 1u : 0u);
+                                tc_commit(bar_addr(smem, B_WR_EMPTY + k));
+                                if (jh == 1 && sl == 3) tc_commit(bar_addr(smem, B_ACC_FULL + 1));
+                            }
                         }
                     }
-                    tc_commit(bar_addr(smem, B_ACC_FULL + 1));
                     if (ch < 3) pass_over(4);
                 }
                 st.accn[1]++;
@@ -1763,9 +1773,9 @@ __global__ void __launch_bounds__(kThreads, 1) encoder_kernel(const Params p) {
         c.t_last = c.prof_on ? clock64() : 0;
         for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) row_warps_tile<kDbg, kRJ, kAr>(c, p, tile);
     } else if (warp == kProducerWarp) {
-        if (elect_one()) producer_loop<kAr>(smem, abort_flag, p, blockIdx.x, gridDim.x, n_tiles);
+        producer_loop<kAr>(smem, abort_flag, p, blockIdx.x, gridDim.x, n_tiles);
     } else {
-        if (elect_one()) mma_loop<kAr>(smem, tmem, abort_flag, p, blockIdx.x, gridDim.x, n_tiles, warp - kMmaWarp);
+        mma_loop<kAr>(smem, tmem, abort_flag, p, blockIdx.x, gridDim.x, n_tiles, warp - kMmaWarp);
     }
     __syncwarp();
     tc_fence_before();

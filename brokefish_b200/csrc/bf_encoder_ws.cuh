@@ -847,36 +847,39 @@ __device__ __forceinline__ void row_tile(Row& c, const Params& p, int first) {
 // ---- weight stream ----
 // The blob's stages are the four-board kernel's: per head pair [Q 64 | K 64 | V 64 rows], then 128-row
 // units, two to each 256-row product.  A stage here is 256 rows of one K-slab, put together from four
-// or two of their pieces.
+// or two of their pieces.  The whole warp walks the stages and waits; one elected lane issues.
 template <int kAr>
 __device__ __forceinline__ void producer(uint32_t smem, volatile int* abort_flag, const Params& p, int n_tiles) {
     using C = Cfg<kAr>;
     constexpr uint32_t kStages = Map<kAr>::kStages, kRing = Map<kAr>::SM_RING;
     uint32_t i = 0;
-    auto begin = [&](uint32_t bytes) -> uint32_t {
+    // the next stage: `copies(dst, barrier)` of `bytes` in all
+    auto stage = [&](uint32_t bytes, auto&& copies) {
         const uint32_t k = i % kStages;
         mbar_wait(bar(smem, B_EMPTY + k), (i / kStages - 1u) & 1u, abort_flag, kErrProducer);
-        mbar_arrive_expect_tx(bar(smem, B_FULL + k), bytes);
+        if (elect_one()) {
+            mbar_arrive_expect_tx(bar(smem, B_FULL + k), bytes);
+            copies(smem + kRing + k * kStage, bar(smem, B_FULL + k));
+        }
         ++i;
-        return k;
     };
     // K-slab s of the product whose two 128-row units start at `u0` and `u1`
     auto two_units = [&](const uint8_t* u0, const uint8_t* u1, int s) {
-        const uint32_t k = begin(kStage), dst = smem + kRing + k * kStage;
-        bulk_g2s(dst, u0 + s * kRStage, kRStage, bar(smem, B_FULL + k));
-        bulk_g2s(dst + kRStage, u1 + s * kRStage, kRStage, bar(smem, B_FULL + k));
+        stage(kStage, [&](uint32_t dst, uint32_t full) {
+            bulk_g2s(dst, u0 + s * kRStage, kRStage, full);
+            bulk_g2s(dst + kRStage, u1 + s * kRStage, kRStage, full);
+        });
     };
     for (int tile = 0; tile < n_tiles; ++tile) {
         const uint8_t* src = p.wstream;
         for (int layer = 0; layer < p.n_layers; ++layer, src += C::kLayerStream) {
             for (int m = 0; m < 3; ++m)                                     // Q, K, V
-                for (int s = 0; s < C::kQkvSlabs; ++s) {
-                    const uint32_t k = begin(kStage), dst = smem + kRing + k * kStage;
-                    const uint8_t* from = src + s * kQStage + m * 8192;
+                for (int s = 0; s < C::kQkvSlabs; ++s)
+                    stage(kStage, [&](uint32_t dst, uint32_t full) {
+                        const uint8_t* from = src + s * kQStage + m * 8192;
 #pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        bulk_g2s(dst + 8192 * j, from + C::kQkvSlabs * j * kQStage, 8192, bar(smem, B_FULL + k));
-                }
+                        for (int j = 0; j < 4; ++j) bulk_g2s(dst + 8192 * j, from + C::kQkvSlabs * j * kQStage, 8192, full);
+                    });
             const uint8_t* out = src + 4 * C::kQkvSlabs * kQStage;
             for (int s = 0; s < C::kOutSlabs; ++s) two_units(out, out + C::kOutSlabs * kRStage, s);
             // ff1 chunks 0-3, then ff2 chunks 0-3; where their two units lie in the packed order
@@ -895,10 +898,8 @@ __device__ __forceinline__ void producer(uint32_t smem, volatile int* abort_flag
                     two_units(ffn + u0 * C::kFfnSlabs * kRStage, ffn + u1 * C::kFfnSlabs * kRStage, s);
             }
         }
-        for (uint32_t st = 0; st < kHeadStages; ++st, src += kHeadStage) {
-            const uint32_t k = begin(kHeadStage);
-            bulk_g2s(smem + kRing + k * kStage, src, kHeadStage, bar(smem, B_FULL + k));
-        }
+        for (uint32_t st = 0; st < kHeadStages; ++st, src += kHeadStage)
+            stage(kHeadStage, [&](uint32_t dst, uint32_t full) { bulk_g2s(dst, src, kHeadStage, full); });
     }
     // after a time-out copies may still be in flight: a bounded while for them to land
     if (*abort_flag != 0) {
@@ -913,28 +914,33 @@ struct Issue {
     volatile int* abort_flag;
     uint32_t i, a, h;           // weight stages, A operands, hidden pairs consumed
 };
-// One product: `slabs` K-slabs of 128 bytes; `more`: on top of what the slot holds.
+// One product: `slabs` K-slabs of 128 bytes; `more`: on top of what the slot holds; `done`: the slot's
+// barrier that its completion goes to (-1: none).  The whole warp walks the schedule and waits; one
+// elected lane -- the same every time -- issues.  (A loop inside the elected branch keeps its addresses
+// in the warp's uniform registers while the other lanes run on to the branch's end, at any time.)
 template <int kAr, int kKind>
 __device__ __forceinline__ void issue_unit(Issue& st, uint32_t d, uint32_t a_base, uint32_t slab, int slabs, uint32_t idesc,
-                                           bool more = false) {
+                                           int done, bool more = false) {
     constexpr uint32_t kStages = Map<kAr>::kStages;
     for (int s = 0; s < slabs; ++s) {
         const uint32_t k = st.i % kStages;
         mbar_wait(bar(st.smem, B_FULL + k), (st.i / kStages) & 1u, st.abort_flag, kErrMmaWeights);
         tc_fence_after();
-        const uint64_t ad = umma_desc_k128(a_base + s * slab), bd = umma_desc_k128(st.smem + Map<kAr>::SM_RING + k * kStage);
+        if (elect_one()) {
+            const uint64_t ad = umma_desc_k128(a_base + s * slab), bd = umma_desc_k128(st.smem + Map<kAr>::SM_RING + k * kStage);
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-            const uint32_t accumulate = (more || (s | kk) != 0) ? 1u : 0u;
-            if (kKind == kKindF16)     umma_ws_f16(d, ad + 2 * kk, bd + 2 * kk, idesc, accumulate);
-            else if (kKind == kKindF8) umma_ws_f8(d, ad + 2 * kk, bd + 2 * kk, idesc, accumulate);
-            else                       umma_ws_i8(d, ad + 2 * kk, bd + 2 * kk, idesc, accumulate);
+            for (int kk = 0; kk < 4; ++kk) {
+                const uint32_t accumulate = (more || (s | kk) != 0) ? 1u : 0u;
+                if (kKind == kKindF16)     umma_ws_f16(d, ad + 2 * kk, bd + 2 * kk, idesc, accumulate);
+                else if (kKind == kKindF8) umma_ws_f8(d, ad + 2 * kk, bd + 2 * kk, idesc, accumulate);
+                else                       umma_ws_i8(d, ad + 2 * kk, bd + 2 * kk, idesc, accumulate);
+            }
+            tc_commit(bar(st.smem, B_EMPTY + k));
+            if (s == slabs - 1 && done >= 0) tc_commit(bar(st.smem, B_ACC + done));
         }
-        tc_commit(bar(st.smem, B_EMPTY + k));
         st.i++;
     }
 }
-__device__ __forceinline__ void issue_done(const Issue& st, int slot) { tc_commit(bar(st.smem, B_ACC + slot)); }
 __device__ __forceinline__ void issue_wait(const Issue& st, int b, uint32_t n) {
     mbar_wait(bar(st.smem, b), n & 1u, st.abort_flag, kErrMmaOperand);
     tc_fence_after();
@@ -956,35 +962,27 @@ __device__ __forceinline__ void issue_tile(Issue& st, int n_layers) {
     const uint32_t a = st.smem + SM_A, h = st.smem + Map<kAr>::SM_H;
     for (int layer = 0; layer < n_layers; ++layer) {
         issue_wait(st, B_A, st.a++);
-        for (int m = 0; m < 3; ++m) {
-            issue_unit<kAr, kQkvKind>(st, st.tmem + O::kSlot * m, a, O::kSlab, C::kQkvSlabs, kI_QKV);
-            issue_done(st, m);
-        }
+        for (int m = 0; m < 3; ++m)
+            issue_unit<kAr, kQkvKind>(st, st.tmem + O::kSlot * m, a, O::kSlab, C::kQkvSlabs, kI_QKV, m);
         issue_wait(st, B_A, st.a++);
-        issue_unit<kAr, kOutKind>(st, st.tmem + O::kSlot * 3, a, O::kSlab, C::kOutSlabs, kI_OUT);
-        issue_done(st, 3);
+        issue_unit<kAr, kOutKind>(st, st.tmem + O::kSlot * 3, a, O::kSlab, C::kOutSlabs, kI_OUT, 3);
         issue_wait(st, B_A, st.a++);
-        for (int ch = 0; ch < 4; ++ch) {
-            issue_unit<kAr, kFfnKind>(st, st.tmem + O::kSlot * ch, a, O::kSlab, C::kFfnSlabs, kI_FF1);
-            issue_done(st, ch);
-        }
+        for (int ch = 0; ch < 4; ++ch)
+            issue_unit<kAr, kFfnKind>(st, st.tmem + O::kSlot * ch, a, O::kSlab, C::kFfnSlabs, kI_FF1, ch);
         for (int ch = 0; ch < 4; ++ch) {
             if ((ch & 1) == 0) issue_wait(st, B_H + (ch >> 1), st.h);
             if (kAr == kArF16) {
-                issue_unit<kAr, kFfnKind>(st, st.tmem, h + (ch & 1) * 4 * O::kSlab, O::kSlab, C::kFfnSlabs, kI_FF2, ch > 0);
-                if (ch == 1) issue_done(st, 0);
+                issue_unit<kAr, kFfnKind>(st, st.tmem, h + (ch & 1) * 4 * O::kSlab, O::kSlab, C::kFfnSlabs, kI_FF2, ch == 1 ? 0 : -1, ch > 0);
             } else {
-                issue_unit<kAr, kFfnKind>(st, st.tmem + O::kSlot * ch, h + ch * 2 * O::kSlab, O::kSlab, C::kFfnSlabs, kI_FF2);
-                issue_done(st, ch);
+                issue_unit<kAr, kFfnKind>(st, st.tmem + O::kSlot * ch, h + ch * 2 * O::kSlab, O::kSlab, C::kFfnSlabs, kI_FF2, ch);
             }
         }
-        if (kAr == kArF16)
-            for (int slot = 1; slot < 4; ++slot) issue_done(st, slot);
+        if (kAr == kArF16 && elect_one())
+            for (int slot = 1; slot < 4; ++slot) tc_commit(bar(st.smem, B_ACC + slot));
         st.h++;
     }
     issue_wait(st, B_A, st.a++);
-    issue_unit<kAr, kKindF16>(st, st.tmem, h + kHeadA, O::kSlab, kHeadStages, kI_HEAD);
-    issue_done(st, 0);
+    issue_unit<kAr, kKindF16>(st, st.tmem, h + kHeadA, O::kSlab, kHeadStages, kI_HEAD, 0);
 }
 
 // launch bounds: 640 threads, so that a scheduler's five warps fit its registers (96 each)
@@ -1029,16 +1027,14 @@ __global__ void __launch_bounds__(640, 1) encoder_ws_kernel(const Params p) {
             else             row_tile<2, kAr>(c, p, first);
         }
     } else if (warp == kProducerWarp) {
-        if (elect_one()) producer<kAr>(smem, abort_flag, p, n_tiles);
+        producer<kAr>(smem, abort_flag, p, n_tiles);
     } else {
-        if (elect_one()) {
-            Issue st = {smem, tmem, abort_flag, 0, 0, 0};
-            for (int k = 0; k < n_tiles; ++k) {
-                int first, boards;
-                tiles.at(k, first, boards);
-                if (boards == 1) issue_tile<1, kAr>(st, p.n_layers);
-                else             issue_tile<2, kAr>(st, p.n_layers);
-            }
+        Issue st = {smem, tmem, abort_flag, 0, 0, 0};
+        for (int k = 0; k < n_tiles; ++k) {
+            int first, boards;
+            tiles.at(k, first, boards);
+            if (boards == 1) issue_tile<1, kAr>(st, p.n_layers);
+            else             issue_tile<2, kAr>(st, p.n_layers);
         }
     }
     __syncwarp();

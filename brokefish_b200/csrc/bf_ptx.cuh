@@ -12,10 +12,12 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-// One lane of the warp (all 32 converged), chosen by `elect.sync`.  A region entered through this
-// predicate is one the compiler knows to be executed by a single thread: the descriptors of the
-// tensor-core and bulk-copy instructions in it are built in uniform registers.  Under `lane == 0` it
-// cannot know that and wraps every such instruction in a loop over the active lanes.
+// One lane of the warp (all 32 take part), chosen by `elect.sync`, the same one every time.  A region
+// entered through this predicate is one the compiler knows to be executed by a single thread: the
+// descriptors of the tensor-core and bulk-copy instructions in it are built in uniform registers.
+// Under `lane == 0` it cannot know that and wraps every such instruction in a loop over the active
+// lanes.  Keep such a region free of waits: the uniform registers belong to the whole warp, whose other
+// lanes run on to the end of the branch meanwhile.
 __device__ __forceinline__ bool elect_one() {
     uint32_t pred;
     asm volatile(
@@ -58,9 +60,6 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity)
 // out of time it is set, and every later wait returns at once, so a lost arrival ends
 // the kernel with an error status instead of a hang.  Returns false on time-out.
 //
-// All of it inline: the single-thread regions of the weight stream and the MMA issuers keep addresses
-// and descriptors in uniform registers, and a function call in the middle of such a region is not
-// something to build on.
 constexpr unsigned kWaitCycles = 400000000u;     // ~0.2 s at 2 GHz
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity,
                                           volatile int* abort_flag, int code) {
