@@ -50,11 +50,13 @@ constexpr uint32_t kHeadA = 32768;                 // the head operand's place i
 constexpr uint32_t SM_STAT = 16384 + 65536 + 4 * kStage;
 constexpr uint32_t SM_MAX = SM_STAT + 1024;        // row maxima: attention output, four hidden chunks
 constexpr uint32_t SM_LIST = SM_MAX + 5 * 256;     // fused expansion: 1 KB per board
-constexpr uint32_t SM_BAR = SM_LIST + 2048;
-constexpr uint32_t SM_MISC = SM_BAR + 128;
+constexpr uint32_t SM_PAR = SM_LIST + 2048;        // scales and biases of two layers
+constexpr uint32_t SM_BAR = SM_PAR + 2 * kLparamStride;
+constexpr uint32_t SM_MISC = SM_BAR + 192;
 constexpr uint32_t SM_BYTES = SM_MISC + 64, kSmemRequest = SM_BYTES + 1024;
+static_assert(kSmemRequest <= 232448 && kLparamStride % 16 == 0 && SM_PAR % 16 == 0, "shared memory map");
 static_assert(Map<kArF16>::SM_RING + 3 * kStage <= SM_STAT && Map<kArInt8>::SM_RING + 4 * kStage <= SM_STAT, "shared memory map");
-enum { B_FULL = 0, B_EMPTY = 4, B_ACC = 8, B_A = 12, B_H = 13, B_COUNT = 15 };
+enum { B_FULL = 0, B_EMPTY = 4, B_ACC = 8, B_PAR = 12, B_A = 14, B_H = 15, B_COUNT = 17 };
 __device__ __forceinline__ uint32_t bar(uint32_t smem, int i) { return smem + SM_BAR + 8u * i; }
 
 // Which boards a CTA evaluates, tile by tile.  At most `one_most` boards per CTA: one-board tiles alone.
@@ -125,13 +127,23 @@ __device__ __forceinline__ void wait_acc(const Row& c, int slot, int use) {
     __syncwarp();                                            // what follows is for a converged warp
     tc_fence_after();
 }
+// The scales and biases of the layer this thread is at (two copies, filled by the weight stream a layer
+// ahead): shared address of the layer's block.  From L1 they came late: beside 228 KB of shared memory
+// the eight layers' 37 KB do not stay there, and the loads could not be issued ahead of the wait for
+// the product they go with (3 to 6 % of a tile).
+__device__ __forceinline__ uint32_t layer_params(const Row& c) {
+    return c.smem + SM_PAR + (c.layers & 1u) * kLparamStride;
+}
+__device__ __forceinline__ void wait_params(const Row& c) {
+    mbar_wait(bar(c.smem, B_PAR + (c.layers & 1u)), (c.layers >> 1) & 1u, c.abort_flag, kErrRowAcc);
+    __syncwarp();
+}
 // This warp's operand rows are written and what it read of tensor memory has arrived: publish.
 __device__ __forceinline__ void publish(const Row& c, int b) {
     tc_fence_before();
     fence_proxy_async_smem();
     __syncwarp();
     if (c.lane == 0) mbar_arrive(bar(c.smem, b));
-    __syncwarp();
 }
 __device__ __forceinline__ float lds_f(uint32_t addr) {
     float v;
@@ -172,6 +184,27 @@ __device__ __forceinline__ Scale row_scale(float amax, float q_max, float q_inv)
 __device__ __forceinline__ Scale scale_s8(float amax) { return row_scale(amax, kQMaxS8, 1.0f / kQMaxS8); }
 __device__ __forceinline__ Scale scale_u8(float amax) { return row_scale(amax, kQMaxU8, 1.0f / kQMaxU8); }
 __device__ __forceinline__ Scale scale_e4m3(float amax) { return row_scale(amax, kQMaxE4M3, 1.0f / kQMaxE4M3); }
+// Sixteen columns' biases (a broadcast: a warp's threads share their columns).
+struct Bias { uint4 lo, hi; };
+__device__ __forceinline__ Bias load_bias(uint32_t addr) { return {lds128(addr), lds128(addr + 16)}; }
+// `(float(acc) * sa) * sw` -> fp16, + fp16 bias, optional ReLU, for sixteen columns: `descale`'s arithmetic.
+template <bool kRelu, int kAcc>
+__device__ __forceinline__ void descale16(const uint32_t (&acc)[16], float sa, float sw, const Bias& bias, uint32_t* out) {
+    const uint32_t bw[8] = {bias.lo.x, bias.lo.y, bias.lo.z, bias.lo.w, bias.hi.x, bias.hi.y, bias.hi.z, bias.hi.w};
+    const uint64_t sw2 = pk2(sw, sw);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        uint32_t h;
+        if (kAcc == kAccPlain) {
+            h = __byte_perm(acc[2 * i], acc[2 * i + 1], 0x5410);
+        } else {
+            const float a0 = kAcc == kAccInt ? static_cast<float>(static_cast<int>(acc[2 * i])) : __uint_as_float(acc[2 * i]);
+            const float a1 = kAcc == kAccInt ? static_cast<float>(static_cast<int>(acc[2 * i + 1])) : __uint_as_float(acc[2 * i + 1]);
+            h = f2_to_h2(mul2(pk2(__fmul_rn(a0, sa), __fmul_rn(a1, sa)), sw2));
+        }
+        out[i] = kRelu ? hfma2_relu(h, 0x3C003C00u, bw[i]) : as_u32(__hadd2(as_h2(h), as_h2(bw[i])));
+    }
+}
 // This thread's columns of a slot, 16 at a time: `use(piece, words)`.  No load is left in flight while
 // another piece is worked on: the registers that one lands in are then free of pressure from the code
 // around them, and the scheduler's other warps cover its latency.
@@ -344,9 +377,6 @@ __device__ __forceinline__ void scores(const uint32_t (&qa)[2][4], uint32_t ks, 
         mma_f16_f16(s[nt], qa[1], kb[2], kb[3]);
     }
 }
-// e^x as 2^(x log2 e) on the hardware's 2^x.  `__expf` is the same but for results below 2^-126, which it
-// keeps as denormals: beside a row sum of at least 1 they change neither the sum nor a probability.
-__device__ __forceinline__ float exp_fast(float x) { return ex2_approx(__fmul_rn(x, 1.44269504088896340736f)); }
 __device__ __forceinline__ void softmax(uint32_t (&s)[4][2], const uint32_t (&dead)[4]) {
 #pragma unroll
     for (int hi = 0; hi < 2; ++hi) {
@@ -364,8 +394,8 @@ __device__ __forceinline__ void softmax(uint32_t (&s)[4][2], const uint32_t (&de
         float sum = 0.f;
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) {
-            pv[nt][0] = exp_fast(pv[nt][0] - mx);     // an all-dead row keeps the reference's NaN
-            pv[nt][1] = exp_fast(pv[nt][1] - mx);
+            pv[nt][0] = __expf(pv[nt][0] - mx);     // an all-dead row keeps the reference's NaN
+            pv[nt][1] = __expf(pv[nt][1] - mx);
             sum += pv[nt][0] + pv[nt][1];
         }
         sum += __shfl_xor_sync(0xffffffffu, sum, 1);
@@ -406,15 +436,17 @@ __device__ __forceinline__ void store_outputs(const uint32_t (&o)[4][2], uint32_
 
 // This thread's columns of product `m` (0 Q, 1 K, 2 V) as fp16 into its head's block.
 template <int NB, int kAr>
-__device__ __forceinline__ void stage_qkv(const Row& c, const LayerParams& lp, float sa, int m, uint32_t block) {
+__device__ __forceinline__ void stage_qkv(const Row& c, uint32_t lp, float sa, int m, uint32_t block) {
     using O = Own<NB>;
     const int col = O::col(c);
+    const uint32_t bias_at = lp + LP_B_QKV + 2u * ((col >> 6) * 192 + m * 64 + (col & 63));
+    const float sw = lds_f(lp + LP_SW_QKV + 4u * (m * 2 + (col >> 7)));
+    Bias bias = load_bias(bias_at);
     wait_acc(c, m, 0);
-    const float sw = __ldg(lp.sw_qkv + m * 2 + (col >> 7));
-    const __half* bias = lp.b_qkv + (col >> 6) * 192 + m * 64 + (col & 63);
     each_piece<NB>(O::slot(c, m), [&](int k, const uint32_t (&acc)[16]) {
         uint32_t h[8];
-        descale<16, false, Cfg<kAr>::kQkvF16 ? kAccPlain : kAccInt>(acc, sa, sw, bias + 16 * k, h);
+        if (k > 0) bias = load_bias(bias_at + 32 * k);
+        descale16<false, Cfg<kAr>::kQkvF16 ? kAccPlain : kAccInt>(acc, sa, sw, bias, h);
         if (k == 0) __syncwarp();
         const int group = ((col & 31) >> 3) + 2 * k;
         sts128(block + head_off(c.lane, group), make_uint4(h[0], h[1], h[2], h[3]));
@@ -423,7 +455,7 @@ __device__ __forceinline__ void stage_qkv(const Row& c, const LayerParams& lp, f
 }
 
 template <int NB, int kAr>
-__device__ __forceinline__ void attention_block(const Row& c, const LayerParams& lp, float sa, uint32_t alive, uint32_t (&x)[8 * NB]) {
+__device__ __forceinline__ void attention_block(const Row& c, uint32_t lp, float sa, uint32_t alive, uint32_t (&x)[8 * NB]) {
     using O = Own<NB>;
     const int lane = c.lane, col = O::col(c);
     uint32_t dead[4];
@@ -491,11 +523,13 @@ __device__ __forceinline__ void attention_block(const Row& c, const LayerParams&
     }
     publish(c, B_A);
     // x = fp16(x + fp16(fp16(descale) + b_o))
+    const float sw = lds_f(lp + LP_SW_O + 4u * (col >> 7));
+    Bias bias = load_bias(lp + LP_B_O + 2u * col);
     wait_acc(c, 3, 0);
-    const float sw = __ldg(lp.sw_o + (col >> 7));
     each_piece<NB>(O::slot(c, 3), [&](int k, const uint32_t (&acc)[16]) {
         uint32_t y[8];
-        descale<16, false, Cfg<kAr>::kOutF16 ? kAccPlain : kAccInt>(acc, so.scale, sw, lp.b_o + col + 16 * k, y);
+        if (k > 0) bias = load_bias(lp + LP_B_O + 2u * col + 32 * k);
+        descale16<false, Cfg<kAr>::kOutF16 ? kAccPlain : kAccInt>(acc, so.scale, sw, bias, y);
 #pragma unroll
         for (int i = 0; i < 8; ++i) x[8 * k + i] = as_u32(__hadd2(as_h2(x[8 * k + i]), as_h2(y[i])));
     });
@@ -506,7 +540,7 @@ __device__ __forceinline__ void attention_block(const Row& c, const LayerParams&
 // board for both maxima, quantisation into the ff2 operand.  ff2's products of the first pair run
 // under the second pair's epilogue; their four sums are added to the fp16 running total in order.
 template <int NB, int kAr>
-__device__ __forceinline__ void ffn_block(const Row& c, const LayerParams& lp, float sa, uint32_t (&x)[8 * NB]) {
+__device__ __forceinline__ void ffn_block(const Row& c, uint32_t lp, float sa, uint32_t (&x)[8 * NB]) {
     using O = Own<NB>;
     const int col = O::col(c), row = O::row(c);
     float s1[4] = {1.f, 1.f, 1.f, 1.f};
@@ -517,10 +551,13 @@ __device__ __forceinline__ void ffn_block(const Row& c, const LayerParams& lp, f
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
             const int ch = 2 * pair + k;
+            const uint32_t bias_at = lp + LP_B_FF1 + 2u * (256 * ch + col);
+            const float sw = lds_f(lp + LP_SW_FF1 + 4u * (2 * ch + (col >> 7)));
+            Bias bias = load_bias(bias_at);
             wait_acc(c, ch, 1);
-            const float sw = __ldg(lp.sw_ff1 + 2 * ch + (col >> 7));
             each_piece<NB>(O::slot(c, ch), [&](int i, const uint32_t (&acc)[16]) {
-                descale<16, true, kAr == kArE4M3 ? kAccFloat : kAccInt>(acc, sa, sw, lp.b_ff1 + 256 * ch + col + 16 * i, &hid[k][8 * i]);
+                if (i > 0) bias = load_bias(bias_at + 32 * i);
+                descale16<true, kAr == kArE4M3 ? kAccFloat : kAccInt>(acc, sa, sw, bias, &hid[k][8 * i]);
             });
             max_to(m + 256u * k, amax_h2<8 * NB>(hid[k], false));
         }
@@ -540,7 +577,7 @@ __device__ __forceinline__ void ffn_block(const Row& c, const LayerParams& lp, f
     uint32_t run[8 * NB];
 #pragma unroll
     for (int i = 0; i < 8 * NB; ++i) run[i] = 0u;
-    const float s2 = __ldg(lp.sw_ff2 + (col >> 7));
+    const float s2 = lds_f(lp + LP_SW_FF2 + 4u * (col >> 7));
     const uint64_t s2_2 = pk2(s2, s2);
 #pragma unroll 1
     for (int ch = 0; ch < 4; ++ch) {
@@ -560,10 +597,9 @@ __device__ __forceinline__ void ffn_block(const Row& c, const LayerParams& lp, f
         });
     }
     // + b_ff2, residual: x = fp16(x + fp16(run + b))
-    const uint4* b4 = reinterpret_cast<const uint4*>(lp.b_ff2 + col);
 #pragma unroll
     for (int v = 0; v < 2 * NB; ++v) {
-        const uint4 bv = __ldg(b4 + v);
+        const uint4 bv = lds128(lp + LP_B_FF2 + 2u * col + 16u * v);
         const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -578,7 +614,7 @@ __device__ __forceinline__ void ffn_block(const Row& c, const LayerParams& lp, f
 // pair is written when the first pair's ff2 products are done (a completion of slot 0 that says no more
 // than that); the last completion, on every slot, says that the sums are there.
 template <int NB>
-__device__ __forceinline__ void ffn_block_f16(const Row& c, const LayerParams& lp, uint32_t (&x)[8 * NB]) {
+__device__ __forceinline__ void ffn_block_f16(const Row& c, uint32_t lp, uint32_t (&x)[8 * NB]) {
     using O = Own<NB>;
     const int col = O::col(c);
 #pragma unroll 1
@@ -586,20 +622,25 @@ __device__ __forceinline__ void ffn_block_f16(const Row& c, const LayerParams& l
 #pragma unroll 1
         for (int k = 0; k < 2; ++k) {
             const int ch = 2 * pair + k;
+            const uint32_t bias_at = lp + LP_B_FF1 + 2u * (256 * ch + col);
+            Bias bias = load_bias(bias_at);
             wait_acc(c, ch, 1);
             if (ch == 2) wait_acc(c, 0, 2);
             each_piece<NB>(O::slot(c, ch), [&](int i, const uint32_t (&acc)[16]) {
                 uint32_t h[8];
-                descale<16, true, kAccPlain>(acc, 1.f, 1.f, lp.b_ff1 + 256 * ch + col + 16 * i, h);
+                if (i > 0) bias = load_bias(bias_at + 32 * i);
+                descale16<true, kAccPlain>(acc, 1.f, 1.f, bias, h);
                 store_operand16<NB>(c, c.h + k * 4 * O::kSlab, i, h);
             });
         }
         publish(c, B_H + pair);
     }
+    Bias bias = load_bias(lp + LP_B_FF2 + 2u * col);
     wait_acc(c, 1, 2);
     each_piece<NB>(O::slot(c, 0), [&](int k, const uint32_t (&acc)[16]) {
         uint32_t y[8];
-        descale<16, false, kAccPlain>(acc, 1.f, 1.f, lp.b_ff2 + col + 16 * k, y);
+        if (k > 0) bias = load_bias(lp + LP_B_FF2 + 2u * col + 32 * k);
+        descale16<false, kAccPlain>(acc, 1.f, 1.f, bias, y);
 #pragma unroll
         for (int i = 0; i < 8; ++i) x[8 * k + i] = as_u32(__hadd2(as_h2(x[8 * k + i]), as_h2(y[i])));
     });
@@ -810,20 +851,10 @@ __device__ __forceinline__ void row_tile(Row& c, const Params& p, int first) {
     const int id = 128 * c.q + 32 * c.s + lane;              // 0 .. 511
     // half-layers, so that the norm's code is there once
     const int n_half = 2 * p.n_layers;
-    const uint8_t* lpb = p.lparams;
 #pragma unroll 1
     for (int half = 0; half < n_half; ++half) {
-        // the layer's scales and biases are asked into L1 a norm ahead of their first use
-        if (id < kLparamStride / 128) prefetch_l1(lpb + 128 * id);
-        LayerParams lp;
-        lp.sw_qkv = reinterpret_cast<const float*>(lpb + LP_SW_QKV);
-        lp.sw_o = reinterpret_cast<const float*>(lpb + LP_SW_O);
-        lp.sw_ff1 = reinterpret_cast<const float*>(lpb + LP_SW_FF1);
-        lp.sw_ff2 = reinterpret_cast<const float*>(lpb + LP_SW_FF2);
-        lp.b_qkv = reinterpret_cast<const __half*>(lpb + LP_B_QKV);
-        lp.b_o = reinterpret_cast<const __half*>(lpb + LP_B_O);
-        lp.b_ff1 = reinterpret_cast<const __half*>(lpb + LP_B_FF1);
-        lp.b_ff2 = reinterpret_cast<const __half*>(lpb + LP_B_FF2);
+        const uint32_t lp = layer_params(c);
+        if ((half & 1) == 0) wait_params(c);
         // the row maxima start at zero: the hidden chunks' are cleared before the attention norm's
         // meetings, the attention output's before the FFN norm's (and at the start), ahead of their use
         const uint32_t mx = c.smem + SM_MAX + 4u * O::row(c);
@@ -836,7 +867,6 @@ __device__ __forceinline__ void row_tile(Row& c, const Params& p, int first) {
             if constexpr (kAr == kArF16) ffn_block_f16<NB>(c, lp, x);
             else ffn_block<NB, kAr>(c, lp, sa, x);
             c.layers++;
-            lpb += kLparamStride;
         }
     }
     if (id < static_cast<int>(kTailBytes / 128)) prefetch_l1(reinterpret_cast<const uint8_t*>(p.tail) + 128 * id);
@@ -870,6 +900,20 @@ __device__ __forceinline__ void producer(uint32_t smem, volatile int* abort_flag
             bulk_g2s(dst + kRStage, u1 + s * kRStage, kRStage, full);
         });
     };
+    // The scales and biases of a layer go into one of two places.  Those of the next layer are sent when
+    // the ring has taken the out-projection's stages: Q of this layer has then been consumed, so every
+    // row warp has published this layer's first operand and is done with the layer before, whose place
+    // they take.
+    uint32_t g = 0;             // layers whose parameters have been sent
+    auto params = [&](int layer) {
+        if (elect_one()) {
+            const uint32_t full = bar(smem, B_PAR + (g & 1u));
+            mbar_arrive_expect_tx(full, kLparamStride);
+            bulk_g2s(smem + SM_PAR + (g & 1u) * kLparamStride, p.lparams + static_cast<size_t>(layer) * kLparamStride, kLparamStride, full);
+        }
+        ++g;
+    };
+    if (n_tiles > 0) params(0);
     for (int tile = 0; tile < n_tiles; ++tile) {
         const uint8_t* src = p.wstream;
         for (int layer = 0; layer < p.n_layers; ++layer, src += C::kLayerStream) {
@@ -882,6 +926,8 @@ __device__ __forceinline__ void producer(uint32_t smem, volatile int* abort_flag
                     });
             const uint8_t* out = src + 4 * C::kQkvSlabs * kQStage;
             for (int s = 0; s < C::kOutSlabs; ++s) two_units(out, out + C::kOutSlabs * kRStage, s);
+            if (layer + 1 < p.n_layers) params(layer + 1);
+            else if (tile + 1 < n_tiles) params(0);
             // ff1 chunks 0-3, then ff2 chunks 0-3; where their two units lie in the packed order
             const uint8_t* ffn = out + 2 * C::kOutSlabs * kRStage;
             for (int u = 0; u < 8; ++u) {
