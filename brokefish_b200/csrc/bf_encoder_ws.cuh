@@ -544,7 +544,7 @@ __device__ __forceinline__ void ffn_block(const Row& c, uint32_t lp, float sa, u
     using O = Own<NB>;
     const int col = O::col(c), row = O::row(c);
     float s1[4] = {1.f, 1.f, 1.f, 1.f};
-#pragma unroll 1
+#pragma unroll
     for (int pair = 0; pair < 2; ++pair) {
         uint32_t hid[2][8 * NB];
         const uint32_t m = c.smem + SM_MAX + 256u * (1 + 2 * pair) + 4u * row;
@@ -579,7 +579,7 @@ __device__ __forceinline__ void ffn_block(const Row& c, uint32_t lp, float sa, u
     for (int i = 0; i < 8 * NB; ++i) run[i] = 0u;
     const float s2 = lds_f(lp + LP_SW_FF2 + 4u * (col >> 7));
     const uint64_t s2_2 = pk2(s2, s2);
-#pragma unroll 1
+#pragma unroll 2
     for (int ch = 0; ch < 4; ++ch) {
         wait_acc(c, ch, 2);
         const uint64_t s1_2 = pk2(s1[0], s1[0]);
