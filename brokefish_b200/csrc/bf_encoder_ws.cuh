@@ -346,12 +346,12 @@ __device__ __forceinline__ float4 row_statistics(const Row& c, const Params& p, 
 template <int NB, int kAr>
 __device__ __forceinline__ float norm_to_operand(const Row& c, const Params& p, const uint32_t (&x)[8 * NB], bool as_f16) {
     const float4 st = row_statistics<NB, kAr>(c, p, x);
-    const uint64_t nmean2 = pk2(st.x, st.x), rstd2 = pk2(st.y, st.y);
+    const uint64_t rstd2 = pk2(st.y, st.y);
 #pragma unroll
     for (int k = 0; k < NB; ++k) {
         uint32_t v[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = f2_to_h2(mul2(add2(h2_to_f2(x[8 * k + i]), nmean2), rstd2));
+        for (int i = 0; i < 8; ++i) v[i] = f2_to_h2(mul2(add_h2_f(x[8 * k + i], st.x), rstd2));
         if (kAr != kArInt8 && kAr != kArI8Qkv && as_f16) store_operand16<NB>(c, c.a(), k, v);
         else store_operand8<NB, kAr == kArE4M3>(c, c.a(), k, v, st.z);
     }
@@ -381,21 +381,19 @@ __device__ __forceinline__ void softmax(uint32_t (&s)[4][2], const uint32_t (&de
 #pragma unroll
     for (int hi = 0; hi < 2; ++hi) {
         float pv[4][2];
-        float mx = -INFINITY;
+        __half2 val[4];
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-            const __half2 val = __hadd2(as_h2(s[nt][hi]), as_h2(dead[nt]));
-            pv[nt][0] = __low2float(val);
-            pv[nt][1] = __high2float(val);
-            mx = fmaxf(mx, fmaxf(pv[nt][0], pv[nt][1]));
-        }
+        for (int nt = 0; nt < 4; ++nt) val[nt] = __hadd2(as_h2(s[nt][hi]), as_h2(dead[nt]));
+        const __half2 m2 = __hmax2(__hmax2(val[0], val[1]), __hmax2(val[2], val[3]));
+        float mx = fmaxf(__low2float(m2), __high2float(m2));
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
         float sum = 0.f;
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) {
-            pv[nt][0] = __expf(pv[nt][0] - mx);     // an all-dead row keeps the reference's NaN
-            pv[nt][1] = __expf(pv[nt][1] - mx);
+            upk2(add_h2_f(as_u32(val[nt]), -mx), pv[nt][0], pv[nt][1]);
+            pv[nt][0] = __expf(pv[nt][0]);           // an all-dead row keeps the reference's NaN
+            pv[nt][1] = __expf(pv[nt][1]);
             sum += pv[nt][0] + pv[nt][1];
         }
         sum += __shfl_xor_sync(0xffffffffu, sum, 1);

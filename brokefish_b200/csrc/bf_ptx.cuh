@@ -342,6 +342,15 @@ __device__ __forceinline__ void mma_f16_f16(uint32_t (&d)[2], const uint32_t (&a
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// c + each half of a packed fp16 pair, one rounding to fp32 (the conversion is exact)
+__device__ __forceinline__ uint64_t add_h2_f(uint32_t h, float c) {
+    uint64_t d;
+    asm("{\n\t.reg .b16 l, h;\n\t.reg .f32 x, y;\n\tmov.b32 {l, h}, %1;\n\t"
+        "add.rn.f32.f16 x, l, %2;\n\tadd.rn.f32.f16 y, h, %2;\n\tmov.b64 %0, {x, y};\n\t}"
+        : "=l"(d) : "r"(h), "f"(c));
+    return d;
+}
+
 // ---------------------------------------------------------------- packed fp32 (sm_100 f32x2)
 // Two fp32 lanes in one 64-bit register; each lane rounds exactly as the scalar op does.
 __device__ __forceinline__ uint64_t pk2(float lo, float hi) {
