@@ -255,18 +255,14 @@ __device__ __forceinline__ float4 row_statistics(const Row& c, const Params& p, 
         uint64_t s2[NB], q2[NB];
 #pragma unroll
         for (int pr = 0; pr < NB; ++pr) {
-            s2[pr] = pk2(0.f, 0.f);
-            q2[pr] = pk2(0.f, 0.f);
+            float sa = 0.f, sb = 0.f, qa = 0.f, qb = 0.f;
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                const uint32_t wa = x[8 * pr + k], wb = x[8 * pr + 4 + k];
-                uint64_t f = h2_to_f2(__byte_perm(wa, wb, 0x5410));
-                s2[pr] = add2(s2[pr], f);
-                q2[pr] = fma2(f, f, q2[pr]);
-                f = h2_to_f2(__byte_perm(wa, wb, 0x7632));
-                s2[pr] = add2(s2[pr], f);
-                q2[pr] = fma2(f, f, q2[pr]);
+                sum_h2(x[8 * pr + k], sa, qa);
+                sum_h2(x[8 * pr + 4 + k], sb, qb);
             }
+            s2[pr] = pk2(sa, sb);
+            q2[pr] = pk2(qa, qb);
         }
         __half2 mn = as_h2(x[0]), mx = as_h2(x[0]);
 #pragma unroll

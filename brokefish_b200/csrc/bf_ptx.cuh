@@ -342,6 +342,14 @@ __device__ __forceinline__ void mma_f16_f16(uint32_t (&d)[2], const uint32_t (&a
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// s + low half, then + high half; q + low half squared, then + high half squared: the bits of the same sums
+// of converted values
+__device__ __forceinline__ void sum_h2(uint32_t h, float& s, float& q) {
+    asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %2;\n\t"
+        "add.rn.f32.f16 %0, l, %0;\n\tadd.rn.f32.f16 %0, h, %0;\n\t"
+        "fma.rn.f32.f16 %1, l, l, %1;\n\tfma.rn.f32.f16 %1, h, h, %1;\n\t}"
+        : "+f"(s), "+f"(q) : "r"(h));
+}
 // c + each half of a packed fp16 pair, one rounding to fp32 (the conversion is exact)
 __device__ __forceinline__ uint64_t add_h2_f(uint32_t h, float c) {
     uint64_t d;
