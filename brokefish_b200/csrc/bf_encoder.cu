@@ -13,8 +13,8 @@
 // fp16-accumulate mma.sync); the 32 x 32 attention products run as mma.sync on the row warps.
 //
 // Plain evaluations run on one- and two-board tiles (bf_encoder_ws.cuh).  The kernel below, on
-// four-board tiles, is the large-batch form of the arithmetics with fp16 products, carries re-injection
-// and is the instrumented arm.  Its shape
+// four-board tiles, is the large-batch form of the fp16 arithmetic, carries re-injection and is the
+// instrumented arm.  Its shape
 //   * persistent grid, one CTA per SM, each CTA loops over tiles of 128 token rows
 //     (4 boards);
 //   * 19 warps: 16 "row" warps, one weight-stream producer, two MMA issuers;
@@ -2214,9 +2214,33 @@ void* mapped_host(const void* p) {
     return a.type == cudaMemoryTypeHost ? a.devicePointer : nullptr;
 }
 
+// A host call on a small batch whose buffers are all pinned and device-mapped runs as one launch on
+// them: no copies, one synchronisation.  B200, us through the Python API, copied / in place:
+//   logits, positions    1: 117/102   16: 118/109   64: 125/124   148: 141/152   296: 194/237
+//   edge lists           1: 112/104   148: 135/121   296: 172/156   592: 305/283
+// Logits are 4.3 KB a position and leave all at once at the end of a tile.
+constexpr int kDirectLogits = 64;        // positions
+constexpr int kDirectEdges = 4;          // positions per SM
+struct MappedInputs {
+    const uint16_t* boards;
+    const int16_t* control;
+    const uint8_t* rep;
+    const uint64_t* legal;
+    bool ok;
+    MappedInputs(const void* b, const void* c, const void* r, const void* l)
+        : boards(static_cast<const uint16_t*>(mapped_host(b))), control(static_cast<const int16_t*>(mapped_host(c))),
+          rep(static_cast<const uint8_t*>(mapped_host(r))), legal(static_cast<const uint64_t*>(mapped_host(l))),
+          ok(boards != nullptr && control != nullptr && rep != nullptr && (legal != nullptr) == (l != nullptr)) {}
+};
+// Whether large batches of this handle run on two-board tiles (a wave is two positions per SM) or on
+// four-board ones.
+bool two_board_waves(const bf_handle* h) { return h->hdr.quant != 0 && h->hdr.rj_mode == 0; }
+
 // bf_forward_host sizes its launches by how many times faster this GPU copies a position's logits
 // to the host than it evaluates a position.
-constexpr double kEvalGBps = 8.8;        // logits a B200 produces per second at full rate (4356 B x 2.03 M)
+constexpr double kEvalGBps = 8.8;        // logits a B200 produces per second at full rate on four-board
+                                         // tiles (4356 B x 2.03 M)
+constexpr double kSmallTileRate = 1.2;   // how much faster two-board tiles are (2.45 M positions/s)
 constexpr double kFastLinkRatio = 6.0;   // a GPU alone on its link: 55 GB/s against those 8.8
 
 // The launch sizes of bf_forward_host for `n` positions on a GPU whose wave is `wave` positions:
@@ -2292,13 +2316,14 @@ struct LeafList {
 // Which form a plain evaluation runs in: one- and two-board tiles (bf_encoder_ws.cuh) or four-board tiles.
 // A tile takes the same time whatever the batch, so the tiles of the busiest SM decide.  Measured, us
 // per one-, two- and four-board tile of an SM (B200):
-//   int8 96 / 141 / 280    int8 FFN+QKV 104 / 143 / 276    int8 FFN 115 / 146 / 277
-//   e4m3 115 / 143 / 270   fp16 143 / 166 / 252
-// The first two never gain from the four-board form.  The others' fp16 products, 32 bytes of K at half
-// the rate, weigh more on fewer rows.
+//   int8 90 / 126    int8 FFN+QKV 96 / 128    int8 FFN 103 / 133 / 273
+//   e4m3 100 / 130 / 270    fp16 129 / 152 / 275
+// Two two-board tiles beat a four-board one everywhere but in fp16, whose products, 32 bytes of K at
+// half the rate and twice the weight bytes, keep the weight stream and the tensor pipe busy for half
+// of a two-board tile's time; there the four-board form takes the batches that fill it.
 bool small_tiles(int quant, int n, int sm_count) {
-    static const int us[5][3] = {{143, 166, 252}, {115, 143, 270}, {115, 146, 277}, {1, 1, 1000}, {1, 1, 1000}};
-    const int* t = us[quant];
+    if (quant != 0) return true;
+    static const int t[3] = {129, 152, 275};
     const long full = n / (2 * sm_count), rest = n - full * 2 * sm_count;
     const long small = full * t[1] + (rest == 0 ? 0 : rest <= sm_count ? t[0] : t[1]);
     const long four = static_cast<long>((n + 4L * sm_count - 1) / (4L * sm_count)) * t[2];
@@ -2352,14 +2377,14 @@ int launch(bf_handle* h, const uint16_t* boards, const int16_t* control, const u
                                                                                                 : bf::ws::encoder_ws_kernel<bf::kArInt8>;
         kernel<<<ctas, bf::ws::kThreads, bf::ws::kSmemRequest, stream>>>(p);
     } else {
-        // four-board tiles: large batches of the arithmetics with fp16 products, re-injection, and the
-        // instrumented arms (dumps, captures, the phase clock, the backbone entry)
+        // four-board tiles: large batches of the fp16 arithmetic, re-injection, and the instrumented arms
+        // (dumps, captures, the phase clock, the backbone entry)
         const auto kernel =
             p.quant == 0 ? (p.rj_mode == 0 ? (dbg ? bf::encoder_kernel<true, false, bf::kArF16> : bf::encoder_kernel<false, false, bf::kArF16>)
                                            : (dbg ? bf::encoder_kernel<true, true, bf::kArF16> : bf::encoder_kernel<false, true, bf::kArF16>))
             : p.quant == 4 ? bf::encoder_kernel<true, false, bf::kArI8Qkv>
-            : p.quant == 2 ? (dbg ? bf::encoder_kernel<true, false, bf::kArI8Ffn> : bf::encoder_kernel<false, false, bf::kArI8Ffn>)
-            : p.quant == 1 ? (dbg ? bf::encoder_kernel<true, false, bf::kArE4M3> : bf::encoder_kernel<false, false, bf::kArE4M3>)
+            : p.quant == 2 ? bf::encoder_kernel<true, false, bf::kArI8Ffn>
+            : p.quant == 1 ? bf::encoder_kernel<true, false, bf::kArE4M3>
             : p.rj_mode == 0 ? bf::encoder_kernel<true, false, bf::kArInt8>
             : dbg            ? bf::encoder_kernel<true, true, bf::kArInt8>
                              : bf::encoder_kernel<false, true, bf::kArInt8>;
@@ -2427,9 +2452,7 @@ int bf_create(const void* blob, size_t blob_bytes, int device, bf_handle** out) 
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->chunk_done, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreate(&h->copy_t0);
     if (e == cudaSuccess) e = cudaEventCreate(&h->copy_t1);
-    for (const void* k : {reinterpret_cast<const void*>(&bf::encoder_kernel<false, false, bf::kArI8Ffn>),
-                          reinterpret_cast<const void*>(&bf::encoder_kernel<false, false, bf::kArE4M3>),
-                          reinterpret_cast<const void*>(&bf::encoder_kernel<false, false, bf::kArF16>),
+    for (const void* k : {reinterpret_cast<const void*>(&bf::encoder_kernel<false, false, bf::kArF16>),
                           reinterpret_cast<const void*>(&bf::encoder_kernel<true, false, bf::kArI8Qkv>),
                           reinterpret_cast<const void*>(&bf::encoder_kernel<true, false, bf::kArI8Ffn>),
                           reinterpret_cast<const void*>(&bf::encoder_kernel<true, false, bf::kArE4M3>),
@@ -2705,6 +2728,21 @@ int bf_forward_host(bf_handle* h, const uint16_t* boards, const int16_t* control
     if (boards == nullptr || control == nullptr || rep == nullptr)
         return fail(BF_EINVAL, "boards, control and rep must be non-null");
     BF_ON_DEVICE(h->device);
+    void* m_policy = mapped_host(policy);
+    void* m_promo = mapped_host(promo);
+    void* m_value = mapped_host(value);
+    const bool all_mapped = policy != nullptr && promo != nullptr && value != nullptr &&
+                            m_policy != nullptr && m_promo != nullptr && m_value != nullptr;
+    if (n <= kDirectLogits && all_mapped) {
+        const MappedInputs in(boards, control, rep, legal);
+        if (in.ok) {
+            const int rc = launch(h, in.boards, in.control, in.rep, in.legal, n, m_policy, m_promo, static_cast<float*>(m_value),
+                                  nullptr, 0, 0, -1, -1, nullptr, nullptr, h->stream);
+            if (rc != BF_OK) return rc;
+            BF_CUDA(cudaStreamSynchronize(h->stream));
+            return BF_OK;
+        }
+    }
     { const int rc = ensure_staging(h, n); if (rc != BF_OK) return rc; }
     const size_t N = static_cast<size_t>(h->cap_n);
     uint8_t* d_legal = h->d_in;                         // 8-byte aligned first
@@ -2728,7 +2766,7 @@ int bf_forward_host(bf_handle* h, const uint16_t* boards, const int16_t* control
     //   r >= 1.5    launches of shrinking size, largest first, the last one a single wave (one
     //               tile per SM), each launch r times the one after it (in whole waves, rounded
     //               down) so that its copy hides behind the next launch; r is capped at 6, a GPU
-    //               alone on its link: [3504, 592] positions for a batch of 4096.  Large launches
+    //               alone on its link: [2320, 1480, 296] positions for a batch of 4096.  Large launches
     //               keep the kernel's tile-to-tile pipelining.
     //   r < 1.5     equal launches of about two waves, so that every copy hides behind the next
     //               launch as long as copying is not slower than evaluating, and the last wave
@@ -2737,12 +2775,9 @@ int bf_forward_host(bf_handle* h, const uint16_t* boards, const int16_t* control
     //               while the wave computes beat a copy that starts when the wave has ended.
     // (Everything through mapped memory was measured 10 % slower on a fast link -- the stores back
     // up behind the bus -- and the last wave alone 4 % slower than copying it.)
-    const int wave = h->sm_count * 4;
-    void* m_policy = mapped_host(policy);
-    void* m_promo = mapped_host(promo);
-    void* m_value = mapped_host(value);
-    const bool all_mapped = policy != nullptr && promo != nullptr && value != nullptr &&
-                            m_policy != nullptr && m_promo != nullptr && m_value != nullptr;
+    // (a wave of two-board tiles is two positions per SM, and they are the faster by kSmallTileRate)
+    const bool two = two_board_waves(h);
+    const int wave = h->sm_count * (two ? 2 : 4);
     cudaStream_t c = h->copy_stream;
     size_t timed_bytes = 0;
     auto copy_out = [&](int lo, int m, bool timed) -> int {
@@ -2756,7 +2791,7 @@ int bf_forward_host(bf_handle* h, const uint16_t* boards, const int16_t* control
     };
     int sizes[16];
     bool slow_link = false;
-    const int n_chunks = host_plan_sizes(n, wave, h->host_plan, h->d2h_gbps, sizes, &slow_link);
+    const int n_chunks = host_plan_sizes(n, wave, h->host_plan, h->d2h_gbps / (two ? kSmallTileRate : 1.0), sizes, &slow_link);
     const bool direct_last = slow_link && all_mapped;
     int lo = 0, k_timed = 0;
     for (int k = 1; k < n_chunks; ++k)
@@ -2806,6 +2841,21 @@ int bf_forward_priors_host(bf_handle* h, const uint16_t* boards, const int16_t* 
     if (prior == nullptr || move == nullptr || nedges == nullptr) return fail(BF_EINVAL, "prior, move and nedges must be non-null");
     if (e_cap < 1 || e_cap > 255) return fail(BF_EINVAL, "e_cap must be in 1..255");
     BF_ON_DEVICE(h->device);
+    void* m_prior = mapped_host(prior);
+    void* m_move = mapped_host(move);
+    void* m_ne = mapped_host(nedges);
+    void* m_value = mapped_host(value);
+    if (n <= h->sm_count * kDirectEdges && m_prior && m_move && m_ne && (value == nullptr || m_value)) {
+        const MappedInputs in(boards, control, rep, legal);
+        if (in.ok) {
+            const PriorOut po{m_prior, static_cast<int16_t*>(m_move), static_cast<int*>(m_ne), e_cap};
+            const int rc = launch(h, in.boards, in.control, in.rep, in.legal, n, nullptr, nullptr, static_cast<float*>(m_value),
+                                  nullptr, 0, 0, -1, -1, nullptr, nullptr, h->stream, &po);
+            if (rc != BF_OK) return rc;
+            BF_CUDA(cudaStreamSynchronize(h->stream));
+            return BF_OK;
+        }
+    }
     { const int rc = ensure_staging(h, n); if (rc != BF_OK) return rc; }
     const size_t N = static_cast<size_t>(h->cap_n), E = static_cast<size_t>(e_cap);
     uint8_t* d_legal = h->d_in;
@@ -2822,26 +2872,12 @@ int bf_forward_priors_host(bf_handle* h, const uint16_t* boards, const int16_t* 
     BF_CUDA(cudaMemcpyAsync(d_control, control, static_cast<size_t>(n) * 2, cudaMemcpyHostToDevice, s));
     BF_CUDA(cudaMemcpyAsync(d_rep, rep, static_cast<size_t>(n), cudaMemcpyHostToDevice, s));
     BF_CUDA(cudaMemcpyAsync(d_legal, legal, static_cast<size_t>(n) * 256, cudaMemcpyHostToDevice, s));
-    {
-        // pinned, mapped outputs: the edge lists are small (392 B per position at e_cap 96), so
-        // one launch writes them across the bus as it goes (measured 2 % faster than staging)
-        void* m_prior = mapped_host(prior);
-        void* m_move = mapped_host(move);
-        void* m_ne = mapped_host(nedges);
-        void* m_value = mapped_host(value);
-        if (m_prior && m_move && m_ne && (value == nullptr || m_value)) {
-            const PriorOut po{m_prior, static_cast<int16_t*>(m_move), static_cast<int*>(m_ne), e_cap};
-            int rc = launch(h, reinterpret_cast<uint16_t*>(d_boards), reinterpret_cast<int16_t*>(d_control), d_rep,
-                            reinterpret_cast<uint64_t*>(d_legal), n, nullptr, nullptr, static_cast<float*>(m_value),
-                            nullptr, 0, 0, -1, -1, nullptr, nullptr, s, &po);
-            if (rc != BF_OK) return rc;
-            BF_CUDA(cudaStreamSynchronize(s));
-            return BF_OK;
-        }
-    }
-    const int wave = h->sm_count * 4;
-    for (int lo = 0; lo < n; lo += wave) {
-        const int m = n - lo < wave ? n - lo : wave;
+    // The edge lists are small (392 B per position at e_cap 96): with the fast-link sizes all but the
+    // last wave's copies hide behind the next launch.
+    int sizes[16];
+    const int n_chunks = host_plan_sizes(n, h->sm_count * (two_board_waves(h) ? 2 : 4), 1, 0.0, sizes, nullptr);
+    for (int k = 0, lo = 0; k < n_chunks; lo += sizes[k], ++k) {
+        const int m = sizes[k];
         const size_t o = static_cast<size_t>(lo), M = static_cast<size_t>(m);
         const PriorOut po{d_prior + o * E * 2, reinterpret_cast<int16_t*>(d_move + o * E * 2),
                           reinterpret_cast<int*>(d_nedges) + o, e_cap};

@@ -27,7 +27,8 @@ constexpr int64_t kMaxHistory = 100;
 
 #define BF_FUNCTIONS(X)                                                                       \
     X(bf_movegen) X(bf_step) X(bf_hash) X(bf_history_push_to) X(bf_repetition_count) X(bf_terminal) \
-    X(bf_terminal_history) X(bf_forward) X(bf_forward_priors) X(bf_forward_leaves)
+    X(bf_terminal_history) X(bf_forward) X(bf_forward_priors) X(bf_forward_leaves) X(bf_forward_host) \
+    X(bf_forward_priors_host)
 struct Api {
 #define X(name) decltype(&::name) name = nullptr;
     BF_FUNCTIONS(X)
@@ -303,6 +304,37 @@ void forward_leaves(int64_t handle, const Tensor& boards, const Tensor& control,
     });
 }
 
+// ---- the host-buffer calls ----
+void check_host(std::initializer_list<const Tensor*> tensors, const char* text) {
+    for (const Tensor* t : tensors)
+        if (t->is_cuda() || !t->is_contiguous()) throw py::value_error(text);
+}
+void forward_host(int64_t handle, const Tensor& boards, const Tensor& control, const Tensor& rep, const Tensor& policy,
+                  const Tensor& promo, const Tensor& value, const std::optional<Tensor>& legal) {
+    const int n = static_cast<int>(check_inputs(boards, control, rep));
+    check_host({&boards, &control, &rep, &policy, &promo, &value}, "forward_host takes contiguous CPU tensors");
+    call("bf_forward_host", [&] {
+        return g_api.bf_forward_host(handle_of(handle), ptr<uint16_t>(boards), ptr<int16_t>(control), ptr<uint8_t>(rep),
+                                     legal ? ptr<uint64_t>(*legal) : nullptr, n, ptr(policy), ptr(promo), ptr<float>(value));
+    });
+}
+void forward_priors_host(int64_t handle, const Tensor& boards, const Tensor& control, const Tensor& rep, const Tensor& legal,
+                         const Tensor& prior, const Tensor& move, const Tensor& nedges, const Tensor& value) {
+    const int64_t n = check_inputs(boards, control, rep);
+    check_host({&boards, &control, &rep, &legal, &prior, &move, &nedges, &value}, "forward_priors_host takes contiguous CPU tensors");
+    const int64_t e_cap = prior.dim() > 1 ? prior.size(1) : -1;
+    if (legal.dim() != 2 || legal.size(0) != n || legal.size(1) != 32 || legal.scalar_type() != at::kLong || move.dim() != 2 ||
+        move.size(0) != n || move.size(1) != e_cap || move.scalar_type() != at::kShort || prior.scalar_type() != at::kHalf ||
+        !is_vector(nedges, n) || nedges.scalar_type() != at::kInt || !is_vector(value, n) || value.scalar_type() != at::kFloat)
+        throw py::value_error("forward_priors_host: legal [n,32] int64, prior [n,E] fp16, move [n,E] int16, "
+                              "nedges [n] int32, value [n] fp32");
+    call("bf_forward_priors_host", [&] {
+        return g_api.bf_forward_priors_host(handle_of(handle), ptr<uint16_t>(boards), ptr<int16_t>(control), ptr<uint8_t>(rep),
+                                            ptr<uint64_t>(legal), static_cast<int>(n), static_cast<int>(e_cap), ptr(prior),
+                                            ptr<int16_t>(move), ptr<int>(nedges), ptr<float>(value));
+    });
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -317,4 +349,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("forward", &forward);
     m.def("forward_priors", &forward_priors);
     m.def("forward_leaves", &forward_leaves);
+    m.def("forward_host", &forward_host);
+    m.def("forward_priors_host", &forward_priors_host);
 }

@@ -427,13 +427,7 @@ class FusedEncoder:
         """End-to-end call on HOST tensors (pinned for speed): copies in, runs, copies the
         three outputs into the given host tensors and synchronises."""
         self._require_net("forward_host")
-        n = self._check_inputs(boards, control, rep)
-        for t in (boards, control, rep, policy, promo, value):
-            if t.is_cuda or not t.is_contiguous():
-                raise ValueError("forward_host takes contiguous CPU tensors")
-        _native.check(_native.lib().bf_forward_host(
-            self._handle, _ptr(boards), _ptr(control), _ptr(rep), _ptr(legal), n, _ptr(policy),
-            _ptr(promo), _ptr(value)), "bf_forward_host")
+        _native.torch_ops().forward_host(self._handle.value, boards, control, rep, policy, promo, value, legal)
         return policy, promo, value
 
     def forward_priors_host(self, boards, control, rep, legal, prior, move, nedges, value):
@@ -441,21 +435,7 @@ class FusedEncoder:
         fp16, ``move [n,E]`` int16, ``nedges [n]`` int32 and ``value [n]`` fp32 are filled;
         ``E = prior.shape[1]``."""
         self._require_net("forward_priors_host")
-        n = self._check_inputs(boards, control, rep)
-        for t in (boards, control, rep, legal, prior, move, nedges, value):
-            if t.is_cuda or not t.is_contiguous():
-                raise ValueError("forward_priors_host takes contiguous CPU tensors")
-        e_cap = int(prior.shape[1])
-        if (tuple(legal.shape) != (n, self.T) or legal.dtype is not torch.int64
-                or tuple(move.shape) != (n, e_cap) or move.dtype is not torch.int16
-                or prior.dtype is not torch.half or tuple(nedges.shape) != (n,)
-                or nedges.dtype is not torch.int32 or tuple(value.shape) != (n,)
-                or value.dtype is not torch.float32):
-            raise ValueError("forward_priors_host: legal [n,32] int64, prior [n,E] fp16, move [n,E] int16, "
-                             "nedges [n] int32, value [n] fp32")
-        _native.check(_native.lib().bf_forward_priors_host(
-            self._handle, _ptr(boards), _ptr(control), _ptr(rep), _ptr(legal), n, e_cap, _ptr(prior),
-            _ptr(move), _ptr(nedges), _ptr(value)), "bf_forward_priors_host")
+        _native.torch_ops().forward_priors_host(self._handle.value, boards, control, rep, legal, prior, move, nedges, value)
         return prior, move, nedges, value
 
     # -- in-kernel phase accounting (the reference's set_profile / read_profile hooks) ----
@@ -499,7 +479,10 @@ class FusedEncoder:
         """The launch sizes ``forward_host`` would use for ``n`` positions now."""
         sizes = (ctypes.c_int * 16)()
         sms = torch.cuda.get_device_properties(self.device).multi_processor_count
-        k = _native.lib().bf_host_plan(int(n), sms, self._host_plan, self.host_link_gbps, sizes)
+        gbps = self.host_link_gbps
+        if self.quant != 0 and not self.rj_mode:         # two-board tiles: half the wave, 1.2 times the rate
+            sms, gbps = max(1, sms // 2), gbps / 1.2
+        k = _native.lib().bf_host_plan(int(n), sms, self._host_plan, gbps, sizes)
         _native.check(min(k, 0), "bf_host_plan")
         return list(sizes[:k])
 

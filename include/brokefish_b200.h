@@ -230,17 +230,16 @@ int bf_forward_capture(bf_handle* h, const uint16_t* boards, const int16_t* cont
 /* End-to-end call with HOST buffers (pinned for best speed): copies the inputs to the
  * device, runs the evaluator as a few launches of shrinking size (the last one a single wave of
  * tiles), copies each launch's three outputs back on a second stream while the next launch
- * computes -- only the last wave's copy is exposed -- and synchronises.
+ * computes -- only the last wave's copy is exposed -- and synchronises.  A small batch in pinned,
+ * device-mapped buffers runs as one launch that reads and writes them in place.
  * Device staging buffers are owned by the handle and grow to the largest `n` seen. */
 int bf_forward_host(bf_handle* h, const uint16_t* boards, const int16_t* control,
                     const uint8_t* rep, const uint64_t* legal, int n, void* policy,
                     void* promo, float* value);
 
-/* bf_forward_priors with HOST buffers, end to end like bf_forward_host: inputs (the legality
- * words included) go to the device, the evaluator runs wave by wave, and each wave's edge
- * lists and values come back on a second stream while the next wave computes; about 11 times
- * fewer bytes return to the host than with the logits (392 B per position at e_cap 96).  When
- * the outputs are pinned, device-mapped host memory the kernel writes them there directly. */
+/* bf_forward_priors with HOST buffers, end to end like bf_forward_host: about 11 times
+ * fewer bytes return to the host than with the logits (392 B per position at e_cap 96), so batches of
+ * up to four positions per SM in pinned, device-mapped buffers run in place. */
 int bf_forward_priors_host(bf_handle* h, const uint16_t* boards, const int16_t* control, const uint8_t* rep,
                            const uint64_t* legal, int n, int e_cap, void* prior, int16_t* move, int* nedges,
                            float* value);
@@ -271,10 +270,11 @@ int bf_set_option(bf_handle* h, int option, int value);
  * first call): what the plan of the next call is chosen by.  No counterpart in the reference. */
 double bf_host_link_gbps(const bf_handle* h);
 
-/* The launch sizes `bf_forward_host` uses for `n` positions on a GPU with `sm_count` SMs under
- * BF_OPT_HOST_PLAN `plan` when the measured copy rate is `gbps` (0: not measured yet): writes up
- * to 16 sizes, in launch order, summing to n, and returns how many; no GPU is touched.  No
- * counterpart in the reference. */
+/* The launch sizes `bf_forward_host` uses for `n` positions under BF_OPT_HOST_PLAN `plan` when the
+ * measured copy rate is `gbps` (0: not measured yet) and a wave of tiles is four positions on each of
+ * `sm_count` SMs; a call that runs on two-board tiles (every arithmetic but fp16, no re-injection)
+ * uses those of half the SMs and gbps / 1.2.  Writes up to 16 sizes, in launch order, summing to n,
+ * and returns how many; no GPU is touched.  No counterpart in the reference. */
 int bf_host_plan(int n, int sm_count, int plan, double gbps, int* sizes);
 
 /* Read (and clear) the device status word; 0 = every launch since the last call ran
