@@ -956,18 +956,17 @@ __device__ __forceinline__ float warp_sum_to_all(float v) {
     return __shfl_sync(0xffffffffu, v, 0);
 }
 __device__ __forceinline__ void expand_board(const Params& p, int board, int lane, bool valid, uint32_t word,
-                                             int ctl, unsigned long long legal, uint32_t stage_pol,
-                                             uint32_t stage_aux, int row, uint8_t* list_buf) {
-    // the staged row of this slot: 16-byte group g of the row lives at sw_off(row, g)
-    const uint32_t row_smem = stage_pol + static_cast<uint32_t>(row) * 128u;
-    const uint32_t row_xor = static_cast<uint32_t>(row & 7);
+                                             int ctl, unsigned long long legal, uint32_t row_smem,
+                                             uint32_t row_xor, uint32_t aux, uint8_t* list_buf) {
+    // the staged logits of this slot: 16-byte group g of the policy row lives at
+    // row_smem + ((g ^ row_xor) << 4), the promotion logits at aux
     const bool pawn = ((word >> 11) & 1u) == 0u && ((word >> 6) & 7u) == 0u;
     const unsigned long long last = ctl < 0 ? 0xffull : (0xffull << 56);
     const unsigned long long promos = pawn ? (legal & last) : 0ull;
     float type_lp[4] = {0.f, 0.f, 0.f, 0.f};
     if (promos != 0ull) {
         uint32_t w0, w1;
-        asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(w0), "=r"(w1) : "r"(stage_aux + sw_off(row, 0)));
+        asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(w0), "=r"(w1) : "r"(aux));
         const float x[4] = {__low2float(as_h2(w0)), __high2float(as_h2(w0)), __low2float(as_h2(w1)),
                             __high2float(as_h2(w1))};
         const float top = fmaxf(fmaxf(x[0], x[1]), fmaxf(x[2], x[3]));
@@ -1247,8 +1246,8 @@ __device__ __forceinline__ void head_epilogue(RowCtx& c, const Params& p, int bo
         if (p.prior != nullptr && c.qt == 1) {
             // the list is put together in this board's rows of the staging region's third block,
             // idle from the head product (which read it) to the next tile's first QKV staging
-            expand_board(p, board, c.lane, c.valid, word, ctl, moves, stage_pol, stage_aux, c.row,
-                         c.smem_gen + (c.sm_r - c.smem) + 32768u + 4096u * c.q);
+            expand_board(p, board, c.lane, c.valid, word, ctl, moves, stage_pol + 128u * c.row, c.row & 7,
+                         stage_aux + sw_off(c.row, 0), c.smem_gen + (c.sm_r - c.smem) + 32768u + 4096u * c.q);
         }
         if (c.qt == 0) {
             if (c.valid && p.promo != nullptr)

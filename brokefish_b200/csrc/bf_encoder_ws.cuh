@@ -33,7 +33,7 @@
 namespace bf {
 namespace ws {
 
-constexpr int kProducerWarp = 16, kMmaWarp = 17, kThreads = 576;
+constexpr int kProducerWarp = 16, kMmaWarp = 17, kExpandWarp = 18, kThreads = 640;
 constexpr uint32_t kStage = 32768;                 // one 128-byte K-slab of 256 weight rows
 // ---- shared memory map ------------------------------------------------------------------
 // A operand: K-slabs of [rows][128 B], two of bytes or (where QKV or the out-projection runs in fp16)
@@ -47,6 +47,9 @@ struct Map {
 };
 constexpr uint32_t SM_A = 0;
 constexpr uint32_t kHeadA = 32768;                 // the head operand's place in H, clear of the other board's partial sums
+// the fused expansion's logits: per board 32 policy rows of 128 bytes, then 16 bytes of promotion logits
+// per slot; the last quarter of H, which the next tile touches in its first FFN
+constexpr uint32_t kStagePolicy = 49152, kStageAux = kStagePolicy + 8192;
 constexpr uint32_t SM_STAT = 16384 + 65536 + 4 * kStage;
 constexpr uint32_t SM_MAX = SM_STAT + 1024;        // row maxima: attention output, four hidden chunks
 constexpr uint32_t SM_LIST = SM_MAX + 5 * 256;     // fused expansion: 1 KB per board
@@ -56,7 +59,7 @@ constexpr uint32_t SM_MISC = SM_BAR + 192;
 constexpr uint32_t SM_BYTES = SM_MISC + 64, kSmemRequest = SM_BYTES + 1024;
 static_assert(kSmemRequest <= 232448 && kLparamStride % 16 == 0 && SM_PAR % 16 == 0, "shared memory map");
 static_assert(Map<kArF16>::SM_RING + 3 * kStage <= SM_STAT && Map<kArInt8>::SM_RING + 4 * kStage <= SM_STAT, "shared memory map");
-enum { B_FULL = 0, B_EMPTY = 4, B_ACC = 8, B_PAR = 12, B_A = 14, B_H = 15, B_COUNT = 17 };
+enum { B_FULL = 0, B_EMPTY = 4, B_ACC = 8, B_PAR = 12, B_A = 14, B_H = 15, B_STAGED = 17, B_EXPANDED = 18, B_COUNT = 19 };
 __device__ __forceinline__ uint32_t bar(uint32_t smem, int i) { return smem + SM_BAR + 8u * i; }
 
 // Which boards a CTA evaluates, tile by tile.  At most `one_most` boards per CTA: one-board tiles alone.
@@ -701,10 +704,9 @@ __device__ __forceinline__ void prenorm_logits(const Row& c, const Params& p, ui
 
 // Final norm into the head product's fp16 operand, then the epilogue: the product's 128 output columns
 // (64 policy, 4 promotion, value, padding) lie 8 NB to a thread.  Policy columns are masked and stored
-// by the threads that hold them; with a fused expansion the board's logits are staged in its own rows
-// of the A operand (which the next tile writes only after a meeting of the board) for one warp.
+// by the threads that hold them; with a fused expansion the logits are staged for the expansion warps.
 template <int NB, int kAr>
-__device__ __forceinline__ void heads(const Row& c, const Params& p, int board, bool valid, uint32_t word, int ctl, uint32_t alive,
+__device__ __forceinline__ void heads(const Row& c, const Params& p, int board, bool valid, int ctl, uint32_t alive,
                                       const uint32_t (&x)[8 * NB]) {
     using O = Own<NB>;
     const int col = O::col(c), row = O::row(c), lane = c.lane;
@@ -730,14 +732,9 @@ __device__ __forceinline__ void heads(const Row& c, const Params& p, int board, 
     }
     // output columns of this thread: hc .. hc + 8 NB - 1
     const int hc = NB == 1 ? 32 * c.q + 8 * c.s : 64 * (c.q >> 1) + 16 * c.s;
-    // while the product runs: the legality words, given or (for the expansion warp, lane = slot) made here
-    const bool expander = p.prior != nullptr && hc == 72 + 8 * (NB - 1);     // a warp whose columns are padding
-    unsigned long long lw = ~0ull, moves = 0ull;
-    if (p.legal != nullptr && valid && (hc < 64 || expander)) lw = p.legal[grow];
-    if (expander && valid) {
-        bool in_check;
-        moves = p.legal != nullptr ? lw : bfmg::legal_word(word, ctl, in_check);
-    }
+    // while the product runs: the legality words
+    unsigned long long lw = ~0ull;
+    if (p.legal != nullptr && p.policy != nullptr && valid && hc < 64) lw = p.legal[grow];
     wait_acc(c, 0, 0);
     uint32_t v[4 * NB];
     {
@@ -748,12 +745,17 @@ __device__ __forceinline__ void heads(const Row& c, const Params& p, int board, 
 #pragma unroll
         for (int i = 0; i < 4 * NB; ++i) v[i] = __byte_perm(acc[2 * i], acc[2 * i + 1], 0x5410);
     }
-    const uint32_t stage_pol = c.a(), stage_aux = c.a() + O::kSlab;
-    if (p.prior != nullptr && hc <= 64) {
+    if (p.prior != nullptr) {
+        if (hc < 64) {
 #pragma unroll
-        for (int k = 0; k < NB; ++k)
-            sts128((hc < 64 ? stage_pol : stage_aux) + sw_off(row, ((hc & 63) >> 3) + k),
-                   make_uint4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]));
+            for (int k = 0; k < NB; ++k)
+                sts128(c.h + kStagePolicy + 4096u * O::board(c) + sw_off(lane, (hc >> 3) + k),
+                       make_uint4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]));
+        } else if (hc == 64) {
+            sts128(c.h + kStageAux + 512u * O::board(c) + 16u * lane, make_uint4(v[0], v[1], v[2], v[3]));
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(c.smem, B_STAGED));
     }
     if (hc < 64) {
         if (valid && p.policy != nullptr) {
@@ -797,11 +799,36 @@ __device__ __forceinline__ void heads(const Row& c, const Params& p, int board, 
             p.value[board] = o;
         }
     }
-    if (p.prior != nullptr) {
-        board_sync<NB>(c);                                   // the board's logits are staged
-        if (expander)
-            expand_board(p, board, lane, valid, word, ctl, moves, stage_pol, stage_aux, row,
-                         c.smem_gen + SM_LIST + 1024u * O::board(c));
+}
+
+// The fused expansion has two warps of its own, one per board of a tile: they make the legal words
+// while the layers run and expand while the next tile begins.  Where the rows' first FFN of the next
+// tile would overwrite the staged logits they wait for B_EXPANDED.
+__device__ __forceinline__ void expander(uint32_t smem, uint8_t* smem_gen, uint32_t h, volatile int* abort_flag, const Params& p,
+                                         const Tiles& tiles, int n_tiles, int which, int lane) {
+    for (int k = 0; k < n_tiles; ++k) {
+        int first, boards;
+        tiles.at(k, first, boards);
+        const int item = first + which;
+        const bool valid = which < boards && item < tiles.n;
+        int board = item, ctl = 1;
+        uint32_t word = 0u;
+        unsigned long long moves = 0ull;
+        if (valid) {
+            if (p.leaf_index != nullptr) board = __ldg(p.leaf_index + item);
+            const long at = static_cast<long>(board) * kT + lane;
+            word = p.boards[at];
+            ctl = static_cast<int>(p.control[board]);
+            bool in_check;
+            moves = p.legal != nullptr ? p.legal[at] : bfmg::legal_word(word, ctl, in_check);
+        }
+        mbar_wait<200>(bar(smem, B_STAGED), k & 1u, abort_flag, kErrRowAcc);
+        __syncwarp();
+        if (valid)
+            expand_board(p, board, lane, true, word, ctl, moves, h + kStagePolicy + 4096u * which + 128u * lane, lane & 7,
+                         h + kStageAux + 512u * which + 16u * lane, smem_gen + SM_LIST + 1024u * which);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(smem, B_EXPANDED));
     }
 }
 
@@ -861,13 +888,17 @@ __device__ __forceinline__ void row_tile(Row& c, const Params& p, int first) {
         if ((half & 1) == 0) {
             attention_block<NB, kAr>(c, lp, sa, alive, x);
         } else {
+            if (half == 1 && p.prior != nullptr && c.tiles != 0) {
+                mbar_wait(bar(c.smem, B_EXPANDED), (c.tiles - 1u) & 1u, c.abort_flag, kErrRowAcc);
+                __syncwarp();
+            }
             if constexpr (kAr == kArF16) ffn_block_f16<NB>(c, lp, x);
             else ffn_block<NB, kAr>(c, lp, sa, x);
             c.layers++;
         }
     }
     if (id < static_cast<int>(kTailBytes / 128)) prefetch_l1(reinterpret_cast<const uint8_t*>(p.tail) + 128 * id);
-    heads<NB, kAr>(c, p, board, valid, word, ctl, alive, x);
+    heads<NB, kAr>(c, p, board, valid, ctl, alive, x);
     c.tiles++;
 }
 
@@ -1038,7 +1069,7 @@ __global__ void __launch_bounds__(640, 1) encoder_ws_kernel(const Params p) {
     volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + SM_MISC + 4);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + SM_MISC);
     if (threadIdx.x == 0) {
-        for (int i = 0; i < B_COUNT; ++i) mbar_init(bar(smem, i), i >= B_A ? kRowWarps : 1);
+        for (int i = 0; i < B_COUNT; ++i) mbar_init(bar(smem, i), i == B_EXPANDED ? 2 : i >= B_A ? kRowWarps : 1);
         *abort_flag = 0;
         fence_barrier_init();
     }
@@ -1071,6 +1102,9 @@ __global__ void __launch_bounds__(640, 1) encoder_ws_kernel(const Params p) {
         }
     } else if (warp == kProducerWarp) {
         producer<kAr>(smem, abort_flag, p, n_tiles);
+    } else if (warp >= kExpandWarp) {
+        if (p.prior != nullptr)
+            expander(smem, sm, smem + Map<kAr>::SM_H, abort_flag, p, tiles, n_tiles, warp - kExpandWarp, lane);
     } else {
         Issue st = {smem, tmem, abort_flag, 0, 0, 0};
         for (int k = 0; k < n_tiles; ++k) {

@@ -62,6 +62,8 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity)
 // the kernel with an error status instead of a hang.  Returns false on time-out.
 //
 constexpr unsigned kWaitCycles = 400000000u;     // ~0.2 s at 2 GHz
+// `kSleep`: nanoseconds between tries, for a warp that waits long beside others that work.
+template <unsigned kSleep = 0>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity,
                                           volatile int* abort_flag, int code) {
     if (mbar_try_wait(bar, parity)) return true;
@@ -70,6 +72,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity,
     asm volatile("mov.u32 %0, %%clock;" : "=r"(t0) :: "memory");
 #pragma unroll 1
     while (!mbar_try_wait(bar, parity)) {
+        if (kSleep != 0) __nanosleep(kSleep);
         int aborted;
         asm volatile("ld.volatile.shared.b32 %0, [%1];" : "=r"(aborted) : "r"(flag) : "memory");
         if (aborted != 0) return false;
