@@ -2329,6 +2329,18 @@ bool small_tiles(int quant, int n, int sm_count) {
     return small <= four;
 }
 
+using Kernel = void (*)(bf::Params);
+template <bool kExpand>
+Kernel small_tile_kernel(int quant) {
+    return quant == 0   ? bf::ws::encoder_ws_kernel<bf::kArF16, kExpand>
+           : quant == 1 ? bf::ws::encoder_ws_kernel<bf::kArE4M3, kExpand>
+           : quant == 2 ? bf::ws::encoder_ws_kernel<bf::kArI8Ffn, kExpand>
+           : quant == 4 ? bf::ws::encoder_ws_kernel<bf::kArI8Qkv, kExpand>
+                        : bf::ws::encoder_ws_kernel<bf::kArInt8, kExpand>;
+}
+// (the expansion has warps of its own: plain evaluations run without them, 1.5 % faster)
+Kernel small_tile_kernel(int quant, bool expand) { return expand ? small_tile_kernel<true>(quant) : small_tile_kernel<false>(quant); }
+
 int launch(bf_handle* h, const uint16_t* boards, const int16_t* control, const uint8_t* rep,
            const uint64_t* legal, int n, void* policy, void* promo, float* value, void* y, int stage,
            int stage_layer, int cap_layer, int cap_op, uint8_t* cap_a, int32_t* cap_acc, cudaStream_t stream,
@@ -2371,10 +2383,8 @@ int launch(bf_handle* h, const uint16_t* boards, const int16_t* control, const u
     if (!dbg && p.rj_mode == 0 && small_tiles(p.quant, n, h->sm_count)) {
         p.one_most = h->one_board_factor;
         const int ctas = n < h->sm_count ? n : h->sm_count;
-        const auto kernel = p.quant == 0 ? bf::ws::encoder_ws_kernel<bf::kArF16> : p.quant == 1 ? bf::ws::encoder_ws_kernel<bf::kArE4M3>
-                          : p.quant == 2 ? bf::ws::encoder_ws_kernel<bf::kArI8Ffn> : p.quant == 4 ? bf::ws::encoder_ws_kernel<bf::kArI8Qkv>
-                                                                                                : bf::ws::encoder_ws_kernel<bf::kArInt8>;
-        kernel<<<ctas, bf::ws::kThreads, bf::ws::kSmemRequest, stream>>>(p);
+        const bool expand = p.prior != nullptr;
+        small_tile_kernel(p.quant, expand)<<<ctas, bf::ws::threads(expand), bf::ws::kSmemRequest, stream>>>(p);
     } else {
         // four-board tiles: large batches of the fp16 arithmetic, re-injection, and the instrumented arms
         // (dumps, captures, the phase clock, the backbone entry)
@@ -2462,12 +2472,10 @@ int bf_create(const void* blob, size_t blob_bytes, int device, bf_handle** out) 
                           reinterpret_cast<const void*>(&bf::encoder_kernel<false, true, bf::kArInt8>),
                           reinterpret_cast<const void*>(&bf::encoder_kernel<true, true, bf::kArInt8>)})
         if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bf::kSmemRequest);
-    for (const void* k : {reinterpret_cast<const void*>(&bf::ws::encoder_ws_kernel<bf::kArInt8>),
-                          reinterpret_cast<const void*>(&bf::ws::encoder_ws_kernel<bf::kArI8Ffn>),
-                          reinterpret_cast<const void*>(&bf::ws::encoder_ws_kernel<bf::kArI8Qkv>),
-                          reinterpret_cast<const void*>(&bf::ws::encoder_ws_kernel<bf::kArE4M3>),
-                          reinterpret_cast<const void*>(&bf::ws::encoder_ws_kernel<bf::kArF16>)})
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bf::ws::kSmemRequest);
+    for (int expand = 0; expand < 2; ++expand)
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(reinterpret_cast<const void*>(small_tile_kernel(static_cast<int>(hdr.quant), expand != 0)),
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, bf::ws::kSmemRequest);
     if (e != cudaSuccess) {
         bf_destroy(h);
         return fail(BF_ECUDA, std::string("bf_create: ") + cudaGetErrorString(e));
@@ -3154,7 +3162,7 @@ int noalloc_setup(int device, NoAllocDevice** out) {
         void* ptr = nullptr;
         BF_CUDA(cudaGetSymbolAddress(&ptr, bf::g_noalloc_scratch));
         BF_CUDA(cudaMemset(ptr, 0, bf::kNoAllocScratchBytes));
-        BF_CUDA(cudaFuncSetAttribute(bf::ws::encoder_ws_kernel<bf::kArInt8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        BF_CUDA(cudaFuncSetAttribute(bf::ws::encoder_ws_kernel<bf::kArInt8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      bf::ws::kSmemRequest));
         d.scratch = ptr;
         d.sm_count = prop.multiProcessorCount;
@@ -3243,8 +3251,8 @@ int bf_forward_noalloc(int device, const void* blob_dev, size_t blob_bytes, cons
     p.status = static_cast<int*>(scratch);         // the device address, not the symbol
     p.prof = nullptr;
     p.one_most = 1;
-    bf::ws::encoder_ws_kernel<bf::kArInt8><<<n < sm_count ? n : sm_count, bf::ws::kThreads, bf::ws::kSmemRequest,
-                                             static_cast<cudaStream_t>(stream)>>>(p);
+    bf::ws::encoder_ws_kernel<bf::kArInt8, false><<<n < sm_count ? n : sm_count, bf::ws::threads(false), bf::ws::kSmemRequest,
+                                                    static_cast<cudaStream_t>(stream)>>>(p);
     BF_CUDA(cudaGetLastError());
     return BF_OK;
 }

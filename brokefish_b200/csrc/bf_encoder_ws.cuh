@@ -33,7 +33,8 @@
 namespace bf {
 namespace ws {
 
-constexpr int kProducerWarp = 16, kMmaWarp = 17, kExpandWarp = 18, kThreads = 640;
+constexpr int kProducerWarp = 16, kMmaWarp = 17, kExpandWarp = 18;
+constexpr int threads(bool expand) { return expand ? 640 : 576; }
 constexpr uint32_t kStage = 32768;                 // one 128-byte K-slab of 256 weight rows
 // ---- shared memory map ------------------------------------------------------------------
 // A operand: K-slabs of [rows][128 B], two of bytes or (where QKV or the out-projection runs in fp16)
@@ -705,7 +706,7 @@ __device__ __forceinline__ void prenorm_logits(const Row& c, const Params& p, ui
 // Final norm into the head product's fp16 operand, then the epilogue: the product's 128 output columns
 // (64 policy, 4 promotion, value, padding) lie 8 NB to a thread.  Policy columns are masked and stored
 // by the threads that hold them; with a fused expansion the logits are staged for the expansion warps.
-template <int NB, int kAr>
+template <int NB, int kAr, bool kExpand>
 __device__ __forceinline__ void heads(const Row& c, const Params& p, int board, bool valid, int ctl, uint32_t alive,
                                       const uint32_t (&x)[8 * NB]) {
     using O = Own<NB>;
@@ -745,7 +746,7 @@ __device__ __forceinline__ void heads(const Row& c, const Params& p, int board, 
 #pragma unroll
         for (int i = 0; i < 4 * NB; ++i) v[i] = __byte_perm(acc[2 * i], acc[2 * i + 1], 0x5410);
     }
-    if (p.prior != nullptr) {
+    if constexpr (kExpand) {
         if (hc < 64) {
 #pragma unroll
             for (int k = 0; k < NB; ++k)
@@ -833,7 +834,7 @@ __device__ __forceinline__ void expander(uint32_t smem, uint8_t* smem_gen, uint3
 }
 
 // One tile of NB boards, from the piece words to the outputs.
-template <int NB, int kAr>
+template <int NB, int kAr, bool kExpand>
 __device__ __forceinline__ void row_tile(Row& c, const Params& p, int first) {
     using O = Own<NB>;
     const int item = first + O::board(c), lane = c.lane, col = O::col(c);
@@ -888,7 +889,7 @@ __device__ __forceinline__ void row_tile(Row& c, const Params& p, int first) {
         if ((half & 1) == 0) {
             attention_block<NB, kAr>(c, lp, sa, alive, x);
         } else {
-            if (half == 1 && p.prior != nullptr && c.tiles != 0) {
+            if (kExpand && half == 1 && c.tiles != 0) {
                 mbar_wait(bar(c.smem, B_EXPANDED), (c.tiles - 1u) & 1u, c.abort_flag, kErrRowAcc);
                 __syncwarp();
             }
@@ -898,7 +899,7 @@ __device__ __forceinline__ void row_tile(Row& c, const Params& p, int first) {
         }
     }
     if (id < static_cast<int>(kTailBytes / 128)) prefetch_l1(reinterpret_cast<const uint8_t*>(p.tail) + 128 * id);
-    heads<NB, kAr>(c, p, board, valid, ctl, alive, x);
+    heads<NB, kAr, kExpand>(c, p, board, valid, ctl, alive, x);
     c.tiles++;
 }
 
@@ -1060,7 +1061,7 @@ __device__ __forceinline__ void issue_tile(Issue& st, int n_layers) {
 }
 
 // launch bounds: 640 threads, so that a scheduler's five warps fit its registers (96 each)
-template <int kAr>
+template <int kAr, bool kExpand>
 __global__ void __launch_bounds__(640, 1) encoder_ws_kernel(const Params p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -1097,13 +1098,13 @@ __global__ void __launch_bounds__(640, 1) encoder_ws_kernel(const Params p) {
         for (int k = 0; k < n_tiles; ++k) {
             int first, boards;
             tiles.at(k, first, boards);
-            if (boards == 1) row_tile<1, kAr>(c, p, first);
-            else             row_tile<2, kAr>(c, p, first);
+            if (boards == 1) row_tile<1, kAr, kExpand>(c, p, first);
+            else             row_tile<2, kAr, kExpand>(c, p, first);
         }
     } else if (warp == kProducerWarp) {
         producer<kAr>(smem, abort_flag, p, n_tiles);
     } else if (warp >= kExpandWarp) {
-        if (p.prior != nullptr)
+        if constexpr (kExpand)
             expander(smem, sm, smem + Map<kAr>::SM_H, abort_flag, p, tiles, n_tiles, warp - kExpandWarp, lane);
     } else {
         Issue st = {smem, tmem, abort_flag, 0, 0, 0};
