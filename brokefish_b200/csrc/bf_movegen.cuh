@@ -324,161 +324,156 @@ __device__ __forceinline__ unsigned long long anti_ex(int sq) {
     return (d >= 0 ? 0x0102040810204080ull << (8 * d) : 0x0102040810204080ull >> (-8 * d)) ^ (1ull << sq);
 }
 
-// Squares one piece `b` (a single bit) sees along the bishop or the rook lines.
-__device__ __forceinline__ unsigned long long piece_diag(unsigned long long b, unsigned long long occ) {
-    const int sq = __ffsll(static_cast<long long>(b)) - 1;
-    return line_attacks(b, occ, diag_ex(sq)) | line_attacks(b, occ, anti_ex(sq));
-}
-__device__ __forceinline__ unsigned long long piece_line(unsigned long long b, unsigned long long occ) {
-    const int sq = __ffsll(static_cast<long long>(b)) - 1;
-    return line_attacks(b, occ, rank_ex(sq)) | line_attacks(b, occ, file_ex(sq));
-}
 
 constexpr int kTpbThreads = 128;
 constexpr int kTpbInStride = 17;      // 32-bit words per board in shared memory (16 + 1: no bank conflicts)
 constexpr int kTpbOutStride = 33;     // 64-bit words per board in shared memory (32 + 1)
 constexpr int kTpbSmem = kTpbThreads * (kTpbInStride * 4 + kTpbOutStride * 8);
 
-// The legal words of one board held by one thread: `my` = the board's 32 piece words as 16
-// 32-bit words, `out[0..31]` receives the legal-target word of every slot.  Returns whether the
-// side to move is in check.
 __device__ __forceinline__ unsigned piece_word(const unsigned* my, int p) {
     return (my[p >> 1] >> (16 * (p & 1))) & 0xFFFFu;
 }
+// x << s of a 64-bit word with a single bit at 0, 0 for s >= 64 (32-bit shifts clamp).
+__device__ __forceinline__ unsigned long long bit_at(unsigned s) {
+    unsigned lo, hi;
+    asm("shl.b32 %0, 1, %1;" : "=r"(lo) : "r"(s));
+    asm("shl.b32 %0, 1, %1;" : "=r"(hi) : "r"(s - 32u));
+    return (static_cast<unsigned long long>(hi) << 32) | lo;
+}
+// The legal words of one board held by one thread: `my` = the board's 32 piece words as 16
+// 32-bit words, `out[0..31]` receives the legal-target word of every slot.  Returns whether the
+// side to move is in check.
+//
+// Bound by the integer pipe.  A board with black to move is turned upside down as it is decoded (and its
+// words on the way out), so that nothing below depends on the side to move; the bitboards are bit planes
+// of the words, without a branch per piece; checks and pins are taken ray by ray from the king without
+// loops.  2^20 boards of random games, B200: FIXME us against 252 with a branch per piece and loops over
+// the pinning pieces.
 __device__ __forceinline__ bool board_moves(const unsigned* my, bool black, unsigned long long* out) {
-    // ---- pass 1: bitboards ----
-    unsigned long long occ = 0, own = 0, e_pawns = 0, e_knights = 0, e_diag = 0, e_line = 0, e_king = 0;
-    unsigned long long ep_pawns = 0, fresh_rooks = 0, my_king = 0;
-    bool by_slot = true;                 // white in slots 0-15, black in 16-31, as the engine keeps them
-#pragma unroll 1
-    for (int p = 0; p < 32; ++p) {
-        const unsigned word = piece_word(my, p);
-        out[p] = 0ull;
-        if ((word >> 11) & 1u) continue;
-        const bool is_black = (word >> 10) & 1u, special = (word >> 9) & 1u;
-        by_slot &= is_black == (p >= 16);
-        const int type = (word >> 6) & 7;
-        const unsigned long long bb = 1ull << (word & 63u);
-        occ |= bb;
-        if (is_black == black) {
-            own |= bb;
-            if (type == KING) my_king |= bb;
-            if (type == ROOK && !special) fresh_rooks |= bb;
-        } else {
-            if (type == PAWN) { e_pawns |= bb; if (special) ep_pawns |= bb; }
-            else if (type == KNIGHT) e_knights |= bb;
-            else if (type == KING) e_king |= bb;
-            else {
-                if (type == BISHOP || type == QUEEN) e_diag |= bb;
-                if (type == ROOK || type == QUEEN) e_line |= bb;
+    // ---- pass 1: bit planes.  A captured piece's square is moved off the board ----
+    const unsigned flip = black ? 0x00380038u : 0u;
+    unsigned long long half[2] = {0ull, 0ull}, t0 = 0, t1 = 0, t2 = 0, sp = 0;
+    unsigned stray = 0u;                 // a live piece whose colour is not its slot's (white 0-15, black 16-31)
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll 4
+        for (int q = 0; q < 8; ++q) {
+            const unsigned two = my[8 * h + q] ^ flip;
+            stray |= (two ^ (h ? 0x04000400u : 0u)) & ~(two >> 1);
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const unsigned w = k ? two >> 16 : two;
+                const unsigned long long bb = bit_at((w & 63u) | ((w >> 5) & 64u));
+                half[h] |= bb;
+                t0 |= (w & 0x040u) ? bb : 0ull;
+                t1 |= (w & 0x080u) ? bb : 0ull;
+                t2 |= (w & 0x100u) ? bb : 0ull;
+                sp |= (w & 0x200u) ? bb : 0ull;
             }
         }
+    const bool by_slot = (stray & 0x04000400u) == 0u;
+    const unsigned long long occ = half[0] | half[1];
+    unsigned long long own = black ? half[1] : half[0];
+    if (!by_slot) {
+        own = 0ull;
+#pragma unroll 1
+        for (int p = 0; p < 32; ++p) {
+            const unsigned w = piece_word(my, p) ^ (flip & 63u);
+            if (((w & 0x400u) != 0u) == black) own |= bit_at((w & 63u) | ((w >> 5) & 64u));
+        }
     }
-    const unsigned long long opp = occ & ~own;
+    const unsigned long long opp = occ & ~own, queens = t2 & ~(t1 | t0), pawns = occ & ~(t0 | t1 | t2);
+    const unsigned long long kings = t2 & t0 & ~t1, rooks = t1 & t0 & ~t2;
+    const unsigned long long e_pawns = opp & pawns, ep_pawns = e_pawns & sp, e_knights = opp & t0 & ~(t1 | t2);
+    const unsigned long long e_diag = opp & ((t1 & ~(t0 | t2)) | queens), e_line = opp & (rooks | queens);
+    const unsigned long long e_king = opp & kings, my_king = own & kings, fresh_rooks = own & rooks & ~sp;
     const int king_sq = my_king ? __ffsll(static_cast<long long>(my_king)) - 1 : 0;
     // ---- what the opponent attacks, with the mover's king lifted off the board ----
     const unsigned long long occ_nk = occ & ~my_king;
-    const unsigned long long danger = pawn_attacks(e_pawns, !black) | knight_pattern(e_knights) |
+    const unsigned long long danger = pawn_attacks(e_pawns, true) | knight_pattern(e_knights) |
                                       king_pattern(e_king) | fill_diag(e_diag, occ_nk) | fill_line(e_line, occ_nk);
-    // ---- checkers and the squares that answer a single check ----
+    // ---- the eight rays from the king: is the first piece a checker (the squares up to it answer the
+    //      check), or an own piece with a slider of the ray's kind next behind it ----
     const unsigned long long kd_ex = diag_ex(king_sq), ka_ex = anti_ex(king_sq), kr_ex = rank_ex(king_sq),
                              kf_ex = file_ex(king_sq);
-    const unsigned long long k_diag = line_attacks(my_king, occ, kd_ex) | line_attacks(my_king, occ, ka_ex);
-    const unsigned long long k_line = line_attacks(my_king, occ, kr_ex) | line_attacks(my_king, occ, kf_ex);
-    const unsigned long long checkers = (knight_pattern(my_king) & e_knights) | (pawn_attacks(my_king, black) & e_pawns) |
-                                        (k_diag & e_diag) | (k_line & e_line);
-    const bool chk = checkers != 0ull;
-    unsigned long long target_mask = ~0ull;
-    if (chk) {
-        if (checkers & (checkers - 1ull)) target_mask = 0ull;               // two checkers: only the king moves
-        else {
-            unsigned long long between = 0ull;
-            if (checkers & k_diag & e_diag) between = k_diag & piece_diag(checkers, occ);
-            else if (checkers & k_line & e_line) between = k_line & piece_line(checkers, occ);
-            target_mask = checkers | between;
-        }
-    }
-    // ---- pieces that shield the king from a slider: the first own piece on a ray from the
-    //      king, with an enemy slider of that ray's kind next behind it ----
-    unsigned long long pinned = 0ull;
-    if (my_king != 0ull) {
-        const unsigned long long shields = (k_diag | k_line) & own;
-        const unsigned long long occ2 = occ & ~shields;
-        const unsigned long long k_diag2 = line_attacks(my_king, occ2, kd_ex) | line_attacks(my_king, occ2, ka_ex);
-        const unsigned long long k_line2 = line_attacks(my_king, occ2, kr_ex) | line_attacks(my_king, occ2, kf_ex);
-        for (unsigned long long pin = (k_diag2 & ~k_diag) & e_diag; pin != 0ull; pin &= pin - 1ull)
-            pinned |= k_diag2 & piece_diag(pin & (0ull - pin), occ2) & shields;
-        for (unsigned long long pin = (k_line2 & ~k_line) & e_line; pin != 0ull; pin &= pin - 1ull)
-            pinned |= k_line2 & piece_line(pin & (0ull - pin), occ2) & shields;
-    }
+    const unsigned long long above = 0ull - (my_king << 1);          // squares above the king's
+    const unsigned long long leapers = (knight_pattern(my_king) & e_knights) | (pawn_attacks(my_king, false) & e_pawns);
+    unsigned long long answers = leapers, pinned = 0ull;
+    int checkers = __popcll(leapers);
+    auto line = [&](unsigned long long ex, unsigned long long sliders) {
+        const unsigned long long seen = line_attacks(my_king, occ, ex), shields = seen & own;
+        const unsigned long long next = line_attacks(my_king, occ & ~shields, ex) & ~seen & sliders, hit = seen & sliders;
+        if (hit & above) { ++checkers; answers |= seen & above; }
+        if (hit & ~above) { ++checkers; answers |= seen & ~above; }
+        if (next & above) pinned |= shields & above;
+        if (next & ~above) pinned |= shields & ~above;
+    };
+    line(kd_ex, e_diag);
+    line(ka_ex, e_diag);
+    line(kr_ex, e_line);
+    line(kf_ex, e_line);
+    const bool chk = checkers != 0;
+    // one checker: the other pieces may only capture it or step between; two: only the king moves
+    const unsigned long long target_mask = checkers == 0 ? ~0ull : (checkers == 1 ? answers : 0ull);
     // ---- the mover's pieces, one by one: its sixteen slots (all thirty-two for a board that
     //      does not keep the colours apart by slot) ----
-    const int p_lo = by_slot ? (black ? 16 : 0) : 0, p_hi = by_slot ? p_lo + 16 : 32;
+    const int p_lo = by_slot ? (black ? 16 : 0) : 0, p_n = by_slot ? 16 : 32;
+    const unsigned sel_lo = black ? 0x4567u : 0x3210u, sel_hi = black ? 0x0123u : 0x7654u;
+    if (by_slot)
+#pragma unroll 4
+        for (int p = 0; p < 16; ++p) out[(p_lo ^ 16) + p] = 0ull;
 #pragma unroll 1
-    for (int p = p_lo; p < p_hi; ++p) {
-        const unsigned word = piece_word(my, p);
-        if (((word >> 11) & 1u) || (((word >> 10) & 1u) != 0u) != black) continue;
-        const bool special = (word >> 9) & 1u;
-        const int type = (word >> 6) & 7, sq = word & 63;
-        const int rank = sq >> 3, file = sq & 7;
-        const unsigned long long bb = 1ull << sq;
-        unsigned long long cand = 0ull, ep_target = 0ull;
-        if (type == KING) {
-            cand = king_pattern(bb) & ~danger;
-            if (!special && !chk) {
-                const int row = black ? 56 : 0;
-                if ((fresh_rooks >> (row + 7)) & 1ull)
-                    if (((occ >> (row + 5)) & 3ull) == 0ull && ((danger >> (row + 5)) & 3ull) == 0ull)
-                        cand |= 1ull << (row + 6);
-                if ((fresh_rooks >> row) & 1ull)
-                    if (((occ >> (row + 1)) & 7ull) == 0ull && ((danger >> (row + 2)) & 3ull) == 0ull)
-                        cand |= 1ull << (row + 2);
-            }
-            out[p] = cand & ~own;
-            continue;
-        }
-        if (type == KNIGHT) {
-            cand = knight_pattern(bb);
-        } else if (type == PAWN) {
-            const int up = black ? -8 : 8;
-            const int f1 = sq + up;
-            if (f1 >= 0 && f1 < 64) {
-                if (!((occ >> f1) & 1ull)) {
-                    cand |= 1ull << f1;
-                    const bool start = black ? rank == 6 : rank == 1;
-                    if (start && !((occ >> (f1 + up)) & 1ull)) cand |= 1ull << (f1 + up);
+    for (int i = 0; i < p_n; ++i) {
+        const int p = p_lo + i;
+        const unsigned word = piece_word(my, p) ^ (flip & 63u);
+        unsigned long long legal = 0ull;
+        if ((word & 0x800u) == 0u && ((word & 0x400u) != 0u) == black) {
+            const bool special = (word & 0x200u) != 0u;
+            const int type = (word >> 6) & 7, sq = word & 63;
+            const unsigned long long bb = bit_at(sq);
+            if (type == KING) {
+                legal = king_pattern(bb) & ~danger;
+                // castling: neither the king's square nor the one it crosses nor the one it lands on may
+                // be attacked
+                if (!special && !chk) {
+                    if ((fresh_rooks & 0x80ull) && ((occ | danger) & 0x60ull) == 0ull) legal |= 0x40ull;
+                    if ((fresh_rooks & 0x01ull) && (occ & 0x0Eull) == 0ull && (danger & 0x0Cull) == 0ull) legal |= 0x04ull;
                 }
-                if (file > 0) cand |= (1ull << (f1 - 1)) & opp;
-                if (file < 7) cand |= (1ull << (f1 + 1)) & opp;
-                if (rank == (black ? 3 : 4)) {
-                    if (file > 0 && ((ep_pawns >> (sq - 1)) & 1ull)) ep_target |= 1ull << (f1 - 1);
-                    if (file < 7 && ((ep_pawns >> (sq + 1)) & 1ull)) ep_target |= 1ull << (f1 + 1);
+                legal &= ~own;
+            } else {
+                unsigned long long cand = 0ull, ep = 0ull;
+                if (type == PAWN) {
+                    const unsigned long long one = (bb << 8) & ~occ, att = pawn_attacks(bb, false);
+                    const unsigned long long two = (sq >> 3) == 1 ? (one << 8) & ~occ : 0ull;
+                    cand = one | two | (att & opp);
+                    // en passant: an enemy pawn that has just made its double step stands beside us
+                    if ((sq >> 3) == 4) ep = att & (ep_pawns << 8) & ~own;
+                } else if (type == KNIGHT) {
+                    cand = knight_pattern(bb);
+                } else {
+                    if (type == BISHOP || type == QUEEN)
+                        cand |= line_attacks(bb, occ, diag_ex(sq)) | line_attacks(bb, occ, anti_ex(sq));
+                    if (type == ROOK || type == QUEEN)
+                        cand |= line_attacks(bb, occ, rank_ex(sq)) | line_attacks(bb, occ, file_ex(sq));
+                }
+                legal = cand & ~own & target_mask;
+                // a piece that shields the king from a slider moves only along that line
+                if (bb & pinned) legal &= (bb & kd_ex) ? kd_ex : (bb & ka_ex) ? ka_ex : (bb & kr_ex) ? kr_ex : kf_ex;
+                // en passant takes two pieces off one rank at once: tested on the position after it
+                for (; ep != 0ull; ep &= ep - 1ull) {
+                    const unsigned long long tb = ep & (0ull - ep), gone = tb >> 8;
+                    const unsigned long long after = ((occ & ~bb) & ~gone) | tb;
+                    const bool hit = (knight_pattern(my_king) & e_knights) != 0ull ||
+                                     (pawn_attacks(my_king, false) & (e_pawns & ~gone)) != 0ull ||
+                                     (king_pattern(my_king) & e_king) != 0ull ||
+                                     ((line_attacks(my_king, after, kd_ex) | line_attacks(my_king, after, ka_ex)) & e_diag) != 0ull ||
+                                     ((line_attacks(my_king, after, kr_ex) | line_attacks(my_king, after, kf_ex)) & e_line) != 0ull;
+                    if (!hit) legal |= tb;
                 }
             }
-        } else {
-            if (type == BISHOP || type == QUEEN)
-                cand |= line_attacks(bb, occ, diag_ex(sq)) | line_attacks(bb, occ, anti_ex(sq));
-            if (type == ROOK || type == QUEEN)
-                cand |= line_attacks(bb, occ, rank_ex(sq)) | line_attacks(bb, occ, file_ex(sq));
         }
-        cand &= ~own;
-        ep_target &= ~own;
-        if (my_king == 0ull) { out[p] = cand | ep_target; continue; }       // no king to protect
-        unsigned long long legal = cand & target_mask;
-        if (bb & pinned) legal &= line_through(king_sq, sq);
-        // en passant takes two pieces off one rank at once: tested on the position after it
-        for (unsigned long long rest = ep_target; rest != 0ull; rest &= rest - 1ull) {
-            const unsigned long long tb = rest & (0ull - rest);
-            const unsigned long long gone = black ? tb << 8 : tb >> 8;
-            const unsigned long long after = ((occ & ~bb) & ~gone) | tb;
-            const bool hit = (knight_pattern(my_king) & e_knights) != 0ull ||
-                             (pawn_attacks(my_king, black) & (e_pawns & ~gone)) != 0ull ||
-                             (king_pattern(my_king) & e_king) != 0ull ||
-                             ((line_attacks(my_king, after, kd_ex) | line_attacks(my_king, after, ka_ex)) & e_diag) != 0ull ||
-                             ((line_attacks(my_king, after, kr_ex) | line_attacks(my_king, after, kf_ex)) & e_line) != 0ull;
-            if (!hit) legal |= tb;
-        }
-        out[p] = legal;
+        const unsigned lo = static_cast<unsigned>(legal), hi = static_cast<unsigned>(legal >> 32);
+        out[p] = (static_cast<unsigned long long>(__byte_perm(lo, hi, sel_hi)) << 32) | __byte_perm(lo, hi, sel_lo);
     }
     return chk;
 }
