@@ -2279,17 +2279,17 @@ int host_plan_sizes(int n, int wave, int plan, double gbps, int* sizes, bool* sl
 }
 
 // The engine kernels have two forms (bf_movegen.cuh).  Eight lanes per board: an eighth of the chain,
-// so a launch that does not fill the GPU ends sooner.  A thread per board: two thirds of the
-// instructions.  B200, us per launch, eight lanes / thread:
-//   boards                       1     4096    32768    65536   131072   1048576
-//   legal words             < 4.5/10  6.2/18   16/21    29/27    53/43    404/273
-//   move                    < 5.1/8   5.0/12   10/14    15/16    27/27    221/158
-//   move, words and key     < 5.7/23  8.2/39   29/42    51/53    98/92    762/614
-constexpr int kEngineGroupMostMoves = 49152, kEngineGroupMostStep = 98304;
+// so a launch that does not fill the GPU ends sooner.  A thread per board: half of the instructions.
+// B200, us per launch, eight lanes / thread:
+//   boards                       1     4096    16384    32768    49152    98304   131072   1048576
+//   legal words             4.2/7.7  6.2/10    10/10    16/12    23/14    41/23    51/27    385/160
+//   move                    4.8/8.2  4.6/12   6.2/12   8.2/12    10/14    18/23    23/25    168/148
+//   move, words and key     6.2/18   8.2/29    16/29    27/33    37/37    70/66    90/72    688/482
+constexpr int kGroupMostWords = 16384, kGroupMostMove = 131072, kGroupMostBoth = 49152;
 template <bool kStep, bool kPick, class... Args>
-void launch_engine(cudaStream_t stream, const uint16_t* boards, const int16_t* control, const int* move,
+void launch_engine(cudaStream_t stream, bool words_or_key, const uint16_t* boards, const int16_t* control, const int* move,
                    const signed char* promo, const float* r, int n, Args... rest) {
-    if (n <= (kStep ? kEngineGroupMostStep : kEngineGroupMostMoves))
+    if (n <= (!kStep ? kGroupMostWords : words_or_key ? kGroupMostBoth : kGroupMostMove))
         bfmg::engine_group_kernel<kStep, kPick><<<(n + bfmg::kEngineBoards - 1) / bfmg::kEngineBoards,
                                                   bfmg::kEngineThreads, 0, stream>>>(boards, control, move, promo, r, n, rest...);
     else
@@ -2549,7 +2549,7 @@ int bf_movegen(int device, const uint16_t* boards, const int16_t* control, int n
     if (boards == nullptr || control == nullptr || mask == nullptr)
         return fail(BF_EINVAL, "boards, control and mask must be non-null");
     BF_ON_DEVICE(device);
-    launch_engine<false, false>(static_cast<cudaStream_t>(stream),
+    launch_engine<false, false>(static_cast<cudaStream_t>(stream), true,
         boards, control, nullptr, nullptr, nullptr, n, nullptr, nullptr, nullptr,
         reinterpret_cast<unsigned long long*>(mask), in_check, nullptr, nullptr);
     BF_CUDA(cudaGetLastError());
@@ -2562,7 +2562,7 @@ int bf_hash(int device, const uint16_t* boards, const int16_t* control, int n, u
     if (boards == nullptr || control == nullptr || hash == nullptr)
         return fail(BF_EINVAL, "boards, control and hash must be non-null");
     BF_ON_DEVICE(device);
-    launch_engine<false, false>(static_cast<cudaStream_t>(stream),
+    launch_engine<false, false>(static_cast<cudaStream_t>(stream), true,
         boards, control, nullptr, nullptr, nullptr, n, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
         reinterpret_cast<unsigned long long*>(hash));
     BF_CUDA(cudaGetLastError());
@@ -2627,7 +2627,7 @@ int bf_step(int device, const uint16_t* boards, const int16_t* control, const in
     if (boards == nullptr || control == nullptr || move == nullptr || boards_out == nullptr || control_out == nullptr)
         return fail(BF_EINVAL, "boards, control, move, boards_out and control_out must be non-null");
     BF_ON_DEVICE(device);
-    launch_engine<true, false>(static_cast<cudaStream_t>(stream),
+    launch_engine<true, false>(static_cast<cudaStream_t>(stream), mask != nullptr || hash != nullptr,
         boards, control, move, promo, nullptr, n, boards_out, control_out, irreversible,
         reinterpret_cast<unsigned long long*>(mask), in_check, nullptr, reinterpret_cast<unsigned long long*>(hash));
     BF_CUDA(cudaGetLastError());
@@ -2675,7 +2675,7 @@ int bf_random_ply(int device, uint16_t* boards, int16_t* control, uint64_t* mask
     if (boards == nullptr || control == nullptr || mask == nullptr || r == nullptr)
         return fail(BF_EINVAL, "boards, control, mask and r must be non-null");
     BF_ON_DEVICE(device);
-    launch_engine<true, true>(static_cast<cudaStream_t>(stream),
+    launch_engine<true, true>(static_cast<cudaStream_t>(stream), true,
         boards, control, nullptr, promo, r, n, boards, control, nullptr,
         reinterpret_cast<unsigned long long*>(mask), nullptr, move, nullptr);
     BF_CUDA(cudaGetLastError());
