@@ -23,11 +23,11 @@
 // The arithmetic is the four-board kernel's, bit for bit (the order of every sum included).
 //
 // Measured on one B200, int8, against the forms before it (four boards per tile; one board per tile
-// with its rows written four times into a 128-row operand): batch 1-148 94-97 us (167), 149-296 141 us
-// (281), 333 233 us (281), 4096 1.92 ms (1.95).  What bounds it: the element-wise work of the row warps,
-// four to a scheduler and all in the same phase; of a two-board tile's 35,000 cycles per layer 22,000
-// are that work at the rate the CUDA cores sustain on it, 6,000 waits for a product whose operand has
-// only just been written (of a one-board tile's 23,000: 11,000 and 5,000).
+// with its rows written four times into a 128-row operand), through the device-pointer call: batch 1
+// 90 us (176), 64 92 us (176), 149-296 127 us (281), 333 215 us (285), 4096 1.69 ms (1.98).  What bounds
+// it: the row warps, four to a scheduler and all in the same phase.  Issue slots are about half busy,
+// the tensor pipe a fifth; the rest is the latency of a phase's first loads and of the three products
+// per layer that start only when their operand has been written (about 1,100 cycles each).
 #pragma once
 
 namespace bf {

@@ -240,15 +240,12 @@ __device__ __forceinline__ unsigned long long legal_word(unsigned word, int cont
 }
 
 // ------------------------------------------------------------------------------------------
-// One THREAD per board: the stand-alone generator.  A board is 64 bytes; with a warp per board
-// every bitboard costs warp-wide reductions over 32 lanes that hold one piece each, and the
-// kernel is bound by instruction issue far below the memory roof.  A thread that keeps the whole
-// board needs no reductions at all: attacks of all the opponent's sliders come out of eight
-// loop-free fills over the set of them at once, checkers and shielding pieces out of the same
-// fills started at the king, and only the mover's own pieces are visited one by one.  Slot p has
-// the same piece type on almost every board (promotions aside), so the threads of a warp take
-// the same branch as they walk the slots.  Boards come in and legal words go out through shared
-// memory so that global accesses stay coalesced.
+// One THREAD per board: the stand-alone generator for launches that fill the GPU.  A board is 64
+// bytes; with a warp per board every bitboard costs warp-wide reductions over 32 lanes that hold
+// one piece each.  A thread that keeps the whole board needs none, and only the mover's own pieces
+// are visited one by one; slot p has the same piece type on almost every board (promotions aside),
+// so the threads of a warp take the same branch as they walk the slots.  Boards come in and legal
+// words go out through shared memory so that global accesses stay coalesced.
 // ------------------------------------------------------------------------------------------
 template <int kShift>
 __device__ __forceinline__ unsigned long long fill_ray(unsigned long long gen, unsigned long long occ,
