@@ -1489,7 +1489,10 @@ struct MmaState {
     uint32_t aready, a2n[2];  // operand-ready phases consumed
 };
 
-// One GEMM unit: `n_stages` K-slabs of 128 bytes, 4 MMAs each.
+// One GEMM unit: `n_stages` K-slabs of 128 bytes, 4 MMAs each.  Two stages at a time (every unit and
+// every run that is passed over has an even number of them): both in place, then one elected region,
+// because what surrounds a stage's MMAs -- a wait, the election, the descriptors -- is of the order of
+// their time on the tensor pipe.  fp16, B200: 592 positions 277.8 -> 273.0 us, 1000 551 -> 542.
 template <int kAr>
 __device__ __forceinline__ void mma_unit(uint32_t smem, volatile int* abort_flag, MmaState& st,
                                          uint32_t tmem_d, int slot, uint32_t a_base, bool qring,
@@ -1502,32 +1505,38 @@ __device__ __forceinline__ void mma_unit(uint32_t smem, volatile int* abort_flag
         mbar_wait(bar_addr(smem, B_ACC_EMPTY + slot), (st.accn[slot] - 1u) & 1u, abort_flag, kErrMmaAcc);
         tc_fence_after();
     }
-    for (int s = 0; s < n_stages; ++s) {
-        uint32_t w_empty, w_addr;
-        const bool seen = pre && s == 0;
-        if (qring) {
-            const uint32_t k = st.qc % C::kQSlots;
-            if (!seen) mbar_wait(bar_addr(smem, B_WQ_FULL + k), (st.qc / C::kQSlots) & 1u, abort_flag, kErrMmaWeights);
-            w_empty = bar_addr(smem, B_WQ_EMPTY + k); w_addr = smem + C::SM_RING + k * kQStage;
-            st.qc++;
-        } else {
-            const uint32_t k = st.rc % C::kRSlots;
-            if (!seen) mbar_wait(bar_addr(smem, B_WR_FULL + k), (st.rc / C::kRSlots) & 1u, abort_flag, kErrMmaWeights);
-            w_empty = bar_addr(smem, B_WR_EMPTY + k); w_addr = smem + C::SM_RING + k * kRStage;
-            st.rc++;
-        }
-        if (!seen) tc_fence_after();
-        if (elect_one()) {
-            const uint64_t ad = umma_desc_k128(a_base + s * 16384), bd = umma_desc_k128(w_addr);
+    for (int s = 0; s < n_stages; s += 2) {
+        uint32_t w_empty[2], w_addr[2];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const uint32_t accumulate = (s > 0 || k > 0) ? 1u : 0u;
-                if (kind == kKindF16)     umma_f16(tmem_d, ad + 2 * k, bd + 2 * k, idesc, accumulate);
-                else if (kind == kKindF8) umma_f8(tmem_d, ad + 2 * k, bd + 2 * k, idesc, accumulate);
-                else                      umma_i8(tmem_d, ad + 2 * k, bd + 2 * k, idesc, accumulate);
+        for (int e = 0; e < 2; ++e) {
+            const bool seen = pre && s + e == 0;
+            if (qring) {
+                const uint32_t k = st.qc % C::kQSlots;
+                if (!seen) mbar_wait(bar_addr(smem, B_WQ_FULL + k), (st.qc / C::kQSlots) & 1u, abort_flag, kErrMmaWeights);
+                w_empty[e] = bar_addr(smem, B_WQ_EMPTY + k); w_addr[e] = smem + C::SM_RING + k * kQStage;
+                st.qc++;
+            } else {
+                const uint32_t k = st.rc % C::kRSlots;
+                if (!seen) mbar_wait(bar_addr(smem, B_WR_FULL + k), (st.rc / C::kRSlots) & 1u, abort_flag, kErrMmaWeights);
+                w_empty[e] = bar_addr(smem, B_WR_EMPTY + k); w_addr[e] = smem + C::SM_RING + k * kRStage;
+                st.rc++;
             }
-            tc_commit(w_empty);
-            if (s == n_stages - 1) tc_commit(bar_addr(smem, B_ACC_FULL + slot));
+        }
+        tc_fence_after();
+        if (elect_one()) {
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const uint64_t ad = umma_desc_k128(a_base + (s + e) * 16384), bd = umma_desc_k128(w_addr[e]);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const uint32_t accumulate = (s > 0 || e > 0 || k > 0) ? 1u : 0u;
+                    if (kind == kKindF16)     umma_f16(tmem_d, ad + 2 * k, bd + 2 * k, idesc, accumulate);
+                    else if (kind == kKindF8) umma_f8(tmem_d, ad + 2 * k, bd + 2 * k, idesc, accumulate);
+                    else                      umma_i8(tmem_d, ad + 2 * k, bd + 2 * k, idesc, accumulate);
+                }
+                tc_commit(w_empty[e]);
+            }
+            if (s == n_stages - 2) tc_commit(bar_addr(smem, B_ACC_FULL + slot));
         }
     }
     st.accn[slot]++;
@@ -1567,11 +1576,17 @@ template <int kAr>
 __device__ __forceinline__ void mma_pass_over(uint32_t smem, volatile int* abort_flag, MmaState& st, int n_stages) {
     using C = Cfg<kAr>;
 #pragma unroll 1
-    for (int i = 0; i < n_stages; ++i) {
-        const uint32_t k = st.rc % C::kRSlots;
-        mbar_wait(bar_addr(smem, B_WR_FULL + k), (st.rc / C::kRSlots) & 1u, abort_flag, kErrMmaWeights);
-        if (elect_one()) mbar_arrive(bar_addr(smem, B_WR_EMPTY + k));
-        st.rc++;
+    for (int i = 0; i < n_stages; i += 2) {
+        uint32_t k[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e, ++st.rc) {
+            k[e] = st.rc % C::kRSlots;
+            mbar_wait(bar_addr(smem, B_WR_FULL + k[e]), (st.rc / C::kRSlots) & 1u, abort_flag, kErrMmaWeights);
+        }
+        if (elect_one()) {
+            mbar_arrive(bar_addr(smem, B_WR_EMPTY + k[0]));
+            mbar_arrive(bar_addr(smem, B_WR_EMPTY + k[1]));
+        }
     }
 }
 
@@ -1667,19 +1682,25 @@ __device__ __forceinline__ void mma_loop(uint32_t smem, uint32_t tmem, volatile 
                     for (int jh = 0; jh < 2; ++jh) {
                         const uint32_t dst = jh ? acc1 : tmem + TM_OY;
 #pragma unroll 1
-                        for (int sl = 0; sl < 4; ++sl) {
-                            const uint32_t k = st.rc % C::kRSlots;
-                            mbar_wait(bar_addr(smem, B_WR_FULL + k), (st.rc / C::kRSlots) & 1u, abort_flag, kErrMmaWeights);
-                            st.rc++;
+                        for (int sl = 0; sl < 4; sl += 2) {
+                            uint32_t k[2];
+#pragma unroll
+                            for (int e = 0; e < 2; ++e, ++st.rc) {
+                                k[e] = st.rc % C::kRSlots;
+                                mbar_wait(bar_addr(smem, B_WR_FULL + k[e]), (st.rc / C::kRSlots) & 1u, abort_flag, kErrMmaWeights);
+                            }
                             tc_fence_after();
                             if (elect_one()) {
-                                const uint64_t ad = umma_desc_k128(sm_r + sl * 16384);
-                                const uint64_t bd = umma_desc_k128(smem + C::SM_RING + k * kRStage);
 #pragma unroll
-                                for (int kk = 0; kk < 4; ++kk)
-                                    umma_f16(dst, ad + 2 * kk, bd + 2 * kk, kI_FF2, (ch > 0 || sl > 0 || kk > 0) ? 1u : 0u);
-                                tc_commit(bar_addr(smem, B_WR_EMPTY + k));
-                                if (jh == 1 && sl == 3) tc_commit(bar_addr(smem, B_ACC_FULL + 1));
+                                for (int e = 0; e < 2; ++e) {
+                                    const uint64_t ad = umma_desc_k128(sm_r + (sl + e) * 16384);
+                                    const uint64_t bd = umma_desc_k128(smem + C::SM_RING + k[e] * kRStage);
+#pragma unroll
+                                    for (int kk = 0; kk < 4; ++kk)
+                                        umma_f16(dst, ad + 2 * kk, bd + 2 * kk, kI_FF2, (ch > 0 || sl > 0 || e > 0 || kk > 0) ? 1u : 0u);
+                                    tc_commit(bar_addr(smem, B_WR_EMPTY + k[e]));
+                                }
+                                if (jh == 1 && sl == 2) tc_commit(bar_addr(smem, B_ACC_FULL + 1));
                             }
                         }
                     }
@@ -2316,13 +2337,13 @@ struct LeafList {
 // A tile takes the same time whatever the batch, so the tiles of the busiest SM decide.  Measured, us
 // per one-, two- and four-board tile of an SM (B200):
 //   int8 90 / 126    int8 FFN+QKV 96 / 128    int8 FFN 103 / 133 / 273
-//   e4m3 100 / 130 / 270    fp16 129 / 152 / 275
+//   e4m3 100 / 130 / 270    fp16 129 / 152 / 272
 // Two two-board tiles beat a four-board one everywhere but in fp16, whose products, 32 bytes of K at
 // half the rate and twice the weight bytes, keep the weight stream and the tensor pipe busy for half
 // of a two-board tile's time; there the four-board form takes the batches that fill it.
 bool small_tiles(int quant, int n, int sm_count) {
     if (quant != 0) return true;
-    static const int t[3] = {129, 152, 275};
+    static const int t[3] = {129, 152, 272};
     const long full = n / (2 * sm_count), rest = n - full * 2 * sm_count;
     const long small = full * t[1] + (rest == 0 ? 0 : rest <= sm_count ? t[0] : t[1]);
     const long four = static_cast<long>((n + 4L * sm_count - 1) / (4L * sm_count)) * t[2];
