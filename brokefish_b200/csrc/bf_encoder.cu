@@ -2234,13 +2234,15 @@ void* mapped_host(const void* p) {
     return a.type == cudaMemoryTypeHost ? a.devicePointer : nullptr;
 }
 
-// A host call on a small batch whose buffers are all pinned and device-mapped runs as one launch on
+// A host call on a small batch whose buffers are all pinned, device-mapped and aligned runs as one launch on
 // them: no copies, one synchronisation.  B200, us through the Python API, copied / in place:
 //   logits, positions    1: 117/102   16: 118/109   64: 125/124   148: 141/152   296: 194/237
 //   edge lists           1: 112/104   148: 135/121   296: 172/156   592: 305/283
 // Logits are 4.3 KB a position and leave all at once at the end of a tile.
 constexpr int kDirectLogits = 64;        // positions
 constexpr int kDirectEdges = 4;          // positions per SM
+// (a host buffer may start anywhere: one that the kernels' loads and stores cannot use goes through the
+// copies, as one that is not mapped does)
 struct MappedInputs {
     const uint16_t* boards;
     const int16_t* control;
@@ -2250,7 +2252,8 @@ struct MappedInputs {
     MappedInputs(const void* b, const void* c, const void* r, const void* l)
         : boards(static_cast<const uint16_t*>(mapped_host(b))), control(static_cast<const int16_t*>(mapped_host(c))),
           rep(static_cast<const uint8_t*>(mapped_host(r))), legal(static_cast<const uint64_t*>(mapped_host(l))),
-          ok(boards != nullptr && control != nullptr && rep != nullptr && (legal != nullptr) == (l != nullptr)) {}
+          ok(boards != nullptr && control != nullptr && rep != nullptr && (legal != nullptr) == (l != nullptr) &&
+             bf_host_aligned(b, c, l, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr) != 0) {}
 };
 // Whether large batches of this handle run on two-board tiles (a wave is two positions per SM) or on
 // four-board ones.
@@ -2759,9 +2762,9 @@ int bf_forward_host(bf_handle* h, const uint16_t* boards, const int16_t* control
     void* m_policy = mapped_host(policy);
     void* m_promo = mapped_host(promo);
     void* m_value = mapped_host(value);
-    const bool all_mapped = policy != nullptr && promo != nullptr && value != nullptr &&
-                            m_policy != nullptr && m_promo != nullptr && m_value != nullptr;
-    if (n <= kDirectLogits && all_mapped) {
+    const bool in_place = m_policy != nullptr && m_promo != nullptr && m_value != nullptr &&
+                          bf_host_aligned(nullptr, nullptr, nullptr, policy, promo, value, nullptr, nullptr, nullptr) != 0;
+    if (n <= kDirectLogits && in_place) {
         const MappedInputs in(boards, control, rep, legal);
         if (in.ok) {
             const int rc = launch(h, in.boards, in.control, in.rep, in.legal, n, m_policy, m_promo, static_cast<float*>(m_value),
@@ -2798,8 +2801,8 @@ int bf_forward_host(bf_handle* h, const uint16_t* boards, const int16_t* control
     //               keep the kernel's tile-to-tile pipelining.
     //   r < 1.5     equal launches of about two waves, so that every copy hides behind the next
     //               launch as long as copying is not slower than evaluating, and the last wave
-    //               writes its logits straight into the caller's buffers when these are pinned
-    //               and device-mapped: the link is the bottleneck then, and stores that cross it
+    //               writes its logits straight into the caller's buffers when these are pinned,
+    //               device-mapped and aligned for it: the link is the bottleneck then, and stores that cross it
     //               while the wave computes beat a copy that starts when the wave has ended.
     // (Everything through mapped memory was measured 10 % slower on a fast link -- the stores back
     // up behind the bus -- and the last wave alone 4 % slower than copying it.)
@@ -2820,7 +2823,7 @@ int bf_forward_host(bf_handle* h, const uint16_t* boards, const int16_t* control
     int sizes[16];
     bool slow_link = false;
     const int n_chunks = host_plan_sizes(n, wave, h->host_plan, h->d2h_gbps / (two ? kSmallTileRate : 1.0), sizes, &slow_link);
-    const bool direct_last = slow_link && all_mapped;
+    const bool direct_last = slow_link && in_place;
     int lo = 0, k_timed = 0;
     for (int k = 1; k < n_chunks; ++k)
         if (sizes[k] > sizes[k_timed]) k_timed = k;
@@ -2873,7 +2876,8 @@ int bf_forward_priors_host(bf_handle* h, const uint16_t* boards, const int16_t* 
     void* m_move = mapped_host(move);
     void* m_ne = mapped_host(nedges);
     void* m_value = mapped_host(value);
-    if (n <= h->sm_count * kDirectEdges && m_prior && m_move && m_ne && (value == nullptr || m_value)) {
+    if (n <= h->sm_count * kDirectEdges && m_prior && m_move && m_ne && (value == nullptr || m_value) &&
+        bf_host_aligned(nullptr, nullptr, nullptr, nullptr, nullptr, value, prior, move, nedges)) {
         const MappedInputs in(boards, control, rep, legal);
         if (in.ok) {
             const PriorOut po{m_prior, static_cast<int16_t*>(m_move), static_cast<int*>(m_ne), e_cap};
@@ -2956,6 +2960,14 @@ int bf_status(bf_handle* h, int* status) {
 long long bf_launch_count(const bf_handle* h) { return h ? h->launches : 0; }
 
 double bf_host_link_gbps(const bf_handle* h) { return h ? h->d2h_gbps : 0.0; }
+
+int bf_host_aligned(const void* boards, const void* control, const void* legal, const void* policy, const void* promo,
+                    const void* value, const void* prior, const void* move, const void* nedges) {
+    const auto at = [](const void* p, uintptr_t bytes) { return reinterpret_cast<uintptr_t>(p) % bytes == 0; };
+    // (the expansion writes its lists in 16-byte pieces only where they are aligned for it)
+    return at(boards, 2) && at(control, 2) && at(legal, 8) && at(policy, 16) && at(promo, 8) && at(value, 4) &&
+           at(prior, 2) && at(move, 2) && at(nedges, 4);
+}
 
 int bf_host_plan(int n, int sm_count, int plan, double gbps, int* sizes) {
     if (n < 1 || sm_count < 1 || plan < 0 || plan > 2 || sizes == nullptr)

@@ -231,7 +231,8 @@ int bf_forward_capture(bf_handle* h, const uint16_t* boards, const int16_t* cont
  * device, runs the evaluator as a few launches of shrinking size (the last one a single wave of
  * tiles), copies each launch's three outputs back on a second stream while the next launch
  * computes -- only the last wave's copy is exposed -- and synchronises.  A small batch in pinned,
- * device-mapped buffers runs as one launch that reads and writes them in place.
+ * device-mapped and aligned buffers (bf_host_aligned) runs as one launch that reads and writes them
+ * in place; the buffers may start anywhere otherwise.
  * Device staging buffers are owned by the handle and grow to the largest `n` seen. */
 int bf_forward_host(bf_handle* h, const uint16_t* boards, const int16_t* control,
                     const uint8_t* rep, const uint64_t* legal, int n, void* policy,
@@ -239,7 +240,7 @@ int bf_forward_host(bf_handle* h, const uint16_t* boards, const int16_t* control
 
 /* bf_forward_priors with HOST buffers, end to end like bf_forward_host: about 11 times
  * fewer bytes return to the host than with the logits (392 B per position at e_cap 96), so batches of
- * up to four positions per SM in pinned, device-mapped buffers run in place. */
+ * up to four positions per SM in pinned, device-mapped and aligned buffers run in place. */
 int bf_forward_priors_host(bf_handle* h, const uint16_t* boards, const int16_t* control, const uint8_t* rep,
                            const uint64_t* legal, int n, int e_cap, void* prior, int16_t* move, int* nedges,
                            float* value);
@@ -269,6 +270,13 @@ int bf_set_option(bf_handle* h, int option, int value);
 /* GB/s the first device-to-host copy of the last `bf_forward_host` call reached (0 before the
  * first call): what the plan of the next call is chosen by.  No counterpart in the reference. */
 double bf_host_link_gbps(const bf_handle* h);
+
+/* Whether the kernels can read and write host buffers at these addresses themselves (1) or the host
+ * calls copy them (0): boards, control, prior and move on 2 bytes, value and nedges on 4, legal and
+ * promo on 8, policy on 16; null pointers do not count.  No GPU is touched.  No counterpart in the
+ * reference. */
+int bf_host_aligned(const void* boards, const void* control, const void* legal, const void* policy, const void* promo,
+                    const void* value, const void* prior, const void* move, const void* nedges);
 
 /* The launch sizes `bf_forward_host` uses for `n` positions under BF_OPT_HOST_PLAN `plan` when the
  * measured copy rate is `gbps` (0: not measured yet) and a wave of tiles is four positions on each of

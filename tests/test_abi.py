@@ -76,3 +76,17 @@ def test_host_call_launch_plans():
                     assert got[1:] == sorted(got[1:], reverse=True)
     assert L.bf_host_plan(0, 148, 0, 0.0, sizes) == -1
     assert L.bf_host_plan(10, 148, 3, 0.0, sizes) == -1
+
+
+def test_which_host_addresses_the_kernels_use_themselves():
+    """Each buffer of the host calls has the alignment that the kernels' widest access to it needs, and
+    only that: one at any other address goes through the copies."""
+    L = _native.lib()
+    need = dict(boards=2, control=2, legal=8, policy=16, promo=8, value=4, prior=2, move=2, nedges=4)
+    base = 1 << 20
+    assert L.bf_host_aligned(*[None] * 9) == 1 == L.bf_host_aligned(*[base] * 9)
+    for i, (name, bytes_) in enumerate(need.items()):
+        for off in range(1, 33):
+            at = [None] * 9
+            at[i] = base + off
+            assert L.bf_host_aligned(*at) == int(off % bytes_ == 0), (name, off)
