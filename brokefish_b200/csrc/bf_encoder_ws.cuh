@@ -94,8 +94,8 @@ struct Row {
     uint8_t* smem_gen;
     volatile int* abort_flag;
     uint64_t one2;
-    uint32_t layers, tiles;     // layers and tiles finished so far: three products per layer go through
-                                // each slot, and one per tile (the heads') through slot 0
+    uint32_t layers, tiles;     // layers and tiles finished so far: a slot's barrier completes `completions`
+                                // times per layer, and slot 0's once per tile for the heads
     int n;
     uint32_t h;                 // shared address of H
     __device__ uint32_t a() const { return smem + SM_A; }
@@ -123,10 +123,15 @@ __device__ __forceinline__ void board_sync(const Row& c) { __syncwarp(); named_b
 // The two warps of a head (one-board tiles).
 __device__ __forceinline__ void pair_sync(int head) { __syncwarp(); named_bar_sync(3 + head, 64); }
 
-// The `use`-th product of the layer in slot `slot` (0: Q, K, V, out-projection, or the heads; 1: ff1;
-// 2: ff2).
+// How often a slot's barrier completes in a layer: with Q, K, V or the out-projection, with ff1's chunk,
+// with ff2's (in fp16, whose ff2 has one sum, slot 0 with its first half and slot 1 with all of it).  Every
+// completion is one that all row warps wait for: a parity wait tells a phase only from the one before it.
+template <int kAr>
+__host__ __device__ constexpr uint32_t completions(int slot) { return kAr == kArF16 && slot >= 2 ? 2u : 3u; }
+// The `use`-th of them in this layer; of slot 0, use 0 after the last layer is the heads' product.
+template <int kAr>
 __device__ __forceinline__ void wait_acc(const Row& c, int slot, int use) {
-    const uint32_t n = 3u * c.layers + use + (slot == 0 ? c.tiles : 0u);
+    const uint32_t n = completions<kAr>(slot) * c.layers + use + (slot == 0 ? c.tiles : 0u);
     mbar_wait(bar(c.smem, B_ACC + slot), n & 1u, c.abort_flag, kErrRowAcc);
     __syncwarp();                                            // what follows is for a converged warp
     tc_fence_after();
@@ -443,7 +448,7 @@ __device__ __forceinline__ void stage_qkv(const Row& c, uint32_t lp, float sa, i
     const uint32_t bias_at = lp + LP_B_QKV + 2u * ((col >> 6) * 192 + m * 64 + (col & 63));
     const float sw = lds_f(lp + LP_SW_QKV + 4u * (m * 2 + (col >> 7)));
     Bias bias = load_bias(bias_at);
-    wait_acc(c, m, 0);
+    wait_acc<kAr>(c, m, 0);
     each_piece<NB>(O::slot(c, m), [&](int k, const uint32_t (&acc)[16]) {
         uint32_t h[8];
         if (k > 0) bias = load_bias(bias_at + 32 * k);
@@ -526,7 +531,7 @@ __device__ __forceinline__ void attention_block(const Row& c, uint32_t lp, float
     // x = fp16(x + fp16(fp16(descale) + b_o))
     const float sw = lds_f(lp + LP_SW_O + 4u * (col >> 7));
     Bias bias = load_bias(lp + LP_B_O + 2u * col);
-    wait_acc(c, 3, 0);
+    wait_acc<kAr>(c, 3, 0);
     each_piece<NB>(O::slot(c, 3), [&](int k, const uint32_t (&acc)[16]) {
         uint32_t y[8];
         if (k > 0) bias = load_bias(lp + LP_B_O + 2u * col + 32 * k);
@@ -555,7 +560,7 @@ __device__ __forceinline__ void ffn_block(const Row& c, uint32_t lp, float sa, u
             const uint32_t bias_at = lp + LP_B_FF1 + 2u * (256 * ch + col);
             const float sw = lds_f(lp + LP_SW_FF1 + 4u * (2 * ch + (col >> 7)));
             Bias bias = load_bias(bias_at);
-            wait_acc(c, ch, 1);
+            wait_acc<kAr>(c, ch, 1);
             each_piece<NB>(O::slot(c, ch), [&](int i, const uint32_t (&acc)[16]) {
                 if (i > 0) bias = load_bias(bias_at + 32 * i);
                 descale16<true, kAr == kArE4M3 ? kAccFloat : kAccInt>(acc, sa, sw, bias, &hid[k][8 * i]);
@@ -582,7 +587,7 @@ __device__ __forceinline__ void ffn_block(const Row& c, uint32_t lp, float sa, u
     const uint64_t s2_2 = pk2(s2, s2);
 #pragma unroll
     for (int ch = 0; ch < 4; ++ch) {
-        wait_acc(c, ch, 2);
+        wait_acc<kAr>(c, ch, 2);
         const uint64_t s1_2 = pk2(s1[0], s1[0]);
         s1[0] = s1[1]; s1[1] = s1[2]; s1[2] = s1[3];
         each_piece<NB>(O::slot(c, ch), [&](int k, const uint32_t (&acc)[16]) {
@@ -613,7 +618,7 @@ __device__ __forceinline__ void ffn_block(const Row& c, uint32_t lp, float sa, u
 // The fp16 arithmetic's FFN: ff1's epilogue is bias and ReLU, a chunk goes out as ff2's fp16 operand, and
 // ff2's fp16 accumulators (slot 0) run on through the four chunks.  H holds two chunks, so the second
 // pair is written when the first pair's ff2 products are done (a completion of slot 0 that says no more
-// than that); the last completion, on every slot, says that the sums are there.
+// than that); a completion of slot 1 says that the sums are there.
 template <int NB>
 __device__ __forceinline__ void ffn_block_f16(const Row& c, uint32_t lp, uint32_t (&x)[8 * NB]) {
     using O = Own<NB>;
@@ -625,8 +630,8 @@ __device__ __forceinline__ void ffn_block_f16(const Row& c, uint32_t lp, uint32_
             const int ch = 2 * pair + k;
             const uint32_t bias_at = lp + LP_B_FF1 + 2u * (256 * ch + col);
             Bias bias = load_bias(bias_at);
-            wait_acc(c, ch, 1);
-            if (ch == 2) wait_acc(c, 0, 2);
+            wait_acc<kArF16>(c, ch, 1);
+            if (ch == 2) wait_acc<kArF16>(c, 0, 2);
             each_piece<NB>(O::slot(c, ch), [&](int i, const uint32_t (&acc)[16]) {
                 uint32_t h[8];
                 if (i > 0) bias = load_bias(bias_at + 32 * i);
@@ -637,7 +642,7 @@ __device__ __forceinline__ void ffn_block_f16(const Row& c, uint32_t lp, uint32_
         publish(c, B_H + pair);
     }
     Bias bias = load_bias(lp + LP_B_FF2 + 2u * col);
-    wait_acc(c, 1, 2);
+    wait_acc<kArF16>(c, 1, 2);
     each_piece<NB>(O::slot(c, 0), [&](int k, const uint32_t (&acc)[16]) {
         uint32_t y[8];
         if (k > 0) bias = load_bias(lp + LP_B_FF2 + 2u * col + 32 * k);
@@ -736,7 +741,7 @@ __device__ __forceinline__ void heads(const Row& c, const Params& p, int board, 
     // while the product runs: the legality words
     unsigned long long lw = ~0ull;
     if (p.legal != nullptr && p.policy != nullptr && valid && hc < 64) lw = p.legal[grow];
-    wait_acc(c, 0, 0);
+    wait_acc<kAr>(c, 0, 0);
     uint32_t v[4 * NB];
     {
         uint32_t acc[8 * NB];
@@ -1051,13 +1056,12 @@ __device__ __forceinline__ void issue_tile(Issue& st, int n_layers) {
         for (int ch = 0; ch < 4; ++ch) {
             if ((ch & 1) == 0) issue_wait(st, B_H + (ch >> 1), st.h);
             if (kAr == kArF16) {
-                issue_unit<kAr, kFfnKind>(st, st.tmem, h + (ch & 1) * 4 * O::kSlab, O::kSlab, C::kFfnSlabs, kI_FF2, ch == 1 ? 0 : -1, ch > 0);
+                issue_unit<kAr, kFfnKind>(st, st.tmem, h + (ch & 1) * 4 * O::kSlab, O::kSlab, C::kFfnSlabs, kI_FF2,
+                                            ch == 1 ? 0 : ch == 3 ? 1 : -1, ch > 0);
             } else {
                 issue_unit<kAr, kFfnKind>(st, st.tmem + O::kSlot * ch, h + ch * 2 * O::kSlab, O::kSlab, C::kFfnSlabs, kI_FF2, ch);
             }
         }
-        if (kAr == kArF16 && elect_one())
-            for (int slot = 1; slot < 4; ++slot) tc_commit(bar(st.smem, B_ACC + slot));
         st.h++;
     }
     issue_wait(st, B_A, st.a++);
