@@ -2049,12 +2049,12 @@ __global__ void __launch_bounds__(64, 1) timeout_kernel(int code, int* status, l
 
 // ------------------------------------------------------------------------------------------
 // Scale self test: the row scales and reciprocals of bf_encoder_ws.cuh against IEEE division over
-// every value they can be given: all positive fp16 maxima with the three operand ranges (counts 0-2:
-// scale or reciprocal differs), and every fp32 softmax sum from 1 to 32 (count 3).
+// every value they can be given: all non-negative fp16 maxima, infinity and a NaN included, with the three
+// operand ranges (counts 0-2: scale or reciprocal differs), and every fp32 softmax sum from 1 to 32 (count 3).
 // ------------------------------------------------------------------------------------------
 __global__ void scales_kernel(unsigned long long* differ) {
     const unsigned first = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
-    for (unsigned i = first; i <= 0x7bffu; i += step) {
+    for (unsigned i = first; i <= 0x7c01u; i += step) {
         const float amax = __half2float(__ushort_as_half(static_cast<unsigned short>(i)));
         const float range[3] = {kQMaxS8, kQMaxU8, kQMaxE4M3};
         const ws::Scale got[3] = {ws::scale_s8(amax), ws::scale_u8(amax), ws::scale_e4m3(amax)};

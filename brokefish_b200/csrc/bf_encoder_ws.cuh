@@ -173,26 +173,38 @@ __device__ __forceinline__ uint64_t lds_u64(uint32_t addr) {
 __device__ __forceinline__ void max_to(uint32_t addr, float v) {
     asm volatile("red.shared.max.u32 [%0], %1;" ::"r"(addr), "r"(__float_as_uint(v)) : "memory");
 }
-// A row's scale amax / Q and its reciprocal, both correctly rounded, amax being a positive fp16 value: a
-// quotient corrected by its own remainder, and one Newton step on the hardware's reciprocal with the
-// residual taken by fma (Markstein 1990).  Neither leaves the normal range here, and every one of the
-// 31,743 values of amax gives the bits of `__fdiv_rn` for each of the three ranges, as does the
-// reciprocal of every fp32 value from 1 to 32, a softmax row's sum (`scales_kernel`).  Two divisions one after the other
+// A row's scale amax / Q and its reciprocal, both correctly rounded, amax being a non-negative fp16 value.  The
+// scale is a product with 1 / Q held in two words (Brisebarre and Muller 2008), the upper one rounded down so
+// that an infinite amax, a row that has overflowed, stays infinite; the reciprocal one Newton step on the
+// hardware's, the residual taken by fma (Markstein 1990), its minimum leaving infinity's reciprocal zero.
+// Every fp16 amax gives the bits of `__fdiv_rn` for each of the three ranges, as does the reciprocal of
+// every fp32 value from 1 to 32, a softmax row's sum (`scales_kernel`).  Two divisions one after the other
 // took 300 cycles, this takes 45.
 struct Scale { float scale, inverse; };
-__device__ __forceinline__ float reciprocal(float x) {
+__device__ __forceinline__ float rcp_approx(float x) {
     float y;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float reciprocal(float x) {
+    const float y = rcp_approx(x);
     return __fmaf_rn(__fmaf_rn(-x, y, 1.0f), y, y);
 }
-__device__ __forceinline__ Scale row_scale(float amax, float q_max, float q_inv) {
-    const float q = __fmul_rn(amax, q_inv);
-    const float sc = amax > 0.f ? __fmaf_rn(__fmaf_rn(-q, q_max, amax), q_inv, q) : 1.0f;
-    return {sc, reciprocal(sc)};
+__device__ __forceinline__ Scale with_inverse(float sc) {
+    const float y = rcp_approx(sc);
+    return {sc, __fmaf_rn(fminf(__fmaf_rn(-sc, y, 1.0f), 1.0f), y, y)};
 }
-__device__ __forceinline__ Scale scale_s8(float amax) { return row_scale(amax, kQMaxS8, 1.0f / kQMaxS8); }
-__device__ __forceinline__ Scale scale_u8(float amax) { return row_scale(amax, kQMaxU8, 1.0f / kQMaxU8); }
-__device__ __forceinline__ Scale scale_e4m3(float amax) { return row_scale(amax, kQMaxE4M3, 1.0f / kQMaxE4M3); }
+__device__ __forceinline__ Scale scale_s8(float amax) {
+    constexpr float hi = 0x1.020408p-7f, lo = static_cast<float>(1.0 / kQMaxS8 - hi);
+    return with_inverse(amax > 0.f ? __fmaf_rn(amax, hi, __fmul_rn(amax, lo)) : 1.0f);
+}
+__device__ __forceinline__ Scale scale_u8(float amax) {
+    constexpr float hi = 0x1.01010p-8f, lo = static_cast<float>(1.0 / kQMaxU8 - hi);
+    return with_inverse(amax > 0.f ? __fmaf_rn(amax, hi, __fmul_rn(amax, lo)) : 1.0f);
+}
+__device__ __forceinline__ Scale scale_e4m3(float amax) {
+    return with_inverse(amax > 0.f ? __fmul_rn(amax, 1.0f / kQMaxE4M3) : 1.0f);      // a power of two: exact
+}
 // Sixteen columns' biases (a broadcast: a warp's threads share their columns).
 struct Bias { uint4 lo, hi; };
 __device__ __forceinline__ Bias load_bias(uint32_t addr) { return {lds128(addr), lds128(addr + 16)}; }

@@ -382,8 +382,8 @@ int bf_selftest_timeout(int device, int code, int* status, long long* waited_cyc
 
 /* Scale self test; no counterpart in the reference.  The evaluator's row scales and reciprocals are
  * corrected approximations instead of divisions; this compares them with IEEE division over every
- * value they can be given and counts the differences: `differ[0..2]` over all positive fp16 row maxima
- * for the s8, u8 and e4m3 ranges, `differ[3]` over every fp32 softmax sum from 1 to 32. */
+ * value they can be given and counts the differences: `differ[0..2]` over all non-negative fp16 row
+ * maxima, infinity included, for the s8, u8 and e4m3 ranges, `differ[3]` over every fp32 softmax sum from 1 to 32. */
 int bf_selftest_scales(int device, unsigned long long* differ);
 
 /* Tensor-core self test (no network): one 128-row tile times a packed weight tile.
