@@ -1115,6 +1115,17 @@ __device__ __forceinline__ void ffn_block_f16(RowCtx& c, const Params& p, const 
 // over this thread's 64 columns: with a = the column means, the k-th logit is
 // rstd * (sum a*g*w_k - mean * sum g*w_k) + sum b*w_k, so no vector has to be kept.
 // Every thread of the board returns the same three logits.
+//
+// `v + x . y` of one column pair and the logit, with their roundings spelled out: a position's value must
+// not depend on which of the two kernels it runs in (bf_encoder_ws.cuh adds in this order, too).
+__device__ __forceinline__ float prenorm_add(float v, float2 x, float2 y) {
+    return __fadd_rn(v, __fmaf_rn(x.x, y.x, __fmul_rn(x.y, y.y)));
+}
+__device__ __forceinline__ float prenorm_logit(float tot, float totq, float t1, float t2, float t3, float eps) {
+    const float mean = __fmul_rn(tot, 1.0f / 256.0f);
+    const float var = fmaxf(__fsub_rn(__fmul_rn(totq, 1.0f / 256.0f), __fmul_rn(mean, mean)), 0.f);
+    return __fmaf_rn(rsqrtf(__fadd_rn(var, eps)), __fmaf_rn(-mean, t2, t1), t3);
+}
 __device__ __forceinline__ void prenorm_value(RowCtx& c, const Params& p, uint32_t alive, float (&logit)[3]) {
     const bool live = (alive >> c.lane) & 1u;
     const int nlive = __popc(alive);
@@ -1135,18 +1146,18 @@ __device__ __forceinline__ void prenorm_value(RowCtx& c, const Params& p, uint32
                 a0 += __shfl_xor_sync(0xffffffffu, a0, off);
                 a1 += __shfl_xor_sync(0xffffffffu, a1, off);
             }
-            a0 *= inv_live; a1 *= inv_live;
-            s += a0 + a1;
-            q += a0 * a0 + a1 * a1;
+            const float2 a = make_float2(__fmul_rn(a0, inv_live), __fmul_rn(a1, inv_live));
+            s = prenorm_add(s, a, make_float2(1.f, 1.f));
+            q = prenorm_add(q, a, a);
             const float2 g = __half22float2(as_h2(__ldg(reinterpret_cast<const uint32_t*>(p.tail + col) + i)));
             const float2 b = __half22float2(as_h2(__ldg(reinterpret_cast<const uint32_t*>(p.tail + kD + col) + i)));
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
                 const float2 w = __half22float2(
                     as_h2(__ldg(reinterpret_cast<const uint32_t*>(p.tail + 2 * kD + k * kD + col) + i)));
-                s1[k] += a0 * g.x * w.x + a1 * g.y * w.y;
-                s2[k] += g.x * w.x + g.y * w.y;
-                s3[k] += b.x * w.x + b.y * w.y;
+                s1[k] = prenorm_add(s1[k], make_float2(__fmul_rn(a.x, g.x), __fmul_rn(a.y, g.y)), w);
+                s2[k] = prenorm_add(s2[k], g, w);
+                s3[k] = prenorm_add(s3[k], b, w);
             }
         }
     }
@@ -1154,8 +1165,6 @@ __device__ __forceinline__ void prenorm_value(RowCtx& c, const Params& p, uint32
     exchange4(c, make_float4(s, q, 0.f, 0.f), all);
     const float tot = (all[0].x + all[1].x) + (all[2].x + all[3].x);
     const float totq = (all[0].y + all[1].y) + (all[2].y + all[3].y);
-    const float mean = tot * (1.0f / 256.0f);
-    const float rstd = rsqrtf(fmaxf(__fsub_rn(totq * (1.0f / 256.0f), __fmul_rn(mean, mean)), 0.f) + p.eps);
     float t1[3], t2[3], t3[3];
     exchange4(c, make_float4(s1[0], s1[1], s1[2], 0.f), all);
     t1[0] = (all[0].x + all[1].x) + (all[2].x + all[3].x);
@@ -1170,7 +1179,7 @@ __device__ __forceinline__ void prenorm_value(RowCtx& c, const Params& p, uint32
     t3[1] = (all[0].y + all[1].y) + (all[2].y + all[3].y);
     t3[2] = (all[0].z + all[1].z) + (all[2].z + all[3].z);
 #pragma unroll
-    for (int k = 0; k < 3; ++k) logit[k] = rstd * (t1[k] - mean * t2[k]) + t3[k];
+    for (int k = 0; k < 3; ++k) logit[k] = prenorm_logit(tot, totq, t1[k], t2[k], t3[k], p.eps);
 }
 
 // The head epilogue of one board: accumulators of the head product -> staged logits -> legality

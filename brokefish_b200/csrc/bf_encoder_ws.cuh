@@ -665,59 +665,60 @@ __device__ __forceinline__ void ffn_block_f16(const Row& c, uint32_t lp, uint32_
 }
 
 // ---- heads ----
-// The "prenorm" value head (see `prenorm_value`): column means over the board's live tokens, one
-// LayerNorm with affine of that vector, dotted with the value rows; every thread returns the logits.
+// The "prenorm" value head (see `prenorm_value`, whose order of sums this keeps): the column means over the
+// board's live tokens go into the board's list buffer, which the expansion warp touches only once this
+// tile's logits are staged.
 template <int NB>
-__device__ __forceinline__ void prenorm_logits(const Row& c, const Params& p, uint32_t alive, const uint32_t (&x)[8 * NB], float (&logit)[3]) {
+__device__ __forceinline__ void prenorm_means(const Row& c, uint32_t alive, const uint32_t (&x)[8 * NB]) {
     using O = Own<NB>;
     const bool live = (alive >> c.lane) & 1u;
     const int nlive = __popc(alive);
     const float inv_live = 1.0f / static_cast<float>(nlive > 0 ? nlive : 1);
-    const uint32_t xch = c.h + 16384u * O::board(c);
-    float v[11];
+    const uint32_t means = c.smem + SM_LIST + 1024u * O::board(c) + 4u * O::col(c);
 #pragma unroll
-    for (int piece = 0; piece < NB; ++piece) {               // sixteen columns at a time, whatever NB: one order of sums
-        const int col = O::col(c) + 16 * piece;
+    for (int i = 0; i < 8 * NB; ++i) {
+        const float2 f = __half22float2(as_h2(x[i]));
+        float a0 = live ? f.x : 0.f, a1 = live ? f.y : 0.f;
 #pragma unroll
-        for (int i = 0; i < 11; ++i) v[i] = 0.f;             // s, q, s1[3], s2[3], s3[3]
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const float2 f = __half22float2(as_h2(x[8 * piece + i]));
-            float a0 = live ? f.x : 0.f, a1 = live ? f.y : 0.f;
-#pragma unroll
-            for (int off = 16; off; off >>= 1) {
-                a0 += __shfl_xor_sync(0xffffffffu, a0, off);
-                a1 += __shfl_xor_sync(0xffffffffu, a1, off);
-            }
-            a0 *= inv_live; a1 *= inv_live;
-            v[0] += a0 + a1;
-            v[1] += a0 * a0 + a1 * a1;
-            const float2 g = __half22float2(as_h2(__ldg(reinterpret_cast<const uint32_t*>(p.tail + col) + i)));
-            const float2 b = __half22float2(as_h2(__ldg(reinterpret_cast<const uint32_t*>(p.tail + kD + col) + i)));
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                const float2 w = __half22float2(as_h2(__ldg(reinterpret_cast<const uint32_t*>(p.tail + 2 * kD + k * kD + col) + i)));
-                v[2 + k] += a0 * g.x * w.x + a1 * g.y * w.y;
-                v[5 + k] += g.x * w.x + g.y * w.y;
-                v[8 + k] += b.x * w.x + b.y * w.y;
-            }
+        for (int off = 16; off; off >>= 1) {
+            a0 += __shfl_xor_sync(0xffffffffu, a0, off);
+            a1 += __shfl_xor_sync(0xffffffffu, a1, off);
         }
-        if (c.lane == 0)
-#pragma unroll
-            for (int i = 0; i < 11; ++i) sts32(xch + 4u * col + 4u * i, __float_as_uint(v[i]));    // 64 bytes per piece
+        if (c.lane == 0) {
+            sts32(means + 8u * i, __float_as_uint(__fmul_rn(a0, inv_live)));
+            sts32(means + 8u * i + 4u, __float_as_uint(__fmul_rn(a1, inv_live)));
+        }
     }
-    board_sync<NB>(c);
-#pragma unroll
-    for (int i = 0; i < 11; ++i) v[i] = 0.f;
+}
+// The three logits, in one warp, while the head product runs: lane & 3 is the quarter of the columns
+// (32 q .. + 31 and 128 + 32 q .. + 31), lane >> 2 the sum: of the means, of their squares, of
+// means x gamma x value row k (with it gamma x value row k), of beta x value row k.
+template <int NB>
+__device__ __forceinline__ void prenorm_logits(const Row& c, const Params& p, float (&logit)[3]) {
+    const uint32_t means = c.smem + SM_LIST + 1024u * Own<NB>::board(c);
+    const int quarter = c.lane & 3, kind = c.lane >> 2, k = kind < 2 ? 0 : (kind - 2) % 3;
+    float t = 0.f, t2 = 0.f;
 #pragma unroll 1
-    for (int t = 0; t < 16; ++t)
+    for (int i = 0; i < 32; ++i) {
+        const int col = 128 * (i >> 4) + 32 * quarter + 2 * (i & 15);
+        const float2 a = make_float2(lds_f(means + 4u * col), lds_f(means + 4u * col + 4u));
+        const float2 g = __half22float2(as_h2(__ldg(reinterpret_cast<const uint32_t*>(p.tail + col))));
+        const float2 b = __half22float2(as_h2(__ldg(reinterpret_cast<const uint32_t*>(p.tail + kD + col))));
+        const float2 w = __half22float2(as_h2(__ldg(reinterpret_cast<const uint32_t*>(p.tail + (2 + k) * kD + col))));
+        const float2 u = kind < 2 ? a : kind < 5 ? make_float2(__fmul_rn(a.x, g.x), __fmul_rn(a.y, g.y)) : b;
+        t = prenorm_add(t, u, kind == 0 ? make_float2(1.f, 1.f) : kind == 1 ? a : w);
+        t2 = prenorm_add(t2, g, w);
+    }
 #pragma unroll
-        for (int i = 0; i < 11; ++i) v[i] += lds_f(xch + 64u * t + 4u * i);
-    board_sync<NB>(c);
-    const float mean = v[0] * (1.0f / 256.0f);
-    const float rstd = rsqrtf(fmaxf(__fsub_rn(v[1] * (1.0f / 256.0f), __fmul_rn(mean, mean)), 0.f) + p.eps);
+    for (int off = 1; off < 4; off <<= 1) {
+        t = __fadd_rn(t, __shfl_xor_sync(0xffffffffu, t, off));
+        t2 = __fadd_rn(t2, __shfl_xor_sync(0xffffffffu, t2, off));
+    }
+    const float tot = __shfl_sync(0xffffffffu, t, 0), totq = __shfl_sync(0xffffffffu, t, 4);
 #pragma unroll
-    for (int k = 0; k < 3; ++k) logit[k] = rstd * (v[2 + k] - mean * v[5 + k]) + v[8 + k];
+    for (int i = 0; i < 3; ++i)
+        logit[i] = prenorm_logit(tot, totq, __shfl_sync(0xffffffffu, t, 8 + 4 * i), __shfl_sync(0xffffffffu, t2, 8 + 4 * i),
+                                 __shfl_sync(0xffffffffu, t, 20 + 4 * i), p.eps);
 }
 
 // Final norm into the head product's fp16 operand, then the epilogue: the product's 128 output columns
@@ -729,8 +730,7 @@ __device__ __forceinline__ void heads(const Row& c, const Params& p, int board, 
     using O = Own<NB>;
     const int col = O::col(c), row = O::row(c), lane = c.lane;
     const long grow = static_cast<long>(board) * kT + lane;
-    float pre[3] = {0.f, 0.f, 0.f};
-    if (p.vmode == 2) prenorm_logits<NB>(c, p, alive, x, pre);
+    if (p.vmode == 2) prenorm_means<NB>(c, alive, x);         // (the norm's meetings make them everybody's)
     {
         const float4 st = row_statistics<NB, kAr>(c, p, x);
         const uint64_t nmean2 = pk2(st.x, st.x), rstd2 = pk2(st.y, st.y);
@@ -753,6 +753,8 @@ __device__ __forceinline__ void heads(const Row& c, const Params& p, int board, 
     // while the product runs: the legality words
     unsigned long long lw = ~0ull;
     if (p.legal != nullptr && p.policy != nullptr && valid && hc < 64) lw = p.legal[grow];
+    float pre[3] = {0.f, 0.f, 0.f};
+    if (p.vmode == 2 && hc == 64) prenorm_logits<NB>(c, p, pre);
     wait_acc<kAr>(c, 0, 0);
     uint32_t v[4 * NB];
     {

@@ -48,3 +48,34 @@ def test_scales_and_reciprocals_equal_division():
     differ = (ctypes.c_ulonglong * 4)()
     _native.check(_native.lib().bf_selftest_scales(0, differ), "bf_selftest_scales")
     assert list(differ) == [0, 0, 0, 0]
+
+
+@pytest.mark.parametrize("n_value", [1, 3])
+@pytest.mark.parametrize("head", ["king", "pooled", "prenorm"])
+@pytest.mark.parametrize("arithmetic", ["int8", "f16"])
+def test_a_value_does_not_depend_on_the_tile(arithmetic, head, n_value, pos4096):
+    """Every value head on one-, two- and four-board tiles, to the bit: fp16 batches change kernels with
+    their size, the int8 ones under the phase clock."""
+    from brokefish_b200.nn.cuda_impl import FusedEncoder
+    from brokefish_b200.nn.model import net_for_state, seeded_state
+    state = seeded_state(seed=11, std=None, perturb_norms=True, n_value=n_value, value_head=head)
+    net = net_for_state(state).eval()
+    net.load_state_dict(state)
+    enc = FusedEncoder(net, **ARITHMETICS[arithmetic])
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    b, c, r = (cu(pos4096[k]) for k in ("boards", "control", "rep"))
+    legal = cu(pos4096["legal"].view(np.int64))
+    want = [t.clone() for t in enc.forward_full(b, c, r)]
+    assert float(want[2].abs().max()) > 0.05
+    for n in (1, sms, sms + 1, 2 * sms + 1, 4 * sms, 4 * sms + 1):
+        for got, w in zip(enc.forward_full(b[:n], c[:n], r[:n]), want):
+            assert torch.equal(got, w[:n]), n
+    # the expansion's warps share a buffer with the prenorm head
+    n = 2 * sms + 5
+    assert torch.equal(enc.forward_priors(b[:n], c[:n], r[:n], legal[:n], 96)[3], want[2][:n])
+    enc.set_profile(True)
+    for got, w in zip(enc.forward_full(b[:n], c[:n], r[:n]), want):
+        assert torch.equal(got, w[:n])
+    enc.set_profile(False)
+    enc.check_status()
+    enc.close()
