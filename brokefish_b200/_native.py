@@ -42,7 +42,7 @@ EXPORTS = ["bf_version", "bf_last_error", "bf_create", "bf_destroy", "bf_info", 
            "bf_forward_leaves", "bf_measure_elementwise", "bf_forward_backbone", "bf_int8_q_max",
            "bf_fp8_q_max", "bf_terminal", "bf_hash", "bf_history_push",
            "bf_repetition_count", "bf_history_push_to", "bf_terminal_history",
-           "bf_selftest_scales", "bf_host_aligned"]
+           "bf_selftest_scales", "bf_host_aligned", "bf_tile_boards"]
 
 
 def nvcc_path() -> str:
@@ -151,6 +151,7 @@ def lib() -> ctypes.CDLL:
     L.bf_host_link_gbps.argtypes = [vp]
     L.bf_host_link_gbps.restype = ctypes.c_double
     L.bf_host_plan.argtypes = [i32, i32, i32, ctypes.c_double, ctypes.POINTER(i32)]
+    L.bf_tile_boards.argtypes = [i32, i32, i32, i32]
     L.bf_host_aligned.argtypes = [vp] * 9
     L.bf_selftest_scales.argtypes = [i32, ctypes.POINTER(ctypes.c_ulonglong)]
     L.bf_selftest_umma.argtypes = [i32, i32, vp, vp, vp]

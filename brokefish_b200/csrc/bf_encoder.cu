@@ -2345,23 +2345,6 @@ struct LeafList {
     const int* count;           // device: how many of them (read by the kernel when it starts)
 };
 
-// Which form a plain evaluation runs in: one- and two-board tiles (bf_encoder_ws.cuh) or four-board tiles.
-// A tile takes the same time whatever the batch, so the tiles of the busiest SM decide.  Measured, us
-// per one-, two- and four-board tile of an SM (B200):
-//   int8 90 / 126    int8 FFN+QKV 96 / 128    int8 FFN 103 / 133 / 273
-//   e4m3 100 / 130 / 270    fp16 129 / 152 / 272
-// Two two-board tiles beat a four-board one everywhere but in fp16, whose products, 32 bytes of K at
-// half the rate and twice the weight bytes, keep the weight stream and the tensor pipe busy for half
-// of a two-board tile's time; there the four-board form takes the batches that fill it.
-bool small_tiles(int quant, int n, int sm_count) {
-    if (quant != 0) return true;
-    static const int t[3] = {129, 152, 272};
-    const long full = n / (2 * sm_count), rest = n - full * 2 * sm_count;
-    const long small = full * t[1] + (rest == 0 ? 0 : rest <= sm_count ? t[0] : t[1]);
-    const long four = static_cast<long>((n + 4L * sm_count - 1) / (4L * sm_count)) * t[2];
-    return small <= four;
-}
-
 using Kernel = void (*)(bf::Params);
 template <bool kExpand>
 Kernel small_tile_kernel(int quant) {
@@ -2413,7 +2396,7 @@ int launch(bf_handle* h, const uint16_t* boards, const int16_t* control, const u
     // the instrumented instantiation only when a dump, a capture or the phase clock is asked for
     const bool dbg = stage != 0 || cap_layer >= 0 || p.prof != nullptr;
     if (cap_layer >= 0 && p.quant != 3) return fail(BF_ENOTSUP, "operand capture is for the int8 arithmetic");
-    if (!dbg && p.rj_mode == 0 && small_tiles(p.quant, n, h->sm_count)) {
+    if (!dbg && p.rj_mode == 0 && bf_tile_boards(p.quant, n, h->sm_count, h->one_board_factor) < 4) {
         p.one_most = h->one_board_factor;
         const int ctas = n < h->sm_count ? n : h->sm_count;
         const bool expand = p.prior != nullptr;
@@ -2969,6 +2952,26 @@ int bf_status(bf_handle* h, int* status) {
 long long bf_launch_count(const bf_handle* h) { return h ? h->launches : 0; }
 
 double bf_host_link_gbps(const bf_handle* h) { return h ? h->d2h_gbps : 0.0; }
+
+// Which form a plain evaluation runs in: one- and two-board tiles (bf_encoder_ws.cuh) or four-board tiles.
+// A tile takes the same time whatever the batch, so the tiles of the busiest SM decide.  Measured, us
+// per one-, two- and four-board tile of an SM (B200):
+//   int8 90 / 126    int8 FFN+QKV 96 / 128    int8 FFN 103 / 133 / 273
+//   e4m3 100 / 130 / 270    fp16 129 / 152 / 272
+// Two two-board tiles beat a four-board one everywhere but in fp16, whose products, 32 bytes of K at
+// half the rate and twice the weight bytes, keep the weight stream and the tensor pipe busy for half
+// of a two-board tile's time; there the four-board form takes the batches that fill it.  Of a leaf list
+// only the capacity is known here, and that decides.
+int bf_tile_boards(int quant, int n, int sm_count, int one_board) {
+    if (n < 1 || sm_count < 1) return fail(BF_EINVAL, "n and sm_count must be positive");
+    if (n <= static_cast<long>(one_board) * sm_count) return 1;
+    if (quant != 0) return 2;
+    static const int t[3] = {129, 152, 272};
+    const long full = n / (2 * sm_count), rest = n - full * 2 * sm_count;
+    const long small = full * t[1] + (rest == 0 ? 0 : rest <= sm_count && one_board > 0 ? t[0] : t[1]);
+    const long four = static_cast<long>((n + 4L * sm_count - 1) / (4L * sm_count)) * t[2];
+    return small <= four ? 2 : 4;
+}
 
 int bf_host_aligned(const void* boards, const void* control, const void* legal, const void* policy, const void* promo,
                     const void* value, const void* prior, const void* move, const void* nedges) {

@@ -102,7 +102,9 @@ int bf_forward_priors(bf_handle* h, const uint16_t* boards, const int16_t* contr
  * kernel starts, so the caller needs no host synchronisation to know it.  `capacity` is the most
  * the list can hold (the grid is sized for it; a larger count is clamped, a negative one is 0);
  * CTAs beyond the count's tiles leave at once, so a short list runs short, and a list of at
- * most one position per SM runs on one-board tiles (BF_OPT_ONE_BOARD).  Every output is
+ * most one position per SM runs on one-board tiles (BF_OPT_ONE_BOARD) -- except where the capacity
+ * has put the launch on four-board tiles (bf_tile_boards; large capacities in fp16, and every launch
+ * with re-injection).  Every output is
  * written at the position's own place in the staged arrays (policy [place,32,64], value [place],
  * prior [place,e_cap] ...); places not in the list are not touched.  Any of policy / promo /
  * value may be NULL; pass prior, move and nedges (all three, else all NULL) for the fused
@@ -270,6 +272,12 @@ int bf_set_option(bf_handle* h, int option, int value);
 /* GB/s the first device-to-host copy of the last `bf_forward_host` call reached (0 before the
  * first call): what the plan of the next call is chosen by.  No counterpart in the reference. */
 double bf_host_link_gbps(const bf_handle* h);
+
+/* How many positions the largest tiles of a plain evaluation of `n` positions (of a leaf list: of that
+ * capacity) hold, without re-injection, on a GPU with `sm_count` SMs under BF_OPT_ONE_BOARD
+ * `one_board`: 1, 2 or 4; `quant` is the blob's arithmetic (0 fp16).  No GPU is touched.  No counterpart
+ * in the reference. */
+int bf_tile_boards(int quant, int n, int sm_count, int one_board);
 
 /* Whether the kernels can read and write host buffers at these addresses themselves (1) or the host
  * calls copy them (0): boards, control, prior and move on 2 bytes, value and nedges on 4, legal and

@@ -86,6 +86,33 @@ def test_fused_expansion_over_a_leaf_list(enc, pos4096):
         assert (ne[idx[-2:].long()] == -1).all() and (ne[1::3] == -1).all()
 
 
+@pytest.mark.parametrize("capacity", [200, 4096])
+@pytest.mark.parametrize("arithmetic", [dict(), dict(fp8=True)], ids=["f16", "e4m3"])
+def test_lists_of_the_other_arithmetics(arithmetic, capacity, nets, pos4096):
+    """Short and full lists in a small and a large staging area (fp16 changes kernels with the capacity),
+    logits and edges: the dense call's bits, and nothing at other places."""
+    from brokefish_b200.nn.cuda_impl import FusedEncoder
+    e = FusedEncoder(nets["B"], **arithmetic)
+    boards, control, rep, legal = staged(pos4096, capacity)
+    want = [x.clone() for x in e.forward_full(boards, control, rep)]
+    edges = [x.clone() for x in e.forward_priors(boards, control, rep, legal, 96)]
+    idx = torch.randperm(capacity, generator=torch.Generator().manual_seed(5)).to(torch.int32).cuda()
+    for live in (1, 7, 149, capacity):
+        count = torch.tensor([live], dtype=torch.int32, device="cuda")
+        listed = torch.zeros(capacity, dtype=torch.bool, device="cuda")
+        listed[idx[:live].long()] = True
+        e.value_out.fill_(float("nan"))
+        for got, w in zip(e.forward_leaves(boards, control, rep, idx, count), want):
+            assert torch.equal(got[listed], w[listed])
+        assert torch.isnan(e.value_out[~listed]).all()
+        e.nedges_out.fill_(-1)
+        for got, w in zip(e.forward_leaves(boards, control, rep, idx, count, legal, 96), edges):
+            assert torch.equal(got[listed], w[listed])
+        assert (e.nedges_out[~listed] == -1).all()
+    e.check_status()
+    e.close()
+
+
 def test_a_short_list_runs_short(enc, pos4096):
     """128 live leaves of a 4096-place staging area against the dense call on all 4096: the
     reference's evaluator would cost the full batch either way."""
