@@ -83,3 +83,43 @@ def test_pinned_buffers_may_start_anywhere(offset, n, plan, enc, pos4096):
         edges_call(enc, n, 96, ins, outs)
         assert all(o.same(w) for o, w in zip(outs, edges)), (ins is moved, off)
     enc.set_host_plan(0)
+
+
+@pytest.mark.parametrize("n", [1, 63, 64, 65, 2500])
+def test_logits_on_every_way(n, enc, pos4096):
+    """Work in the caller's buffers (all pinned, up to 64 positions) and the copies (more, or any buffer
+    pageable), with and without legality words, every output or some."""
+    b, c, r, lg = device_inputs(pos4096, n)
+    want = {True: [t.clone() for t in enc.forward_full(b, c, r, lg)]}
+    want[False] = [t.clone() for t in enc.forward_full(b, c, r)]
+    for legal in (True, False):
+        ways = [[True] * 7, [False] * 7] + [[i != k for i in range(7)] for k in range(7)]
+        for pinned in ways:
+            ins = [Buffer(pos4096[k][:n], pinned=p) for k, p in zip(("boards", "control", "rep", "legal"), pinned)]
+            outs = [Buffer(nbytes=n * k, pinned=p) for k, p in zip((4096, 256, 4), pinned[4:])]
+            logits_call(enc, n, ins, outs, legal)
+            assert all(o.same(w) for o, w in zip(outs, want[legal])), (legal, pinned)
+        for keep in range(1, 7):
+            outs = [o if keep >> i & 1 else None for i, o in enumerate(logits_buffers(n))]
+            logits_call(enc, n, inputs(pos4096, n), outs, legal)
+            assert all(o.same(w) for o, w in zip(outs, want[legal]) if o), (legal, keep)
+
+
+@pytest.mark.parametrize("waves", ["one", "last in place", "first copied", "several"])
+def test_edge_lists_on_every_way(waves, enc, pos4096):
+    """The same for edge lists, which are written in place up to four positions per SM; an edge cap that is
+    no multiple of eight has its rows off the 16-byte boundaries."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    n = {"one": 1, "last in place": 4 * sms, "first copied": 4 * sms + 1, "several": 2500}[waves]
+    for e_cap in (96, 13):
+        want = [t.clone() for t in enc.forward_priors(*device_inputs(pos4096, n), e_cap)]
+        ways = [[True] * 8, [False] * 8] + [[i != k for i in range(8)] for k in range(8)]
+        for pinned in ways:
+            ins = [Buffer(pos4096[k][:n], pinned=p) for k, p in zip(("boards", "control", "rep", "legal"), pinned)]
+            outs = [Buffer(nbytes=n * k, pinned=p) for k, p in zip((2 * e_cap, 2 * e_cap, 4, 4), pinned[4:])]
+            edges_call(enc, n, e_cap, ins, outs)
+            assert all(o.same(w) for o, w in zip(outs, want)), (e_cap, pinned)
+        for pinned in (True, False):
+            outs = edges_buffers(n, e_cap, pinned=pinned)[:3] + [None]       # no values wanted
+            edges_call(enc, n, e_cap, inputs(pos4096, n, pinned=pinned), outs)
+            assert all(o.same(w) for o, w in zip(outs[:3], want)), (e_cap, pinned)

@@ -180,8 +180,8 @@ def test_fused_expansion_equals_the_expansion_of_its_own_logits(cap, pos4096):
 @pytest.mark.gpu
 @pytest.mark.parametrize("pinned", [True, False])
 def test_fused_expansion_host_call_matches_the_device_call(pinned, pos256):
-    """Pinned outputs are written by the kernel straight into host memory; pageable ones go
-    through the staged path (wave-sized launches, copies on a second stream)."""
+    """With every buffer pinned a batch this small is read and written by the kernel in host memory;
+    pageable buffers go through the copies."""
     from brokefish_b200.nn import encoder_impl
     from brokefish_b200.nn.model import seeded_state
     from oracle.torch_net import TorchNet
@@ -195,6 +195,7 @@ def test_fused_expansion_host_call_matches_the_device_call(pinned, pos256):
     dp, dm, dn, dv = (x.cpu().clone() for x in enc.forward_priors(boards.cuda(), control.cuda(), rep.cuda(),
                                                                   legal.cuda(), cap))
     pin = (lambda t: t.pin_memory()) if pinned else (lambda t: t)
+    boards, control, rep, legal = (pin(x) for x in (boards, control, rep, legal))
     hp = pin(torch.zeros(n, cap, dtype=torch.half))
     hm = pin(torch.zeros(n, cap, dtype=torch.int16))
     hn = pin(torch.zeros(n, dtype=torch.int32))
