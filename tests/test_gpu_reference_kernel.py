@@ -3,7 +3,8 @@
 ``oracle/build_ref.py`` compiles the reference's ``csrc/encoder.cu`` for sm_100a from the
 reference checkout and saves the weight slabs the reference's constructor derives; this file
 runs that kernel (``oracle/ref_kernel.py``) and the product on identical seeded positions and
-weights.  Skipped when the built reference is not present (it is not part of the history).
+weights.  The built reference is not part of the history: on a machine with a GPU these tests fail
+without it, after all others have run.
 
 Bar for the int8 arithmetic (the path the metric is quoted on): BIT IDENTITY.  The product
 keeps the reference kernel's own rounding points and summation orders -- LayerNorm partial
