@@ -2312,17 +2312,25 @@ int host_plan_sizes(int n, int wave, int plan, double gbps, int* sizes, bool* sl
 }
 
 // The engine kernels have two forms (bf_movegen.cuh).  Eight lanes per board: an eighth of the chain,
-// so a launch that does not fill the GPU ends sooner.  A thread per board: half of the instructions.
-// B200, us per launch, eight lanes / thread:
-//   boards                       1     4096    16384    32768    49152    98304   131072   1048576
-//   legal words             4.2/7.7  6.2/10    10/10    16/12    23/14    41/23    51/27    385/160
-//   move                    4.8/8.2  4.6/12   6.2/12   8.2/12    10/14    18/23    23/25    168/148
-//   move, words and key     6.2/18   8.2/29    16/29    27/33    37/37    70/66    90/72    688/482
-constexpr int kGroupMostWords = 16384, kGroupMostMove = 131072, kGroupMostBoth = 49152;
+// so a launch that does not fill the GPU ends sooner.  A thread per board: half of the instructions, most
+// of all where legal words are made.  B200, us per launch in a graph, eight lanes / thread:
+//   boards                      1       4096      16384      32768      49152      65536     131072    1048576
+//   legal words              3.1/6.8   4.2/8.6   8.6/8.6    15/11      21/13      27/16      50/24     384/159
+//   key                      2.2/7.6   3.1/12    5.8/12     8.8/13     12/14      15/16      27/27     203/176
+//   move                     2.1/7.2   2.6/11    4.4/11     6.7/11     9.0/12     11/13      21/24     166/146
+//   move and key             3.5/14    4.4/20    8.7/20     14/22      20/24      25/27      47/50     364/314
+//   move and words           4.3/13    5.4/17    11/18      19.7/20.2  28/23      37/27      70/47     541/304
+//   move, words and key      5.3/20    6.9/27    15/27      25/31      35.6/35.8  46/42      89/70     684/480
+//   random move and words    5.2/17    6.4/25    13/26      23/29      32.7/32.6  42/37      81/62
+int group_form_most(bool step, bool pick, bool words, bool key) {
+    if (!words) return 131072;
+    if (!step) return 16384;
+    return pick || key ? 49152 : 32768;
+}
 template <bool kStep, bool kPick, class... Args>
-void launch_engine(cudaStream_t stream, bool words_or_key, const uint16_t* boards, const int16_t* control, const int* move,
+void launch_engine(cudaStream_t stream, bool words, bool key, const uint16_t* boards, const int16_t* control, const int* move,
                    const signed char* promo, const float* r, int n, Args... rest) {
-    if (n <= (!kStep ? kGroupMostWords : words_or_key ? kGroupMostBoth : kGroupMostMove))
+    if (n <= group_form_most(kStep, kPick, words, key))
         bfmg::engine_group_kernel<kStep, kPick><<<(n + bfmg::kEngineBoards - 1) / bfmg::kEngineBoards,
                                                   bfmg::kEngineThreads, 0, stream>>>(boards, control, move, promo, r, n, rest...);
     else
@@ -2565,7 +2573,7 @@ int bf_movegen(int device, const uint16_t* boards, const int16_t* control, int n
     if (boards == nullptr || control == nullptr || mask == nullptr)
         return fail(BF_EINVAL, "boards, control and mask must be non-null");
     BF_ON_DEVICE(device);
-    launch_engine<false, false>(static_cast<cudaStream_t>(stream), true,
+    launch_engine<false, false>(static_cast<cudaStream_t>(stream), true, false,
         boards, control, nullptr, nullptr, nullptr, n, nullptr, nullptr, nullptr,
         reinterpret_cast<unsigned long long*>(mask), in_check, nullptr, nullptr);
     BF_CUDA(cudaGetLastError());
@@ -2578,7 +2586,7 @@ int bf_hash(int device, const uint16_t* boards, const int16_t* control, int n, u
     if (boards == nullptr || control == nullptr || hash == nullptr)
         return fail(BF_EINVAL, "boards, control and hash must be non-null");
     BF_ON_DEVICE(device);
-    launch_engine<false, false>(static_cast<cudaStream_t>(stream), true,
+    launch_engine<false, false>(static_cast<cudaStream_t>(stream), false, true,
         boards, control, nullptr, nullptr, nullptr, n, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
         reinterpret_cast<unsigned long long*>(hash));
     BF_CUDA(cudaGetLastError());
@@ -2643,7 +2651,7 @@ int bf_step(int device, const uint16_t* boards, const int16_t* control, const in
     if (boards == nullptr || control == nullptr || move == nullptr || boards_out == nullptr || control_out == nullptr)
         return fail(BF_EINVAL, "boards, control, move, boards_out and control_out must be non-null");
     BF_ON_DEVICE(device);
-    launch_engine<true, false>(static_cast<cudaStream_t>(stream), mask != nullptr || hash != nullptr,
+    launch_engine<true, false>(static_cast<cudaStream_t>(stream), mask != nullptr, hash != nullptr,
         boards, control, move, promo, nullptr, n, boards_out, control_out, irreversible,
         reinterpret_cast<unsigned long long*>(mask), in_check, nullptr, reinterpret_cast<unsigned long long*>(hash));
     BF_CUDA(cudaGetLastError());
@@ -2691,7 +2699,7 @@ int bf_random_ply(int device, uint16_t* boards, int16_t* control, uint64_t* mask
     if (boards == nullptr || control == nullptr || mask == nullptr || r == nullptr)
         return fail(BF_EINVAL, "boards, control, mask and r must be non-null");
     BF_ON_DEVICE(device);
-    launch_engine<true, true>(static_cast<cudaStream_t>(stream), true,
+    launch_engine<true, true>(static_cast<cudaStream_t>(stream), true, false,
         boards, control, nullptr, promo, r, n, boards, control, nullptr,
         reinterpret_cast<unsigned long long*>(mask), nullptr, move, nullptr);
     BF_CUDA(cudaGetLastError());

@@ -272,7 +272,7 @@ def test_position_keys_repetition_ring_and_threefold_rule():
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("n", [1, 3, 4097, 16384, 16385, 49152, 49153, 131072, 131073])
+@pytest.mark.parametrize("n", [1, 3, 4097, 16384, 16385, 32768, 32769, 49152, 49153, 131072, 131073])
 def test_both_forms_of_the_engine_kernels_agree_at_every_size(n, pos4096):
     """The launches pick eight lanes or one thread per board by their size: on either side of the
     line, and with a ragged last block, every board gets the answer it gets in a batch of 4096."""
@@ -295,3 +295,9 @@ def test_both_forms_of_the_engine_kernels_agree_at_every_size(n, pos4096):
         assert torch.equal(g, w[place])
     for g, w in zip(env.step(b, c, move[place], promo[place])[:2], want[3:5]):      # the move alone
         assert torch.equal(g, w[place])
+    moved = env.step(b, c, move[place], promo[place], hash=key[place])              # ... with its key
+    words = env.step(b, c, move[place], promo[place], with_moves=True)              # ... with legal words
+    for g, w in zip(moved, want[3:7]):
+        assert torch.equal(g, w[place])
+    for k in (0, 1, 3, 4, 5):
+        assert torch.equal(words[k], want[3 + k][place])
