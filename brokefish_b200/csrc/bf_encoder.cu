@@ -2081,19 +2081,29 @@ __global__ void scales_kernel(unsigned long long* differ) {
 }
 
 // ------------------------------------------------------------------------------------------
-// Tensor-core self test: one tile, one GEMM, no network.
+// Tensor-core self test: one tile, one GEMM, no network.  Modes 0-4 are the four-board kernel's products (128
+// rows), the others the small tiles' weight-stationary ones (32 or 64 rows), read out of tensor memory where
+// bf_encoder_ws.cuh looks for them.
 // ------------------------------------------------------------------------------------------
+constexpr int kSelftestModes = 15;
+constexpr uint32_t kSelftestW = 65536, kSelftestBar = kSelftestW + 131072, kSelftestSmem = kSelftestBar + 128 + 1024;
 __global__ void __launch_bounds__(128, 1) selftest_kernel(int mode, const uint8_t* a, const uint8_t* w,
                                                           uint32_t* out, int* status) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const uint32_t smem = smem_u32(sm);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, row = threadIdx.x;
-    const int n = mode == 2 ? 192 : (mode == 3 ? 96 : 128);
-    const int slabs = mode == 3 ? 4 : 2;
-    const uint32_t w_stage = n * 128;
-    // layout: A slabs at 0 (slabs x 16 KB), W at 65536, barriers at 163840
-    constexpr uint32_t kW = 65536, kBar = 163840;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool ws = mode >= 5;
+    const int rows = ws ? 32 << ((mode - 5) & 1) : 128;
+    enum { kS8, kU8, kF16to32, kE4M3, kF16 };
+    const int what = ws ? (mode < 7 ? kS8 : mode < 9 ? kU8 : mode < 11 ? kF16 : mode < 13 ? kE4M3 : kF16)
+                        : (mode == 1 ? kU8 : mode == 3 ? kF16to32 : mode == 4 ? kE4M3 : kS8);
+    const int n = ws ? (mode < 13 ? 256 : 128) : mode == 2 ? 192 : (mode == 3 ? 96 : 128);
+    const bool halves = what == kF16to32 || what == kF16;
+    const int slabs = halves ? 4 : 2;
+    const uint32_t w_stage = n * 128, a_slab = rows * 128;
+    // layout: A slabs at 0 (up to 64 KB), W after them (up to 128 KB), barriers
+    constexpr uint32_t kW = kSelftestW, kBar = kSelftestBar;
     volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + kBar + 64);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + kBar + 68);
     if (threadIdx.x == 0) {
@@ -2103,11 +2113,12 @@ __global__ void __launch_bounds__(128, 1) selftest_kernel(int mode, const uint8_
         fence_barrier_init();
     }
     if (warp == 0) { tmem_alloc(smem + kBar + 68, 256); tmem_relinquish(); }
-    // A: row-major [128][slabs*128 B] -> swizzled slabs, written by the generic proxy
-    for (int s = 0; s < slabs; ++s)
-        for (int k = 0; k < 8; ++k)
-            *reinterpret_cast<uint4*>(sm + s * 16384 + sw_off(row, k)) =
-                *reinterpret_cast<const uint4*>(a + static_cast<size_t>(row) * slabs * 128 + s * 128 + k * 16);
+    // A: row-major [rows][slabs*128 B] -> swizzled slabs, written by the generic proxy
+    if (static_cast<int>(threadIdx.x) < rows)
+        for (int s = 0; s < slabs; ++s)
+            for (int k = 0; k < 8; ++k)
+                *reinterpret_cast<uint4*>(sm + s * a_slab + sw_off(threadIdx.x, k)) =
+                    *reinterpret_cast<const uint4*>(a + static_cast<size_t>(threadIdx.x) * slabs * 128 + s * 128 + k * 16);
     fence_proxy_async_smem();
     tc_fence_before();
     __syncthreads();
@@ -2118,30 +2129,38 @@ __global__ void __launch_bounds__(128, 1) selftest_kernel(int mode, const uint8_
         for (int s = 0; s < slabs; ++s) bulk_g2s(smem + kW + s * w_stage, w + s * w_stage, w_stage, smem + kBar);
         mbar_wait(smem + kBar, 0, abort_flag, kErrMmaWeights);
         tc_fence_after();
-        const uint32_t idesc = mode == 0 ? umma_idesc(kAccS32, kFmtS8, kFmtS8, 128, 128)
-                             : mode == 1 ? umma_idesc(kAccS32, kFmtU8, kFmtS8, 128, 128)
-                             : mode == 2 ? umma_idesc(kAccS32, kFmtS8, kFmtS8, 128, 192)
-                             : mode == 3 ? umma_idesc(kAccF32, kFmtF16, kFmtF16, 128, 96)
-                                         : umma_idesc(kAccF32, kFmtE4M3, kFmtE4M3, 128, 128);
+        const uint32_t idesc = what == kS8        ? umma_idesc(kAccS32, kFmtS8, kFmtS8, rows, n)
+                             : what == kU8        ? umma_idesc(kAccS32, kFmtU8, kFmtS8, rows, n)
+                             : what == kF16to32   ? umma_idesc(kAccF32, kFmtF16, kFmtF16, rows, n)
+                             : what == kF16       ? umma_idesc(kAccF16, kFmtF16, kFmtF16, rows, n)
+                                                  : umma_idesc(kAccF32, kFmtE4M3, kFmtE4M3, rows, n);
         for (int s = 0; s < slabs; ++s) {
-            const uint64_t ad = umma_desc_k128(smem + s * 16384), bd = umma_desc_k128(smem + kW + s * w_stage);
+            const uint64_t ad = umma_desc_k128(smem + s * a_slab), bd = umma_desc_k128(smem + kW + s * w_stage);
             for (int k = 0; k < 4; ++k) {
-                if (mode == 3)      umma_f16(tmem, ad + 2 * k, bd + 2 * k, idesc, (s | k) ? 1u : 0u);
-                else if (mode == 4) umma_f8(tmem, ad + 2 * k, bd + 2 * k, idesc, (s | k) ? 1u : 0u);
-                else                umma_i8(tmem, ad + 2 * k, bd + 2 * k, idesc, (s | k) ? 1u : 0u);
+                const uint32_t more = (s | k) ? 1u : 0u;
+                if (ws && halves)             umma_ws_f16(tmem, ad + 2 * k, bd + 2 * k, idesc, more);
+                else if (ws && what == kE4M3) umma_ws_f8(tmem, ad + 2 * k, bd + 2 * k, idesc, more);
+                else if (ws)                  umma_ws_i8(tmem, ad + 2 * k, bd + 2 * k, idesc, more);
+                else if (halves)              umma_f16(tmem, ad + 2 * k, bd + 2 * k, idesc, more);
+                else if (what == kE4M3)       umma_f8(tmem, ad + 2 * k, bd + 2 * k, idesc, more);
+                else                          umma_i8(tmem, ad + 2 * k, bd + 2 * k, idesc, more);
             }
         }
         tc_commit(smem + kBar + 8);
     }
     mbar_wait(smem + kBar + 8, 0, abort_flag, kErrRowAcc);
+    __syncwarp();
     tc_fence_after();
-    for (int c0 = 0; c0 < n; c0 += 32) {
+    // lane quadrant `warp`: its rows, and its first column and how many of them
+    const int row = rows == 128 ? 32 * warp + lane : rows == 64 ? 32 * (warp & 1) + lane : lane;
+    const int columns = rows == 128 ? n : rows == 64 ? n / 2 : n / 4;
+    const int first = rows == 128 ? 0 : rows == 64 ? columns * (warp >> 1) : columns * warp;
+    for (int c0 = 0; c0 < columns; c0 += 32) {
         uint32_t acc[32];
         tmem_ld32(tmem + (static_cast<uint32_t>(32 * warp) << 16) + c0, acc);
         tmem_wait_ld();
-        for (int i = 0; i < 32; ++i) out[static_cast<size_t>(row) * n + c0 + i] = acc[i];
+        for (int i = 0; i < 32; ++i) out[static_cast<size_t>(row) * n + first + c0 + i] = acc[i];
     }
-    (void)lane;
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -3144,15 +3163,14 @@ int bf_selftest_scales(int device, unsigned long long* differ) {
 }
 
 int bf_selftest_umma(int device, int mode, const void* a, const void* w_image, void* out) {
-    if (mode < 0 || mode > 4 || a == nullptr || w_image == nullptr || out == nullptr)
+    if (mode < 0 || mode >= bf::kSelftestModes || a == nullptr || w_image == nullptr || out == nullptr)
         return fail(BF_EINVAL, "bad self-test argument");
     BF_ON_DEVICE(device);
     int* status = nullptr;
     BF_CUDA(cudaMalloc(&status, sizeof(int)));
     BF_CUDA(cudaMemset(status, 0, sizeof(int)));
-    constexpr int kSmem = 163840 + 128 + 1024;
-    BF_CUDA(cudaFuncSetAttribute(bf::selftest_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
-    bf::selftest_kernel<<<1, 128, kSmem>>>(mode, static_cast<const uint8_t*>(a),
+    BF_CUDA(cudaFuncSetAttribute(bf::selftest_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bf::kSelftestSmem));
+    bf::selftest_kernel<<<1, 128, bf::kSelftestSmem>>>(mode, static_cast<const uint8_t*>(a),
                                            static_cast<const uint8_t*>(w_image),
                                            static_cast<uint32_t*>(out), status);
     cudaError_t e = cudaGetLastError();

@@ -409,7 +409,7 @@ class FusedEncoder:
 
     def capture_gemm(self, boards, control, rep, layer: int, op: int):
         """``(A bytes [n*32,256] uint8, accumulators [n*32,N] int32)`` of one GEMM of one
-        layer, exactly as the tensor cores saw and produced them."""
+        layer, exactly as the tensor cores saw and produced them (in the four-board kernel)."""
         self._require_net("capture_gemm")
         n = self._check_inputs(boards, control, rep)
         width = _OP_WIDTH.get(op, 256)
@@ -440,6 +440,7 @@ class FusedEncoder:
 
     # -- in-kernel phase accounting (the reference's set_profile / read_profile hooks) ----
     def set_profile(self, on: bool) -> None:
+        """The phase clock, and with it the four-board kernel for every call while it is on."""
         _native.check(_native.lib().bf_profile(self._handle, int(bool(on))), "bf_profile")
 
     def read_profile(self) -> dict:

@@ -210,7 +210,10 @@ int bf_forward_backbone(bf_handle* h, const void* x, const int8_t* alive, int n,
 /* Activations at an intermediate stage as [n,32,256] fp16.  Replaces
  * `model_forward(..., debug_stage=stage)` (csrc/encoder.cu:1315-1427, 1575-1598):
  * 9 embedding; layer 0: 1 LN1 out, 5/6/7 Q/K/V after bias, 4 attention out,
- * 2 residual after attention, 3 LN2 out; 8 final norm out. */
+ * 2 residual after attention, 3 LN2 out; 8 final norm out.  This call, bf_forward_stage_at,
+ * bf_forward_capture and bf_profile run the four-board kernel, whatever tiles bf_forward would take
+ * (bf_tile_boards): the outputs of both are equal bit for bit, the phase clock's cycles are not those
+ * of the small tiles. */
 int bf_forward_stage(bf_handle* h, const uint16_t* boards, const int16_t* control,
                      const uint8_t* rep, int n, int stage, void* y, void* stream);
 
@@ -305,7 +308,8 @@ long long bf_launch_count(const bf_handle* h);
  * 1886-1916).  While enabled, one thread of every CTA charges its clock cycles to the phase
  * it is in; `bf_profile_read` synchronises, returns the cycle sums since the last read (up
  * to 16 values, in the order `bf_profile_phases()` names them, comma separated) and clears
- * them.  Enabling or disabling also clears. */
+ * them.  Enabling or disabling also clears.  Enabled, every call runs the four-board kernel, which alone
+ * has the clock. */
 int bf_profile(bf_handle* h, int enable);
 int bf_profile_read(bf_handle* h, long long* cycles, int n);
 const char* bf_profile_phases(void);
@@ -394,13 +398,18 @@ int bf_selftest_timeout(int device, int code, int* status, long long* waited_cyc
  * maxima, infinity included, for the s8, u8 and e4m3 ranges, `differ[3]` over every fp32 softmax sum from 1 to 32. */
 int bf_selftest_scales(int device, unsigned long long* differ);
 
-/* Tensor-core self test (no network): one 128-row tile times a packed weight tile.
+/* Tensor-core self test (no network): one tile times a packed weight tile.  128-row products, the
+ * four-board kernel's:
  *   mode 0: s8 x s8, N=128, K=256     mode 1: u8 x s8, N=128, K=256
  *   mode 2: s8 x s8, N=192, K=256     mode 3: f16 x f16 -> f32, N=96, K=256
  *   mode 4: e4m3 x e4m3 -> f32, N=128, K=256
- *   a        device, [128, K] row-major (1 byte or 2 bytes per element)
+ * and the small tiles' weight-stationary ones, of M = 32 rows in the odd modes and 64 in the even ones:
+ *   modes 5, 6: s8 x s8, N=256        modes 7, 8: u8 x s8, N=256
+ *   modes 9, 10: f16 x f16 -> f16, N=256     modes 11, 12: e4m3 x e4m3 -> f32, N=256
+ *   modes 13, 14: f16 x f16 -> f16, N=128
+ *   a        device, [M, K] row-major (1 byte or 2 bytes per element)
  *   w_image  device, K/ (128 B) stage images of [N, 128 B] (pack.py: sw128_image)
- *   out      device, [128, N] s32 (modes 0-2) or f32 (modes 3, 4)
+ *   out      device, [M, N] words: s32, f32, or f16 in the low half
  * Follows the exact-integer method of the reference's csrc/tests/tint8.cu:268-337. */
 int bf_selftest_umma(int device, int mode, const void* a, const void* w_image, void* out);
 

@@ -196,7 +196,9 @@ def test_layer0_stages(name, encoders, oracle_weights, pos256):
 @pytest.mark.parametrize("name,layer", [("A", 0), ("B", 0), ("A", 5), ("B", 7)])
 def test_s32_accumulators_are_bit_exact(name, layer, encoders, oracle_weights, pos256):
     """Every weight GEMM of a layer: the captured A bytes times the packed s8 weights,
-    recomputed on the host in int64, equals the captured tensor-core accumulators."""
+    recomputed on the host in int64, equals the captured tensor-core accumulators.  The capture runs the
+    four-board kernel; the small tiles' products are held by test_gpu_tiles.py, against the host and by
+    outputs equal to this kernel's."""
     from brokefish_b200.nn.pack import qkv_chunk_rows
     enc = encoders[name]
     lw = oracle_weights[name].layers[layer]
@@ -424,8 +426,8 @@ def test_input_rejection_and_empty_batch(encoders):
 
 
 def test_phase_profile_hooks(encoders, pos256):
-    """The in-kernel phase clock: off by default, sums cycles per phase when on, and leaves
-    the outputs untouched (the reference's bench/bench_phases.py protocol)."""
+    """The in-kernel phase clock (of the four-board kernel): off by default, sums cycles per phase when
+    on, and leaves the outputs untouched (the reference's bench/bench_phases.py protocol)."""
     enc = encoders["A"]
     args = inputs(pos256, slice(0, 256))
     base = enc.forward_full(*args)[0].cpu().numpy().copy()

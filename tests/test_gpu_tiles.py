@@ -1,5 +1,6 @@
 """The evaluator on one- and two-board tiles: at every size where the tiling changes, a position's
-outputs are those it gets in any other batch, in every arithmetic; and the arithmetic helpers the tiles
+outputs are those it gets in any other batch, in every arithmetic, and those of the four-board kernel,
+which carries the dumps and captures; the tiles' products are exact; and the arithmetic helpers the tiles
 use instead of divisions equal division on everything they can be given."""
 import ctypes
 
@@ -41,6 +42,56 @@ def test_every_tiling_gives_a_position_the_same_outputs(arithmetic, nets, pos409
             for got, w in zip(enc.forward_full(*(t[:n] for t in (b, c, r, legal))), want):
                 assert torch.equal(got, w[:n]), (one, n)
     enc.check_status()
+
+
+@pytest.mark.parametrize("arithmetic", ARITHMETICS)
+def test_the_instrumented_kernel_gives_the_small_tiles_outputs(arithmetic, nets, pos4096):
+    """Stage dumps, operand captures and the phase clock exist in the four-board kernel alone: what they show
+    holds for the kernel that evaluates because both give the same bits."""
+    from brokefish_b200.nn.cuda_impl import FusedEncoder
+    enc = FusedEncoder(nets["B"], **ARITHMETICS[arithmetic])
+    n = 301
+    args = [cu(pos4096[k][:n]) for k in ("boards", "control", "rep")] + [cu(pos4096["legal"][:n].view(np.int64))]
+    want = [t.clone() for t in enc.forward_full(*args)]
+    enc.set_profile(True)
+    for got, w in zip(enc.forward_full(*args), want):
+        assert torch.equal(got, w)
+    enc.set_profile(False)
+    enc.check_status()
+
+
+@pytest.mark.parametrize("rows", [32, 64])
+@pytest.mark.parametrize("what", ["s8", "u8", "f16", "e4m3", "f16 heads"])
+def test_weight_stationary_products(what, rows):
+    """The small tiles' tensor-core products, read where the kernel reads them, against exact host products:
+    bytes over their full range, fp16 and e4m3 operands whose sums are all representable."""
+    from brokefish_b200 import _native
+    from brokefish_b200.nn.pack import sw128_image
+    rng = np.random.default_rng(rows)
+    n = 128 if what == "f16 heads" else 256
+    if what in ("s8", "u8"):
+        a = rng.integers(0 if what == "u8" else -128, 256 if what == "u8" else 128, size=(rows, 256))
+        w = rng.integers(-128, 128, size=(n, 256))
+        a[0, :], w[0, :] = (255 if what == "u8" else -128), -128
+        a_bytes, w_bytes = a.astype(np.uint8 if what == "u8" else np.int8).view(np.uint8), w.astype(np.int8).view(np.uint8)
+    else:
+        a, w = rng.integers(-2, 3, size=(rows, 256)), rng.integers(-2, 3, size=(n, 256))
+        if what == "e4m3":
+            a_bytes, w_bytes = (torch.from_numpy(m.astype(np.float32)).to(torch.float8_e4m3fn).view(torch.uint8).numpy()
+                                for m in (a, w))
+        else:
+            a_bytes, w_bytes = a.astype(np.float16).view(np.uint8), w.astype(np.float16).view(np.uint8)
+    image = np.concatenate([sw128_image(np.ascontiguousarray(w_bytes[:, s:s + 128])) for s in range(0, w_bytes.shape[1], 128)])
+    d_a, d_w, d_out = cu(a_bytes), cu(image), torch.zeros(rows, n, dtype=torch.int32, device="cuda")
+    mode = 5 + 2 * ["s8", "u8", "f16", "e4m3", "f16 heads"].index(what) + (rows == 64)
+    _native.check(_native.lib().bf_selftest_umma(0, mode, *(ctypes.c_void_p(t.data_ptr()) for t in (d_a, d_w, d_out))),
+                  "bf_selftest_umma")
+    got = d_out.cpu().numpy()
+    if what == "e4m3":
+        got = got.view(np.float32)
+    elif what.startswith("f16"):
+        got = np.ascontiguousarray(got.view(np.float16)[:, ::2])
+    assert np.array_equal(got.astype(np.int64), a.astype(np.int64) @ w.astype(np.int64).T)
 
 
 def test_scales_and_reciprocals_equal_division():
