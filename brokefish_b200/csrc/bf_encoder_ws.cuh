@@ -25,9 +25,10 @@
 // Measured on one B200, int8, against the forms before it (four boards per tile; one board per tile
 // with its rows written four times into a 128-row operand), through the device-pointer call: batch 1
 // 90 us (176), 64 92 us (176), 149-296 127 us (281), 333 215 us (285), 4096 1.69 ms (1.98).  What bounds
-// it: the row warps, four to a scheduler and all in the same phase.  Issue slots are about half busy,
-// the tensor pipe a fifth; the rest is the latency of a phase's first loads and of the three products
-// per layer that start only when their operand has been written (about 1,100 cycles each).
+// it: the row warps, four to a scheduler and all in the same phase.  At 4096 issue slots are 58 % busy, the
+// tensor pipe 25 %.  Of a one-board tile's 19,800 cycles per layer a row warp waits 5,400 for products
+// (1,000 to 1,350 after each norm and after attention, whose operand has just been written), of a
+// two-board tile's 27,000 5,500; the rest is its own dependent instructions and the board's meetings.
 #pragma once
 
 namespace bf {
@@ -137,9 +138,8 @@ __device__ __forceinline__ void wait_acc(const Row& c, int slot, int use) {
     tc_fence_after();
 }
 // The scales and biases of the layer this thread is at (two copies, filled by the weight stream a layer
-// ahead): shared address of the layer's block.  From L1 they came late: beside 228 KB of shared memory
-// the eight layers' 37 KB do not stay there, and the loads could not be issued ahead of the wait for
-// the product they go with (3 to 6 % of a tile).
+// ahead): shared address of the layer's block.  Read through L1, beside 228 KB of shared memory, they
+// cost 3 to 6 % of a tile more.
 __device__ __forceinline__ uint32_t layer_params(const Row& c) {
     return c.smem + SM_PAR + (c.layers & 1u) * kLparamStride;
 }
@@ -1012,9 +1012,7 @@ struct Issue {
 };
 // One product: `slabs` K-slabs of 128 bytes; `more`: on top of what the slot holds; `done`: the slot's
 // barrier that its completion goes to (-1: none).  The whole warp walks the schedule and waits; one
-// elected lane -- the same every time -- issues.  (A loop inside the elected branch keeps its addresses
-// in the warp's uniform registers while the other lanes run on to the branch's end, at any time.)  Stage
-// by stage: waiting for two at once, which the four-board form gains from, costs 5 % of a one-board
+// elected lane -- the same every time -- issues.  Stage by stage: waiting for two at once, which the four-board form gains from, costs 5 % of a one-board
 // tile and 19 % of a two-board one in fp16, where the stages arrive no sooner than they are wanted.
 template <int kAr, int kKind>
 __device__ __forceinline__ void issue_unit(Issue& st, uint32_t d, uint32_t a_base, uint32_t slab, int slabs, uint32_t idesc,

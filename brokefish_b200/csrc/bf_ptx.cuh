@@ -12,12 +12,10 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-// One lane of the warp (all 32 take part), chosen by `elect.sync`, the same one every time.  A region
-// entered through this predicate is one the compiler knows to be executed by a single thread: the
-// descriptors of the tensor-core and bulk-copy instructions in it are built in uniform registers.
-// Under `lane == 0` it cannot know that and wraps every such instruction in a loop over the active
-// lanes.  Keep such a region free of waits: the uniform registers belong to the whole warp, whose other
-// lanes run on to the end of the branch meanwhile.
+// One lane of the warp (all 32 take part), chosen by `elect.sync`, the same one every time.  Tensor-core
+// and bulk-copy instructions issued in a region entered through this predicate take 60 to 100 cycles
+// each, under `lane == 0` 134 (measured).  Such a region holds no wait: the whole warp waits, then one lane
+// issues.
 __device__ __forceinline__ bool elect_one() {
     uint32_t pred;
     asm volatile(
@@ -43,8 +41,8 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t byt
                  : "memory");
 }
 // One try: the thread is parked by the hardware until the phase completes or the hardware's own time
-// limit has passed.  (With a suspend-time hint the instruction becomes a check and a timed sleep, which
-// wakes later: 4 % of a one-board tile, 2 % of a batch of 4096.)
+// limit has passed.  (With a suspend-time hint waiting warps come back later: 4 % of a one-board tile, 2 %
+// of a batch of 4096.)
 __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
@@ -201,18 +199,6 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8])
         ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
         : "memory");
 }
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]),
-          "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]),
-          "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]),
-          "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]),
-          "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
-        : "memory");
-}
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
@@ -324,15 +310,6 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t sad
                  : "r"(saddr)
                  : "memory");
 }
-// D(16x8, f32) += A(16x16, f16) * B(16x8, f16)
-__device__ __forceinline__ void mma_f16_f32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0,
-                                            uint32_t b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 "
-        "{%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
 // D(16x8, f16) += A(16x16, f16) * B(16x8, f16): fp16 accumulators (two packed pairs: row g
 // and row g + 8 of this lane's two columns), the form the reference's attention and head
 // products use (csrc/mma.cuh), so the same operands give the same bits.
@@ -388,7 +365,7 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
     return d;
 }
 // Note on two-step roundings: a packed multiply followed by a packed add (also when the add is
-// written as fma(x, 1.0, b) with a literal 1.0) may come out of the assembler as one fused
+// written as fma(x, 1.0, b) with a literal 1.0) has given the results of one fused
 // multiply-add.  Where the product must be rounded on its own, feed the add an fma whose unit
 // multiplier is a run-time value (see `quant16` in bf_encoder.cu).
 __device__ __forceinline__ uint64_t h2_to_f2(uint32_t h) {
