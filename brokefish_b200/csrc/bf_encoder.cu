@@ -1821,9 +1821,9 @@ __global__ void __launch_bounds__(kThreads, 1) encoder_kernel(const Params p) {
 // CUDA-core probe: what one SM sustains on the element-wise building blocks of the row warps when
 // nothing else is in the way -- operands in shared memory, sixteen warps resident as in the
 // evaluator, no tensor-memory loads, no exchanges, no barriers.  The same device functions the
-// evaluator calls.  Block 0: ff1 epilogue (s32 -> descale -> bias + ReLU -> row maximum -> u8);
+// small tiles call, sixteen columns at a time, biases from shared memory.  Block 0: ff1 epilogue (s32 -> descale -> bias + ReLU -> row maximum -> u8);
 // 1: descale + bias -> fp16 (QKV and out-projection epilogues); 2: ff2 step (descale, fused add
-// to the fp16 running total); 3: norm statistics (sum, sum of squares, minimum, maximum); 4:
+// to the fp16 running total); 3: norm statistics (sums, sums of squares, minimum, maximum); 4:
 // normalise -> fp16 -> s8; 5: fp16 -> int8 quantisation alone; 8-11: the cheaper forms of blocks 0,
 // 4, 1 and 2 that a not-bit-exact arithmetic could use (one combined scale, the requantisation in
 // fp16 or fused into the normalise), to measure what giving up the reference's bits would buy.
@@ -1837,33 +1837,39 @@ __global__ void __launch_bounds__(kProbeThreads, 1) elementwise_probe_kernel(con
     extern __shared__ uint32_t probe_sm[];
     const int tid = threadIdx.x;
     for (int i = tid; i < 32 * kProbeThreads; i += kProbeThreads) probe_sm[i] = 0x3c003800u + ((i * 2654435761u) >> 20);
+    if (tid < 16) probe_sm[32 * kProbeThreads + tid] = __ldg(reinterpret_cast<const uint32_t*>(bias) + tid);
+    const uint32_t bias_at = smem_u32(probe_sm + 32 * kProbeThreads);
     __syncthreads();
     const uint64_t one2 = pk2(one, one), sa2 = pk2(sa, sa), sw2 = pk2(sw, sw);
     float m = 0.f;
     uint32_t keep = 0;
-    uint64_t sum2 = pk2(0.f, 0.f), sq2 = pk2(0.f, 0.f);
+    float part[4] = {0.f, 0.f, 0.f, 0.f}, square[4] = {0.f, 0.f, 0.f, 0.f};
     __half2 mn = __float2half2_rn(65504.0f), mx = __float2half2_rn(-65504.0f);
     uint32_t run[16];
 #pragma unroll
     for (int i = 0; i < 16; ++i) run[i] = 0;
     for (int it = 0; it < iters; ++it) {
-        uint32_t acc[32], o[16];
+        uint32_t acc[32], lower[16], upper[16], o[16];
         if (kBlock <= 2 || kBlock == 8 || kBlock >= 10) {
 #pragma unroll
             for (int k = 0; k < 32; ++k) acc[k] = probe_sm[k * kProbeThreads + tid] + it;
+#pragma unroll
+            for (int k = 0; k < 16; ++k) { lower[k] = acc[k]; upper[k] = acc[16 + k]; }
         } else {
 #pragma unroll
             for (int k = 0; k < 16; ++k) o[k] = probe_sm[k * kProbeThreads + tid] ^ (it & 1);
         }
         if (kBlock == 0) {
-            descale<32, true, kAccInt>(acc, sa, sw, bias, o);
+            ws::descale16<true, kAccInt>(lower, sa, sw, ws::load_bias(bias_at), &o[0]);
+            ws::descale16<true, kAccInt>(upper, sa, sw, ws::load_bias(bias_at + 32), &o[8]);
             const float am = amax_h2<16>(o, false);
             m = fmaxf(m, am);
-            const float inv = 255.0f / fmaxf(am, 1e-3f);
+            const float inv = ws::scale_u8(am).inverse;
             const uint4 a = quant16(&o[0], inv, one2), b = quant16(&o[8], inv, one2);
             keep ^= a.x ^ a.y ^ a.z ^ a.w ^ b.x ^ b.y ^ b.z ^ b.w;
         } else if (kBlock == 1) {
-            descale<32, false, kAccInt>(acc, sa, sw, bias, o);
+            ws::descale16<false, kAccInt>(lower, sa, sw, ws::load_bias(bias_at), &o[0]);
+            ws::descale16<false, kAccInt>(upper, sa, sw, ws::load_bias(bias_at + 32), &o[8]);
 #pragma unroll
             for (int k = 0; k < 16; ++k) probe_sm[(16 + k) * kProbeThreads + tid] = o[k];
         } else if (kBlock == 2) {
@@ -1877,15 +1883,17 @@ __global__ void __launch_bounds__(kProbeThreads, 1) elementwise_probe_kernel(con
         } else if (kBlock == 3) {
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
-                const uint64_t f = h2_to_f2(o[i]);
-                sum2 = add2(sum2, f);
-                sq2 = fma2(f, f, sq2);
+                sum_h2(o[i], part[i >> 2], square[i >> 2]);
                 mn = __hmin2(mn, as_h2(o[i]));
                 mx = __hmax2(mx, as_h2(o[i]));
             }
         } else if (kBlock == 4) {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) o[i] = f2_to_h2(mul2(add2(h2_to_f2(o[i]), sa2), sw2));
+            for (int i = 0; i < 16; ++i) {
+                float a0, a1;
+                upk2(add_h2_f(o[i], sa), a0, a1);
+                o[i] = pack_h2(__fmul_rn(a0, sw), __fmul_rn(a1, sw));
+            }
             const uint4 a = quant16(&o[0], sa, one2), b = quant16(&o[8], sa, one2);
             keep ^= a.x ^ a.y ^ a.z ^ a.w ^ b.x ^ b.y ^ b.z ^ b.w;
         } else if (kBlock == 5) {
@@ -1962,13 +1970,11 @@ __global__ void __launch_bounds__(kProbeThreads, 1) elementwise_probe_kernel(con
             }
         }
     }
-    float a, b, c, d;
-    upk2(sum2, a, b);
-    upk2(sq2, c, d);
 #pragma unroll
     for (int i = 0; i < 16; ++i) keep ^= run[i];
-    out[blockIdx.x * kProbeThreads + tid] =
-        m + a + b + c + d + __low2float(mn) + __high2float(mx) + __uint_as_float(keep & 0xffu);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) m += part[i] + square[i];
+    out[blockIdx.x * kProbeThreads + tid] = m + __low2float(mn) + __high2float(mx) + __uint_as_float(keep & 0xffu);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -2289,9 +2295,11 @@ bool two_board_waves(const bf_handle* h) { return h->hdr.quant != 0 && h->hdr.rj
 
 // bf_forward_host sizes its launches by how many times faster this GPU copies a position's logits
 // to the host than it evaluates a position.
+// (Of int8; one pair of figures serves every arithmetic: e4m3 produces 10.1 GB/s on two-board tiles where
+// int8 produces 10.6, fp16 9.4 on four-board ones, which moves the ratio, and a launch's size, by 5 to 7 %.)
 constexpr double kEvalGBps = 8.8;        // logits a B200 produces per second at full rate on four-board
                                          // tiles (4356 B x 2.03 M)
-constexpr double kSmallTileRate = 1.2;   // how much faster two-board tiles are (2.45 M positions/s)
+constexpr double kSmallTileRate = 1.2;   // how much faster two-board tiles are (2.42 M positions/s)
 constexpr double kFastLinkRatio = 6.0;   // a GPU alone on its link: 55 GB/s against those 8.8
 
 // The launch sizes of bf_forward_host for `n` positions on a GPU whose wave is `wave` positions:
@@ -3093,7 +3101,7 @@ int bf_measure_elementwise(int device, int block, int iters, double* elements_pe
                                        bf::elementwise_probe_kernel<8, 512>, bf::elementwise_probe_kernel<9, 512>,
                                        bf::elementwise_probe_kernel<10, 512>, bf::elementwise_probe_kernel<11, 512>};
     const int threads = block == 6 ? 256 : (block == 7 ? 1024 : 512);
-    const int kSmem = 32 * threads * 4;
+    const int kSmem = 32 * threads * 4 + 64;
     BF_CUDA(cudaFuncSetAttribute(kernels[block], cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
     const int sms = prop.multiProcessorCount;
     __half* bias = nullptr;
