@@ -674,7 +674,7 @@ __device__ __forceinline__ void prenorm_means(const Row& c, uint32_t alive, cons
     const bool live = (alive >> c.lane) & 1u;
     const int nlive = __popc(alive);
     const float inv_live = 1.0f / static_cast<float>(nlive > 0 ? nlive : 1);
-    const uint32_t means = c.smem + SM_LIST + 1024u * O::board(c) + 4u * O::col(c);
+    float2 mine = make_float2(0.f, 0.f);                     // lane i keeps column pair i
 #pragma unroll
     for (int i = 0; i < 8 * NB; ++i) {
         const float2 f = __half22float2(as_h2(x[i]));
@@ -684,17 +684,21 @@ __device__ __forceinline__ void prenorm_means(const Row& c, uint32_t alive, cons
             a0 += __shfl_xor_sync(0xffffffffu, a0, off);
             a1 += __shfl_xor_sync(0xffffffffu, a1, off);
         }
-        if (c.lane == 0) {
-            sts32(means + 8u * i, __float_as_uint(__fmul_rn(a0, inv_live)));
-            sts32(means + 8u * i + 4u, __float_as_uint(__fmul_rn(a1, inv_live)));
-        }
+        if (c.lane == i) mine = make_float2(__fmul_rn(a0, inv_live), __fmul_rn(a1, inv_live));
+    }
+    if (c.lane < 8 * NB) {
+        const uint32_t at = c.smem + SM_LIST + 1024u * O::board(c) + 4u * O::col(c) + 8u * c.lane;
+        sts32(at, __float_as_uint(mine.x));
+        sts32(at + 4u, __float_as_uint(mine.y));
     }
 }
 // The three logits, in one warp, while the head product runs: lane & 3 is the quarter of the columns
 // (32 q .. + 31 and 128 + 32 q .. + 31), lane >> 2 the sum: of the means, of their squares, of
-// means x gamma x value row k (with it gamma x value row k), of beta x value row k.
+// means x gamma x value row k (with it gamma x value row k), of beta x value row k.  Out of line: inlined, this
+// head's code slows the networks that do not have it (4096 positions, int8 1690 us against 1675, with edge
+// lists 1748 against 1727).
 template <int NB>
-__device__ __forceinline__ void prenorm_logits(const Row& c, const Params& p, float (&logit)[3]) {
+__device__ __noinline__ void prenorm_logits(const Row& c, const Params& p, float (&logit)[3]) {
     const uint32_t means = c.smem + SM_LIST + 1024u * Own<NB>::board(c);
     const int quarter = c.lane & 3, kind = c.lane >> 2, k = kind < 2 ? 0 : (kind - 2) % 3;
     float t = 0.f, t2 = 0.f;
