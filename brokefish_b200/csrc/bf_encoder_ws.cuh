@@ -24,9 +24,9 @@
 //
 // Measured on one B200, int8, against the forms before it (four boards per tile; one board per tile
 // with its rows written four times into a 128-row operand), through the device-pointer call: batch 1
-// 90 us (176), 64 92 us (176), 149-296 127 us (281), 333 215 us (285), 4096 1.69 ms (1.98).  What bounds
-// it: the row warps, four to a scheduler and all in the same phase.  At 4096 issue slots are 58 % busy, the
-// tensor pipe 25 %.  Of a one-board tile's 19,800 cycles per layer a row warp waits 5,400 for products
+// 88 us (176), 64 90 us (176), 149-296 127 us (281), 333 213 us (285), 4096 1.68 ms (1.98).  What bounds
+// it: the row warps, four to a scheduler and all in the same phase.  At 4096 issue slots are 57 % busy, the
+// tensor pipe 26 %.  Of a one-board tile's 19,800 cycles per layer a row warp waits 5,400 for products
 // (1,000 to 1,350 after each norm and after attention, whose operand has just been written), of a
 // two-board tile's 27,000 5,500; the rest is its own dependent instructions and the board's meetings.
 #pragma once
