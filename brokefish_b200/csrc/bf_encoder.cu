@@ -2356,13 +2356,17 @@ int group_form_most(bool step, bool pick, bool words, bool key) {
 }
 template <bool kStep, bool kPick, class... Args>
 void launch_engine(cudaStream_t stream, bool words, bool key, const uint16_t* boards, const int16_t* control, const int* move,
-                   const signed char* promo, const float* r, int n, Args... rest) {
-    if (n <= group_form_most(kStep, kPick, words, key))
+                   const signed char* promo, const float* r, int n, uint16_t* boards_out, Args... rest) {
+    // (a thread per board moves boards in 16-byte pieces; eight lanes take them wherever they start)
+    const bool pieces = ((reinterpret_cast<uintptr_t>(boards) | reinterpret_cast<uintptr_t>(boards_out)) & 15u) == 0;
+    if (n <= group_form_most(kStep, kPick, words, key) || !pieces)
         bfmg::engine_group_kernel<kStep, kPick><<<(n + bfmg::kEngineBoards - 1) / bfmg::kEngineBoards,
-                                                  bfmg::kEngineThreads, 0, stream>>>(boards, control, move, promo, r, n, rest...);
+                                                  bfmg::kEngineThreads, 0, stream>>>(boards, control, move, promo, r, n, boards_out,
+                                                                                     rest...);
     else
         bfmg::engine_board_kernel<kStep, kPick><<<(n + bfmg::kTpbThreads - 1) / bfmg::kTpbThreads, bfmg::kTpbThreads,
-                                                  bfmg::kTpbSmem, stream>>>(boards, control, move, promo, r, n, rest...);
+                                                  bfmg::kTpbSmem, stream>>>(boards, control, move, promo, r, n, boards_out,
+                                                                                  rest...);
 }
 
 struct PriorOut {

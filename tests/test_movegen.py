@@ -301,3 +301,23 @@ def test_both_forms_of_the_engine_kernels_agree_at_every_size(n, pos4096):
         assert torch.equal(g, w[place])
     for k in (0, 1, 3, 4, 5):
         assert torch.equal(words[k], want[3 + k][place])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [40000, 140000])
+def test_boards_may_start_anywhere(n, pos4096):
+    """A view of boards off the 16-byte boundaries gets the answers of an aligned copy at every size."""
+    from brokefish_b200 import env
+    place = torch.arange(n) % 4096
+    boards = torch.from_numpy(np.ascontiguousarray(pos4096["boards"])).view(torch.int16)[place].cuda()
+    control = torch.from_numpy(np.ascontiguousarray(pos4096["control"])).view(torch.int16)[place].cuda()
+    whole = torch.zeros(n * 32 + 1, dtype=torch.int16, device="cuda")
+    moved = whole[1:].view(n, 32)
+    moved.copy_(boards)
+    move = torch.full((n,), -1, dtype=torch.int32, device="cuda")
+    key = torch.zeros(n, dtype=torch.int64, device="cuda")
+    calls = (lambda b: env.movegen(b, control), lambda b: (env.hash_position(b, control),),
+             lambda b: env.step(b, control, move, with_moves=True, hash=key))
+    for call in calls:
+        for got, want in zip(call(moved), call(boards)):
+            assert torch.equal(got, want)
