@@ -2365,7 +2365,7 @@ void launch_engine(cudaStream_t stream, bool words, bool key, const uint16_t* bo
                                                                                      rest...);
     else
         bfmg::engine_board_kernel<kStep, kPick><<<(n + bfmg::kTpbThreads - 1) / bfmg::kTpbThreads, bfmg::kTpbThreads,
-                                                  bfmg::kTpbSmem, stream>>>(boards, control, move, promo, r, n, boards_out,
+                                                  bfmg::tpb_smem_bytes(kPick, words), stream>>>(boards, control, move, promo, r, n, boards_out,
                                                                                   rest...);
 }
 

@@ -324,8 +324,8 @@ __device__ __forceinline__ unsigned long long anti_ex(int sq) {
 
 constexpr int kTpbThreads = 128;
 constexpr int kTpbInStride = 17;      // 32-bit words per board in shared memory (16 + 1: no bank conflicts)
-constexpr int kTpbOutStride = 33;     // 64-bit words per board in shared memory (32 + 1)
-constexpr int kTpbSmem = kTpbThreads * (kTpbInStride * 4 + kTpbOutStride * 8);
+constexpr int kTpbOutStride = 17;     // 64-bit words per board in shared memory: the mover's (16 + 1)
+constexpr int kTpbMaskStride = 33;    // a random ply's incoming words (32 + 1)
 
 __device__ __forceinline__ unsigned piece_word(const unsigned* my, int p) {
     return (my[p >> 1] >> (16 * (p & 1))) & 0xFFFFu;
@@ -339,14 +339,13 @@ __device__ __forceinline__ unsigned long long bit_at(unsigned s) {
 }
 // The legal words of one board held by one thread: `my` = the board's 32 piece words as 16
 // 32-bit words, `out[0..31]` receives the legal-target word of every slot.  Returns whether the
-// side to move is in check.
+// side to move is in check.  This form takes any board; `board_moves` below is the faster one for boards
+// whose pieces are in the slots they start in.
 //
-// Bound by the integer pipe.  A board with black to move is turned upside down as it is decoded (and its
-// words on the way out), so that nothing below depends on the side to move; the bitboards are bit planes
-// of the words, without a branch per piece; checks and pins are taken ray by ray from the king without
-// loops.  2^20 boards of random games, B200: 160 us against 252 with a branch per piece and loops over
-// the pinning pieces (323 bytes a board: 2.1 TB/s of the 6.5 a copy reaches).
-__device__ __forceinline__ bool board_moves(const unsigned* my, bool black, unsigned long long* out) {
+// A board with black to move is turned upside down as it is decoded (and its words on the way out), so that
+// nothing below depends on the side to move; the bitboards are bit planes of the words, without a branch per
+// piece; checks and pins are taken ray by ray from the king without loops.
+__device__ __noinline__ bool board_moves_any(const unsigned* my, bool black, unsigned long long* out) {
     // ---- pass 1: bit planes.  A captured piece's square is moved off the board ----
     const unsigned flip = black ? 0x00380038u : 0u;
     unsigned long long half[2] = {0ull, 0ull}, t0 = 0, t1 = 0, t2 = 0, sp = 0;
@@ -471,6 +470,295 @@ __device__ __forceinline__ bool board_moves(const unsigned* my, bool black, unsi
         }
         const unsigned lo = static_cast<unsigned>(legal), hi = static_cast<unsigned>(legal >> 32);
         out[p] = (static_cast<unsigned long long>(__byte_perm(lo, hi, sel_hi)) << 32) | __byte_perm(lo, hi, sel_lo);
+    }
+    return chk;
+}
+
+// ---- the faster form of the same, for boards whose pieces are in the slots they start in ----
+// What a slider sees along one line, looked up: the line's squares are folded into one byte (a rank, a
+// diagonal and an antidiagonal hold one square of each file, so the fold is two logical operations and a
+// multiplication), whose inner six bits pick the answer for the slider's file.  A file is folded by rank.
+// Row 64 of the tables by square, and rank 8 of `up`, are empty: a captured piece looks there.
+struct alignas(16) MoveTables {
+    unsigned long long up[9 * 64];               // [rank][ranks 2-7 occupied]: squares of the a file
+    unsigned long long diag[65][2];              // both diagonals through a square, the square included
+    unsigned along[8 * 64];                      // [file][files b-g occupied]: a byte of files, four times
+    unsigned long long rank[65], knight[65], king[65], pawn[65];   // pawn: what a white pawn attacks
+    unsigned long long pad[1];
+};
+constexpr MoveTables make_move_tables() {
+    MoveTables t{};
+    for (int at = 0; at < 8; ++at)
+        for (int inner = 0; inner < 64; ++inner) {
+            const int occ = inner << 1;
+            unsigned bits = 0;
+            for (int i = at + 1; i < 8; ++i) { bits |= 1u << i; if ((occ >> i) & 1) break; }
+            for (int i = at - 1; i >= 0; --i) { bits |= 1u << i; if ((occ >> i) & 1) break; }
+            t.along[at * 64 + inner] = bits * 0x01010101u;
+            for (int i = 0; i < 8; ++i)
+                if ((bits >> i) & 1u) t.up[at * 64 + inner] |= 1ull << (8 * i);
+        }
+    for (int sq = 0; sq < 64; ++sq)
+        for (int to = 0; to < 64; ++to) {
+            const int dr = (to >> 3) - (sq >> 3), df = (to & 7) - (sq & 7);
+            const int r = dr < 0 ? -dr : dr, f = df < 0 ? -df : df;
+            const unsigned long long b = 1ull << to;
+            if (dr == df) t.diag[sq][0] |= b;
+            if (dr == -df) t.diag[sq][1] |= b;
+            if (dr == 0) t.rank[sq] |= b;
+            if ((r == 1 && f == 2) || (r == 2 && f == 1)) t.knight[sq] |= b;
+            if (r <= 1 && f <= 1 && r + f > 0) t.king[sq] |= b;
+            if (dr == 1 && f == 1) t.pawn[sq] |= b;
+        }
+    return t;
+}
+__device__ const MoveTables kMoveTables = make_move_tables();
+
+// Along a rank or a diagonal (`line`, which holds the slider's square) from a square of file sq & 7.
+__device__ __forceinline__ unsigned long long see_along(const MoveTables& t, unsigned long long occ, unsigned long long line,
+                                                        unsigned sq) {
+    const unsigned long long o = occ & line;
+    const unsigned fold = static_cast<unsigned>(o) | static_cast<unsigned>(o >> 32);
+    const unsigned f = t.along[(sq & 7u) * 64u + (fold * 0x02020202u >> 26)];
+    return line & ((static_cast<unsigned long long>(f) << 32) | f);
+}
+// Along the file of a square (64: nothing).
+__device__ __forceinline__ unsigned long long see_file(const MoveTables& t, unsigned long long occ, unsigned sq) {
+    const unsigned f = sq & 7u;
+    const unsigned lo = (static_cast<unsigned>(occ) >> f) & 0x01010101u, hi = (static_cast<unsigned>(occ >> 32) >> f) & 0x01010101u;
+    const unsigned long long u = t.up[(sq >> 3) * 64u + ((hi * 16u + lo) * 0x02040810u >> 26)];
+    return (static_cast<unsigned long long>(static_cast<unsigned>(u >> 32) << f) << 32) | (static_cast<unsigned>(u) << f);
+}
+__device__ __forceinline__ unsigned long long see_diag(const MoveTables& t, unsigned long long occ, unsigned sq) {
+    const ulonglong2 d = *reinterpret_cast<const ulonglong2*>(t.diag[sq]);
+    return see_along(t, occ, d.x, sq) | see_along(t, occ, d.y, sq);
+}
+__device__ __forceinline__ unsigned long long see_line(const MoveTables& t, unsigned long long occ, unsigned sq) {
+    return see_along(t, occ, t.rank[sq], sq) | see_file(t, occ, sq);
+}
+
+// A piece word with its slot's expected colour and type taken out: its square when the piece is there, 64
+// or more when it has been captured or is not the piece expected, so that `bit_at` of it is its bit or 0.
+constexpr unsigned kIndexBits = 0x0DFF0DFFu;
+
+// The legal words of one board held by one thread: the mover's sixteen into `to`, the other side's are
+// zero -- or, where the board takes the general form, all thirty-two into `all`, and `by_slot` is false.
+//
+// A colour's sixteen slots are eight pawns, two knights, two bishops, two rooks, the queen and the king,
+// and only pawns ever change their type.  So a piece's plane is known before its word is looked at, its
+// bit falls out of the word and the expectation in five operations, and each slot has code of its own, with no
+// branch on what it holds.  Promoted pawns (one board in thirty of random games) are found by
+// counting: the planes must hold as many squares as there are pieces left.  They are put in one by one; a board
+// that does not add up then (colours or types in other slots, two pieces on a square) takes the general form.
+//
+// Bound by the integer pipe (the general form keeps it busy 87 % of the time with 3,600 instructions a board), which is why
+// every attack is a table's.  2^20 boards of random games, B200: 123 us, 161 in the general form (323 bytes a board: 2.8
+// and 2.1 TB/s of the 6.5 a copy reaches).
+__device__ __forceinline__ bool board_moves(const unsigned* my, bool black, unsigned long long* to, unsigned long long* all,
+                                            const MoveTables& t, bool& by_slot) {
+    by_slot = true;
+    const unsigned flip = black ? 0x04380438u : 0u;             // the mover is white: squares turned, colour changed
+    const unsigned* mine = my + (black ? 8 : 0);
+    const unsigned* theirs = my + (black ? 0 : 8);
+    constexpr unsigned kTheirs = 0x04000400u, kN = 0x00400040u, kB = 0x00800080u, kR = 0x00C000C0u, kQK = 0x01400100u;
+    auto lo_of = [](unsigned x) { return x & 0xFFFFu; };
+    auto hi_of = [](unsigned x) { return x >> 16; };
+    auto expect = [&](unsigned two, unsigned e) { return (two ^ (flip ^ e)) & kIndexBits; };
+    auto both = [&](unsigned x) { return bit_at(lo_of(x)) | bit_at(hi_of(x)); };
+    auto on_board = [](unsigned i) { return min(i, 64u); };
+    // ---- the planes ----
+    unsigned long long own_pawns = 0ull, e_pawns = 0ull;
+    unsigned gone = 0u, stepped = 0u;                            // captured pieces, counted; enemy pawns that are flagged
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const unsigned a = mine[q], b = theirs[q];
+        own_pawns |= both(expect(a, 0u));
+        e_pawns |= both(expect(b, kTheirs));
+        gone += (a & 0x08000800u) + (b & 0x08000800u);
+        stepped |= b & 0x02000200u;
+    }
+    const unsigned w_n = mine[4], w_b = mine[5], w_r = mine[6], w_qk = mine[7];
+    const unsigned v_n = theirs[4], v_b = theirs[5], v_r = theirs[6], v_qk = theirs[7];
+    gone += (w_n & 0x08000800u) + (w_b & 0x08000800u) + (w_r & 0x08000800u) + (w_qk & 0x08000800u);
+    gone += (v_n & 0x08000800u) + (v_b & 0x08000800u) + (v_r & 0x08000800u) + (v_qk & 0x08000800u);
+    const unsigned x_qk = expect(w_qk, kQK), y_n = expect(v_n, kTheirs | kN), y_b = expect(v_b, kTheirs | kB),
+                   y_r = expect(v_r, kTheirs | kR), y_qk = expect(v_qk, kTheirs | kQK);
+    const unsigned long long my_king = bit_at(hi_of(x_qk)), e_king = bit_at(hi_of(y_qk)), e_queen = bit_at(lo_of(y_qk));
+    unsigned long long e_knights = both(y_n), e_diag = both(y_b) | e_queen, e_line = both(y_r) | e_queen;
+    unsigned long long own = own_pawns | both(expect(w_n, kN)) | both(expect(w_b, kB)) | both(expect(w_r, kR)) |
+                             bit_at(lo_of(x_qk)) | my_king;
+    unsigned long long occ = own | e_pawns | e_knights | e_diag | e_line | e_king;
+    // castling rooks: not moved, on their corners
+    const unsigned r_lo = lo_of(w_r ^ flip ^ kR) & 0xFFFu, r_hi = hi_of(w_r ^ flip ^ kR) & 0xFFFu;
+    bool fresh_a = r_lo == 0u || r_hi == 0u, fresh_h = r_lo == 7u || r_hi == 7u;
+    const int live = 32 - static_cast<int>((gone & 0xFFFFu) >> 11) - static_cast<int>(gone >> 27);
+    // ---- promoted pawns ----
+    unsigned own_promoted = 0u;                                  // the mover's, by slot
+    unsigned long long e_promoted = 0ull;                        // the opponent's sliders
+    if (__popcll(occ) != live) {
+        unsigned todo = 0u;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const unsigned a = (mine[q] & 0x01C001C0u) + 0x01C001C0u, b = (theirs[q] & 0x01C001C0u) + 0x01C001C0u;
+            todo |= ((a & 0x02000200u) >> (9 - q)) | ((b & 0x02000200u) >> (5 - q));
+        }
+        for (; todo != 0u; todo &= todo - 1u) {
+            const int i = __ffs(static_cast<int>(todo)) - 1, q = i & 3;
+            const bool enemy = (i & 4) != 0;
+            const unsigned word = ((enemy ? theirs : mine)[q] >> (i & 16)) ^ (flip & 0x438u);
+            const int type = (word >> 6) & 7;
+            if ((word & 0x800u) != 0u || ((word & 0x400u) != 0u) != enemy || type < KNIGHT || type > QUEEN) continue;
+            const unsigned long long bb = bit_at(word & 63u);
+            occ |= bb;
+            if (enemy) {
+                if (type == KNIGHT) e_knights |= bb;
+                if (type == BISHOP || type == QUEEN) e_diag |= bb;
+                if (type == ROOK || type == QUEEN) e_line |= bb;
+                if (type != KNIGHT) e_promoted |= bb;
+            } else {
+                own |= bb;
+                own_promoted |= 1u << (2 * q + (i >> 4));
+                if (type == ROOK && (word & 0x200u) == 0u) { fresh_a |= (word & 63u) == 0u; fresh_h |= (word & 63u) == 7u; }
+            }
+        }
+        by_slot = __popcll(occ) == live;
+        if (!by_slot) return board_moves_any(my, black, all);
+    }
+    const unsigned long long opp = occ & ~own;
+    // ---- what the opponent attacks, with the mover's king lifted off the board ----
+    const unsigned long long occ_nk = occ & ~my_king;
+    unsigned long long danger = pawn_attacks(e_pawns, true) | knight_pattern(e_knights) | t.king[on_board(hi_of(y_qk))];
+    {
+        const unsigned b0 = on_board(lo_of(y_b)), b1 = on_board(hi_of(y_b)), r0 = on_board(lo_of(y_r)), r1 = on_board(hi_of(y_r)),
+                       qq = on_board(lo_of(y_qk));
+        danger |= see_diag(t, occ_nk, b0) | see_diag(t, occ_nk, b1) | see_diag(t, occ_nk, qq);
+        danger |= see_line(t, occ_nk, r0) | see_line(t, occ_nk, r1) | see_line(t, occ_nk, qq);
+        for (; e_promoted != 0ull; e_promoted &= e_promoted - 1ull) {
+            const unsigned sq = static_cast<unsigned>(__ffsll(static_cast<long long>(e_promoted)) - 1);
+            const unsigned long long bb = e_promoted & (0ull - e_promoted);
+            if (bb & e_diag) danger |= see_diag(t, occ_nk, sq);
+            if (bb & e_line) danger |= see_line(t, occ_nk, sq);
+        }
+    }
+    // ---- the four lines through the king: is the first piece on either side a checker (the squares up to it answer the
+    //      check), or an own piece with a slider of the line's kind next behind it ----
+    const unsigned ks = on_board(hi_of(x_qk));
+    const unsigned long long above = 0ull - (my_king << 1);          // squares above the king's
+    const ulonglong2 k_diag = *reinterpret_cast<const ulonglong2*>(t.diag[ks]);
+    const unsigned long long k_rank = t.rank[ks], k_file = kFileA << (ks & 7u);
+    const unsigned long long leapers = (t.knight[ks] & e_knights) | (t.pawn[ks] & e_pawns);
+    unsigned long long answers = 0ull, pinned = 0ull, hits = 0ull;
+    auto line = [&](unsigned long long sliders, auto&& see) {
+        const unsigned long long seen = see(occ), shields = seen & own, hit = seen & sliders;
+        const unsigned long long next = see(occ & ~shields) & ~seen & sliders;
+        hits |= hit;
+        if (hit != 0ull) answers |= seen;
+        if (next & above) pinned |= shields & above;
+        if (next & ~above) pinned |= shields & ~above;
+    };
+    line(e_diag, [&](unsigned long long o) { return see_along(t, o, k_diag.x, ks); });
+    line(e_diag, [&](unsigned long long o) { return see_along(t, o, k_diag.y, ks); });
+    line(e_line, [&](unsigned long long o) { return see_along(t, o, k_rank, ks); });
+    line(e_line, [&](unsigned long long o) { return see_file(t, o, ks); });
+    const int checkers = __popcll(hits) + __popcll(leapers);
+    const bool chk = checkers != 0;
+    // one checker: the other pieces may only capture it or step between; two: only the king moves
+    const unsigned long long target_mask = checkers == 0 ? ~0ull
+                                           : checkers == 1 ? leapers | (answers & ((hits & above) ? above : ~above)) : 0ull;
+    // ---- the mover's pieces ----
+    const unsigned long long allowed = target_mask & ~own;
+    const unsigned sel_lo = black ? 0x4567u : 0x3210u, sel_hi = black ? 0x0123u : 0x7654u;
+    auto put = [&](int slot, unsigned long long legal) {
+        const unsigned lo = static_cast<unsigned>(legal), hi = static_cast<unsigned>(legal >> 32);
+        to[slot] = (static_cast<unsigned long long>(__byte_perm(lo, hi, sel_hi)) << 32) | __byte_perm(lo, hi, sel_lo);
+    };
+    // a piece that shields the king from a slider moves only along that line
+    auto held = [&](unsigned long long bb, unsigned long long legal) {
+        if (bb & pinned)
+            legal &= (bb & k_diag.x) ? k_diag.x : (bb & k_diag.y) ? k_diag.y : (bb & k_rank) ? k_rank : k_file;
+        return legal;
+    };
+    {
+        const unsigned long long step = ~occ & target_mask, takes = opp & target_mask;
+        const unsigned long long two = ~occ & (~occ << 8) & target_mask & 0xFF000000ull;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const unsigned x = expect(mine[q], 0u);
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const unsigned i = k ? hi_of(x) : lo_of(x);
+                const unsigned long long bb = bit_at(i);
+                put(2 * q + k, held(bb, ((bb << 8) & step) | ((bb << 16) & two) | (t.pawn[on_board(i)] & takes)));
+            }
+        }
+    }
+    {
+        const unsigned x_n = expect(w_n, kN), x_b = expect(w_b, kB), x_r = expect(w_r, kR);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const unsigned i = k ? hi_of(x_n) : lo_of(x_n);
+            put(8 + k, held(bit_at(i), t.knight[on_board(i)] & allowed));
+        }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const unsigned i = k ? hi_of(x_b) : lo_of(x_b);
+            put(10 + k, held(bit_at(i), see_diag(t, occ, on_board(i)) & allowed));
+        }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const unsigned i = k ? hi_of(x_r) : lo_of(x_r);
+            put(12 + k, held(bit_at(i), see_line(t, occ, on_board(i)) & allowed));
+        }
+        const unsigned i = lo_of(x_qk);
+        put(14, held(bit_at(i), (see_diag(t, occ, on_board(i)) | see_line(t, occ, on_board(i))) & allowed));
+    }
+    {
+        unsigned long long legal = t.king[ks] & ~danger;
+        // castling: neither the king's square nor the one it crosses nor the one it lands on may be attacked
+        if (my_king != 0ull && (w_qk & 0x02000000u) == 0u && !chk) {
+            if (fresh_h && ((occ | danger) & 0x60ull) == 0ull) legal |= 0x40ull;
+            if (fresh_a && (occ & 0x0Eull) == 0ull && (danger & 0x0Cull) == 0ull) legal |= 0x04ull;
+        }
+        put(15, legal & ~own);
+    }
+    // ---- the mover's promoted pawns ----
+    for (; own_promoted != 0u; own_promoted &= own_promoted - 1u) {
+        const int slot = __ffs(static_cast<int>(own_promoted)) - 1;
+        const unsigned word = (mine[slot >> 1] >> (16 * (slot & 1))) ^ (flip & 63u), sq = word & 63u;
+        const int type = (word >> 6) & 7;
+        unsigned long long cand = 0ull;
+        if (type == KNIGHT) cand = t.knight[sq];
+        if (type == BISHOP || type == QUEEN) cand |= see_diag(t, occ, sq);
+        if (type == ROOK || type == QUEEN) cand |= see_line(t, occ, sq);
+        put(slot, held(bit_at(sq), cand & allowed));
+    }
+    // ---- en passant takes two pieces off one rank at once: tested on the position after it ----
+    if (stepped != 0u) {
+        unsigned long long targets = 0ull;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const unsigned b = theirs[q], x = expect(b, kTheirs);
+            if (b & 0x0200u) targets |= bit_at(lo_of(x)) << 8;
+            if (b & 0x02000000u) targets |= bit_at(hi_of(x)) << 8;
+        }
+        targets &= ~own & 0x0000FF0000000000ull;
+        if (pawn_attacks(targets, true) & own_pawns)
+#pragma unroll 1
+            for (int slot = 0; slot < 8; ++slot) {
+                const unsigned x = expect(mine[slot >> 1], 0u), i = (slot & 1) ? hi_of(x) : lo_of(x);
+                const unsigned long long bb = bit_at(i);
+                unsigned long long legal = 0ull;
+                for (unsigned long long ep = t.pawn[on_board(i)] & targets; ep != 0ull; ep &= ep - 1ull) {
+                    const unsigned long long tb = ep & (0ull - ep), victim = tb >> 8;
+                    const unsigned long long after = ((occ & ~bb) & ~victim) | tb;
+                    const bool hit = (t.knight[ks] & e_knights) != 0ull || (t.pawn[ks] & (e_pawns & ~victim)) != 0ull ||
+                                     (t.king[ks] & e_king) != 0ull ||
+                                     (see_diag(t, after, ks) & e_diag) != 0ull || (see_line(t, after, ks) & e_line) != 0ull;
+                    if (!hit) legal |= tb;
+                }
+                const unsigned lo = static_cast<unsigned>(legal), hi = static_cast<unsigned>(legal >> 32);
+                to[slot] |= (static_cast<unsigned long long>(__byte_perm(lo, hi, sel_hi)) << 32) | __byte_perm(lo, hi, sel_lo);
+            }
     }
     return chk;
 }
@@ -625,6 +913,18 @@ __device__ __forceinline__ unsigned long long board_hash(const unsigned* my, boo
     return h;
 }
 
+// Shared memory: the boards; the tables and the words that go out, or before them a random ply's incoming
+// words.  (Launches without words need the boards only.)
+constexpr int kTpbIn = kTpbThreads * kTpbInStride * 4;
+constexpr int kTpbTables = static_cast<int>(sizeof(MoveTables));
+constexpr int tpb_smem_bytes(bool pick, bool words) {
+    const int made = kTpbTables + kTpbThreads * kTpbOutStride * 8, incoming = kTpbThreads * kTpbMaskStride * 8;
+    return kTpbIn + (!words ? 0 : pick && incoming > made ? incoming : made);
+}
+static_assert(kTpbIn % 16 == 0 && kTpbTables % 16 == 0 && tpb_smem_bytes(true, true) <= 49152, "shared memory map");
+// What becomes of a board's words: the first two are the side to move, whose words lie in shared memory.
+enum { WORDS_WHITE = 0, WORDS_BLACK = 1, WORDS_STORED = 2, WORDS_KEPT = 3 };
+
 // One thread per board, boards and legal words staged through shared memory for coalescing.
 // `hash_out` non-null: the position key of the resulting board.
 // kStep: play `move` first (or, with kPick, the floor(r * count)-th legal move of the incoming
@@ -638,11 +938,17 @@ __global__ void __launch_bounds__(kTpbThreads) engine_board_kernel(
         int16_t* control_out, unsigned char* __restrict__ irreversible, unsigned long long* mask,
         unsigned char* __restrict__ in_check, int* __restrict__ move_out, unsigned long long* __restrict__ hash_out) {
     extern __shared__ unsigned long long tpb_smem[];
-    unsigned long long* s_out = tpb_smem;                                        // [128][33]
-    unsigned* s_in = reinterpret_cast<unsigned*>(tpb_smem + kTpbThreads * kTpbOutStride);   // [128][17]
+    unsigned* s_in = reinterpret_cast<unsigned*>(tpb_smem);                                 // [128][17]
+    MoveTables* s_tables = reinterpret_cast<MoveTables*>(reinterpret_cast<uint8_t*>(tpb_smem) + kTpbIn);
+    unsigned long long* s_mask = reinterpret_cast<unsigned long long*>(s_tables);           // [128][33], before the tables
+    unsigned long long* s_out = reinterpret_cast<unsigned long long*>(s_tables + 1);        // [128][17]
     const int tid = threadIdx.x;
     const long first = static_cast<long>(blockIdx.x) * kTpbThreads;
     const int here = static_cast<int>(min(static_cast<long>(kTpbThreads), n - first));
+    auto load_tables = [&] {
+        for (int j = tid; j < kTpbTables / 16; j += kTpbThreads)
+            reinterpret_cast<uint4*>(s_tables)[j] = __ldg(reinterpret_cast<const uint4*>(&kMoveTables) + j);
+    };
     {
         // coalesced load: the block's boards are one contiguous run of 16-byte pieces
         const uint4* src = reinterpret_cast<const uint4*>(boards + first * 32);
@@ -653,52 +959,63 @@ __global__ void __launch_bounds__(kTpbThreads) engine_board_kernel(
         }
         if (kPick)
             for (int j = tid; j < here * 32; j += kTpbThreads)
-                s_out[(j >> 5) * kTpbOutStride + (j & 31)] = mask[first * 32 + j];
+                s_mask[(j >> 5) * kTpbMaskStride + (j & 31)] = mask[first * 32 + j];
+        else if (mask != nullptr)
+            load_tables();
     }
     __syncthreads();
-    bool moved = false;
-    if (tid < here) {
-        unsigned* my = s_in + tid * kTpbInStride;
-        unsigned long long* out = s_out + tid * kTpbOutStride;
+    const bool mine = tid < here;
+    unsigned* my = s_in + tid * kTpbInStride;
+    int mv = -1;
+    if (kPick) {
+        if (mine) {
+            const unsigned long long* words = s_mask + tid * kTpbMaskStride;
+            int total = 0;
+#pragma unroll 1
+            for (int p = 0; p < 32; ++p) total += __popcll(words[p]);
+            if (total > 0) {
+                int pick = static_cast<int>(__fmul_rn(r[first + tid], static_cast<float>(total)));
+                pick = pick < total - 1 ? pick : total - 1;
+#pragma unroll 1
+                for (int p = 0; p < 32 && mv < 0; ++p) {
+                    unsigned long long m = words[p];
+                    const int cnt = __popcll(m);
+                    if (pick < cnt) {
+                        for (int i = 0; i < pick; ++i) m &= m - 1ull;
+                        mv = p * 64 + __ffsll(static_cast<long long>(m)) - 1;
+                    }
+                    pick -= cnt;
+                }
+            }
+            if (move_out != nullptr) move_out[first + tid] = mv;
+        }
+        __syncthreads();                              // the incoming words' place is the tables'
+        load_tables();
+        __syncthreads();
+    }
+    if (mine) {
         int ctl = control[first + tid];
         bool generate = mask != nullptr;
         if (kStep) {
-            int mv = kPick ? -1 : move[first + tid];
-            if (kPick) {
-                int total = 0;
-#pragma unroll 1
-                for (int p = 0; p < 32; ++p) total += __popcll(out[p]);
-                if (total > 0) {
-                    int pick = static_cast<int>(__fmul_rn(r[first + tid], static_cast<float>(total)));
-                    pick = pick < total - 1 ? pick : total - 1;
-#pragma unroll 1
-                    for (int p = 0; p < 32 && mv < 0; ++p) {
-                        unsigned long long m = out[p];
-                        const int cnt = __popcll(m);
-                        if (pick < cnt) {
-                            for (int i = 0; i < pick; ++i) m &= m - 1ull;
-                            mv = p * 64 + __ffsll(static_cast<long long>(m)) - 1;
-                        }
-                        pick -= cnt;
-                    }
-                }
-                if (move_out != nullptr) move_out[first + tid] = mv;
-                generate = mv >= 0;                   // a finished game keeps its (empty) legal words
-            }
+            if (!kPick) mv = move[first + tid];
+            if (kPick) generate = mv >= 0;            // a finished game keeps its (empty) legal words
             int nc;
             bool irr;
             board_step(my, ctl, mv, promo != nullptr ? promo[first + tid] : -1, nc, irr);
-            moved = !kPick || mv >= 0;
-            if (moved) {
+            if (!kPick || mv >= 0) {
                 control_out[first + tid] = static_cast<int16_t>(nc);
                 if (irreversible != nullptr) irreversible[first + tid] = irr ? 1 : 0;
             }
             ctl = nc;
         }
+        unsigned words = WORDS_KEPT;
         if (generate) {
-            const bool chk = board_moves(my, ctl < 0, out);
+            bool by_slot;
+            const bool chk = board_moves(my, ctl < 0, s_out + tid * kTpbOutStride, mask + (first + tid) * 32, *s_tables, by_slot);
             if (in_check != nullptr) in_check[first + tid] = chk ? 1 : 0;
+            words = !by_slot ? WORDS_STORED : ctl < 0 ? WORDS_BLACK : WORDS_WHITE;
         }
+        my[16] = words;                               // (the row's padding)
         if (hash_out != nullptr) hash_out[first + tid] = board_hash(my, ctl < 0);
     }
     __syncthreads();
@@ -710,9 +1027,16 @@ __global__ void __launch_bounds__(kTpbThreads) engine_board_kernel(
             dst[j] = make_uint4(d[0], d[1], d[2], d[3]);
         }
     }
-    if (mask != nullptr)
-        for (int j = tid; j < here * 32; j += kTpbThreads)
-            mask[first * 32 + j] = s_out[(j >> 5) * kTpbOutStride + (j & 31)];
+    if (mask != nullptr) {
+        // a warp stores a board's words; the side that is not to move has none
+        const unsigned p = tid & 31, side = p >> 4;
+#pragma unroll 4
+        for (int b = tid >> 5; b < here; b += kTpbThreads / 32) {
+            const unsigned words = s_in[b * kTpbInStride + 16];
+            const unsigned long long v = s_out[b * kTpbOutStride + (p & 15)];
+            if (words <= WORDS_BLACK) mask[(first + b) * 32 + p] = words == side ? v : 0ull;
+        }
+    }
 }
 
 // ------------------------------------------------------------------------------------------
