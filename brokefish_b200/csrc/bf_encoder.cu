@@ -2338,6 +2338,27 @@ int host_plan_sizes(int n, int wave, int plan, double gbps, int* sizes, bool* sl
     return n_chunks;
 }
 
+// Launches a kernel that takes the grid before it in its stream to be still running: it calls
+// `griddepcontrol.wait` before it touches what that grid may write or read, and before that does
+// what depends on nothing (barriers, tensor memory, the first weights, tables).  `cluster`: CTAs to a cluster.
+template <class... P, class... A>
+cudaError_t launch_early(void (*kernel)(P...), unsigned grid, int threads, size_t smem, int cluster, cudaStream_t stream, bool early, A... args) {
+    cudaLaunchAttribute attributes[2] = {};
+    attributes[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attributes[0].val.programmaticStreamSerializationAllowed = early ? 1 : 0;
+    attributes[1].id = cudaLaunchAttributeClusterDimension;
+    attributes[1].val.clusterDim.x = cluster;
+    attributes[1].val.clusterDim.y = attributes[1].val.clusterDim.z = 1;
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(grid);
+    config.blockDim = dim3(threads);
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    config.attrs = attributes;
+    config.numAttrs = cluster > 1 ? 2 : 1;
+    return cudaLaunchKernelEx(&config, kernel, static_cast<P>(args)...);
+}
+
 // The engine kernels have two forms (bf_movegen.cuh).  Eight lanes per board: an eighth of the chain,
 // so a launch that does not fill the GPU ends sooner.  A thread per board: half of the instructions, most
 // of all where legal words are made.  B200, us per launch in a graph, eight lanes / thread:
@@ -2355,18 +2376,15 @@ int group_form_most(bool step, bool pick, bool words, bool key) {
     return pick || key ? 49152 : 32768;
 }
 template <bool kStep, bool kPick, class... Args>
-void launch_engine(cudaStream_t stream, bool words, bool key, const uint16_t* boards, const int16_t* control, const int* move,
-                   const signed char* promo, const float* r, int n, uint16_t* boards_out, Args... rest) {
+cudaError_t launch_engine(cudaStream_t stream, bool words, bool key, const uint16_t* boards, const int16_t* control, const int* move,
+                          const signed char* promo, const float* r, int n, uint16_t* boards_out, Args... rest) {
     // (a thread per board moves boards in 16-byte pieces; eight lanes take them wherever they start)
     const bool pieces = ((reinterpret_cast<uintptr_t>(boards) | reinterpret_cast<uintptr_t>(boards_out)) & 15u) == 0;
     if (n <= group_form_most(kStep, kPick, words, key) || !pieces)
-        bfmg::engine_group_kernel<kStep, kPick><<<(n + bfmg::kEngineBoards - 1) / bfmg::kEngineBoards,
-                                                  bfmg::kEngineThreads, 0, stream>>>(boards, control, move, promo, r, n, boards_out,
-                                                                                     rest...);
-    else
-        bfmg::engine_board_kernel<kStep, kPick><<<(n + bfmg::kTpbThreads - 1) / bfmg::kTpbThreads, bfmg::kTpbThreads,
-                                                  bfmg::tpb_smem_bytes(kPick, words), stream>>>(boards, control, move, promo, r, n, boards_out,
-                                                                                  rest...);
+        return launch_early(bfmg::engine_group_kernel<kStep, kPick>, (n + bfmg::kEngineBoards - 1) / bfmg::kEngineBoards,
+                            bfmg::kEngineThreads, 0, 1, stream, true, boards, control, move, promo, r, n, boards_out, rest...);
+    return launch_early(bfmg::engine_board_kernel<kStep, kPick>, (n + bfmg::kTpbThreads - 1) / bfmg::kTpbThreads, bfmg::kTpbThreads,
+                        bfmg::tpb_smem_bytes(kPick, words), 1, stream, true, boards, control, move, promo, r, n, boards_out, rest...);
 }
 
 struct PriorOut {
@@ -2604,10 +2622,9 @@ int bf_movegen(int device, const uint16_t* boards, const int16_t* control, int n
     if (boards == nullptr || control == nullptr || mask == nullptr)
         return fail(BF_EINVAL, "boards, control and mask must be non-null");
     BF_ON_DEVICE(device);
-    launch_engine<false, false>(static_cast<cudaStream_t>(stream), true, false,
+    BF_CUDA((launch_engine<false, false>(static_cast<cudaStream_t>(stream), true, false,
         boards, control, nullptr, nullptr, nullptr, n, nullptr, nullptr, nullptr,
-        reinterpret_cast<unsigned long long*>(mask), in_check, nullptr, nullptr);
-    BF_CUDA(cudaGetLastError());
+        reinterpret_cast<unsigned long long*>(mask), in_check, nullptr, nullptr)));
     return BF_OK;
 }
 
@@ -2617,10 +2634,9 @@ int bf_hash(int device, const uint16_t* boards, const int16_t* control, int n, u
     if (boards == nullptr || control == nullptr || hash == nullptr)
         return fail(BF_EINVAL, "boards, control and hash must be non-null");
     BF_ON_DEVICE(device);
-    launch_engine<false, false>(static_cast<cudaStream_t>(stream), false, true,
+    BF_CUDA((launch_engine<false, false>(static_cast<cudaStream_t>(stream), false, true,
         boards, control, nullptr, nullptr, nullptr, n, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
-        reinterpret_cast<unsigned long long*>(hash));
-    BF_CUDA(cudaGetLastError());
+        reinterpret_cast<unsigned long long*>(hash))));
     return BF_OK;
 }
 
@@ -2631,10 +2647,9 @@ int bf_history_push(int device, uint64_t* ring, long long* length, const uint64_
     if (ring == nullptr || length == nullptr || hash == nullptr || irreversible == nullptr)
         return fail(BF_EINVAL, "ring, length, hash and irreversible must be non-null");
     BF_ON_DEVICE(device);
-    bfmg::history_push_kernel<<<(n + 127) / 128, 128, 0, static_cast<cudaStream_t>(stream)>>>(
+    BF_CUDA(launch_early(bfmg::history_push_kernel, (n + 127) / 128, 128, 0, 1, static_cast<cudaStream_t>(stream), true, 
         reinterpret_cast<unsigned long long*>(ring), length, reinterpret_cast<const unsigned long long*>(hash),
-        irreversible, n);
-    BF_CUDA(cudaGetLastError());
+        irreversible, n));
     return BF_OK;
 }
 
@@ -2654,9 +2669,8 @@ int bf_history_push_to(int device, const uint64_t* ring, const long long* length
     const long pieces = static_cast<long>(n) * (wide ? bfmg::kMaxHistory / 2 : bfmg::kMaxHistory);
     const unsigned blocks = static_cast<unsigned>((pieces + 255) / 256);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (wide) bfmg::history_push_to_kernel<2><<<blocks, 256, 0, s>>>(src, length, key, irreversible, n, dst, new_length);
-    else      bfmg::history_push_to_kernel<1><<<blocks, 256, 0, s>>>(src, length, key, irreversible, n, dst, new_length);
-    BF_CUDA(cudaGetLastError());
+    BF_CUDA(launch_early(wide ? bfmg::history_push_to_kernel<2> : bfmg::history_push_to_kernel<1>, blocks, 256, 0, 1, s, true, src, length,
+                         key, irreversible, n, dst, new_length));
     return BF_OK;
 }
 
@@ -2667,10 +2681,9 @@ int bf_repetition_count(int device, const uint64_t* hash, const uint64_t* ring, 
     if (ring == nullptr || length == nullptr || hash == nullptr || count == nullptr)
         return fail(BF_EINVAL, "hash, ring, length and count must be non-null");
     BF_ON_DEVICE(device);
-    bfmg::repetition_kernel<<<(n + 3) / 4, 128, 0, static_cast<cudaStream_t>(stream)>>>(
+    BF_CUDA(launch_early(bfmg::repetition_kernel, (n + 3) / 4, 128, 0, 1, static_cast<cudaStream_t>(stream), true, 
         reinterpret_cast<const unsigned long long*>(hash), reinterpret_cast<const unsigned long long*>(ring), length,
-        n, count);
-    BF_CUDA(cudaGetLastError());
+        n, count));
     return BF_OK;
 }
 
@@ -2682,10 +2695,9 @@ int bf_step(int device, const uint16_t* boards, const int16_t* control, const in
     if (boards == nullptr || control == nullptr || move == nullptr || boards_out == nullptr || control_out == nullptr)
         return fail(BF_EINVAL, "boards, control, move, boards_out and control_out must be non-null");
     BF_ON_DEVICE(device);
-    launch_engine<true, false>(static_cast<cudaStream_t>(stream), mask != nullptr, hash != nullptr,
+    BF_CUDA((launch_engine<true, false>(static_cast<cudaStream_t>(stream), mask != nullptr, hash != nullptr,
         boards, control, move, promo, nullptr, n, boards_out, control_out, irreversible,
-        reinterpret_cast<unsigned long long*>(mask), in_check, nullptr, reinterpret_cast<unsigned long long*>(hash));
-    BF_CUDA(cudaGetLastError());
+        reinterpret_cast<unsigned long long*>(mask), in_check, nullptr, reinterpret_cast<unsigned long long*>(hash))));
     return BF_OK;
 }
 
@@ -2696,11 +2708,10 @@ int launch_terminal(int device, const uint64_t* mask, const unsigned char* in_ch
     if (mask == nullptr || in_check == nullptr || control == nullptr || boards == nullptr || code == nullptr)
         return fail(BF_EINVAL, "mask, in_check, control, boards and code must be non-null");
     BF_ON_DEVICE(device);
-    bfmg::terminal_kernel<<<(n + 3) / 4, 128, 0, static_cast<cudaStream_t>(stream)>>>(
+    BF_CUDA(launch_early(bfmg::terminal_kernel, (n + 3) / 4, 128, 0, 1, static_cast<cudaStream_t>(stream), true, 
         reinterpret_cast<const unsigned long long*>(mask), in_check, control, boards, rep_count,
         reinterpret_cast<const unsigned long long*>(hash), reinterpret_cast<const unsigned long long*>(ring), length, n,
-        code, result);
-    BF_CUDA(cudaGetLastError());
+        code, result));
     return BF_OK;
 }
 }  // namespace
@@ -2730,10 +2741,9 @@ int bf_random_ply(int device, uint16_t* boards, int16_t* control, uint64_t* mask
     if (boards == nullptr || control == nullptr || mask == nullptr || r == nullptr)
         return fail(BF_EINVAL, "boards, control, mask and r must be non-null");
     BF_ON_DEVICE(device);
-    launch_engine<true, true>(static_cast<cudaStream_t>(stream), true, false,
+    BF_CUDA((launch_engine<true, true>(static_cast<cudaStream_t>(stream), true, false,
         boards, control, nullptr, promo, r, n, boards, control, nullptr,
-        reinterpret_cast<unsigned long long*>(mask), nullptr, move, nullptr);
-    BF_CUDA(cudaGetLastError());
+        reinterpret_cast<unsigned long long*>(mask), nullptr, move, nullptr)));
     return BF_OK;
 }
 

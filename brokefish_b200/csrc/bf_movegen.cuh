@@ -28,6 +28,14 @@
 
 namespace bfmg {
 
+// These kernels are launched while the grid before them in the stream may still be running: they wait for it
+// before they touch its memory, and let the grid after them start at once.  (No __restrict__ on what they read: the
+// compiler may move a load from memory that it takes to be constant above the wait.)
+__device__ __forceinline__ void begin_after_previous_grid() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 constexpr unsigned long long kFileA = 0x0101010101010101ull, kFileH = kFileA << 7;
 constexpr unsigned kFull = 0xffffffffu;
 enum { PAWN = 0, KNIGHT = 1, BISHOP = 2, ROOK = 3, QUEEN = 4, KING = 5 };
@@ -552,7 +560,7 @@ constexpr unsigned kIndexBits = 0x0DFF0DFFu;
 // that does not add up then (colours or types in other slots, two pieces on a square) takes the general form.
 //
 // Bound by the integer pipe (the general form keeps it busy 87 % of the time with 3,600 instructions a board), which is why
-// every attack is a table's.  2^20 boards of random games, B200: 123 us, 161 in the general form (323 bytes a board: 2.8
+// every attack is a table's.  2^20 boards of random games, B200: 121 us, 161 in the general form (323 bytes a board: 2.8
 // and 2.1 TB/s of the 6.5 a copy reaches).
 __device__ __forceinline__ bool board_moves(const unsigned* my, bool black, unsigned long long* to, unsigned long long* all,
                                             const MoveTables& t, bool& by_slot) {
@@ -933,10 +941,10 @@ enum { WORDS_WHITE = 0, WORDS_BLACK = 1, WORDS_STORED = 2, WORDS_KEPT = 3 };
 // board follow.  In place (boards_out == boards) is safe: a block reads all its boards first.
 template <bool kStep, bool kPick>
 __global__ void __launch_bounds__(kTpbThreads) engine_board_kernel(
-        const uint16_t* __restrict__ boards, const int16_t* __restrict__ control, const int* __restrict__ move,
-        const signed char* __restrict__ promo, const float* __restrict__ r, int n, uint16_t* boards_out,
-        int16_t* control_out, unsigned char* __restrict__ irreversible, unsigned long long* mask,
-        unsigned char* __restrict__ in_check, int* __restrict__ move_out, unsigned long long* __restrict__ hash_out) {
+        const uint16_t* boards, const int16_t* control, const int* move,
+        const signed char* promo, const float* r, int n, uint16_t* boards_out,
+        int16_t* control_out, unsigned char* irreversible, unsigned long long* mask,
+        unsigned char* in_check, int* move_out, unsigned long long* hash_out) {
     extern __shared__ unsigned long long tpb_smem[];
     unsigned* s_in = reinterpret_cast<unsigned*>(tpb_smem);                                 // [128][17]
     MoveTables* s_tables = reinterpret_cast<MoveTables*>(reinterpret_cast<uint8_t*>(tpb_smem) + kTpbIn);
@@ -949,19 +957,19 @@ __global__ void __launch_bounds__(kTpbThreads) engine_board_kernel(
         for (int j = tid; j < kTpbTables / 16; j += kTpbThreads)
             reinterpret_cast<uint4*>(s_tables)[j] = __ldg(reinterpret_cast<const uint4*>(&kMoveTables) + j);
     };
+    if (!kPick && mask != nullptr) load_tables();
+    begin_after_previous_grid();
     {
         // coalesced load: the block's boards are one contiguous run of 16-byte pieces
         const uint4* src = reinterpret_cast<const uint4*>(boards + first * 32);
         for (int j = tid; j < here * 4; j += kTpbThreads) {
-            const uint4 v = __ldg(src + j);
+            const uint4 v = src[j];
             unsigned* d = s_in + (j >> 2) * kTpbInStride + (j & 3) * 4;
             d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
         }
         if (kPick)
             for (int j = tid; j < here * 32; j += kTpbThreads)
                 s_mask[(j >> 5) * kTpbMaskStride + (j & 31)] = mask[first * 32 + j];
-        else if (mask != nullptr)
-            load_tables();
     }
     __syncthreads();
     const bool mine = tid < here;
@@ -1381,10 +1389,11 @@ __device__ __forceinline__ unsigned long long group_hash(const unsigned (&w)[4],
 // lanes read all of it first.
 template <bool kStep, bool kPick>
 __global__ void __launch_bounds__(kEngineThreads) engine_group_kernel(
-        const uint16_t* boards, const int16_t* control, const int* __restrict__ move,
-        const signed char* __restrict__ promo, const float* __restrict__ r, int n, uint16_t* boards_out,
-        int16_t* control_out, unsigned char* __restrict__ irreversible, unsigned long long* mask,
-        unsigned char* __restrict__ in_check, int* __restrict__ move_out, unsigned long long* __restrict__ hash_out) {
+        const uint16_t* boards, const int16_t* control, const int* move,
+        const signed char* promo, const float* r, int n, uint16_t* boards_out,
+        int16_t* control_out, unsigned char* irreversible, unsigned long long* mask,
+        unsigned char* in_check, int* move_out, unsigned long long* hash_out) {
+    begin_after_previous_grid();
     const int lane = threadIdx.x & 31, j = lane & 7;
     const long board = static_cast<long>(blockIdx.x) * kEngineBoards + (threadIdx.x >> 3);
     const bool valid = board < n;
@@ -1469,7 +1478,7 @@ __global__ void __launch_bounds__(kEngineThreads) engine_group_kernel(
 
 // How many of the first `length` entries of a game's ring equal `hash`: warp-collective.
 constexpr int kMaxHistory = 100;
-__device__ __forceinline__ int ring_matches(const unsigned long long* __restrict__ ring, long long length,
+__device__ __forceinline__ int ring_matches(const unsigned long long* ring, long long length,
                                             unsigned long long hash, int lane) {
     const int len = static_cast<int>(length < kMaxHistory ? length : kMaxHistory);
     int c = 0;
@@ -1492,15 +1501,16 @@ __device__ __forceinline__ int ring_matches(const unsigned long long* __restrict
 // One WARP per game, lane = slot: a game's words, board and ring are contiguous runs that a warp
 // reads whole, where a thread per game walked 1.1 KB of its own (4096 games with rings of up to
 // forty entries: 4 us instead of 12 us for the two launches this one replaces).
-__global__ void __launch_bounds__(128) terminal_kernel(const unsigned long long* __restrict__ mask,
-                                                       const unsigned char* __restrict__ in_check,
-                                                       const int16_t* __restrict__ control,
-                                                       const uint16_t* __restrict__ boards,
-                                                       const int* __restrict__ rep_count,
-                                                       const unsigned long long* __restrict__ hash,
-                                                       const unsigned long long* __restrict__ ring,
-                                                       const long long* __restrict__ length, int n,
-                                                       unsigned char* __restrict__ code, signed char* __restrict__ result) {
+__global__ void __launch_bounds__(128) terminal_kernel(const unsigned long long* mask,
+                                                       const unsigned char* in_check,
+                                                       const int16_t* control,
+                                                       const uint16_t* boards,
+                                                       const int* rep_count,
+                                                       const unsigned long long* hash,
+                                                       const unsigned long long* ring,
+                                                       const long long* length, int n,
+                                                       unsigned char* code, signed char* result) {
+    begin_after_previous_grid();
     const int lane = threadIdx.x & 31;
     const long board = static_cast<long>(blockIdx.x) * 4 + (threadIdx.x >> 5);
     if (board >= n) return;
@@ -1530,10 +1540,11 @@ __global__ void __launch_bounds__(128) terminal_kernel(const unsigned long long*
 // since the last irreversible move, `length` [n].  Push: record the position being left (`hash`
 // is the key BEFORE the move, `irreversible` describes the move); an irreversible move empties
 // the ring, because nothing at or before it can recur.
-__global__ void __launch_bounds__(128) history_push_kernel(unsigned long long* __restrict__ ring,
-                                                           long long* __restrict__ length,
-                                                           const unsigned long long* __restrict__ hash,
-                                                           const unsigned char* __restrict__ irreversible, int n) {
+__global__ void __launch_bounds__(128) history_push_kernel(unsigned long long* ring,
+                                                           long long* length,
+                                                           const unsigned long long* hash,
+                                                           const unsigned char* irreversible, int n) {
+    begin_after_previous_grid();
     const long g = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (g >= n) return;
     if (irreversible[g]) { length[g] = 0; return; }
@@ -1545,12 +1556,13 @@ __global__ void __launch_bounds__(128) history_push_kernel(unsigned long long* _
 // (1,632 bytes per game); a thread copies 16 bytes (a ring is fifty of them), or 8 where an array
 // does not start on a 16-byte boundary.
 template <int kWords>
-__global__ void __launch_bounds__(256) history_push_to_kernel(const unsigned long long* __restrict__ ring,
-                                                              const long long* __restrict__ length,
-                                                              const unsigned long long* __restrict__ hash,
-                                                              const unsigned char* __restrict__ irreversible, int n,
-                                                              unsigned long long* __restrict__ new_ring,
-                                                              long long* __restrict__ new_length) {
+__global__ void __launch_bounds__(256) history_push_to_kernel(const unsigned long long* ring,
+                                                              const long long* length,
+                                                              const unsigned long long* hash,
+                                                              const unsigned char* irreversible, int n,
+                                                              unsigned long long* new_ring,
+                                                              long long* new_length) {
+    begin_after_previous_grid();
     constexpr unsigned kPieces = kMaxHistory / kWords;
     const long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
     const long g = i / kPieces;
@@ -1574,10 +1586,11 @@ __global__ void __launch_bounds__(256) history_push_to_kernel(const unsigned lon
     if (piece == 0) new_length[g] = empties ? 0 : (len + 1 < kMaxHistory ? len + 1 : kMaxHistory);
 }
 // How many times the position has occurred, counting the present one: one warp per game.
-__global__ void __launch_bounds__(128) repetition_kernel(const unsigned long long* __restrict__ hash,
-                                                         const unsigned long long* __restrict__ ring,
-                                                         const long long* __restrict__ length, int n,
-                                                         int* __restrict__ count) {
+__global__ void __launch_bounds__(128) repetition_kernel(const unsigned long long* hash,
+                                                         const unsigned long long* ring,
+                                                         const long long* length, int n,
+                                                         int* count) {
+    begin_after_previous_grid();
     const int lane = threadIdx.x & 31;
     const long g = static_cast<long>(blockIdx.x) * 4 + (threadIdx.x >> 5);
     if (g >= n) return;
