@@ -151,6 +151,8 @@ struct Params {
     // staged arrays; `n` is then the capacity (the most the list can hold) the grid was sized for
     const int* leaf_index;
     const int* leaf_count;
+    int wave_ctas;              // one- and two-board tiles: CTAs of a whole wave
+    int after_waves;            // one-board tiles: launched beside this call's own two-board tiles
     int* status;
     unsigned long long* prof;   // 16 phase counters (cycles of warp 0, lane 0 of every CTA) or null
 };
@@ -2232,6 +2234,7 @@ struct bf_handle {
     bool prof_on = false;
     bool rsqrt_rn = false;        // BF_OPT_RSQRT_RN
     int sm_count = 0;
+    int wave_ctas = 0;            // CTAs of the one- and two-board tiles' kernels that run at a time
     long long launches = 0;
     // staging for bf_forward_host
     int cap_n = 0;
@@ -2289,17 +2292,17 @@ struct MappedInputs {
           ok(boards != nullptr && control != nullptr && rep != nullptr && (legal != nullptr) == (l != nullptr) &&
              bf_host_aligned(b, c, l, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr) != 0) {}
 };
-// Whether large batches of this handle run on two-board tiles (a wave is two positions per SM) or on
-// four-board ones.
-bool two_board_waves(const bf_handle* h) { return h->hdr.quant != 0 && h->hdr.rj_mode == 0; }
+// Whether large batches of this handle run on two-board tiles (a wave is two positions per SM) or, with
+// re-injection, on four-board ones.
+bool two_board_waves(const bf_handle* h) { return h->hdr.rj_mode == 0; }
 
 // bf_forward_host sizes its launches by how many times faster this GPU copies a position's logits
 // to the host than it evaluates a position.
-// (Of int8; one pair of figures serves every arithmetic: e4m3 produces 10.1 GB/s on two-board tiles where
-// int8 produces 10.6, fp16 9.4 on four-board ones, which moves the ratio, and a launch's size, by 5 to 7 %.)
+// (Of int8; one pair of figures serves every arithmetic: two-board tiles produce 11.2 GB/s in int8, 11.5 in e4m3,
+// 10.8 in fp16, which moves the ratio, and a launch's size, by 4 %.)
 constexpr double kEvalGBps = 8.8;        // logits a B200 produces per second at full rate on four-board
                                          // tiles (4356 B x 2.03 M)
-constexpr double kSmallTileRate = 1.2;   // how much faster two-board tiles are (2.42 M positions/s)
+constexpr double kSmallTileRate = 1.27;  // how much faster two-board tiles are (2.58 M positions/s)
 constexpr double kFastLinkRatio = 6.0;   // a GPU alone on its link: 55 GB/s against those 8.8
 
 // The launch sizes of bf_forward_host for `n` positions on a GPU whose wave is `wave` positions:
@@ -2403,16 +2406,72 @@ struct LeafList {
 };
 
 using Kernel = void (*)(bf::Params);
-template <bool kExpand>
+template <bool kExpand, int NB>
 Kernel small_tile_kernel(int quant) {
-    return quant == 0   ? bf::ws::encoder_ws_kernel<bf::kArF16, kExpand>
-           : quant == 1 ? bf::ws::encoder_ws_kernel<bf::kArE4M3, kExpand>
-           : quant == 2 ? bf::ws::encoder_ws_kernel<bf::kArI8Ffn, kExpand>
-           : quant == 4 ? bf::ws::encoder_ws_kernel<bf::kArI8Qkv, kExpand>
-                        : bf::ws::encoder_ws_kernel<bf::kArInt8, kExpand>;
+    return quant == 0   ? bf::ws::encoder_ws_kernel<bf::kArF16, kExpand, NB>
+           : quant == 1 ? bf::ws::encoder_ws_kernel<bf::kArE4M3, kExpand, NB>
+           : quant == 2 ? bf::ws::encoder_ws_kernel<bf::kArI8Ffn, kExpand, NB>
+           : quant == 4 ? bf::ws::encoder_ws_kernel<bf::kArI8Qkv, kExpand, NB>
+                        : bf::ws::encoder_ws_kernel<bf::kArInt8, kExpand, NB>;
 }
 // (the expansion has warps of its own: plain evaluations run without them, 1.5 % faster)
-Kernel small_tile_kernel(int quant, bool expand) { return expand ? small_tile_kernel<true>(quant) : small_tile_kernel<false>(quant); }
+Kernel small_tile_kernel(int quant, bool expand, int boards) {
+    return boards == 1 ? (expand ? small_tile_kernel<true, 1>(quant) : small_tile_kernel<false, 1>(quant))
+                       : (expand ? small_tile_kernel<true, 2>(quant) : small_tile_kernel<false, 2>(quant));
+}
+// Sets a handle's or device's kernels up; how many of their CTAs run at a time, in pairs: all SMs, but for
+// one of a GPC with an odd number of them.
+cudaError_t pairs_at_a_time(int quant, int sm_count, int* wave) {
+    for (int arm = 0; arm < 4; ++arm) {
+        const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(small_tile_kernel(quant, (arm & 1) != 0, 1 + (arm >> 1))),
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, bf::ws::kSmemRequest);
+        if (e != cudaSuccess) return e;
+    }
+    cudaLaunchAttribute cluster = {};
+    cluster.id = cudaLaunchAttributeClusterDimension;
+    cluster.val.clusterDim.x = 2;
+    cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(sm_count & ~1);
+    config.blockDim = dim3(bf::ws::threads(true));
+    config.dynamicSmemBytes = bf::ws::kSmemRequest;
+    config.attrs = &cluster;
+    config.numAttrs = 1;
+    int pairs = 0;
+    const cudaError_t e = cudaOccupancyMaxActiveClusters(&pairs, reinterpret_cast<const void*>(small_tile_kernel(quant, true, 2)), &config);
+    *wave = pairs > 0 && 2 * pairs < sm_count ? 2 * pairs : sm_count & ~1;
+    return e;
+}
+
+// An evaluation on one- and two-board tiles: one launch, or two where a batch ends in one-board tiles or where only
+// the device knows a leaf list's length (`Tiles`).  The one-board tiles then start as SMs become free, without
+// waiting for the launch beside them, and wait for it when they are done: what comes after them in the
+// stream comes after both.
+// `wave`: CTAs that run at a time (`pairs_at_a_time`).
+cudaError_t launch_tiles(bf::Params p, int wave, int one_board, cudaStream_t stream, bool early) {
+    const int n = p.n, quant = static_cast<int>(p.quant);
+    const bool expand = p.prior != nullptr;
+    p.wave_ctas = wave;
+    p.one_most = one_board;
+    const int full = n / (2 * wave), rest = n - full * 2 * wave;
+    const bool singles = n <= static_cast<long>(one_board) * wave;
+    const bool list = p.leaf_count != nullptr;
+    const bool twos = !singles, ones = singles || (one_board > 0 && (list || (rest > 0 && rest <= wave)));
+    auto ctas = [&](int boards, int per) {
+        const long pairs = (boards + 2L * per - 1) / (2 * per);
+        return static_cast<int>(2 * pairs < wave ? 2 * pairs : wave);
+    };
+    cudaError_t e = cudaSuccess;
+    if (twos)
+        e = launch_early(small_tile_kernel(quant, expand, 2), ctas(n, 2), bf::ws::threads(expand), bf::ws::kSmemRequest, 2, stream,
+                         early, p);
+    if (ones && e == cudaSuccess) {
+        p.after_waves = twos ? 1 : 0;
+        e = launch_early(small_tile_kernel(quant, expand, 1), ctas(singles || list ? n : rest, 1), bf::ws::threads(expand),
+                         bf::ws::kSmemRequest, 2, stream, early || twos, p);
+    }
+    return e;
+}
 
 int launch(bf_handle* h, const uint16_t* boards, const int16_t* control, const uint8_t* rep,
            const uint64_t* legal, int n, void* policy, void* promo, float* value, void* y, int stage,
@@ -2453,16 +2512,13 @@ int launch(bf_handle* h, const uint16_t* boards, const int16_t* control, const u
     // the instrumented instantiation only when a dump, a capture or the phase clock is asked for
     const bool dbg = stage != 0 || cap_layer >= 0 || p.prof != nullptr;
     if (cap_layer >= 0 && p.quant != 3) return fail(BF_ENOTSUP, "operand capture is for the int8 arithmetic");
-    if (!dbg && p.rj_mode == 0 && bf_tile_boards(p.quant, n, h->sm_count, h->one_board_factor) < 4) {
-        p.one_most = h->one_board_factor;
-        const int ctas = n < h->sm_count ? n : h->sm_count;
-        const bool expand = p.prior != nullptr;
-        small_tile_kernel(p.quant, expand)<<<ctas, bf::ws::threads(expand), bf::ws::kSmemRequest, stream>>>(p);
+    if (!dbg && p.rj_mode == 0) {
+        BF_CUDA(launch_tiles(p, h->wave_ctas, h->one_board_factor, stream, true));
     } else {
-        // four-board tiles: large batches of the fp16 arithmetic, re-injection, and the instrumented arms
-        // (dumps, captures, the phase clock, the backbone entry)
+        // four-board tiles: re-injection, and the instrumented arms (dumps, captures, the phase clock, the
+        // backbone entry)
         const auto kernel =
-            p.quant == 0 ? (p.rj_mode == 0 ? (dbg ? bf::encoder_kernel<true, false, bf::kArF16> : bf::encoder_kernel<false, false, bf::kArF16>)
+            p.quant == 0 ? (p.rj_mode == 0 ? bf::encoder_kernel<true, false, bf::kArF16>
                                            : (dbg ? bf::encoder_kernel<true, true, bf::kArF16> : bf::encoder_kernel<false, true, bf::kArF16>))
             : p.quant == 4 ? bf::encoder_kernel<true, false, bf::kArI8Qkv>
             : p.quant == 2 ? bf::encoder_kernel<true, false, bf::kArI8Ffn>
@@ -2534,8 +2590,7 @@ int bf_create(const void* blob, size_t blob_bytes, int device, bf_handle** out) 
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->chunk_done, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreate(&h->copy_t0);
     if (e == cudaSuccess) e = cudaEventCreate(&h->copy_t1);
-    for (const void* k : {reinterpret_cast<const void*>(&bf::encoder_kernel<false, false, bf::kArF16>),
-                          reinterpret_cast<const void*>(&bf::encoder_kernel<true, false, bf::kArI8Qkv>),
+    for (const void* k : {reinterpret_cast<const void*>(&bf::encoder_kernel<true, false, bf::kArI8Qkv>),
                           reinterpret_cast<const void*>(&bf::encoder_kernel<true, false, bf::kArI8Ffn>),
                           reinterpret_cast<const void*>(&bf::encoder_kernel<true, false, bf::kArE4M3>),
                           reinterpret_cast<const void*>(&bf::encoder_kernel<true, false, bf::kArF16>),
@@ -2545,10 +2600,7 @@ int bf_create(const void* blob, size_t blob_bytes, int device, bf_handle** out) 
                           reinterpret_cast<const void*>(&bf::encoder_kernel<false, true, bf::kArInt8>),
                           reinterpret_cast<const void*>(&bf::encoder_kernel<true, true, bf::kArInt8>)})
         if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bf::kSmemRequest);
-    for (int expand = 0; expand < 2; ++expand)
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(reinterpret_cast<const void*>(small_tile_kernel(static_cast<int>(hdr.quant), expand != 0)),
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, bf::ws::kSmemRequest);
+    if (e == cudaSuccess) e = pairs_at_a_time(static_cast<int>(hdr.quant), h->sm_count, &h->wave_ctas);
     if (e != cudaSuccess) {
         bf_destroy(h);
         return fail(BF_ECUDA, std::string("bf_create: ") + cudaGetErrorString(e));
@@ -3002,15 +3054,10 @@ long long bf_launch_count(const bf_handle* h) { return h ? h->launches : 0; }
 
 double bf_host_link_gbps(const bf_handle* h) { return h ? h->d2h_gbps : 0.0; }
 
-// Which form a plain evaluation runs in: one- and two-board tiles (bf_encoder_ws.cuh) or four-board tiles.
-// A tile takes the same time whatever the batch, so the tiles of the busiest SM decide.  Measured, us
-// per one-, two- and four-board tile of an SM (B200):
-//   int8 90 / 126    int8 FFN+QKV 96 / 128    int8 FFN 103 / 133 / 273
-//   e4m3 100 / 130 / 270    fp16 129 / 152 / 272
-// Two two-board tiles beat a four-board one everywhere but in fp16, whose products, 32 bytes of K at
-// half the rate and twice the weight bytes, keep the weight stream and the tensor pipe busy for half
-// of a two-board tile's time; there the four-board form takes the batches that fill it.  Of a leaf list
-// only the capacity is known here, and that decides.
+// The tiles of evaluations whose SMs work by themselves, by the tiles of the busiest SM: what launches went by
+// before SMs worked in pairs, kept with its results for callers that size their batches by it.  Pairs of SMs take one- and
+// two-board tiles in every arithmetic (`launch_tiles`): four boards took an SM 272 us in fp16, a pair's two-board tile
+// takes 116.
 int bf_tile_boards(int quant, int n, int sm_count, int one_board) {
     if (n < 1 || sm_count < 1) return fail(BF_EINVAL, "n and sm_count must be positive");
     if (n <= static_cast<long>(one_board) * sm_count) return 1;
@@ -3230,7 +3277,7 @@ constexpr int kNoAllocMaxDevices = 64;
 struct NoAllocDevice {
     bool ready = false;
     void* scratch = nullptr;      // device address of bf::g_noalloc_scratch on this device
-    int sm_count = 0;
+    int wave_ctas = 0;            // CTAs of the evaluator that run at a time
     const void* blob = nullptr;   // blob whose header is cached below
     size_t blob_bytes = 0;
     BlobHeader hdr{};
@@ -3255,10 +3302,8 @@ int noalloc_setup(int device, NoAllocDevice** out) {
         void* ptr = nullptr;
         BF_CUDA(cudaGetSymbolAddress(&ptr, bf::g_noalloc_scratch));
         BF_CUDA(cudaMemset(ptr, 0, bf::kNoAllocScratchBytes));
-        BF_CUDA(cudaFuncSetAttribute(bf::ws::encoder_ws_kernel<bf::kArInt8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     bf::ws::kSmemRequest));
+        BF_CUDA(pairs_at_a_time(3, prop.multiProcessorCount, &d.wave_ctas));
         d.scratch = ptr;
-        d.sm_count = prop.multiProcessorCount;
         d.ready = true;
     }
     *out = &d;
@@ -3314,7 +3359,7 @@ int bf_forward_noalloc(int device, const void* blob_dev, size_t blob_bytes, cons
     BF_ON_DEVICE(device);
     BlobHeader hdr;
     void* scratch = nullptr;
-    int sm_count = 0;
+    int wave = 0;
     {
         std::lock_guard<std::mutex> lock(g_noalloc_mutex);
         NoAllocDevice* d = nullptr;
@@ -3322,7 +3367,7 @@ int bf_forward_noalloc(int device, const void* blob_dev, size_t blob_bytes, cons
         if (rc == BF_OK) rc = noalloc_header(d, blob_dev, blob_bytes, &hdr);
         if (rc != BF_OK) return rc;
         scratch = d->scratch;
-        sm_count = d->sm_count;
+        wave = d->wave_ctas;
     }
     if (n == 0) return BF_OK;
     const uint8_t* base = static_cast<const uint8_t*>(blob_dev);
@@ -3343,10 +3388,8 @@ int bf_forward_noalloc(int device, const void* blob_dev, size_t blob_bytes, cons
     p.cap_layer = -1; p.cap_op = -1; p.cap_a = nullptr; p.cap_acc = nullptr;
     p.status = static_cast<int*>(scratch);         // the device address, not the symbol
     p.prof = nullptr;
-    p.one_most = 1;
-    bf::ws::encoder_ws_kernel<bf::kArInt8, false><<<n < sm_count ? n : sm_count, bf::ws::threads(false), bf::ws::kSmemRequest,
-                                                    static_cast<cudaStream_t>(stream)>>>(p);
-    BF_CUDA(cudaGetLastError());
+    // (the caller's own blob may be an output of the grid before)
+    BF_CUDA(launch_tiles(p, wave, 1, static_cast<cudaStream_t>(stream), false));
     return BF_OK;
 }
 

@@ -1,14 +1,16 @@
-// The evaluator kernel on weight-stationary tensor-core tiles of one or two boards (included by
-// bf_encoder.cu): the form every plain evaluation runs in.
+// The evaluator kernel on tensor-core tiles of one or two boards, by pairs of SMs (included by bf_encoder.cu): the
+// form every plain evaluation runs in.
 //
-// Why one or two boards.  `tcgen05.mma.ws` takes an M of 32 or 64 and lays the product out over all
-// 128 lanes of tensor memory: lane quadrant q holds, for M = 32, all 32 rows and output columns
-// 64 q .. 64 q + 63 of an N = 256 product; for M = 64, the 32 rows of board q & 1 and output columns
-// 128 (q >> 1) .. + 127.  So sixteen row warps (four per quadrant, thread = row x 16 or 32 columns)
-// share the element-wise work of one or two boards, where a 128-row tile gives a board four warps,
-// and an N = 256 product of 32 / 64 / 128 rows costs 84 / 92 / 166 cycles per 32 bytes of K (measured;
-// the weights' way out of shared memory alone is 64).  A board then takes as long as its own chain
-// of phases, and that chain is a quarter as long.
+// Why one or two boards, and why pairs.  A 128-row tile takes as long as one board's chain of phases, with four warps
+// to a board; sixteen row warps on one or two boards make that chain a quarter as long.  A product then
+// has 32 or 64 rows, and two things bound it: the weights' way out of shared memory (an N = 256 product of 64 rows
+// by `tcgen05.mma.ws` takes 80.7 cycles per 32 bytes of K, of which the weights are 64) and their way into the SM (at
+// 64 bytes a cycle, 12.3 k cycles of a layer in int8, 24.6 k in fp16).  `tcgen05.mma.cta_group::2` halves
+// both: two SMs share a product, M = 128 rows, 64 of each; each loads and keeps half of the weight rows (64.8 cycles per
+// 32 bytes of K).  An SM's tensor memory gets the product of its own rows over all 128 lanes: lane quadrant q holds
+// rows 32 (q & 1) .. + 31 and output columns 128 (q >> 1) .. + 127.  So sixteen row warps (four per quadrant,
+// thread = row x 32 columns) share the element-wise work of two boards; a single board's operand rows are there
+// twice, and the two quadrants that hold its product take half of the columns each (thread = row x 16).
 //
 // What follows from a thread's columns being the same in every product:
 //   * the residual stream x stays in the owning thread's registers from the embedding to the heads;
@@ -22,13 +24,10 @@
 //
 // The arithmetic is the four-board kernel's, bit for bit (the order of every sum included).
 //
-// Measured on one B200, int8, against the forms before it (four boards per tile; one board per tile
-// with its rows written four times into a 128-row operand), through the device-pointer call: batch 1
-// 88 us (176), 64 90 us (176), 149-296 127 us (281), 333 213 us (285), 4096 1.68 ms (1.98).  What bounds
-// it: the row warps, four to a scheduler and all in the same phase.  At 4096 issue slots are 57 % busy, the
-// tensor pipe 26 %.  Of a one-board tile's 19,800 cycles per layer a row warp waits 5,400 for products
-// (1,000 to 1,350 after each norm and after attention, whose operand has just been written), of a
-// two-board tile's 27,000 5,500; the rest is its own dependent instructions and the board's meetings.
+// Measured on one B200, us, against tiles of one SM (M = 32 and 64 by `tcgen05.mma.ws`): a one-board tile
+// int8 85 (91), e4m3 91 (101), fp16 109 (129); a two-board tile 117 (127), 117 (130), 116 (152); batch 4096 1586
+// (1675), 1547 (1727), 1650 (1870, then on four-board tiles).  What bounds it: the row warps, four to a scheduler and all in the same
+// phase.
 #pragma once
 
 namespace bf {
@@ -36,14 +35,14 @@ namespace ws {
 
 constexpr int kProducerWarp = 16, kMmaWarp = 17, kExpandWarp = 18;
 constexpr int threads(bool expand) { return expand ? 640 : 576; }
-constexpr uint32_t kStage = 32768;                 // one 128-byte K-slab of 256 weight rows
+constexpr uint32_t kStage = 16384;                 // one 128-byte K-slab of this SM's 128 rows of a product's weights
 // ---- shared memory map ------------------------------------------------------------------
 // A operand: K-slabs of [rows][128 B], two of bytes or (where QKV or the out-projection runs in fp16)
 // four of halves.  H: the ff2 operand's chunks; before and after that the attention scratch, the norms'
 // partial sums, the head operand.
 template <int kAr>
 struct Map {
-    static constexpr int kStages = Cfg<kAr>::kHalfA ? 3 : 4;
+    static constexpr int kStages = Cfg<kAr>::kHalfA ? 6 : 8;
     static constexpr uint32_t SM_H = Cfg<kAr>::kHalfA ? 32768 : 16384;
     static constexpr uint32_t SM_RING = SM_H + 65536;
 };
@@ -52,41 +51,59 @@ constexpr uint32_t kHeadA = 32768;                 // the head operand's place i
 // the fused expansion's logits: per board 32 policy rows of 128 bytes, then 16 bytes of promotion logits
 // per slot; the last quarter of H, which the next tile touches in its first FFN
 constexpr uint32_t kStagePolicy = 49152, kStageAux = kStagePolicy + 8192;
-constexpr uint32_t SM_STAT = 16384 + 65536 + 4 * kStage;
+constexpr uint32_t SM_STAT = 16384 + 65536 + 8 * kStage;
 constexpr uint32_t SM_MAX = SM_STAT + 1024;        // row maxima: attention output, four hidden chunks
 constexpr uint32_t SM_LIST = SM_MAX + 5 * 256;     // fused expansion: 1 KB per board
 constexpr uint32_t SM_PAR = SM_LIST + 2048;        // scales and biases of two layers
 constexpr uint32_t SM_BAR = SM_PAR + 2 * kLparamStride;
-constexpr uint32_t SM_MISC = SM_BAR + 192;
+constexpr uint32_t SM_MISC = SM_BAR + 8 * 34;
 constexpr uint32_t SM_BYTES = SM_MISC + 64, kSmemRequest = SM_BYTES + 1024;
 static_assert(kSmemRequest <= 232448 && kLparamStride % 16 == 0 && SM_PAR % 16 == 0, "shared memory map");
-static_assert(Map<kArF16>::SM_RING + 3 * kStage <= SM_STAT && Map<kArInt8>::SM_RING + 4 * kStage <= SM_STAT, "shared memory map");
-enum { B_FULL = 0, B_EMPTY = 4, B_ACC = 8, B_PAR = 12, B_A = 14, B_H = 15, B_STAGED = 17, B_EXPANDED = 18, B_COUNT = 19 };
+static_assert(Map<kArF16>::SM_RING + 6 * kStage <= SM_STAT && Map<kArInt8>::SM_RING + 8 * kStage <= SM_STAT, "shared memory map");
+enum { B_FULL = 0, B_EMPTY = 8, B_ACC = 16, B_PAR = 20, B_A = 22, B_H = 23, B_STAGED = 25, B_EXPANDED = 26, B_COUNT = 27 };
 __device__ __forceinline__ uint32_t bar(uint32_t smem, int i) { return smem + SM_BAR + 8u * i; }
 
-// Which boards a CTA evaluates, tile by tile.  At most `one_most` boards per CTA: one-board tiles alone.
-// More: as many whole waves of two-board tiles as there are, then what is left, one board per CTA where
-// that is enough (and allowed), else two.  A one-board tile takes about two thirds of a two-board
-// tile's time.
+// ---- what is different in a pair of SMs ----
+// These take the place of the functions of the same names for one SM in everything below: a product is the pair's,
+// its completion goes to the same barrier in both SMs, and an operand's or a weight stage's arrival to the first
+// SM's barrier, whose MMA warp issues the pair's products.  (Arrivals and waits at their default scope, the
+// operands made visible by the proxy fence before: at cluster scope an arrival costs some 500 cycles, a
+// wait more, and a two-board tile 147 us instead of 118.)
+__device__ __forceinline__ void umma_ws_i8(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    umma_pair_i8(d, a, b, idesc, accumulate);
+}
+__device__ __forceinline__ void umma_ws_f16(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    umma_pair_f16(d, a, b, idesc, accumulate);
+}
+__device__ __forceinline__ void umma_ws_f8(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    umma_pair_f8(d, a, b, idesc, accumulate);
+}
+__device__ __forceinline__ void tc_commit(uint32_t bar) { tc_commit_pair(bar); }
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) { mbar_arrive_cluster(cluster_address(bar, 0)); }
+
+// Which boards a CTA evaluates, tile by tile.  A launch's tiles hold `NB` boards each.  At most `one_most` boards
+// per CTA: one-board tiles alone.  More: as many whole waves of two-board tiles as there are, then what is left, one board
+// per CTA where that is enough (and allowed), else two.  A one-board tile takes about two thirds of a
+// two-board tile's time.  The two forms are kernels of their own -- together they cost each other registers, 2 to
+// 4 % of a tile -- so that a batch takes one launch of either or one of each; of a leaf list, whose length only the
+// kernels know, each makes its own part.  `grid`: CTAs of a whole wave.  Both SMs of a pair have as many tiles.
+template <int NB>
 struct Tiles {
-    int n, grid, cta, full, rest, per;
-    bool singles;
-    __device__ Tiles(int n_, int grid_, int cta_, int one_most) : n(n_), grid(grid_), cta(cta_) {
-        singles = n <= one_most * grid;
-        full = n / (2 * grid);
-        rest = n - full * 2 * grid;
-        per = rest <= grid && one_most > 0 ? 1 : 2;
+    int n, first, step, tiles;       // boards in all; this CTA's first board; boards per round; rounds
+    __device__ Tiles(int n_, int grid, int ctas, int cta, int one_most) : n(n_) {
+        const int full = n / (2 * grid), rest = n - full * 2 * grid, lead = cta & ~1;
+        const bool singles = n <= one_most * grid, one = rest <= grid && one_most > 0;
+        int begin = 0, end = n;      // the boards of this form
+        if (NB == 1) { if (!singles) begin = one ? n - rest : n; }
+        else if (singles) end = 0;
+        else if (one) end = n - rest;
+        step = NB * ctas;
+        first = begin + NB * cta;
+        const int mine = begin + NB * lead;
+        tiles = mine < end ? (end - mine + step - 1) / step : 0;
     }
-    // number of tiles of this CTA; tile k starts at board `first` and holds `boards` (1 or 2)
-    __device__ int count() const {
-        if (singles) return cta < n ? (n - cta + grid - 1) / grid : 0;
-        return full + (cta * per < rest ? 1 : 0);
-    }
-    __device__ void at(int k, int& first, int& boards) const {
-        if (singles) { boards = 1; first = k * grid + cta; return; }
-        boards = k < full ? 2 : per;
-        first = k < full ? 2 * (k * grid + cta) : 2 * full * grid + per * cta;
-    }
+    __device__ int count() const { return tiles; }
+    __device__ int at(int k) const { return first + k * step; }
 };
 
 struct Row {
@@ -106,16 +123,21 @@ struct Row {
 template <int NB>
 struct Own {
     static constexpr int kW = 16 * NB;                       // columns per thread of a 256-wide row
-    static constexpr int kRowsT = 32 * NB;
-    static constexpr uint32_t kSlab = kRowsT * 128;          // bytes of a K-slab of an operand
-    static constexpr uint32_t kSlot = NB == 1 ? 64 : 128;    // tensor-memory columns of a slot
+    static constexpr uint32_t kSlab = 64 * 128;              // bytes of a K-slab of an operand
+    static constexpr uint32_t kSlot = 128;                   // tensor-memory columns of a slot
     static constexpr int kGroup = 16 / NB;                   // threads that share a row
     static __device__ int board(const Row& c) { return NB == 1 ? 0 : c.q & 1; }
-    static __device__ int col(const Row& c) { return NB == 1 ? 64 * c.q + 16 * c.s : 128 * (c.q >> 1) + 32 * c.s; }
-    static __device__ int member(const Row& c) { return NB == 1 ? 4 * c.q + c.s : 4 * (c.q >> 1) + c.s; }
+    static __device__ int col(const Row& c) { return 128 * (c.q >> 1) + 32 * c.s + (NB == 1 ? 16 * (c.q & 1) : 0); }
+    static __device__ int member(const Row& c) { return NB == 1 ? 8 * (c.q >> 1) + 2 * c.s + (c.q & 1) : 4 * (c.q >> 1) + c.s; }
     static __device__ int row(const Row& c) { return 32 * board(c) + c.lane; }
-    static __device__ uint32_t slot(const Row& c, int k) { return c.tm + kSlot * k + kW * c.s; }
+    static __device__ uint32_t slot(const Row& c, int k) { return c.tm + kSlot * k + 32 * c.s + (NB == 1 ? 16 * (c.q & 1) : 0); }
 };
+// 16 bytes of an operand row.  A single board's rows are there twice, so that every quadrant of tensor memory has them.
+template <int NB>
+__device__ __forceinline__ void store_operand(uint32_t at, uint4 v) {
+    sts128(at, v);
+    if (NB == 1) sts128(at + 32 * 128, v);
+}
 // The warps of a board meet here (barriers of their own for one- and two-board tiles: a warp may be a
 // tile ahead).
 template <int NB>
@@ -245,15 +267,15 @@ template <int NB, bool kE4M3 = false>
 __device__ __forceinline__ void store_operand8(const Row& c, uint32_t base, int k, const uint32_t* v, float inv) {
     using O = Own<NB>;
     const int col = O::col(c);
-    sts128(base + (col >> 7) * O::kSlab + sw_off(O::row(c), ((col & 127) >> 4) + k), quant16_any<kE4M3>(v, inv, c.one2));
+    store_operand<NB>(base + (col >> 7) * O::kSlab + sw_off(O::row(c), ((col & 127) >> 4) + k), quant16_any<kE4M3>(v, inv, c.one2));
 }
 template <int NB>
 __device__ __forceinline__ void store_operand16(const Row& c, uint32_t base, int k, const uint32_t* v) {
     using O = Own<NB>;
     const int col = O::col(c), row = O::row(c), group = ((col & 63) >> 3) + 2 * k;
     const uint32_t slab = base + (col >> 6) * O::kSlab;
-    sts128(slab + sw_off(row, group), make_uint4(v[0], v[1], v[2], v[3]));
-    sts128(slab + sw_off(row, group + 1), make_uint4(v[4], v[5], v[6], v[7]));
+    store_operand<NB>(slab + sw_off(row, group), make_uint4(v[0], v[1], v[2], v[3]));
+    store_operand<NB>(slab + sw_off(row, group + 1), make_uint4(v[4], v[5], v[6], v[7]));
 }
 
 // ---- LayerNorm ----
@@ -486,8 +508,8 @@ __device__ __forceinline__ void attention_block(const Row& c, uint32_t lp, float
     // Q, K and V one after the other.  Two boards: one warp per head, whose block serves Q, K, V and the
     // outputs in turn.  One board: two warps per head, each with half the query rows; Q, K and V have
     // blocks of their own and the outputs go over Q.
-    const int head = NB == 1 ? 2 * c.q + (c.s >> 1) : 4 * c.q + c.s;
-    const int first = NB == 1 ? 16 * (c.s & 1) : 0;
+    const int head = NB == 1 ? 4 * (c.q >> 1) + c.s : 4 * c.q + c.s;
+    const int first = NB == 1 ? 16 * (c.q & 1) : 0;
     const uint32_t block = c.h + 2048u * head;
     uint32_t qa[NB][2][4], s[NB][4][2];
 #pragma unroll
@@ -748,12 +770,12 @@ __device__ __forceinline__ void heads(const Row& c, const Params& p, int board, 
 #pragma unroll
             for (int j = 0; j < 4; ++j)
                 y[j] = f2_to_h2(fma2(mul2(add2(h2_to_f2(x[4 * v + j]), nmean2), rstd2), h2_to_f2(gw[j]), h2_to_f2(bw[j])));
-            sts128(c.h + kHeadA + (col >> 6) * O::kSlab + sw_off(row, ((col & 63) >> 3) + v), make_uint4(y[0], y[1], y[2], y[3]));
+            store_operand<NB>(c.h + kHeadA + (col >> 6) * O::kSlab + sw_off(row, ((col & 63) >> 3) + v), make_uint4(y[0], y[1], y[2], y[3]));
         }
         publish(c, B_A);
     }
     // output columns of this thread: hc .. hc + 8 NB - 1
-    const int hc = NB == 1 ? 32 * c.q + 8 * c.s : 64 * (c.q >> 1) + 16 * c.s;
+    const int within = 16 * c.s + (NB == 1 ? 8 * (c.q & 1) : 0), hc = 64 * (c.q >> 1) + within;
     // while the product runs: the legality words
     unsigned long long lw = ~0ull;
     if (p.legal != nullptr && p.policy != nullptr && valid && hc < 64) lw = p.legal[grow];
@@ -763,7 +785,7 @@ __device__ __forceinline__ void heads(const Row& c, const Params& p, int board, 
     uint32_t v[4 * NB];
     {
         uint32_t acc[8 * NB];
-        const uint32_t t = c.tm + 8 * NB * c.s;
+        const uint32_t t = c.tm + within;
         if constexpr (NB == 1) tmem_ld8(t, acc); else tmem_ld16(t, acc);
         tmem_wait_ld();
 #pragma unroll
@@ -779,7 +801,7 @@ __device__ __forceinline__ void heads(const Row& c, const Params& p, int board, 
             sts128(c.h + kStageAux + 512u * O::board(c) + 16u * lane, make_uint4(v[0], v[1], v[2], v[3]));
         }
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar(c.smem, B_STAGED));
+        if (lane == 0) bfptx::mbar_arrive(bar(c.smem, B_STAGED));
     }
     if (hc < 64) {
         if (valid && p.policy != nullptr) {
@@ -830,18 +852,17 @@ __device__ __forceinline__ void heads(const Row& c, const Params& p, int board, 
 // the next tile: 4096 positions 1793 us with the words given, 1839 with the moves generated; here 1743 and
 // 1766.  Where the rows' first FFN of the next
 // tile would overwrite the staged logits they wait for B_EXPANDED.
+template <int NB>
 __device__ __forceinline__ void expander(uint32_t smem, uint8_t* smem_gen, uint32_t h, volatile int* abort_flag, const Params& p,
-                                         const Tiles& tiles, int n_tiles, int which, int lane) {
-    for (int k = 0; k < n_tiles; ++k) {
-        int first, boards;
-        tiles.at(k, first, boards);
-        const int item = first + which;
-        const bool valid = which < boards && item < tiles.n;
+                                         const Tiles<NB>& tiles, int which, int lane) {
+    for (int k = 0; k < tiles.count(); ++k) {
+        const int item = tiles.at(k) + which;
+        const bool valid = which < NB && item < tiles.n;
         int board = item, ctl = 1;
         uint32_t word = 0u;
         unsigned long long moves = 0ull;
         if (valid) {
-            if (p.leaf_index != nullptr) board = __ldg(p.leaf_index + item);
+            if (p.leaf_index != nullptr) board = p.leaf_index[item];
             const long at = static_cast<long>(board) * kT + lane;
             word = p.boards[at];
             ctl = static_cast<int>(p.control[board]);
@@ -854,7 +875,7 @@ __device__ __forceinline__ void expander(uint32_t smem, uint8_t* smem_gen, uint3
             expand_board(p, board, lane, true, word, ctl, moves, h + kStagePolicy + 4096u * which + 128u * lane, lane & 7,
                          h + kStageAux + 512u * which + 16u * lane, smem_gen + SM_LIST + 1024u * which);
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar(smem, B_EXPANDED));
+        if (lane == 0) bfptx::mbar_arrive(bar(smem, B_EXPANDED));
     }
 }
 
@@ -864,7 +885,7 @@ __device__ __forceinline__ void row_tile(Row& c, const Params& p, int first) {
     using O = Own<NB>;
     const int item = first + O::board(c), lane = c.lane, col = O::col(c);
     const bool valid = item < c.n;
-    const int board = (valid && p.leaf_index != nullptr) ? __ldg(p.leaf_index + item) : item;
+    const int board = (valid && p.leaf_index != nullptr) ? p.leaf_index[item] : item;
     const uint32_t word = valid ? p.boards[static_cast<long>(board) * kT + lane] : 0u;
     uint32_t alive = __ballot_sync(0xffffffffu, ((word >> 11) & 1u) == 0u);
     const int ctl = valid ? static_cast<int>(p.control[board]) : 1;
@@ -932,15 +953,17 @@ __device__ __forceinline__ void row_tile(Row& c, const Params& p, int first) {
 // The blob's stages are the four-board kernel's: per head pair [Q 64 | K 64 | V 64 rows], then 128-row
 // units, two to each 256-row product.  A stage here is 256 rows of one K-slab, put together from four
 // or two of their pieces.  The whole warp walks the stages and waits; one elected lane issues.
+// Each SM of the pair loads its half of every product's rows: the first or the second of two units, two of four head pairs.
 template <int kAr>
-__device__ __forceinline__ void producer(uint32_t smem, volatile int* abort_flag, const Params& p, int n_tiles) {
+__device__ __forceinline__ void producer(uint32_t smem, volatile int* abort_flag, const Params& p, int n_tiles, uint32_t rank) {
     using C = Cfg<kAr>;
     constexpr uint32_t kStages = Map<kAr>::kStages, kRing = Map<kAr>::SM_RING;
     uint32_t i = 0;
     // the next stage: `copies(dst, barrier)` of `bytes` in all
     auto stage = [&](uint32_t bytes, auto&& copies) {
         const uint32_t k = i % kStages;
-        mbar_wait(bar(smem, B_EMPTY + k), (i / kStages - 1u) & 1u, abort_flag, kErrProducer);
+        if (i == kStages && !p.after_waves) { previous_grid_wait(); next_grid_may_start(); }   // (before the first wait that has a limit)
+        if (i >= kStages) mbar_wait(bar(smem, B_EMPTY + k), (i / kStages - 1u) & 1u, abort_flag, kErrProducer);
         if (elect_one()) {
             mbar_arrive_expect_tx(bar(smem, B_FULL + k), bytes);
             copies(smem + kRing + k * kStage, bar(smem, B_FULL + k));
@@ -949,15 +972,12 @@ __device__ __forceinline__ void producer(uint32_t smem, volatile int* abort_flag
     };
     // K-slab s of the product whose two 128-row units start at `u0` and `u1`
     auto two_units = [&](const uint8_t* u0, const uint8_t* u1, int s) {
-        stage(kStage, [&](uint32_t dst, uint32_t full) {
-            bulk_g2s(dst, u0 + s * kRStage, kRStage, full);
-            bulk_g2s(dst + kRStage, u1 + s * kRStage, kRStage, full);
-        });
+        stage(kStage, [&](uint32_t dst, uint32_t full) { bulk_g2s(dst, (rank ? u1 : u0) + s * kRStage, kRStage, full); });
     };
     // The scales and biases of a layer go into one of two places.  Those of the next layer are sent when
-    // the ring has taken the out-projection's stages: Q of this layer has then been consumed, so every
-    // row warp has published this layer's first operand and is done with the layer before, whose place
-    // they take.
+    // the ring has taken as many of this layer's stages as it holds and one more: Q's first has then been
+    // consumed, so every row warp has published this layer's first operand and is done with the layer before,
+    // whose place they take.
     uint32_t g = 0;             // layers whose parameters have been sent
     auto params = [&](int layer) {
         if (elect_one()) {
@@ -971,17 +991,19 @@ __device__ __forceinline__ void producer(uint32_t smem, volatile int* abort_flag
     for (int tile = 0; tile < n_tiles; ++tile) {
         const uint8_t* src = p.wstream;
         for (int layer = 0; layer < p.n_layers; ++layer, src += C::kLayerStream) {
+            const uint32_t begin = i;
+            // (an FFN stage: the ring is no deeper than the stages before the FFN and ff1's)
+            constexpr uint32_t kBefore = 3 * C::kQkvSlabs + C::kOutSlabs, kFirstFfn = kBefore > kStages ? kBefore : kStages;
+            static_assert(kFirstFfn < kBefore + 8 * C::kFfnSlabs, "the parameters are sent within the layer");
             for (int m = 0; m < 3; ++m)                                     // Q, K, V
                 for (int s = 0; s < C::kQkvSlabs; ++s)
                     stage(kStage, [&](uint32_t dst, uint32_t full) {
-                        const uint8_t* from = src + s * kQStage + m * 8192;
+                        const uint8_t* from = src + s * kQStage + m * 8192 + 2 * rank * C::kQkvSlabs * kQStage;
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) bulk_g2s(dst + 8192 * j, from + C::kQkvSlabs * j * kQStage, 8192, full);
+                        for (int j = 0; j < 2; ++j) bulk_g2s(dst + 8192 * j, from + C::kQkvSlabs * j * kQStage, 8192, full);
                     });
             const uint8_t* out = src + 4 * C::kQkvSlabs * kQStage;
             for (int s = 0; s < C::kOutSlabs; ++s) two_units(out, out + C::kOutSlabs * kRStage, s);
-            if (layer + 1 < p.n_layers) params(layer + 1);
-            else if (tile + 1 < n_tiles) params(0);
             // ff1 chunks 0-3, then ff2 chunks 0-3; where their two units lie in the packed order
             const uint8_t* ffn = out + 2 * C::kOutSlabs * kRStage;
             for (int u = 0; u < 8; ++u) {
@@ -994,12 +1016,20 @@ __device__ __forceinline__ void producer(uint32_t smem, volatile int* abort_flag
                     u0 = (0xEC84A620u >> (4 * u)) & 15u;
                     u1 = u0 + 1;
                 }
-                for (int s = 0; s < C::kFfnSlabs; ++s)
+                for (int s = 0; s < C::kFfnSlabs; ++s) {
                     two_units(ffn + u0 * C::kFfnSlabs * kRStage, ffn + u1 * C::kFfnSlabs * kRStage, s);
+                    if (i - begin == kFirstFfn + 1u) {
+                        if (layer + 1 < p.n_layers) params(layer + 1);
+                        else if (tile + 1 < n_tiles) params(0);
+                    }
+                }
             }
         }
+        // (the second SM has rows 64 to 95 of the head's; what else its half of the product reads is left from before,
+        // and no output comes from it)
+        const uint32_t skip = rank ? 8192u : 0u, bytes = rank ? kHeadStage - 8192u : 8192u;
         for (uint32_t st = 0; st < kHeadStages; ++st, src += kHeadStage)
-            stage(kHeadStage, [&](uint32_t dst, uint32_t full) { bulk_g2s(dst, src, kHeadStage, full); });
+            stage(bytes, [&](uint32_t dst, uint32_t full) { bulk_g2s(dst, src + skip, bytes, full); });
     }
     // after a time-out copies may still be in flight: a bounded while for them to land
     if (*abort_flag != 0) {
@@ -1041,6 +1071,16 @@ __device__ __forceinline__ void issue_unit(Issue& st, uint32_t d, uint32_t a_bas
         st.i++;
     }
 }
+// The pair's second SM issues nothing: its MMA warp tells the first which weights have arrived.
+template <int kAr>
+__device__ __forceinline__ void relay(uint32_t smem, volatile int* abort_flag, uint32_t stages) {
+    constexpr uint32_t kStages = Map<kAr>::kStages;
+    for (uint32_t i = 0; i < stages; ++i) {
+        const uint32_t k = i % kStages;
+        mbar_wait(bar(smem, B_FULL + k), (i / kStages) & 1u, abort_flag, kErrMmaWeights);
+        if (elect_one()) mbar_arrive(bar(smem, B_FULL + k));
+    }
+}
 __device__ __forceinline__ void issue_wait(const Issue& st, int b, uint32_t n) {
     mbar_wait(bar(st.smem, b), n & 1u, st.abort_flag, kErrMmaOperand);
     tc_fence_after();
@@ -1049,14 +1089,15 @@ template <int NB, int kAr>
 __device__ __forceinline__ void issue_tile(Issue& st, int n_layers) {
     using O = Own<NB>;
     using C = Cfg<kAr>;
-    constexpr uint32_t kI_S8 = umma_idesc(kAccS32, kFmtS8, kFmtS8, 32 * NB, 256);
-    constexpr uint32_t kI_F16 = umma_idesc(kAccF16, kFmtF16, kFmtF16, 32 * NB, 256);
-    constexpr uint32_t kI_E4M3 = umma_idesc(kAccF32, kFmtE4M3, kFmtE4M3, 32 * NB, 256);
+    constexpr uint32_t kM = 128;                             // 64 rows of each SM
+    constexpr uint32_t kI_S8 = umma_idesc(kAccS32, kFmtS8, kFmtS8, kM, 256);
+    constexpr uint32_t kI_F16 = umma_idesc(kAccF16, kFmtF16, kFmtF16, kM, 256);
+    constexpr uint32_t kI_E4M3 = umma_idesc(kAccF32, kFmtE4M3, kFmtE4M3, kM, 256);
     constexpr uint32_t kI_QKV = C::kQkvF16 ? kI_F16 : kI_S8, kI_OUT = C::kOutF16 ? kI_F16 : kI_S8;
     constexpr uint32_t kI_FF1 = kAr == kArF16 ? kI_F16 : kAr == kArE4M3 ? kI_E4M3 : kI_S8;
     constexpr uint32_t kI_FF2 = kAr == kArF16 ? kI_F16 : kAr == kArE4M3 ? kI_E4M3
-                                              : umma_idesc(kAccS32, kFmtU8, kFmtS8, 32 * NB, 256);
-    constexpr uint32_t kI_HEAD = umma_idesc(kAccF16, kFmtF16, kFmtF16, 32 * NB, 128);
+                                              : umma_idesc(kAccS32, kFmtU8, kFmtS8, kM, 256);
+    constexpr uint32_t kI_HEAD = umma_idesc(kAccF16, kFmtF16, kFmtF16, kM, 128);
     constexpr int kQkvKind = C::kQkvF16 ? kKindF16 : kKindI8, kOutKind = C::kOutF16 ? kKindF16 : kKindI8;
     constexpr int kFfnKind = kAr == kArE4M3 ? kKindF8 : (kAr == kArF16 ? kKindF16 : kKindI8);
     const uint32_t a = st.smem + SM_A, h = st.smem + Map<kAr>::SM_H;
@@ -1085,30 +1126,42 @@ __device__ __forceinline__ void issue_tile(Issue& st, int n_layers) {
 }
 
 // launch bounds: 640 threads, so that a scheduler's five warps fit its registers (96 each)
-template <int kAr, bool kExpand>
+template <int kAr, bool kExpand, int NB>
 __global__ void __launch_bounds__(640, 1) encoder_ws_kernel(const Params p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const uint32_t smem = smem_u32(sm);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_rank();
     volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + SM_MISC + 4);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + SM_MISC);
     if (threadIdx.x == 0) {
-        for (int i = 0; i < B_COUNT; ++i) mbar_init(bar(smem, i), i == B_EXPANDED ? 2 : i >= B_A ? kRowWarps : 1);
+        // the operands come from both SMs' warps, and the first SM hears of its own weights and of the second's
+        for (int i = 0; i < B_COUNT; ++i)
+            mbar_init(bar(smem, i), i == B_EXPANDED        ? 2
+                                    : i < B_EMPTY          ? 2 - rank
+                                    : i >= B_A && i < B_STAGED ? 2 * kRowWarps
+                                    : i >= B_STAGED        ? kRowWarps
+                                                           : 1);
         *abort_flag = 0;
         fence_barrier_init();
     }
-    if (warp == kMmaWarp) {
-        tmem_alloc(smem + SM_MISC, TM_COLS);
-        tmem_relinquish();
-    }
+    if (warp == kMmaWarp) tmem_alloc_pair(smem + SM_MISC, TM_COLS);
     tc_fence_before();
     __syncthreads();
+    cluster_sync();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    // The grid before this one may still be running.  Only the producer goes on without it: the first weights are
+    // nobody's output.  One-board tiles beside this call's own two-board ones start without it, since that grid lets
+    // them start only when what came before it has ended; they wait for it at their own end.
+    if (!p.after_waves && (warp != kProducerWarp || p.leaf_count != nullptr)) {
+        previous_grid_wait();
+        next_grid_may_start();
+    }
     int n_eval = p.n;
-    if (p.leaf_count != nullptr) n_eval = min(max(__ldg(p.leaf_count), 0), p.n);
-    const Tiles tiles(n_eval, gridDim.x, blockIdx.x, p.one_most);
+    if (p.leaf_count != nullptr) n_eval = min(max(*p.leaf_count, 0), p.n);
+    const Tiles<NB> tiles(n_eval, p.wave_ctas, gridDim.x, blockIdx.x, p.one_most);
     const int n_tiles = tiles.count();
     if (warp < kRowWarps) {
         Row c;
@@ -1119,32 +1172,27 @@ __global__ void __launch_bounds__(640, 1) encoder_ws_kernel(const Params p) {
         c.one2 = pk2(p.one, p.one);
         c.layers = c.tiles = 0;
         c.n = n_eval;
-        for (int k = 0; k < n_tiles; ++k) {
-            int first, boards;
-            tiles.at(k, first, boards);
-            if (boards == 1) row_tile<1, kAr, kExpand>(c, p, first);
-            else             row_tile<2, kAr, kExpand>(c, p, first);
-        }
+        for (int k = 0; k < n_tiles; ++k) row_tile<NB, kAr, kExpand>(c, p, tiles.at(k));
     } else if (warp == kProducerWarp) {
-        producer<kAr>(smem, abort_flag, p, n_tiles);
+        producer<kAr>(smem, abort_flag, p, n_tiles, rank);
     } else if (warp >= kExpandWarp) {
-        if constexpr (kExpand)
-            expander(smem, sm, smem + Map<kAr>::SM_H, abort_flag, p, tiles, n_tiles, warp - kExpandWarp, lane);
+        if constexpr (kExpand) expander<NB>(smem, sm, smem + Map<kAr>::SM_H, abort_flag, p, tiles, warp - kExpandWarp, lane);
+    } else if (rank != 0) {
+        using C = Cfg<kAr>;
+        relay<kAr>(smem, abort_flag, n_tiles * (p.n_layers * (3 * C::kQkvSlabs + C::kOutSlabs + 8 * C::kFfnSlabs) + kHeadStages));
     } else {
         Issue st = {smem, tmem, abort_flag, 0, 0, 0};
-        for (int k = 0; k < n_tiles; ++k) {
-            int first, boards;
-            tiles.at(k, first, boards);
-            if (boards == 1) issue_tile<1, kAr>(st, p.n_layers);
-            else             issue_tile<2, kAr>(st, p.n_layers);
-        }
+        for (int k = 0; k < n_tiles; ++k) issue_tile<NB, kAr>(st, p.n_layers);
     }
     __syncwarp();
     tc_fence_before();
     __syncthreads();
+    // (the products read both SMs' shared memory, and barriers are written from both)
+    cluster_sync();
     tc_fence_after();
-    if (warp == kMmaWarp) tmem_dealloc(tmem, TM_COLS);
+    if (warp == kMmaWarp) tmem_dealloc_pair(tmem, TM_COLS);
     if (threadIdx.x == 0 && *abort_flag != 0) atomicCAS(p.status, 0, *abort_flag);
+    previous_grid_wait();
 }
 
 }  // namespace ws

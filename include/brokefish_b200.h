@@ -102,9 +102,8 @@ int bf_forward_priors(bf_handle* h, const uint16_t* boards, const int16_t* contr
  * kernel starts, so the caller needs no host synchronisation to know it.  `capacity` is the most
  * the list can hold (the grid is sized for it; a larger count is clamped, a negative one is 0);
  * CTAs beyond the count's tiles leave at once, so a short list runs short, and a list of at
- * most one position per SM runs on one-board tiles (BF_OPT_ONE_BOARD) -- except where the capacity
- * has put the launch on four-board tiles (bf_tile_boards; large capacities in fp16, and every launch
- * with re-injection).  Every output is
+ * most one position per SM runs on one-board tiles (BF_OPT_ONE_BOARD) -- except with re-injection, whose launches
+ * run on four-board tiles.  Every output is
  * written at the position's own place in the staged arrays (policy [place,32,64], value [place],
  * prior [place,e_cap] ...); places not in the list are not touched.  Any of policy / promo /
  * value may be NULL; pass prior, move and nedges (all three, else all NULL) for the fused
@@ -211,9 +210,8 @@ int bf_forward_backbone(bf_handle* h, const void* x, const int8_t* alive, int n,
  * `model_forward(..., debug_stage=stage)` (csrc/encoder.cu:1315-1427, 1575-1598):
  * 9 embedding; layer 0: 1 LN1 out, 5/6/7 Q/K/V after bias, 4 attention out,
  * 2 residual after attention, 3 LN2 out; 8 final norm out.  This call, bf_forward_stage_at,
- * bf_forward_capture and bf_profile run the four-board kernel, whatever tiles bf_forward would take
- * (bf_tile_boards): the outputs of both are equal bit for bit, the phase clock's cycles are not those
- * of the small tiles. */
+ * bf_forward_capture and bf_profile run the four-board kernel, bf_forward one- and two-board tiles: the
+ * outputs of both are equal bit for bit, the phase clock's cycles are not those of the small tiles. */
 int bf_forward_stage(bf_handle* h, const uint16_t* boards, const int16_t* control,
                      const uint8_t* rep, int n, int stage, void* y, void* stream);
 
@@ -276,10 +274,11 @@ int bf_set_option(bf_handle* h, int option, int value);
  * first call): what the plan of the next call is chosen by.  No counterpart in the reference. */
 double bf_host_link_gbps(const bf_handle* h);
 
-/* How many positions the largest tiles of a plain evaluation of `n` positions (of a leaf list: of that
- * capacity) hold, without re-injection, on a GPU with `sm_count` SMs under BF_OPT_ONE_BOARD
- * `one_board`: 1, 2 or 4; `quant` is the blob's arithmetic (0 fp16).  No GPU is touched.  No counterpart
- * in the reference. */
+/* How many positions (1, 2 or 4) the largest tiles of an evaluation of `n` positions would hold if each of a
+ * GPU's `sm_count` SMs worked by itself under BF_OPT_ONE_BOARD `one_board`; `quant` is the blob's arithmetic
+ * (0 fp16).  SMs work in pairs: a plain evaluation runs on one- and two-board tiles in every arithmetic, and
+ * nothing goes by this rule any more; its results are kept.  No GPU is touched.  No counterpart in the
+ * reference. */
 int bf_tile_boards(int quant, int n, int sm_count, int one_board);
 
 /* Whether the kernels can read and write host buffers at these addresses themselves (1) or the host
