@@ -25,8 +25,8 @@
 // The arithmetic is the four-board kernel's, bit for bit (the order of every sum included).
 //
 // Measured on one B200, us, against tiles of one SM (M = 32 and 64 by `tcgen05.mma.ws`): a one-board tile
-// int8 85 (91), e4m3 91 (101), fp16 109 (129); a two-board tile 117 (127), 117 (130), 116 (152); batch 4096 1586
-// (1675), 1547 (1727), 1650 (1870, then on four-board tiles).  What bounds it: the row warps, four to a scheduler and all in the same
+// int8 85 (91), e4m3 91 (101), fp16 109 (129); a two-board tile 117 (127), 117 (130), 116 (152); batch 4096 1589
+// (1677), 1547 (1735), 1660 (1877, then on four-board tiles).  What bounds it: the row warps, four to a scheduler and all in the same
 // phase.
 #pragma once
 
@@ -60,7 +60,7 @@ constexpr uint32_t SM_MISC = SM_BAR + 8 * 34;
 constexpr uint32_t SM_BYTES = SM_MISC + 64, kSmemRequest = SM_BYTES + 1024;
 static_assert(kSmemRequest <= 232448 && kLparamStride % 16 == 0 && SM_PAR % 16 == 0, "shared memory map");
 static_assert(Map<kArF16>::SM_RING + 6 * kStage <= SM_STAT && Map<kArInt8>::SM_RING + 8 * kStage <= SM_STAT, "shared memory map");
-enum { B_FULL = 0, B_EMPTY = 8, B_ACC = 16, B_PAR = 20, B_A = 22, B_H = 23, B_STAGED = 25, B_EXPANDED = 26, B_COUNT = 27 };
+enum { B_FULL = 0, B_EMPTY = 8, B_ACC = 16, B_PAR = 20, B_A = 22, B_H = 23, B_MAX = 27, B_STAGED = 31, B_EXPANDED = 32, B_COUNT = 33 };
 __device__ __forceinline__ uint32_t bar(uint32_t smem, int i) { return smem + SM_BAR + 8u * i; }
 
 // ---- what is different in a pair of SMs ----
@@ -194,6 +194,18 @@ __device__ __forceinline__ uint64_t lds_u64(uint32_t addr) {
 // Row maxima of non-negative values meet in shared memory by an integer maximum of their bits.
 __device__ __forceinline__ void max_to(uint32_t addr, float v) {
     asm volatile("red.shared.max.u32 [%0], %1;" ::"r"(addr), "r"(__float_as_uint(v)) : "memory");
+}
+// The same for a hidden chunk, whose maxima are waited for later: the warp has given its part.
+__device__ __forceinline__ void max_to(uint32_t addr, float v, const Row& c, int chunk) {
+    max_to(addr, v);
+    __syncwarp();
+    if (c.lane == 0) bfptx::mbar_arrive(bar(c.smem, B_MAX + chunk));
+}
+// The chunk's maxima are all there.
+template <int NB>
+__device__ __forceinline__ void board_sync(const Row& c, int chunk) {
+    mbar_wait(bar(c.smem, B_MAX + chunk), c.layers & 1u, c.abort_flag, kErrRowAcc);
+    __syncwarp();
 }
 // A row's scale amax / Q and its reciprocal, both correctly rounded, amax being a non-negative fp16 value.  The
 // scale is a product with 1 / Q held in two words (Brisebarre and Muller 2008), the upper one rounded down so
@@ -576,43 +588,40 @@ __device__ __forceinline__ void attention_block(const Row& c, uint32_t lp, float
 }
 
 // ---- FFN ----
-// Two hidden chunks at a time: ff1's epilogue (descale, bias, ReLU, row maximum), one meeting of the
-// board for both maxima, quantisation into the ff2 operand.  ff2's products of the first pair run
-// under the second pair's epilogue; their four sums are added to the fp16 running total in order.
+// Chunk by chunk: ff1's epilogue (descale, bias, ReLU, row maximum), the meeting of the row's threads for the
+// maximum, quantisation into the ff2 operand, which starts that chunk's ff2 product.  A chunk's epilogue
+// comes before the quantisation of the one before it, so that nobody waits where they meet.  ff2's products
+// run under the epilogues that follow; their four sums are added to the fp16 running total in order.
 template <int NB, int kAr>
 __device__ __forceinline__ void ffn_block(const Row& c, uint32_t lp, float sa, uint32_t (&x)[8 * NB]) {
     using O = Own<NB>;
     const int col = O::col(c), row = O::row(c);
-    float s1[4] = {1.f, 1.f, 1.f, 1.f};
+    float s1[4];
+    uint32_t hid[2][8 * NB];
+    const uint32_t maxima = c.smem + SM_MAX + 256u + 4u * row;
+    auto epilogue = [&](int ch, uint32_t (&h)[8 * NB]) {
+        const uint32_t bias_at = lp + LP_B_FF1 + 2u * (256 * ch + col);
+        const float sw = lds_f(lp + LP_SW_FF1 + 4u * (2 * ch + (col >> 7)));
+        Bias bias = load_bias(bias_at);
+        wait_acc<kAr>(c, ch, 1);
+        each_piece<NB>(O::slot(c, ch), [&](int i, const uint32_t (&acc)[16]) {
+            if (i > 0) bias = load_bias(bias_at + 32 * i);
+            descale16<true, kAr == kArE4M3 ? kAccFloat : kAccInt>(acc, sa, sw, bias, &h[8 * i]);
+        });
+        max_to(maxima + 256u * ch, amax_h2<8 * NB>(h, false), c, ch);
+    };
+    epilogue(0, hid[0]);
 #pragma unroll
-    for (int pair = 0; pair < 2; ++pair) {
-        uint32_t hid[2][8 * NB];
-        const uint32_t m = c.smem + SM_MAX + 256u * (1 + 2 * pair) + 4u * row;
+    for (int ch = 0; ch < 4; ++ch) {
+        if (ch < 3) epilogue(ch + 1, hid[(ch + 1) & 1]);
+        board_sync<NB>(c, ch);
+        const float amax = lds_f(maxima + 256u * ch);
+        const Scale sc = kAr == kArE4M3 ? scale_e4m3(amax) : scale_u8(amax);
+        s1[ch] = sc.scale;
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const int ch = 2 * pair + k;
-            const uint32_t bias_at = lp + LP_B_FF1 + 2u * (256 * ch + col);
-            const float sw = lds_f(lp + LP_SW_FF1 + 4u * (2 * ch + (col >> 7)));
-            Bias bias = load_bias(bias_at);
-            wait_acc<kAr>(c, ch, 1);
-            each_piece<NB>(O::slot(c, ch), [&](int i, const uint32_t (&acc)[16]) {
-                if (i > 0) bias = load_bias(bias_at + 32 * i);
-                descale16<true, kAr == kArE4M3 ? kAccFloat : kAccInt>(acc, sa, sw, bias, &hid[k][8 * i]);
-            });
-            max_to(m + 256u * k, amax_h2<8 * NB>(hid[k], false));
-        }
-        board_sync<NB>(c);
-        s1[0] = s1[2]; s1[1] = s1[3];
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const float amax = lds_f(m + 256u * k);
-            const Scale sc = kAr == kArE4M3 ? scale_e4m3(amax) : scale_u8(amax);
-            s1[2 + k] = sc.scale;
-#pragma unroll
-            for (int i = 0; i < NB; ++i)
-                store_operand8<NB, kAr == kArE4M3>(c, c.h + (2 * pair + k) * 2 * O::kSlab, i, &hid[k][8 * i], sc.inverse);
-        }
-        publish(c, B_H + pair);
+        for (int i = 0; i < NB; ++i)
+            store_operand8<NB, kAr == kArE4M3>(c, c.h + ch * 2 * O::kSlab, i, &hid[ch & 1][8 * i], sc.inverse);
+        publish(c, B_H + ch);
     }
     uint32_t run[8 * NB];
 #pragma unroll
@@ -622,8 +631,7 @@ __device__ __forceinline__ void ffn_block(const Row& c, uint32_t lp, float sa, u
 #pragma unroll
     for (int ch = 0; ch < 4; ++ch) {
         wait_acc<kAr>(c, ch, 2);
-        const uint64_t s1_2 = pk2(s1[0], s1[0]);
-        s1[0] = s1[1]; s1[1] = s1[2]; s1[2] = s1[3];
+        const uint64_t s1_2 = pk2(s1[ch], s1[ch]);
         each_piece<NB>(O::slot(c, ch), [&](int k, const uint32_t (&acc)[16]) {
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
@@ -1111,7 +1119,8 @@ __device__ __forceinline__ void issue_tile(Issue& st, int n_layers) {
         for (int ch = 0; ch < 4; ++ch)
             issue_unit<kAr, kFfnKind>(st, st.tmem + O::kSlot * ch, a, O::kSlab, C::kFfnSlabs, kI_FF1, ch);
         for (int ch = 0; ch < 4; ++ch) {
-            if ((ch & 1) == 0) issue_wait(st, B_H + (ch >> 1), st.h);
+            if (kAr != kArF16)      issue_wait(st, B_H + ch, st.h);
+            else if ((ch & 1) == 0) issue_wait(st, B_H + (ch >> 1), st.h);
             if (kAr == kArF16) {
                 issue_unit<kAr, kFfnKind>(st, st.tmem, h + (ch & 1) * 4 * O::kSlab, O::kSlab, C::kFfnSlabs, kI_FF2,
                                             ch == 1 ? 0 : ch == 3 ? 1 : -1, ch > 0);
@@ -1140,8 +1149,8 @@ __global__ void __launch_bounds__(640, 1) encoder_ws_kernel(const Params p) {
         for (int i = 0; i < B_COUNT; ++i)
             mbar_init(bar(smem, i), i == B_EXPANDED        ? 2
                                     : i < B_EMPTY          ? 2 - rank
-                                    : i >= B_A && i < B_STAGED ? 2 * kRowWarps
-                                    : i >= B_STAGED        ? kRowWarps
+                                    : i >= B_A && i < B_MAX ? 2 * kRowWarps
+                                    : i >= B_MAX           ? kRowWarps
                                                            : 1);
         *abort_flag = 0;
         fence_barrier_init();
