@@ -2363,20 +2363,22 @@ cudaError_t launch_early(void (*kernel)(P...), unsigned grid, int threads, size_
 }
 
 // The engine kernels have two forms (bf_movegen.cuh).  Eight lanes per board: an eighth of the chain,
-// so a launch that does not fill the GPU ends sooner.  A thread per board: half of the instructions, most
+// so a launch that does not fill the GPU ends sooner.  A thread per board: a half to a quarter of the instructions, most
 // of all where legal words are made.  B200, us per launch in a graph, eight lanes / thread:
-//   boards                      1       4096      16384      32768      49152      65536     131072    1048576
-//   legal words              3.1/6.8   4.2/8.6   8.6/8.6    15/11      21/13      27/16      50/24     384/159
-//   key                      2.2/7.6   3.1/12    5.8/12     8.8/13     12/14      15/16      27/27     203/176
-//   move                     2.1/7.2   2.6/11    4.4/11     6.7/11     9.0/12     11/13      21/24     166/146
-//   move and key             3.5/14    4.4/20    8.7/20     14/22      20/24      25/27      47/50     364/314
-//   move and words           4.3/13    5.4/17    11/18      19.7/20.2  28/23      37/27      70/47     541/304
-//   move, words and key      5.3/20    6.9/27    15/27      25/31      35.6/35.8  46/42      89/70     684/480
-//   random move and words    5.2/17    6.4/25    13/26      23/29      32.7/32.6  42/37      81/62
+//   boards                        1      4096     16384     32768     49152     65536    131072    262144   1048576
+//   legal words             2.8/3.5   4.0/6.8   8.6/7.4    14/9.3     21/11     26/12     50/18     99/32   384/109
+//   key                     1.9/7.7    3.0/11    5.5/11    8.6/13     12/14     15/16     27/27     53/46   204/165
+//   move                    2.0/9.3    2.5/12    4.3/12    6.4/13    8.8/14     11/15     20/26     40/41   166/145
+//   move and key             3.1/16    4.2/21    8.4/21     13/24     19/26     24/29     45/50     89/83   350/305
+//   move and words           4.0/12    5.2/16     11/16     19/19     28/20     36/24     70/41    138/70   538/240
+//   move, words and key      4.8/19    6.7/26     14/26     24/30     34/32     45/37     85/66   169/111   659/399
+//   random move and words     4.4/-    5.7/22     12/23     22/24     32/27     41/31     80/55    159/96   630/355
+// and where the lines lie, legal words 11,264 boards 6.7/7.0, move 262,144 40/41 and 393,216 58/56, move and key 131,072 45/50
+// and 196,608 67/65, move and words 30,720 18.4/19.1, move, words and key 45,056 32.1/32.1, random move 36,864 24.9/24.6.
 int group_form_most(bool step, bool pick, bool words, bool key) {
-    if (!words) return 131072;
-    if (!step) return 16384;
-    return pick || key ? 49152 : 32768;
+    if (!words) return !step ? 131072 : key ? 163840 : 327680;
+    if (!step) return 12288;
+    return pick ? 34816 : key ? 45056 : 31744;
 }
 template <bool kStep, bool kPick, class... Args>
 cudaError_t launch_engine(cudaStream_t stream, bool words, bool key, const uint16_t* boards, const int16_t* control, const int* move,

@@ -28,13 +28,13 @@
 
 namespace bfmg {
 
-// These kernels are launched while the grid before them in the stream may still be running: they wait for it
-// before they touch its memory, and let the grid after them start at once.  (No __restrict__ on what they read: the
-// compiler may move a load from memory that it takes to be constant above the wait.)
-__device__ __forceinline__ void begin_after_previous_grid() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
+// These kernels are launched before the grid before them in the stream has quite ended: they wait for it before they
+// touch its memory.  (No __restrict__ on what they read: the compiler may move a load from memory that it takes to
+// be constant above the wait.)  Legal words by a thread per board let the grid after them start when a block
+// has made its words; the others say nothing, and the next grid starts as theirs drains: its blocks, placed among the
+// ones that still run, leave the SMs uneven (a move with words and key of 4096 boards 9.6 us a launch instead of 6.6).
+__device__ __forceinline__ void after_previous_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void next_grid_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 constexpr unsigned long long kFileA = 0x0101010101010101ull, kFileH = kFileA << 7;
 constexpr unsigned kFull = 0xffffffffu;
@@ -560,8 +560,8 @@ constexpr unsigned kIndexBits = 0x0DFF0DFFu;
 // that does not add up then (colours or types in other slots, two pieces on a square) takes the general form.
 //
 // Bound by the integer pipe (the general form keeps it busy 87 % of the time with 3,600 instructions a board), which is why
-// every attack is a table's.  2^20 boards of random games, B200: 121 us, 161 in the general form (323 bytes a board: 2.8
-// and 2.1 TB/s of the 6.5 a copy reaches).
+// every attack is a table's.  2^20 boards of random games, B200: 109 us, 161 in the general form (323 bytes a board: 3.1
+// and 2.1 TB/s of the 6.5 a copy reaches); 2,300 instructions a board, the integer pipe 68 % busy.
 __device__ __forceinline__ bool board_moves(const unsigned* my, bool black, unsigned long long* to, unsigned long long* all,
                                             const MoveTables& t, bool& by_slot) {
     by_slot = true;
@@ -939,8 +939,10 @@ enum { WORDS_WHITE = 0, WORDS_BLACK = 1, WORDS_STORED = 2, WORDS_KEPT = 3 };
 // `mask` in (slot, square) order; a board without legal moves stays as it is) and write the new
 // board, control word and irreversible flag; `mask` non-null: the legal words of the resulting
 // board follow.  In place (boards_out == boards) is safe: a block reads all its boards first.
+// (Six blocks to an SM, at 80 registers: left to itself the compiler takes 122 to 128, which leaves four and costs 10 % of
+// the words of 2^20 boards, 20 % of a move without them.  With five a random ply is the faster.)
 template <bool kStep, bool kPick>
-__global__ void __launch_bounds__(kTpbThreads) engine_board_kernel(
+__global__ void __launch_bounds__(kTpbThreads, kPick ? 5 : 6) engine_board_kernel(
         const uint16_t* boards, const int16_t* control, const int* move,
         const signed char* promo, const float* r, int n, uint16_t* boards_out,
         int16_t* control_out, unsigned char* irreversible, unsigned long long* mask,
@@ -953,23 +955,41 @@ __global__ void __launch_bounds__(kTpbThreads) engine_board_kernel(
     const int tid = threadIdx.x;
     const long first = static_cast<long>(blockIdx.x) * kTpbThreads;
     const int here = static_cast<int>(min(static_cast<long>(kTpbThreads), n - first));
+    // (every load is under way before the first is waited for: one after the other the tables' five alone are 1,500 cycles)
+    constexpr int kTablePieces = (kTpbTables / 16 + kTpbThreads - 1) / kTpbThreads;
+    uint4 piece[kTablePieces];
     auto load_tables = [&] {
-        for (int j = tid; j < kTpbTables / 16; j += kTpbThreads)
-            reinterpret_cast<uint4*>(s_tables)[j] = __ldg(reinterpret_cast<const uint4*>(&kMoveTables) + j);
+#pragma unroll
+        for (int k = 0; k < kTablePieces; ++k)
+            if (tid + k * kTpbThreads < kTpbTables / 16)
+                piece[k] = __ldg(reinterpret_cast<const uint4*>(&kMoveTables) + tid + k * kTpbThreads);
     };
-    if (!kPick && mask != nullptr) load_tables();
-    begin_after_previous_grid();
+    auto store_tables = [&] {
+#pragma unroll
+        for (int k = 0; k < kTablePieces; ++k)
+            if (tid + k * kTpbThreads < kTpbTables / 16) reinterpret_cast<uint4*>(s_tables)[tid + k * kTpbThreads] = piece[k];
+    };
+    const bool tables = mask != nullptr;
+    if (!kPick && tables) load_tables();
+    after_previous_grid();
     {
         // coalesced load: the block's boards are one contiguous run of 16-byte pieces
         const uint4* src = reinterpret_cast<const uint4*>(boards + first * 32);
-        for (int j = tid; j < here * 4; j += kTpbThreads) {
-            const uint4 v = src[j];
-            unsigned* d = s_in + (j >> 2) * kTpbInStride + (j & 3) * 4;
-            d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
-        }
+        uint4 v[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (tid + k * kTpbThreads < here * 4) v[k] = src[tid + k * kTpbThreads];
         if (kPick)
             for (int j = tid; j < here * 32; j += kTpbThreads)
                 s_mask[(j >> 5) * kTpbMaskStride + (j & 31)] = mask[first * 32 + j];
+        else if (tables)
+            store_tables();
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int j = tid + k * kTpbThreads;
+            unsigned* d = s_in + (j >> 2) * kTpbInStride + (j & 3) * 4;
+            if (j < here * 4) { d[0] = v[k].x; d[1] = v[k].y; d[2] = v[k].z; d[3] = v[k].w; }
+        }
     }
     __syncthreads();
     const bool mine = tid < here;
@@ -999,6 +1019,7 @@ __global__ void __launch_bounds__(kTpbThreads) engine_board_kernel(
         }
         __syncthreads();                              // the incoming words' place is the tables'
         load_tables();
+        store_tables();
         __syncthreads();
     }
     if (mine) {
@@ -1026,6 +1047,7 @@ __global__ void __launch_bounds__(kTpbThreads) engine_board_kernel(
         my[16] = words;                               // (the row's padding)
         if (hash_out != nullptr) hash_out[first + tid] = board_hash(my, ctl < 0);
     }
+    if (!kStep) next_grid_may_start();
     __syncthreads();
     if (kStep) {
         // coalesced store of the block's boards (all of them: a board that did not move is rewritten as it was)
@@ -1393,7 +1415,7 @@ __global__ void __launch_bounds__(kEngineThreads) engine_group_kernel(
         const signed char* promo, const float* r, int n, uint16_t* boards_out,
         int16_t* control_out, unsigned char* irreversible, unsigned long long* mask,
         unsigned char* in_check, int* move_out, unsigned long long* hash_out) {
-    begin_after_previous_grid();
+    after_previous_grid();
     const int lane = threadIdx.x & 31, j = lane & 7;
     const long board = static_cast<long>(blockIdx.x) * kEngineBoards + (threadIdx.x >> 3);
     const bool valid = board < n;
@@ -1510,7 +1532,7 @@ __global__ void __launch_bounds__(128) terminal_kernel(const unsigned long long*
                                                        const unsigned long long* ring,
                                                        const long long* length, int n,
                                                        unsigned char* code, signed char* result) {
-    begin_after_previous_grid();
+    after_previous_grid();
     const int lane = threadIdx.x & 31;
     const long board = static_cast<long>(blockIdx.x) * 4 + (threadIdx.x >> 5);
     if (board >= n) return;
@@ -1544,7 +1566,7 @@ __global__ void __launch_bounds__(128) history_push_kernel(unsigned long long* r
                                                            long long* length,
                                                            const unsigned long long* hash,
                                                            const unsigned char* irreversible, int n) {
-    begin_after_previous_grid();
+    after_previous_grid();
     const long g = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (g >= n) return;
     if (irreversible[g]) { length[g] = 0; return; }
@@ -1562,7 +1584,7 @@ __global__ void __launch_bounds__(256) history_push_to_kernel(const unsigned lon
                                                               const unsigned char* irreversible, int n,
                                                               unsigned long long* new_ring,
                                                               long long* new_length) {
-    begin_after_previous_grid();
+    after_previous_grid();
     constexpr unsigned kPieces = kMaxHistory / kWords;
     const long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x;
     const long g = i / kPieces;
@@ -1590,7 +1612,7 @@ __global__ void __launch_bounds__(128) repetition_kernel(const unsigned long lon
                                                          const unsigned long long* ring,
                                                          const long long* length, int n,
                                                          int* count) {
-    begin_after_previous_grid();
+    after_previous_grid();
     const int lane = threadIdx.x & 31;
     const long g = static_cast<long>(blockIdx.x) * 4 + (threadIdx.x >> 5);
     if (g >= n) return;

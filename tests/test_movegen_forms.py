@@ -148,3 +148,35 @@ def test_boards_of_every_kind(kind, turned, compare, pos4096):
         assert (slots != 0).mean() > 0.99 if by_slot else (slots != 0).mean() < 0.01
     else:
         assert slots.any() and not slots.all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [12288, 12289, 31744, 31745, 45056, 45057, 163841, 327681])
+def test_either_side_of_the_lines_between_a_launch_s_forms(n, pos4096):
+    from test_movegen import test_both_forms_of_the_engine_kernels_agree_at_every_size as agree
+    agree(n, pos4096)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [34816, 34817, 40001])
+def test_a_random_ply_either_side_of_its_line(n, pos4096):
+    """The same boards with the same draws in batches of 4096 (eight lanes per board) and in one."""
+    import torch
+    from brokefish_b200 import _native
+    L, at = _native.lib(), lambda t: ctypes.c_void_p(t.data_ptr())
+    place = torch.arange(n) % 4096
+    start = [torch.from_numpy(np.ascontiguousarray(pos4096[k])).view(torch.int16)[place].cuda() for k in ("boards", "control")]
+    start.append(torch.from_numpy(pos4096["legal"].view(np.int64))[place].cuda())
+    gen = torch.Generator().manual_seed(n)
+    draw, promo = torch.rand(n, generator=gen).cuda(), torch.randint(0, 4, (n,), generator=gen).to(torch.int8).cuda()
+
+    def ply(step):
+        b, c, m = (t.clone() for t in start)
+        move = torch.empty(n, dtype=torch.int32, device="cuda")
+        for lo in range(0, n, step):
+            part = [t[lo:lo + step] for t in (b, c, m, draw, promo)]
+            _native.check(L.bf_random_ply(0, *(at(t) for t in part), len(part[0]), at(move[lo:]),
+                                          ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)), "bf_random_ply")
+        return b, c, m, move
+    for got, want in zip(ply(n), ply(4096)):
+        assert torch.equal(got, want)
