@@ -957,6 +957,8 @@ __device__ __forceinline__ float warp_sum_to_all(float v) {
     for (int off = 16; off > 0; off >>= 1) v = __fadd_rn(v, __shfl_down_sync(0xffffffffu, v, off));
     return __shfl_sync(0xffffffffu, v, 0);
 }
+// The list is put together in shared memory: a float for each of at most 255 edges, then their labels.
+constexpr uint32_t kListLabels = 1024, kListBytes = kListLabels + 512;
 __device__ __forceinline__ void expand_board(const Params& p, int board, int lane, bool valid, uint32_t word,
                                              int ctl, unsigned long long legal, uint32_t row_smem,
                                              uint32_t row_xor, uint32_t aux, uint8_t* list_buf) {
@@ -1016,35 +1018,49 @@ __device__ __forceinline__ void expand_board(const Params& p, int board, int lan
         if (k < thr) return false;
         return tie_rank++ < ties_wanted;
     };
+    const int kept = cut ? e_cap : total;
+    // Every slot puts its candidates into the list; what follows goes by the list's places, a place to a lane, but for
+    // the sum, whose order is the slots'.  (Slot by slot throughout, the lane with the queen's twenty moves makes
+    // all the others wait while it computes their exponentials twice and divides: 8 us of a one-board tile's 95.)
+    const uint32_t list = smem_u32(list_buf), labels = list + kListLabels;
+    int end = first;
+    each_candidate(legal, promos, row_smem, row_xor, type_lp, [&](int sq, int t, float lg) {
+        if (!stays(lg)) return;
+        asm volatile("st.shared.f32 [%0], %1;" ::"r"(list + 4u * end), "f"(lg) : "memory");
+        asm volatile("st.shared.u16 [%0], %1;" ::"r"(labels + 2u * end), "h"(static_cast<uint16_t>((lane * 64 + sq) | (t << 11))) : "memory");
+        ++end;
+    });
+    __syncwarp();
+    auto at = [&](int i) { float v; asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(list + 4u * i) : "memory"); return v; };
     float top = -INFINITY;
-    each_candidate(legal, promos, row_smem, row_xor, type_lp, [&](int, int, float lg) { if (stays(lg)) top = fmaxf(top, lg); });
+    for (int i = lane; i < kept; i += 32) top = fmaxf(top, at(i));
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, off));
-    tie_rank = tie_rank0;
+    for (int i = lane; i < kept; i += 32)
+        asm volatile("st.shared.f32 [%0], %1;" ::"r"(list + 4u * i), "f"(expf(__fsub_rn(at(i), top))) : "memory");
+    __syncwarp();
     float part = 0.f;
-    each_candidate(legal, promos, row_smem, row_xor, type_lp, [&](int, int, float lg) {
-        if (stays(lg)) part = __fadd_rn(part, expf(__fsub_rn(lg, top)));
-    });
+#pragma unroll 4
+    for (int i = first; i < end; ++i) part = __fadd_rn(part, at(i));
     const float z = warp_sum_to_all(part);
-    const int kept = cut ? e_cap : total;
     if (valid) {
-        // The edge list is put together in shared memory (`list_buf`: 1 KB, priors in the first
-        // half, labels in the second) and leaves in 16-byte stores: the outputs may be pinned host
+        // The edge list is put together in shared memory (the priors over the first half of what they are made from: a place
+        // is read before its bytes are written) and leaves in 16-byte stores: the outputs may be pinned host
         // memory, where every store is a transaction on the bus.
         __half* out_p = p.prior + static_cast<size_t>(board) * e_cap;
         int16_t* out_m = p.move + static_cast<size_t>(board) * e_cap;
         __half* list_p = reinterpret_cast<__half*>(list_buf);
-        int16_t* list_m = reinterpret_cast<int16_t*>(list_buf + 512);
-        tie_rank = tie_rank0;
-        int at = first;
-        each_candidate(legal, promos, row_smem, row_xor, type_lp, [&](int sq, int t, float lg) {
-            if (!stays(lg)) return;
-            list_p[at] = __float2half_rn(__fdiv_rn(expf(__fsub_rn(lg, top)), z));
-            list_m[at] = static_cast<int16_t>((lane * 64 + sq) | (t << 11));
-            ++at;
-        });
-        for (int i = kept + lane; i < e_cap; i += 32) { list_p[i] = __float2half_rn(0.f); list_m[i] = 0; }
-        __syncwarp();
+        int16_t* list_m = reinterpret_cast<int16_t*>(list_buf + kListLabels);
+        for (int base = 0; base < e_cap; base += 32) {
+            const int i = base + lane;
+            const __half prior = i < kept ? __float2half_rn(__fdiv_rn(at(i), z)) : __float2half_rn(0.f);
+            __syncwarp();
+            if (i < e_cap) {
+                list_p[i] = prior;
+                if (i >= kept) list_m[i] = 0;
+            }
+            __syncwarp();
+        }
         const bool wide = (e_cap & 7) == 0 &&
                           ((reinterpret_cast<uintptr_t>(out_p) | reinterpret_cast<uintptr_t>(out_m)) & 15u) == 0;
         if (wide) {

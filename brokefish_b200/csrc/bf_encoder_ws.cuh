@@ -53,8 +53,8 @@ constexpr uint32_t kHeadA = 32768;                 // the head operand's place i
 constexpr uint32_t kStagePolicy = 49152, kStageAux = kStagePolicy + 8192;
 constexpr uint32_t SM_STAT = 16384 + 65536 + 8 * kStage;
 constexpr uint32_t SM_MAX = SM_STAT + 1024;        // row maxima: attention output, four hidden chunks
-constexpr uint32_t SM_LIST = SM_MAX + 5 * 256;     // fused expansion: 1 KB per board
-constexpr uint32_t SM_PAR = SM_LIST + 2048;        // scales and biases of two layers
+constexpr uint32_t SM_LIST = SM_MAX + 5 * 256;     // fused expansion: a list per board
+constexpr uint32_t SM_PAR = SM_LIST + 2 * kListBytes;        // scales and biases of two layers
 constexpr uint32_t SM_BAR = SM_PAR + 2 * kLparamStride;
 constexpr uint32_t SM_MISC = SM_BAR + 8 * 34;
 constexpr uint32_t SM_BYTES = SM_MISC + 64, kSmemRequest = SM_BYTES + 1024;
@@ -717,7 +717,7 @@ __device__ __forceinline__ void prenorm_means(const Row& c, uint32_t alive, cons
         if (c.lane == i) mine = make_float2(__fmul_rn(a0, inv_live), __fmul_rn(a1, inv_live));
     }
     if (c.lane < 8 * NB) {
-        const uint32_t at = c.smem + SM_LIST + 1024u * O::board(c) + 4u * O::col(c) + 8u * c.lane;
+        const uint32_t at = c.smem + SM_LIST + kListBytes * O::board(c) + 4u * O::col(c) + 8u * c.lane;
         sts32(at, __float_as_uint(mine.x));
         sts32(at + 4u, __float_as_uint(mine.y));
     }
@@ -729,7 +729,7 @@ __device__ __forceinline__ void prenorm_means(const Row& c, uint32_t alive, cons
 // lists 1748 against 1727).
 template <int NB>
 __device__ __noinline__ void prenorm_logits(const Row& c, const Params& p, float (&logit)[3]) {
-    const uint32_t means = c.smem + SM_LIST + 1024u * Own<NB>::board(c);
+    const uint32_t means = c.smem + SM_LIST + kListBytes * Own<NB>::board(c);
     const int quarter = c.lane & 3, kind = c.lane >> 2, k = kind < 2 ? 0 : (kind - 2) % 3;
     float t = 0.f, t2 = 0.f;
 #pragma unroll 1
@@ -881,7 +881,7 @@ __device__ __forceinline__ void expander(uint32_t smem, uint8_t* smem_gen, uint3
         __syncwarp();
         if (valid)
             expand_board(p, board, lane, true, word, ctl, moves, h + kStagePolicy + 4096u * which + 128u * lane, lane & 7,
-                         h + kStageAux + 512u * which + 16u * lane, smem_gen + SM_LIST + 1024u * which);
+                         h + kStageAux + 512u * which + 16u * lane, smem_gen + SM_LIST + kListBytes * which);
         __syncwarp();
         if (lane == 0) bfptx::mbar_arrive(bar(smem, B_EXPANDED));
     }

@@ -55,24 +55,34 @@ __device__ __forceinline__ unsigned long long king_pattern(unsigned long long b)
     const unsigned long long row = b | ((b >> 1) & ~kFileH) | ((b << 1) & ~kFileA);
     return (row | (row << 8) | (row >> 8)) & ~b;
 }
+// One sliding piece along one line without loops or fills: on the line's squares other than the
+// piece's own, subtracting the piece's bit from the occupancy flips exactly the squares up to and
+// including the first occupied one above it; the same on the bit-reversed board gives the squares
+// below it.
+__device__ __forceinline__ unsigned long long line_attacks(unsigned long long s, unsigned long long occ,
+                                                           unsigned long long line_ex) {
+    const unsigned long long o = occ & line_ex;
+    const unsigned long long up = o - s;
+    const unsigned long long down = __brevll(__brevll(o) - __brevll(s));
+    return (up ^ down) & line_ex;
+}
+// The rank, file and two diagonals through a square, without the square itself.
+__device__ __forceinline__ unsigned long long rank_ex(int sq) { return (0xFFull << (sq & 56)) ^ (1ull << sq); }
+__device__ __forceinline__ unsigned long long file_ex(int sq) { return (kFileA << (sq & 7)) ^ (1ull << sq); }
+__device__ __forceinline__ unsigned long long diag_ex(int sq) {
+    const int d = (sq >> 3) - (sq & 7);
+    return (d >= 0 ? 0x8040201008040201ull << (8 * d) : 0x8040201008040201ull >> (-8 * d)) ^ (1ull << sq);
+}
+__device__ __forceinline__ unsigned long long anti_ex(int sq) {
+    const int d = (sq >> 3) + (sq & 7) - 7;
+    return (d >= 0 ? 0x0102040810204080ull << (8 * d) : 0x0102040810204080ull >> (-8 * d)) ^ (1ull << sq);
+}
 // Squares seen from `sq` along the rook (diag = false) or bishop (diag = true) lines, each ray
 // ending on and including its first occupied square.
 __device__ __forceinline__ unsigned long long rays(int sq, unsigned long long occ, bool diag) {
-    const int r0 = sq >> 3, f0 = sq & 7;
-    unsigned long long out = 0ull;
-#pragma unroll
-    for (int d = 0; d < 4; ++d) {
-        const int dr = diag ? ((d & 1) ? 1 : -1) : (d == 0 ? 1 : (d == 1 ? -1 : 0));
-        const int df = diag ? ((d & 2) ? 1 : -1) : (d == 2 ? 1 : (d == 3 ? -1 : 0));
-        int r = r0 + dr, f = f0 + df;
-        while (r >= 0 && r < 8 && f >= 0 && f < 8) {
-            const unsigned long long bit = 1ull << (r * 8 + f);
-            out |= bit;
-            if (occ & bit) break;
-            r += dr; f += df;
-        }
-    }
-    return out;
+    const unsigned long long b = 1ull << sq;
+    return diag ? line_attacks(b, occ, diag_ex(sq)) | line_attacks(b, occ, anti_ex(sq))
+                : line_attacks(b, occ, rank_ex(sq)) | line_attacks(b, occ, file_ex(sq));
 }
 
 // The opponent's pieces by the way they attack.
@@ -305,30 +315,6 @@ __device__ __forceinline__ unsigned long long line_through(int a, int b) {
     }
     return 0ull;
 }
-
-// One sliding piece along one line without loops or fills: on the line's squares other than the
-// piece's own, subtracting the piece's bit from the occupancy flips exactly the squares up to and
-// including the first occupied one above it; the same on the bit-reversed board gives the squares
-// below it.
-__device__ __forceinline__ unsigned long long line_attacks(unsigned long long s, unsigned long long occ,
-                                                           unsigned long long line_ex) {
-    const unsigned long long o = occ & line_ex;
-    const unsigned long long up = o - s;
-    const unsigned long long down = __brevll(__brevll(o) - __brevll(s));
-    return (up ^ down) & line_ex;
-}
-// The rank, file and two diagonals through a square, without the square itself.
-__device__ __forceinline__ unsigned long long rank_ex(int sq) { return (0xFFull << (sq & 56)) ^ (1ull << sq); }
-__device__ __forceinline__ unsigned long long file_ex(int sq) { return (kFileA << (sq & 7)) ^ (1ull << sq); }
-__device__ __forceinline__ unsigned long long diag_ex(int sq) {
-    const int d = (sq >> 3) - (sq & 7);
-    return (d >= 0 ? 0x8040201008040201ull << (8 * d) : 0x8040201008040201ull >> (-8 * d)) ^ (1ull << sq);
-}
-__device__ __forceinline__ unsigned long long anti_ex(int sq) {
-    const int d = (sq >> 3) + (sq & 7) - 7;
-    return (d >= 0 ? 0x0102040810204080ull << (8 * d) : 0x0102040810204080ull >> (-8 * d)) ^ (1ull << sq);
-}
-
 
 constexpr int kTpbThreads = 128;
 constexpr int kTpbInStride = 17;      // 32-bit words per board in shared memory (16 + 1: no bank conflicts)
