@@ -887,6 +887,13 @@ __device__ __forceinline__ void expander(uint32_t smem, uint8_t* smem_gen, uint3
     }
 }
 
+// Where 16-byte piece `part` of a token's columns lies in a warp's block: `kLanes` pieces to a token, moved so that
+// eight tokens' same piece, and what eight lanes next to each other hold, hit all banks.
+template <int kLanes>
+__device__ __forceinline__ uint32_t embed_off(int token, int part) {
+    return 16u * (kLanes * token + (part ^ ((token / (8 / kLanes)) & (kLanes - 1))));
+}
+
 // One tile of NB boards, from the piece words to the outputs.
 template <int NB, int kAr, bool kExpand>
 __device__ __forceinline__ void row_tile(Row& c, const Params& p, int first) {
@@ -907,24 +914,51 @@ __device__ __forceinline__ void row_tile(Row& c, const Params& p, int first) {
         const int sq = word & 63;
         const int ts = min(static_cast<int>(((word >> 6) & 7) * 2 + ((word >> 9) & 1)), kNTypeSpecial - 1);
         const int ct = ((word >> 10) & 1) * 2 + stm;
-        const uint4* e_sq = reinterpret_cast<const uint4*>(p.emb + (EMB_SQUARE + sq) * kD + col);
-        const uint4* e_ts = reinterpret_cast<const uint4*>(p.emb + (EMB_TS + ts) * kD + col);
-        const uint4* e_ct = reinterpret_cast<const uint4*>(p.emb + (EMB_CT + ct) * kD + col);
-        const uint4* e_ck = reinterpret_cast<const uint4*>(p.emb + (EMB_CLOCK + clk) * kD + col);
-        const uint4* e_rp = reinterpret_cast<const uint4*>(p.emb + (EMB_REP + rp) * kD + col);
+        // A token's columns of the three tables that go by token are read by 2 NB lanes next to each other, 16 bytes to a
+        // lane, summed there, and go to the token's own lane through the warp's 1 KB of the last tile's head operand
+        // (32 / NB tokens at a time).  With every lane reading its own token's a warp's load touches 32 lines, one a cycle:
+        // 1 % of a two-board tile more.
+        constexpr int kLanes = 2 * NB, kTokens = 32 / kLanes;
+        const int part = lane & (kLanes - 1);
+        const int rows = (EMB_SQUARE + sq) | (EMB_TS + ts) << 8 | (EMB_CT + ct) << 16;
+        constexpr int kAtOnce = 32 / NB;
+        const uint32_t block = c.h + kHeadA + 1024u * (4 * c.q + c.s);
+        const __half* emb = p.emb + col + 8 * part;
+        const uint4 e = __ldg(reinterpret_cast<const uint4*>(emb + (EMB_CLOCK + clk) * kD));
+        const uint4 f = __ldg(reinterpret_cast<const uint4*>(emb + (EMB_REP + rp) * kD));
+        const uint32_t ew[4] = {e.x, e.y, e.z, e.w}, fw[4] = {f.x, f.y, f.z, f.w};
+        uint4 a[kLanes], b[kLanes], d[kLanes];
 #pragma unroll
-        for (int k = 0; k < 2 * NB; ++k) {
-            const uint4 a = __ldg(e_sq + k), b = __ldg(e_ts + k), d = __ldg(e_ct + k);
-            const uint4 e = __ldg(e_ck + k), f = __ldg(e_rp + k);
-            const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
-            const uint32_t dw[4] = {d.x, d.y, d.z, d.w}, ew[4] = {e.x, e.y, e.z, e.w};
-            const uint32_t fw[4] = {f.x, f.y, f.z, f.w};
+        for (int k = 0; k < kLanes; ++k) {
+            const int r = __shfl_sync(0xffffffffu, rows, kTokens * k + lane / kLanes);
+            a[k] = __ldg(reinterpret_cast<const uint4*>(emb + (r & 255) * kD));
+            b[k] = __ldg(reinterpret_cast<const uint4*>(emb + ((r >> 8) & 255) * kD));
+            d[k] = __ldg(reinterpret_cast<const uint4*>(emb + (r >> 16) * kD));
+        }
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                __half2 v = __hadd2(as_h2(aw[j]), as_h2(bw[j]));
-                v = __hadd2(v, as_h2(dw[j]));
-                x[4 * k + j] = as_u32(__hadd2(v, __hadd2(as_h2(ew[j]), as_h2(fw[j]))));
+        for (int pass = 0; pass < NB; ++pass) {
+#pragma unroll
+            for (int k = 2 * pass; k < 2 * pass + 2; ++k) {
+                const uint32_t aw[4] = {a[k].x, a[k].y, a[k].z, a[k].w}, bw[4] = {b[k].x, b[k].y, b[k].z, b[k].w};
+                const uint32_t dw[4] = {d[k].x, d[k].y, d[k].z, d[k].w};
+                uint32_t y[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    __half2 v = __hadd2(as_h2(aw[j]), as_h2(bw[j]));
+                    v = __hadd2(v, as_h2(dw[j]));
+                    y[j] = as_u32(__hadd2(v, __hadd2(as_h2(ew[j]), as_h2(fw[j]))));
+                }
+                sts128(block + embed_off<kLanes>((kTokens * k + lane / kLanes) & (kAtOnce - 1), part), make_uint4(y[0], y[1], y[2], y[3]));
             }
+            __syncwarp();
+            if (lane / kAtOnce == pass) {
+#pragma unroll
+                for (int k = 0; k < kLanes; ++k) {
+                    const uint4 v = lds128(block + embed_off<kLanes>(lane & (kAtOnce - 1), k));
+                    x[4 * k] = v.x; x[4 * k + 1] = v.y; x[4 * k + 2] = v.z; x[4 * k + 3] = v.w;
+                }
+            }
+            __syncwarp();
         }
     }
     const int id = 128 * c.q + 32 * c.s + lane;              // 0 .. 511
