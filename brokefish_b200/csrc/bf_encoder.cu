@@ -2441,8 +2441,12 @@ Kernel small_tile_kernel(int quant, bool expand, int boards) {
 // one of a GPC with an odd number of them.
 cudaError_t pairs_at_a_time(int quant, int sm_count, int* wave) {
     for (int arm = 0; arm < 4; ++arm) {
-        const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(small_tile_kernel(quant, (arm & 1) != 0, 1 + (arm >> 1))),
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, bf::ws::kSmemRequest);
+        const void* const kernel = reinterpret_cast<const void*>(small_tile_kernel(quant, (arm & 1) != 0, 1 + (arm >> 1)));
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bf::ws::kSmemRequest);
+        // (two-board tiles share out the registers that they are launched with)
+        cudaFuncAttributes a = {};
+        if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, kernel);
+        if (e == cudaSuccess && (arm >> 1) != 0 && a.numRegs < bf::ws::kLaunchRegisters) e = cudaErrorInvalidKernelImage;
         if (e != cudaSuccess) return e;
     }
     cudaLaunchAttribute cluster = {};
@@ -2451,7 +2455,7 @@ cudaError_t pairs_at_a_time(int quant, int sm_count, int* wave) {
     cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3(sm_count & ~1);
-    config.blockDim = dim3(bf::ws::threads(true));
+    config.blockDim = dim3(bf::ws::threads(true, 2));
     config.dynamicSmemBytes = bf::ws::kSmemRequest;
     config.attrs = &cluster;
     config.numAttrs = 1;
@@ -2466,7 +2470,7 @@ cudaError_t pairs_at_a_time(int quant, int sm_count, int* wave) {
 // waiting for the launch beside them, and wait for it when they are done: what comes after them in the
 // stream comes after both.
 // `wave`: CTAs that run at a time (`pairs_at_a_time`).
-cudaError_t launch_tiles(bf::Params p, int wave, int one_board, cudaStream_t stream, bool early) {
+cudaError_t launch_tiles(bf::Params p, int wave, int one_board, cudaStream_t stream, bool early, int* launches) {
     const int n = p.n, quant = static_cast<int>(p.quant);
     const bool expand = p.prior != nullptr;
     p.wave_ctas = wave;
@@ -2480,12 +2484,13 @@ cudaError_t launch_tiles(bf::Params p, int wave, int one_board, cudaStream_t str
         return static_cast<int>(2 * pairs < wave ? 2 * pairs : wave);
     };
     cudaError_t e = cudaSuccess;
+    *launches = (twos ? 1 : 0) + (ones ? 1 : 0);
     if (twos)
-        e = launch_early(small_tile_kernel(quant, expand, 2), ctas(n, 2), bf::ws::threads(expand), bf::ws::kSmemRequest, 2, stream,
+        e = launch_early(small_tile_kernel(quant, expand, 2), ctas(n, 2), bf::ws::threads(expand, 2), bf::ws::kSmemRequest, 2, stream,
                          early, p);
     if (ones && e == cudaSuccess) {
         p.after_waves = twos ? 1 : 0;
-        e = launch_early(small_tile_kernel(quant, expand, 1), ctas(singles || list ? n : rest, 1), bf::ws::threads(expand),
+        e = launch_early(small_tile_kernel(quant, expand, 1), ctas(singles || list ? n : rest, 1), bf::ws::threads(expand, 1),
                          bf::ws::kSmemRequest, 2, stream, early || twos, p);
     }
     return e;
@@ -2530,8 +2535,9 @@ int launch(bf_handle* h, const uint16_t* boards, const int16_t* control, const u
     // the instrumented instantiation only when a dump, a capture or the phase clock is asked for
     const bool dbg = stage != 0 || cap_layer >= 0 || p.prof != nullptr;
     if (cap_layer >= 0 && p.quant != 3) return fail(BF_ENOTSUP, "operand capture is for the int8 arithmetic");
+    int launches = 1;
     if (!dbg && p.rj_mode == 0) {
-        BF_CUDA(launch_tiles(p, h->wave_ctas, h->one_board_factor, stream, true));
+        BF_CUDA(launch_tiles(p, h->wave_ctas, h->one_board_factor, stream, true, &launches));
     } else {
         // four-board tiles: re-injection, and the instrumented arms (dumps, captures, the phase clock, the
         // backbone entry)
@@ -2547,7 +2553,7 @@ int launch(bf_handle* h, const uint16_t* boards, const int16_t* control, const u
         kernel<<<grid, bf::kThreads, bf::kSmemRequest, stream>>>(p);
     }
     BF_CUDA(cudaGetLastError());
-    h->launches++;
+    h->launches += launches;
     return BF_OK;
 }
 
@@ -3407,7 +3413,8 @@ int bf_forward_noalloc(int device, const void* blob_dev, size_t blob_bytes, cons
     p.status = static_cast<int*>(scratch);         // the device address, not the symbol
     p.prof = nullptr;
     // (the caller's own blob may be an output of the grid before)
-    BF_CUDA(launch_tiles(p, wave, 1, static_cast<cudaStream_t>(stream), false));
+    int launches = 0;
+    BF_CUDA(launch_tiles(p, wave, 1, static_cast<cudaStream_t>(stream), false, &launches));
     return BF_OK;
 }
 

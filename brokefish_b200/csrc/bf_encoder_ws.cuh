@@ -34,7 +34,13 @@ namespace bf {
 namespace ws {
 
 constexpr int kProducerWarp = 16, kMmaWarp = 17, kExpandWarp = 18;
-constexpr int threads(bool expand) { return expand ? 640 : 576; }
+// (two-board tiles: a whole warpgroup of the warps that give registers up)
+constexpr int threads(bool expand, int boards) { return expand || boards == 2 ? 640 : 576; }
+// Two-board tiles: a row warp's registers and another's, out of the 96 a thread that the launch comes with.  4096
+// positions int8 1570 us without the split, 1543 with it; 112 and 32 are too few for the producer (e4m3 +2 %, fp16 +10 %),
+// and one-board tiles, which need 95, lose 1 % by it.
+constexpr int kRowRegisters = 104, kHelperRegisters = 64, kLaunchRegisters = 96;
+static_assert(16 * kRowRegisters + 4 * kHelperRegisters <= 20 * kLaunchRegisters, "a larger share would be waited for in vain");
 constexpr uint32_t kStage = 16384;                 // one 128-byte K-slab of this SM's 128 rows of a product's weights
 // ---- shared memory map ------------------------------------------------------------------
 // A operand: K-slabs of [rows][128 B], two of bytes or (where QKV or the out-projection runs in fp16)
@@ -1206,6 +1212,10 @@ __global__ void __launch_bounds__(640, 1) encoder_ws_kernel(const Params p) {
     if (p.leaf_count != nullptr) n_eval = min(max(*p.leaf_count, 0), p.n);
     const Tiles<NB> tiles(n_eval, p.wave_ctas, gridDim.x, blockIdx.x, p.one_most);
     const int n_tiles = tiles.count();
+    if constexpr (NB == 2) {
+        if (warp < kRowWarps) take_registers<kRowRegisters>();
+        else give_registers<kHelperRegisters>();
+    }
     if (warp < kRowWarps) {
         Row c;
         c.lane = lane; c.q = warp & 3; c.s = warp >> 2;

@@ -34,6 +34,13 @@ __device__ __forceinline__ void previous_grid_wait() { asm volatile("griddepcont
 // The grid after this one may start once every CTA of this one has said so.
 __device__ __forceinline__ void next_grid_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// ---------------------------------------------------------------- register shares of a warpgroup's warps
+// The block's shares together must not be above what it was launched with: the taker waits for what is given.
+template <int kCount>
+__device__ __forceinline__ void take_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kCount)); }
+template <int kCount>
+__device__ __forceinline__ void give_registers() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kCount)); }
+
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
