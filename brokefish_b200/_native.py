@@ -81,7 +81,7 @@ def build_ops(force: bool = False, verbose: bool = False) -> str:
     _compile(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=_torch_ops",
               f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
              + [a for i in inc for a in ("-isystem", i)]
-             + [OPS_SOURCE, "-o", OPS_PATH, f"-L{libs}", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda",
+             + [OPS_SOURCE, "-o", OPS_PATH, f"-L{libs}", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda",
                 "-ltorch_python", "-ldl"], verbose)
     return OPS_PATH
 

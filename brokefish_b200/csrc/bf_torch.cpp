@@ -9,6 +9,7 @@
 // (zero fills of buffers that the kernels fill anyway, clones, conversions between bool and bytes)
 // and about 40 us of attribute look-ups, shape tuples and argument boxing.
 #include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAStream.h>
 #include <dlfcn.h>
 #include <torch/csrc/utils/pybind.h>
@@ -77,6 +78,11 @@ T* ptr(const Tensor& t) {
     return t.defined() && t.numel() ? static_cast<T*>(t.data_ptr()) : nullptr;
 }
 void* stream_of(c10::Device d) { return c10::cuda::getCurrentCUDAStream(d.index()).stream(); }
+// An output on the inputs' device.  Straight from the allocator: through the dispatcher, `at::empty`, one takes 0.73 us
+// instead of 0.52, and a ply of games makes ten of them in 20 us.
+Tensor output(at::IntArrayRef size, at::ScalarType type, const Tensor& like) {
+    return at::detail::empty_cuda(size, type, like.device(), std::nullopt);
+}
 bool is_vector(const Tensor& t, int64_t n) { return t.dim() == 1 && t.size(0) == n; }
 
 // ---- the engine ----
@@ -93,8 +99,7 @@ constexpr const char* kNoCpu = "the engine kernels take CUDA tensors on one devi
 
 py::tuple movegen(const Tensor& boards, const Tensor& control) {
     const int64_t n = check_position(boards, control, "movegen takes CUDA tensors on one device; there is no CPU path");
-    const auto o = boards.options();
-    Tensor mask = at::empty({n, 32}, o.dtype(at::kLong)), check = at::empty({n}, o.dtype(at::kBool));
+    Tensor mask = output({n, 32}, at::kLong, boards), check = output({n}, at::kBool, boards);
     if (n) {
         const Tensor b = boards.contiguous(), c = control.contiguous();
         call("bf_movegen", [&] {
@@ -118,12 +123,13 @@ py::tuple step(const Tensor& boards, const Tensor& control, const Tensor& move, 
         pr = promo->to(o.dtype(at::kChar)).contiguous();
         if (!is_vector(pr, n)) throw py::value_error("promo must have shape [" + std::to_string(n) + "]");
     }
-    Tensor nb = at::empty({n, 32}, o), nc = at::empty({n}, o), irr = at::empty({n}, o.dtype(at::kBool)), mask, check, key;
+    Tensor nb = output({n, 32}, at::kShort, boards), nc = output({n}, at::kShort, boards), irr = output({n}, at::kBool, boards);
+    Tensor mask, check, key;
     if (with_moves) {
-        mask = at::empty({n, 32}, o.dtype(at::kLong));
-        check = at::empty({n}, o.dtype(at::kBool));
+        mask = output({n, 32}, at::kLong, boards);
+        check = output({n}, at::kBool, boards);
     }
-    if (with_hash) key = at::empty({n}, o.dtype(at::kLong));
+    if (with_hash) key = output({n}, at::kLong, boards);
     if (n) {
         const Tensor b = boards.contiguous(), c = control.contiguous();
         call("bf_step", [&] {
@@ -138,7 +144,7 @@ py::tuple step(const Tensor& boards, const Tensor& control, const Tensor& move, 
 
 Tensor hash_position(const Tensor& boards, const Tensor& control) {
     const int64_t n = check_position(boards, control, kNoCpu);
-    Tensor key = at::empty({n}, boards.options().dtype(at::kLong));
+    Tensor key = output({n}, at::kLong, boards);
     if (n) {
         const Tensor b = boards.contiguous(), c = control.contiguous();
         call("bf_hash", [&] {
@@ -163,7 +169,7 @@ py::tuple push_history(const Tensor& ring, const Tensor& length, const Tensor& h
         throw py::value_error("length, hash [n] int64 and irreversible [n] are needed");
     if (length.device() != ring.device() || hash.device() != ring.device() || irreversible.device() != ring.device())
         throw py::value_error("ring, length, hash and irreversible must live on one device");
-    Tensor new_ring = at::empty({n, kMaxHistory}, ring.options()), new_length = at::empty({n}, length.options());
+    Tensor new_ring = output({n, kMaxHistory}, at::kLong, ring), new_length = output({n}, at::kLong, ring);
     if (n) {
         const Tensor r = ring.contiguous(), l = length.contiguous(), h = hash.contiguous(), irr = bytes_of(irreversible);
         call("bf_history_push_to", [&] {
@@ -186,7 +192,7 @@ void check_history(const Tensor& hash, const Tensor& ring, const Tensor& length,
 Tensor repetition_count(const Tensor& hash, const Tensor& ring, const Tensor& length) {
     const int64_t n = ring.dim() ? ring.size(0) : 0;
     check_history(hash, ring, length, n);
-    Tensor count = at::empty({n}, ring.options().dtype(at::kInt));
+    Tensor count = output({n}, at::kInt, ring);
     if (n) {
         const Tensor h = hash.contiguous(), r = ring.contiguous(), l = length.contiguous();
         call("bf_repetition_count", [&] {
@@ -207,8 +213,7 @@ py::tuple terminal(const Tensor& mask, const Tensor& in_check, const Tensor& con
         throw py::value_error("mask must be a CUDA int64 tensor of shape [" + std::to_string(n) + ", 32]");
     if (!is_vector(in_check, n) || !in_check.is_cuda())
         throw py::value_error("in_check must be a CUDA tensor of shape [" + std::to_string(n) + "]");
-    const auto o = boards.options();
-    Tensor code = at::empty({n}, o.dtype(at::kByte)), result = at::empty({n}, o.dtype(at::kChar));
+    Tensor code = output({n}, at::kByte, boards), result = output({n}, at::kChar, boards);
     if (n) {
         const Tensor m = mask.contiguous(), chk = bytes_of(in_check), c = control.contiguous(), b = boards.contiguous();
         const int dev = b.device().index(), count = static_cast<int>(n);
