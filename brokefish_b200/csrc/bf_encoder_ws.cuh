@@ -153,10 +153,10 @@ __device__ __forceinline__ void board_sync(const Row& c) { __syncwarp(); named_b
 __device__ __forceinline__ void pair_sync(int head) { __syncwarp(); named_bar_sync(3 + head, 64); }
 
 // How often a slot's barrier completes in a layer: with Q, K, V or the out-projection, with ff1's chunk,
-// with ff2's (in fp16, whose ff2 has one sum, slot 0 with its first half and slot 1 with all of it).  Every
-// completion is one that all row warps wait for: a parity wait tells a phase only from the one before it.
+// with ff2's (in fp16, whose ff2 has one sum, slots 0 and 1 with its first and second chunk and slot 2 with all of
+// it).  Every completion is one that all row warps wait for: a parity wait tells a phase only from the one before it.
 template <int kAr>
-__host__ __device__ constexpr uint32_t completions(int slot) { return kAr == kArF16 && slot >= 2 ? 2u : 3u; }
+__host__ __device__ constexpr uint32_t completions(int slot) { return kAr == kArF16 && slot == 3 ? 2u : 3u; }
 // The `use`-th of them in this layer; of slot 0, use 0 after the last layer is the heads' product.
 template <int kAr>
 __device__ __forceinline__ void wait_acc(const Row& c, int slot, int use) {
@@ -664,33 +664,31 @@ __device__ __forceinline__ void ffn_block(const Row& c, uint32_t lp, float sa, u
 }
 
 // The fp16 arithmetic's FFN: ff1's epilogue is bias and ReLU, a chunk goes out as ff2's fp16 operand, and
-// ff2's fp16 accumulators (slot 0) run on through the four chunks.  H holds two chunks, so the second
-// pair is written when the first pair's ff2 products are done (a completion of slot 0 that says no more
-// than that); a completion of slot 1 says that the sums are there.
+// ff2's fp16 accumulators (slot 0) run on through the four chunks.  H holds two chunks, so the third and the fourth
+// are written when ff2 is done with the first and the second (completions of slots 0 and 1 that say no more than
+// that); a completion of slot 2 says that the sums are there.  The products follow one another in the order ff1 0, 1,
+// ff2 0, ff1 2, ff2 1, ff1 3, ff2 2, 3: each has its operand when its turn comes, and a chunk's place is free when
+// the chunk is (all of ff1 first, and two chunks to an arrival: 1,000 cycles of a two-board layer's 23,400 more).
 template <int NB>
 __device__ __forceinline__ void ffn_block_f16(const Row& c, uint32_t lp, uint32_t (&x)[8 * NB]) {
     using O = Own<NB>;
     const int col = O::col(c);
 #pragma unroll 1
-    for (int pair = 0; pair < 2; ++pair) {
-#pragma unroll 1
-        for (int k = 0; k < 2; ++k) {
-            const int ch = 2 * pair + k;
-            const uint32_t bias_at = lp + LP_B_FF1 + 2u * (256 * ch + col);
-            Bias bias = load_bias(bias_at);
-            wait_acc<kArF16>(c, ch, 1);
-            if (ch == 2) wait_acc<kArF16>(c, 0, 2);
-            each_piece<NB>(O::slot(c, ch), [&](int i, const uint32_t (&acc)[16]) {
-                uint32_t h[8];
-                if (i > 0) bias = load_bias(bias_at + 32 * i);
-                descale16<true, kAccPlain>(acc, 1.f, 1.f, bias, h);
-                store_operand16<NB>(c, c.h + k * 4 * O::kSlab, i, h);
-            });
-        }
-        publish(c, B_H + pair);
+    for (int ch = 0; ch < 4; ++ch) {
+        const uint32_t bias_at = lp + LP_B_FF1 + 2u * (256 * ch + col);
+        Bias bias = load_bias(bias_at);
+        wait_acc<kArF16>(c, ch, 1);
+        if (ch >= 2) wait_acc<kArF16>(c, ch - 2, 2);
+        each_piece<NB>(O::slot(c, ch), [&](int i, const uint32_t (&acc)[16]) {
+            uint32_t h[8];
+            if (i > 0) bias = load_bias(bias_at + 32 * i);
+            descale16<true, kAccPlain>(acc, 1.f, 1.f, bias, h);
+            store_operand16<NB>(c, c.h + (ch & 1) * 4 * O::kSlab, i, h);
+        });
+        publish(c, B_H + ch);
     }
     Bias bias = load_bias(lp + LP_B_FF2 + 2u * col);
-    wait_acc<kArF16>(c, 1, 2);
+    wait_acc<kArF16>(c, 2, 2);
     each_piece<NB>(O::slot(c, 0), [&](int k, const uint32_t (&acc)[16]) {
         uint32_t y[8];
         if (k > 0) bias = load_bias(lp + LP_B_FF2 + 2u * col + 32 * k);
@@ -1052,16 +1050,16 @@ __device__ __forceinline__ void producer(uint32_t smem, volatile int* abort_flag
                     });
             const uint8_t* out = src + 4 * C::kQkvSlabs * kQStage;
             for (int s = 0; s < C::kOutSlabs; ++s) two_units(out, out + C::kOutSlabs * kRStage, s);
-            // ff1 chunks 0-3, then ff2 chunks 0-3; where their two units lie in the packed order
+            // ff1 chunks 0-3, then ff2 chunks 0-3 (fp16: see `ffn_block_f16`); where their two units lie in the packed order
             const uint8_t* ffn = out + 2 * C::kOutSlabs * kRStage;
-            for (int u = 0; u < 8; ++u) {
+            for (int k = 0; k < 8; ++k) {
                 int u0, u1;
                 if (kAr == kArF16) {
-                    const int ch = u & 3;
+                    const int u = (0x76352410u >> (4 * k)) & 7, ch = u & 3;
                     u0 = u < 4 ? (ch == 0 ? 0 : 4 * ch - 2) : (ch < 3 ? 4 * ch + 3 : 14);
                     u1 = u < 4 ? 4 * ch + 1 : (ch < 3 ? 4 * ch + 4 : 15);
                 } else {
-                    u0 = (0xEC84A620u >> (4 * u)) & 15u;
+                    u0 = (0xEC84A620u >> (4 * k)) & 15u;
                     u1 = u0 + 1;
                 }
                 for (int s = 0; s < C::kFfnSlabs; ++s) {
@@ -1156,14 +1154,16 @@ __device__ __forceinline__ void issue_tile(Issue& st, int n_layers) {
         issue_wait(st, B_A, st.a++);
         issue_unit<kAr, kOutKind>(st, st.tmem + O::kSlot * 3, a, O::kSlab, C::kOutSlabs, kI_OUT, 3);
         issue_wait(st, B_A, st.a++);
-        for (int ch = 0; ch < 4; ++ch)
+        auto ff1 = [&](int ch) {
             issue_unit<kAr, kFfnKind>(st, st.tmem + O::kSlot * ch, a, O::kSlab, C::kFfnSlabs, kI_FF1, ch);
+        };
+        for (int ch = 0; ch < (kAr == kArF16 ? 2 : 4); ++ch) ff1(ch);
         for (int ch = 0; ch < 4; ++ch) {
-            if (kAr != kArF16)      issue_wait(st, B_H + ch, st.h);
-            else if ((ch & 1) == 0) issue_wait(st, B_H + (ch >> 1), st.h);
+            issue_wait(st, B_H + ch, st.h);
             if (kAr == kArF16) {
                 issue_unit<kAr, kFfnKind>(st, st.tmem, h + (ch & 1) * 4 * O::kSlab, O::kSlab, C::kFfnSlabs, kI_FF2,
-                                            ch == 1 ? 0 : ch == 3 ? 1 : -1, ch > 0);
+                                          ch < 2 ? ch : ch == 3 ? 2 : -1, ch > 0);
+                if (ch < 2) ff1(ch + 2);
             } else {
                 issue_unit<kAr, kFfnKind>(st, st.tmem + O::kSlot * ch, h + ch * 2 * O::kSlab, O::kSlab, C::kFfnSlabs, kI_FF2, ch);
             }
