@@ -965,6 +965,7 @@ __global__ void __launch_bounds__(kTpbThreads, kPick ? 5 : 6) engine_board_kerne
 #pragma unroll
         for (int k = 0; k < 4; ++k)
             if (tid + k * kTpbThreads < here * 4) v[k] = src[tid + k * kTpbThreads];
+        const int word = tid < here ? control[first + tid] : 1;
         if (kPick)
             for (int j = tid; j < here * 32; j += kTpbThreads)
                 s_mask[(j >> 5) * kTpbMaskStride + (j & 31)] = mask[first * 32 + j];
@@ -976,6 +977,7 @@ __global__ void __launch_bounds__(kTpbThreads, kPick ? 5 : 6) engine_board_kerne
             unsigned* d = s_in + (j >> 2) * kTpbInStride + (j & 3) * 4;
             if (j < here * 4) { d[0] = v[k].x; d[1] = v[k].y; d[2] = v[k].z; d[3] = v[k].w; }
         }
+        s_in[tid * kTpbInStride + 16] = static_cast<unsigned>(word);      // (the row's padding)
     }
     __syncthreads();
     const bool mine = tid < here;
@@ -1009,7 +1011,7 @@ __global__ void __launch_bounds__(kTpbThreads, kPick ? 5 : 6) engine_board_kerne
         __syncthreads();
     }
     if (mine) {
-        int ctl = control[first + tid];
+        int ctl = static_cast<int>(my[16]);
         bool generate = mask != nullptr;
         if (kStep) {
             if (!kPick) mv = move[first + tid];
@@ -1030,7 +1032,7 @@ __global__ void __launch_bounds__(kTpbThreads, kPick ? 5 : 6) engine_board_kerne
             if (in_check != nullptr) in_check[first + tid] = chk ? 1 : 0;
             words = !by_slot ? WORDS_STORED : ctl < 0 ? WORDS_BLACK : WORDS_WHITE;
         }
-        my[16] = words;                               // (the row's padding)
+        my[16] = words;
         if (hash_out != nullptr) hash_out[first + tid] = board_hash(my, ctl < 0);
     }
     if (!kStep) next_grid_may_start();
