@@ -25,9 +25,11 @@
 // The arithmetic is the four-board kernel's, bit for bit (the order of every sum included).
 //
 // Measured on one B200, us, against tiles of one SM (M = 32 and 64 by `tcgen05.mma.ws`): a one-board tile
-// int8 85 (91), e4m3 91 (101), fp16 109 (129); a two-board tile 117 (127), 117 (130), 116 (152); batch 4096 1589
-// (1677), 1547 (1735), 1660 (1877, then on four-board tiles).  What bounds it: the row warps, four to a scheduler and all in the same
-// phase.
+// int8 85 (91), e4m3 91 (101), fp16 103 (129); a two-board tile 114 (127), 115 (130), 117 (152); batch 4096 1544
+// (1677), 1547 (1735), 1620 (1877, then on four-board tiles).  What bounds it: the row warps, four to a scheduler and all
+// in the same phase, at 61 % of the issue slots in int8; of a one-board tile's 18,900 cycles per layer a row warp waits 3,600
+// for products, of a two-board tile's 26,000 4,800.  In fp16 and e4m3 a loop of large batches also runs into
+// the 1000 W power cap (1.75 to 1.87 GHz; int8 stays at 890 W and 1.965 GHz).
 #pragma once
 
 namespace bf {
@@ -1203,8 +1205,11 @@ __global__ void __launch_bounds__(640, 1) encoder_ws_kernel(const Params p) {
     const uint32_t tmem = *tmem_slot;
     // The grid before this one may still be running.  Only the producer goes on without it: the first weights are
     // nobody's output.  One-board tiles beside this call's own two-board ones start without it, since that grid lets
-    // them start only when what came before it has ended; they wait for it at their own end.
-    if (!p.after_waves && (warp != kProducerWarp || p.leaf_count != nullptr)) {
+    // them start only when what came before it has ended (the fence is for what that left in this SM's cache); they wait
+    // for it at their own end.
+    if (p.after_waves) {
+        __threadfence();
+    } else if (warp != kProducerWarp || p.leaf_count != nullptr) {
         previous_grid_wait();
         next_grid_may_start();
     }
