@@ -12,9 +12,8 @@
 // integers; fp16 x fp16 with fp16 accumulators, which carries the bits of the reference's
 // fp16-accumulate mma.sync); the 32 x 32 attention products run as mma.sync on the row warps.
 //
-// Plain evaluations run on one- and two-board tiles (bf_encoder_ws.cuh).  The kernel below, on
-// four-board tiles, is the large-batch form of the fp16 arithmetic, carries re-injection and is the
-// instrumented arm.  Its shape
+// Plain evaluations run on one- and two-board tiles, by pairs of SMs (bf_encoder_ws.cuh).  The kernel below, on
+// four-board tiles, carries re-injection and is the instrumented arm.  Its shape
 //   * persistent grid, one CTA per SM, each CTA loops over tiles of 128 token rows
 //     (4 boards);
 //   * 19 warps: 16 "row" warps, one weight-stream producer, two MMA issuers;
@@ -2106,8 +2105,8 @@ __global__ void scales_kernel(unsigned long long* differ) {
 
 // ------------------------------------------------------------------------------------------
 // Tensor-core self test: one tile, one GEMM, no network.  Modes 0-4 are the four-board kernel's products (128
-// rows), the others the small tiles' weight-stationary ones (32 or 64 rows), read out of tensor memory where
-// bf_encoder_ws.cuh looks for them.
+// rows), the others weight-stationary ones of one SM (32 or 64 rows; those of 64 read out of tensor memory where
+// bf_encoder_ws.cuh looks for its pairs').
 // ------------------------------------------------------------------------------------------
 constexpr int kSelftestModes = 15;
 constexpr uint32_t kSelftestW = 65536, kSelftestBar = kSelftestW + 131072, kSelftestSmem = kSelftestBar + 128 + 1024;
@@ -2318,7 +2317,7 @@ bool two_board_waves(const bf_handle* h) { return h->hdr.rj_mode == 0; }
 // 10.8 in fp16, which moves the ratio, and a launch's size, by 4 %.)
 constexpr double kEvalGBps = 8.8;        // logits a B200 produces per second at full rate on four-board
                                          // tiles (4356 B x 2.03 M)
-constexpr double kSmallTileRate = 1.27;  // how much faster two-board tiles are (2.58 M positions/s)
+constexpr double kSmallTileRate = 1.27;  // how much faster two-board tiles are (2.58 to 2.65 M positions/s)
 constexpr double kFastLinkRatio = 6.0;   // a GPU alone on its link: 55 GB/s against those 8.8
 
 // The launch sizes of bf_forward_host for `n` positions on a GPU whose wave is `wave` positions:
@@ -2914,7 +2913,7 @@ int bf_forward_host(bf_handle* h, const uint16_t* boards, const int16_t* control
     //   r >= 1.5    launches of shrinking size, largest first, the last one a single wave (one
     //               tile per SM), each launch r times the one after it (in whole waves, rounded
     //               down) so that its copy hides behind the next launch; r is capped at 6, a GPU
-    //               alone on its link: [2320, 1480, 296] positions for a batch of 4096.  Large launches
+    //               alone on its link: [2616, 1184, 296] positions for a batch of 4096.  Large launches
     //               keep the kernel's tile-to-tile pipelining.
     //   r < 1.5     equal launches of about two waves, so that every copy hides behind the next
     //               launch as long as copying is not slower than evaluating, and the last wave

@@ -481,8 +481,8 @@ class FusedEncoder:
         sizes = (ctypes.c_int * 16)()
         sms = torch.cuda.get_device_properties(self.device).multi_processor_count
         gbps = self.host_link_gbps
-        if self.quant != 0 and not self.rj_mode:         # two-board tiles: half the wave, 1.2 times the rate
-            sms, gbps = max(1, sms // 2), gbps / 1.2
+        if not self.rj_mode:                             # two-board tiles: half the wave, 1.27 times the rate
+            sms, gbps = max(1, sms // 2), gbps / 1.27
         k = _native.lib().bf_host_plan(int(n), sms, self._host_plan, gbps, sizes)
         _native.check(min(k, 0), "bf_host_plan")
         return list(sizes[:k])

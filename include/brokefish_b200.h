@@ -290,8 +290,8 @@ int bf_host_aligned(const void* boards, const void* control, const void* legal, 
 
 /* The launch sizes `bf_forward_host` uses for `n` positions under BF_OPT_HOST_PLAN `plan` when the
  * measured copy rate is `gbps` (0: not measured yet) and a wave of tiles is four positions on each of
- * `sm_count` SMs; a call that runs on two-board tiles (every arithmetic but fp16, no re-injection)
- * uses those of half the SMs and gbps / 1.2.  Writes up to 16 sizes, in launch order, summing to n,
+ * `sm_count` SMs; a call that runs on two-board tiles (without re-injection)
+ * uses those of half the SMs and gbps / 1.27.  Writes up to 16 sizes, in launch order, summing to n,
  * and returns how many; no GPU is touched.  No counterpart in the reference. */
 int bf_host_plan(int n, int sm_count, int plan, double gbps, int* sizes);
 
@@ -402,7 +402,8 @@ int bf_selftest_scales(int device, unsigned long long* differ);
  *   mode 0: s8 x s8, N=128, K=256     mode 1: u8 x s8, N=128, K=256
  *   mode 2: s8 x s8, N=192, K=256     mode 3: f16 x f16 -> f32, N=96, K=256
  *   mode 4: e4m3 x e4m3 -> f32, N=128, K=256
- * and the small tiles' weight-stationary ones, of M = 32 rows in the odd modes and 64 in the even ones:
+ * and weight-stationary ones of one SM, whose layout the small tiles' products by pairs of SMs share, of M = 32
+ * rows in the odd modes and 64 in the even ones:
  *   modes 5, 6: s8 x s8, N=256        modes 7, 8: u8 x s8, N=256
  *   modes 9, 10: f16 x f16 -> f16, N=256     modes 11, 12: e4m3 x e4m3 -> f32, N=256
  *   modes 13, 14: f16 x f16 -> f16, N=128
