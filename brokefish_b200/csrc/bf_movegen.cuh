@@ -546,8 +546,9 @@ constexpr unsigned kIndexBits = 0x0DFF0DFFu;
 // that does not add up then (colours or types in other slots, two pieces on a square) takes the general form.
 //
 // Bound by the integer pipe (the general form keeps it busy 87 % of the time with 3,600 instructions a board), which is why
-// every attack is a table's.  2^20 boards of random games, B200: 109 us, 161 in the general form (323 bytes a board: 3.1
-// and 2.1 TB/s of the 6.5 a copy reaches); 2,300 instructions a board, the integer pipe 68 % busy.
+// every attack is a table's.  The loops over the pawns stay loops: unrolled, the code misses the instruction cache (107 us).
+// 2^20 boards of random games, B200: 102 us, 161 in the general form (323 bytes a board: 3.3 and 2.1 TB/s of the 6.5 a
+// copy reaches); 2,400 instructions a board, the integer pipe 76 % busy.
 __device__ __forceinline__ bool board_moves(const unsigned* my, bool black, unsigned long long* to, unsigned long long* all,
                                             const MoveTables& t, bool& by_slot) {
     by_slot = true;
@@ -563,7 +564,7 @@ __device__ __forceinline__ bool board_moves(const unsigned* my, bool black, unsi
     // ---- the planes ----
     unsigned long long own_pawns = 0ull, e_pawns = 0ull;
     unsigned gone = 0u, stepped = 0u;                            // captured pieces, counted; enemy pawns that are flagged
-#pragma unroll
+#pragma unroll 1
     for (int q = 0; q < 4; ++q) {
         const unsigned a = mine[q], b = theirs[q];
         own_pawns |= both(expect(a, 0u));
@@ -675,7 +676,7 @@ __device__ __forceinline__ bool board_moves(const unsigned* my, bool black, unsi
     {
         const unsigned long long step = ~occ & target_mask, takes = opp & target_mask;
         const unsigned long long two = ~occ & (~occ << 8) & target_mask & 0xFF000000ull;
-#pragma unroll
+#pragma unroll 1
         for (int q = 0; q < 4; ++q) {
             const unsigned x = expect(mine[q], 0u);
 #pragma unroll
