@@ -2191,6 +2191,81 @@ __global__ void __launch_bounds__(128, 1) selftest_kernel(int mode, const uint8_
     if (threadIdx.x == 0 && *abort_flag != 0) atomicCAS(status, 0, *abort_flag);
 }
 
+// The same for the small tiles' products, of a pair of SMs: modes 15-19, 64 rows of A and half of the weight rows
+// in each, read out of tensor memory where bf_encoder_ws.cuh looks for them.
+constexpr int kPairSelftestModes = 20;
+__global__ void __launch_bounds__(128, 1) pair_selftest_kernel(int mode, const uint8_t* a, const uint8_t* w, uint32_t* out,
+                                                               int* status) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    const uint32_t smem = smem_u32(sm), rank = cluster_rank();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool halves = mode == 17 || mode == 19;                   // 15 s8, 16 u8, 17 f16, 18 e4m3, 19 f16 with N = 128
+    const int n = mode == 19 ? 128 : 256, slabs = halves ? 4 : 2;
+    const uint32_t w_half = n * 64, a_slab = 64 * 128;
+    constexpr uint32_t kW = kSelftestW, kBar = kSelftestBar;
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + kBar + 64);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + kBar + 68);
+    if (threadIdx.x == 0) {
+        mbar_init(smem + kBar, 2 - rank);                           // weights: the first SM hears of the second's
+        mbar_init(smem + kBar + 8, 1);
+        *abort_flag = 0;
+        fence_barrier_init();
+    }
+    if (warp == 0) tmem_alloc_pair(smem + kBar + 68, 256);
+    if (threadIdx.x < 64)
+        for (int s = 0; s < slabs; ++s)
+            for (int k = 0; k < 8; ++k)
+                *reinterpret_cast<uint4*>(sm + s * a_slab + sw_off(threadIdx.x, k)) =
+                    *reinterpret_cast<const uint4*>(a + static_cast<size_t>(64 * rank + threadIdx.x) * slabs * 128 + s * 128 + k * 16);
+    fence_proxy_async_smem();
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    if (threadIdx.x == 0) {
+        mbar_arrive_expect_tx(smem + kBar, w_half * slabs);
+        for (int s = 0; s < slabs; ++s) bulk_g2s(smem + kW + s * w_half, w + (2 * s + rank) * w_half, w_half, smem + kBar);
+        mbar_wait(smem + kBar, 0, abort_flag, kErrMmaWeights);
+        if (rank != 0) {
+            mbar_arrive_cluster(cluster_address(smem + kBar, 0));
+        } else {
+            tc_fence_after();
+            const uint32_t idesc = mode == 15   ? umma_idesc(kAccS32, kFmtS8, kFmtS8, 128, n)
+                                   : mode == 16 ? umma_idesc(kAccS32, kFmtU8, kFmtS8, 128, n)
+                                   : halves     ? umma_idesc(kAccF16, kFmtF16, kFmtF16, 128, n)
+                                                : umma_idesc(kAccF32, kFmtE4M3, kFmtE4M3, 128, n);
+            for (int s = 0; s < slabs; ++s) {
+                const uint64_t ad = umma_desc_k128(smem + s * a_slab), bd = umma_desc_k128(smem + kW + s * w_half);
+                for (int k = 0; k < 4; ++k) {
+                    const uint32_t more = (s | k) ? 1u : 0u;
+                    if (halves)          umma_pair_f16(tmem, ad + 2 * k, bd + 2 * k, idesc, more);
+                    else if (mode == 18) umma_pair_f8(tmem, ad + 2 * k, bd + 2 * k, idesc, more);
+                    else                 umma_pair_i8(tmem, ad + 2 * k, bd + 2 * k, idesc, more);
+                }
+            }
+            tc_commit_pair(smem + kBar + 8);
+        }
+    }
+    mbar_wait(smem + kBar + 8, 0, abort_flag, kErrRowAcc);
+    __syncwarp();
+    tc_fence_after();
+    const int row = 64 * rank + 32 * (warp & 1) + lane, first = (n / 2) * (warp >> 1);
+    for (int c0 = 0; c0 < n / 2; c0 += 32) {
+        uint32_t acc[32];
+        tmem_ld32(tmem + (static_cast<uint32_t>(32 * warp) << 16) + c0, acc);
+        tmem_wait_ld();
+        for (int i = 0; i < 32; ++i) out[static_cast<size_t>(row) * n + first + c0 + i] = acc[i];
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();
+    tc_fence_after();
+    if (warp == 0) tmem_dealloc_pair(tmem, 256);
+    if (threadIdx.x == 0 && *abort_flag != 0) atomicCAS(status, 0, *abort_flag);
+}
+
 }  // namespace bf
 
 // ==========================================================================================
@@ -2381,7 +2456,7 @@ cudaError_t launch_early(void (*kernel)(P...), unsigned grid, int threads, size_
 // so a launch that does not fill the GPU ends sooner.  A thread per board: a half to a quarter of the instructions, most
 // of all where legal words are made.  B200, us per launch in a graph, eight lanes / thread:
 //   boards                        1      4096     16384     32768     49152     65536    131072    262144   1048576
-//   legal words             2.8/3.5   4.0/6.8   8.6/7.4    14/9.3     21/11     26/12     50/18     99/32   384/109
+//   legal words             2.8/3.5   4.0/6.8   8.6/7.4    14/9.3     21/11     26/12     50/18     99/31   384/102
 //   key                     1.9/7.7    3.0/11    5.5/11    8.6/13     12/14     15/16     27/27     53/46   204/165
 //   move                    2.0/9.3    2.5/12    4.3/12    6.4/13    8.8/14     11/15     20/26     40/41   166/145
 //   move and key             3.1/16    4.2/21    8.4/21     13/24     19/26     24/29     45/50     89/83   350/305
@@ -3255,17 +3330,18 @@ int bf_selftest_scales(int device, unsigned long long* differ) {
 }
 
 int bf_selftest_umma(int device, int mode, const void* a, const void* w_image, void* out) {
-    if (mode < 0 || mode >= bf::kSelftestModes || a == nullptr || w_image == nullptr || out == nullptr)
+    if (mode < 0 || mode >= bf::kPairSelftestModes || a == nullptr || w_image == nullptr || out == nullptr)
         return fail(BF_EINVAL, "bad self-test argument");
+    const bool pair = mode >= bf::kSelftestModes;
     BF_ON_DEVICE(device);
     int* status = nullptr;
     BF_CUDA(cudaMalloc(&status, sizeof(int)));
     BF_CUDA(cudaMemset(status, 0, sizeof(int)));
-    BF_CUDA(cudaFuncSetAttribute(bf::selftest_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bf::kSelftestSmem));
-    bf::selftest_kernel<<<1, 128, bf::kSelftestSmem>>>(mode, static_cast<const uint8_t*>(a),
-                                           static_cast<const uint8_t*>(w_image),
-                                           static_cast<uint32_t*>(out), status);
-    cudaError_t e = cudaGetLastError();
+    const auto kernel = pair ? bf::pair_selftest_kernel : bf::selftest_kernel;
+    BF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bf::kSelftestSmem));
+    cudaError_t e = launch_early(kernel, pair ? 2 : 1, 128, bf::kSelftestSmem, pair ? 2 : 1, nullptr, false, mode,
+                                 static_cast<const uint8_t*>(a), static_cast<const uint8_t*>(w_image),
+                                 static_cast<uint32_t*>(out), status);
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     int st = 0;
     if (e == cudaSuccess) e = cudaMemcpy(&st, status, sizeof(int), cudaMemcpyDeviceToHost);

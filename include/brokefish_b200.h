@@ -407,6 +407,10 @@ int bf_selftest_scales(int device, unsigned long long* differ);
  *   modes 5, 6: s8 x s8, N=256        modes 7, 8: u8 x s8, N=256
  *   modes 9, 10: f16 x f16 -> f16, N=256     modes 11, 12: e4m3 x e4m3 -> f32, N=256
  *   modes 13, 14: f16 x f16 -> f16, N=128
+ * and the small tiles', of a pair of SMs with 64 rows in each, M = 128:
+ *   mode 15: s8 x s8, N=256           mode 16: u8 x s8, N=256
+ *   mode 17: f16 x f16 -> f16, N=256  mode 18: e4m3 x e4m3 -> f32, N=256
+ *   mode 19: f16 x f16 -> f16, N=128
  *   a        device, [M, K] row-major (1 byte or 2 bytes per element)
  *   w_image  device, K/ (128 B) stage images of [N, 128 B] (pack.py: sw128_image)
  *   out      device, [M, N] words: s32, f32, or f16 in the low half
