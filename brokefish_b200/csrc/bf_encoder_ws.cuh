@@ -998,6 +998,15 @@ __device__ __forceinline__ void row_tile(Row& c, const Params& p, int first) {
 }
 
 // ---- weight stream ----
+// Of `sent` stages the last ones' consumption, which no further stage is sent for, arrives too, from the first SM's
+// products at both SMs' barriers: waited for, so that no arrival is on its way when the next grid has its own barriers
+// here.  (Once a launch, beside the heads: 0.3 us of a batch of 1 (81.0), 5 us of 4096 (1538).)
+template <uint32_t kStages>
+__device__ __forceinline__ void drain(uint32_t smem, volatile int* abort_flag, uint32_t sent) {
+#pragma unroll 1
+    for (uint32_t i = sent > kStages ? sent - kStages : 0u; i < sent; ++i)
+        mbar_wait(bar(smem, B_EMPTY + i % kStages), (i / kStages) & 1u, abort_flag, kErrProducer);
+}
 // The blob's stages are the four-board kernel's: per head pair [Q 64 | K 64 | V 64 rows], then 128-row
 // units, two to each 256-row product.  A stage here is 256 rows of one K-slab, put together from four
 // or two of their pieces.  The whole warp walks the stages and waits; one elected lane issues.
@@ -1079,6 +1088,7 @@ __device__ __forceinline__ void producer(uint32_t smem, volatile int* abort_flag
         for (uint32_t st = 0; st < kHeadStages; ++st, src += kHeadStage)
             stage(bytes, [&](uint32_t dst, uint32_t full) { bulk_g2s(dst, src + skip, bytes, full); });
     }
+    drain<kStages>(smem, abort_flag, i);
     // after a time-out copies may still be in flight: a bounded while for them to land
     if (*abort_flag != 0) {
         const long long t0 = clock64();

@@ -136,3 +136,58 @@ def test_every_phase_is_waited_for(arithmetic, boards, source, tmp_path):
     assert set(waits) == set(done) and len(done) >= 7          # four slots, the operand, two hidden pairs
     for b, parities in waits.items():
         assert parities == [i & 1 for i in range(done[b])], b
+
+
+# ---- the weight ring ----
+
+RING = r"""
+#include <vector>
+struct Params { const uint8_t *wstream = nullptr, *lparams = nullptr; int n_layers = LAYERS, after_waves = 0; };
+enum { kErrProducer = 100, kQStage = 0, kRStage = 0, kHeadStage = 16384, kLparamStride = 0, SM_PAR = 0 };
+template <int AR_> struct RingCfg : Cfg<AR_> { static constexpr int kLayerStream = 0; };
+#define Cfg RingCfg
+static std::vector<int> sent(64), waited(64);
+static bool wrong = false;
+bool ring_wait(uint32_t b, uint32_t parity, volatile int*, int) {
+    if (b >= B_EMPTY && b < B_ACC) wrong |= ((unsigned)(waited[b - B_EMPTY]++) & 1u) != parity;
+    return true;
+}
+void ring_send(uint32_t b, uint32_t) { if (b < B_EMPTY) ++sent[b - B_FULL]; }
+template <class... T> void bulk_g2s(T&&...) {}
+void previous_grid_wait() {}
+void next_grid_may_start() {}
+long long clock64() { return 1ll << 40; }
+#define mbar_wait ring_wait
+#define mbar_arrive_expect_tx ring_send
+"""
+
+RING_MAIN = r"""
+int main() {
+    volatile int abort_flag = 0;
+    Params p;
+    producer<AR>(0, &abort_flag, p, TILES, RANK);
+    for (int k = 0; k < B_EMPTY; ++k)
+        if (sent[k] != waited[k]) { std::printf("place %d: sent %d times, waited for %d\n", k, sent[k], waited[k]); return 1; }
+    if (wrong) std::puts("a wait's parity is not the next phase's");
+    return wrong;
+}
+"""
+
+
+@pytest.mark.parametrize("tiles", [0, 1, 3])
+@pytest.mark.parametrize("stages", [6, 8])
+@pytest.mark.parametrize("arithmetic", ["kArInt8", "kArF16"])
+def test_the_weight_ring_is_drained(arithmetic, stages, tiles, tmp_path):
+    """Each stage's consumption arrives at a barrier of both SMs of a pair.  The producer waits for every one of
+    them, the last ones too: none may be on its way when the shared memory is another grid's."""
+    text = open(os.path.join(ROOT, "brokefish_b200", "csrc", "bf_encoder_ws.cuh")).read()
+    stubs = STUBS.replace("kStages = 4", f"kStages = {stages}")
+    parts = [definition(text, start) for start in ("__device__ __forceinline__ void drain(", "__device__ __forceinline__ void producer(")]
+    main = "\n".join([re.search(r"enum \{ B_FULL.*?\};", text).group(0), stubs, RING, *parts, RING_MAIN])
+    for rank in (0, 1):
+        src, exe = tmp_path / "ring.cpp", tmp_path / f"ring{rank}"
+        src.write_text(main)
+        subprocess.run(["g++", "-std=c++17", "-w", f"-DAR={arithmetic}", f"-DLAYERS={LAYERS}", f"-DTILES={tiles}", f"-DRANK={rank}",
+                        str(src), "-o", str(exe)], check=True)
+        out = subprocess.run([str(exe)], capture_output=True, text=True)
+        assert out.returncode == 0, out.stdout
