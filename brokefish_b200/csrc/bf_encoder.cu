@@ -2227,7 +2227,7 @@ __global__ void __launch_bounds__(128, 1) pair_selftest_kernel(int mode, const u
     if (threadIdx.x == 0) {
         mbar_arrive_expect_tx(smem + kBar, w_half * slabs);
         for (int s = 0; s < slabs; ++s) bulk_g2s(smem + kW + s * w_half, w + (2 * s + rank) * w_half, w_half, smem + kBar);
-        mbar_wait(smem + kBar, 0, abort_flag, kErrMmaWeights);
+        mbar_wait_cluster(smem + kBar, 0, abort_flag, kErrMmaWeights);
         if (rank != 0) {
             mbar_arrive_cluster(cluster_address(smem + kBar, 0));
         } else {

@@ -74,9 +74,9 @@ __device__ __forceinline__ uint32_t bar(uint32_t smem, int i) { return smem + SM
 // ---- what is different in a pair of SMs ----
 // These take the place of the functions of the same names for one SM in everything below: a product is the pair's,
 // its completion goes to the same barrier in both SMs, and an operand's or a weight stage's arrival to the first
-// SM's barrier, whose MMA warp issues the pair's products.  (Arrivals and waits at their default scope, the
-// operands made visible by the proxy fence before: at cluster scope an arrival costs some 500 cycles, a
-// wait more, and a two-board tile 147 us instead of 118.)
+// SM's barrier, whose MMA warp issues the pair's products.  What crosses from SM to SM -- an operand's rows, a weight stage --
+// is written or copied into the writer's own shared memory and read by the product's asynchronous proxy: a writer's proxy fence,
+// the arrival's release and the MMA warp's acquire at cluster scope.
 __device__ __forceinline__ void umma_ws_i8(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
     umma_pair_i8(d, a, b, idesc, accumulate);
 }
@@ -1112,7 +1112,7 @@ __device__ __forceinline__ void issue_unit(Issue& st, uint32_t d, uint32_t a_bas
     constexpr uint32_t kStages = Map<kAr>::kStages;
     for (int s = 0; s < slabs; ++s) {
         const uint32_t k = st.i % kStages;
-        mbar_wait(bar(st.smem, B_FULL + k), (st.i / kStages) & 1u, st.abort_flag, kErrMmaWeights);
+        mbar_wait_cluster(bar(st.smem, B_FULL + k), (st.i / kStages) & 1u, st.abort_flag, kErrMmaWeights);
         tc_fence_after();
         if (elect_one()) {
             const uint64_t ad = umma_desc_k128(a_base + s * slab), bd = umma_desc_k128(st.smem + Map<kAr>::SM_RING + k * kStage);
@@ -1140,7 +1140,7 @@ __device__ __forceinline__ void relay(uint32_t smem, volatile int* abort_flag, u
     }
 }
 __device__ __forceinline__ void issue_wait(const Issue& st, int b, uint32_t n) {
-    mbar_wait(bar(st.smem, b), n & 1u, st.abort_flag, kErrMmaOperand);
+    mbar_wait_cluster(bar(st.smem, b), n & 1u, st.abort_flag, kErrMmaOperand);
     tc_fence_after();
 }
 template <int NB, int kAr>

@@ -70,21 +70,37 @@ __device__ __forceinline__ uint32_t cluster_address(uint32_t saddr, uint32_t ran
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// An arrival that hands over what this SM's shared memory holds, at the barrier of any SM of the cluster;
+// `mbar_wait_cluster` there takes it.  At CTA scope, the default, neither orders memory between SMs.  Each is in two halves,
+// a fence for shared memory alone and a relaxed access to the barrier: `mbarrier.arrive.release.cluster` and a wait with
+// `.acquire.cluster` order global memory too (evaluations of 1 and 4096 positions, us: 107 and 1948; this way 82 and 1558,
+// of which the arrivals' fences are 1 and 15 and the waits' nothing).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
-    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+    asm volatile("fence.release.sync_restrict::shared::cta.cluster;" ::: "memory");
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
 // One try: the thread is parked by the hardware until the phase completes or the hardware's own time
 // limit has passed.  (With a suspend-time hint waiting warps come back later: 4 % of a one-board tile, 2 %
 // of a batch of 4096.)
+template <bool kCluster = false>
 __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity) {
     uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
+    if (kCluster)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
     return ok;
 }
 
@@ -94,15 +110,15 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity)
 //
 constexpr unsigned kWaitCycles = 400000000u;     // ~0.2 s at 2 GHz
 // `kSleep`: nanoseconds between tries, for a warp that waits long beside others that work.
-template <unsigned kSleep = 0>
+template <unsigned kSleep = 0, bool kCluster = false>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity,
                                           volatile int* abort_flag, int code) {
-    if (mbar_try_wait(bar, parity)) return true;
+    if (mbar_try_wait<kCluster>(bar, parity)) return true;
     const uint32_t flag = smem_u32(const_cast<int*>(abort_flag));
     uint32_t t0, t;
     asm volatile("mov.u32 %0, %%clock;" : "=r"(t0) :: "memory");
 #pragma unroll 1
-    while (!mbar_try_wait(bar, parity)) {
+    while (!mbar_try_wait<kCluster>(bar, parity)) {
         if (kSleep != 0) __nanosleep(kSleep);
         int aborted;
         asm volatile("ld.volatile.shared.b32 %0, [%1];" : "=r"(aborted) : "r"(flag) : "memory");
@@ -114,6 +130,13 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity,
         }
     }
     return true;
+}
+
+// The same where other SMs of the cluster arrive (`mbar_arrive_cluster`).
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, volatile int* abort_flag, int code) {
+    const bool there = mbar_wait<0, true>(bar, parity, abort_flag, code);
+    asm volatile("fence.acquire.sync_restrict::shared::cluster.cluster;" ::: "memory");
+    return there;
 }
 
 // Ask a 128-byte line of global memory into L1 (no register, no wait).

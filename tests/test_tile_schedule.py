@@ -34,7 +34,10 @@ template <int> struct Map { static constexpr uint32_t kStages = 4, SM_RING = 0, 
 struct Any { template <class T> operator T() const { return T(); } };
 uint32_t bar(uint32_t, int i) { return i; }
 void say(const char* what, int b, int parity) { if (b >= B_ACC) std::printf("%s %d %d\n", what, b, parity); }
-bool mbar_wait(uint32_t b, uint32_t parity, volatile int*, int) { say("wait", b, parity); return true; }
+// (barriers that both SMs of a pair arrive at are waited for across them, no others)
+void check(bool across, int b) { if (across != (b < B_EMPTY || (b >= B_A && b < B_MAX))) std::printf("scope %d 0\n", b); }
+bool mbar_wait(uint32_t b, uint32_t parity, volatile int*, int) { check(false, b); say("wait", b, parity); return true; }
+bool mbar_wait_cluster(uint32_t b, uint32_t parity, volatile int*, int) { check(true, b); say("wait", b, parity); return true; }
 void mbar_arrive(uint32_t b) { say("done", b, 0); }
 void tc_commit(uint32_t b) { say("done", b, 0); }
 bool elect_one() { return true; }
@@ -129,6 +132,7 @@ def test_every_phase_is_waited_for(arithmetic, boards, source, tmp_path):
     for lines in (rows, issue):
         for line in filter(None, lines):
             what, b, parity = line.split()
+            assert what != "scope", f"barrier {b} is waited for at the wrong scope"
             if what == "wait":
                 waits.setdefault(int(b), []).append(int(parity))
             else:
@@ -136,6 +140,16 @@ def test_every_phase_is_waited_for(arithmetic, boards, source, tmp_path):
     assert set(waits) == set(done) and len(done) >= 7          # four slots, the operand, two hidden pairs
     for b, parities in waits.items():
         assert parities == [i & 1 for i in range(done[b])], b
+
+
+def test_what_crosses_between_sms_is_ordered_at_cluster_scope():
+    """At the default scope, the CTA's, an arrival and a wait order nothing between two SMs."""
+    text = open(os.path.join(ROOT, "brokefish_b200", "csrc", "bf_ptx.cuh")).read()
+    arrive = definition(text, "__device__ __forceinline__ void mbar_arrive_cluster(")
+    assert arrive.index("fence.release.sync_restrict::shared::cta.cluster") < arrive.index("mbarrier.arrive.relaxed.cluster.shared::cluster")
+    wait = definition(text, "__device__ __forceinline__ bool mbar_wait_cluster(")
+    assert wait.index("mbar_wait<0, true>") < wait.index("fence.acquire.sync_restrict::shared::cluster.cluster")
+    assert "mbarrier.try_wait.parity.relaxed.cluster" in definition(text, "__device__ __forceinline__ uint32_t mbar_try_wait(")
 
 
 # ---- the weight ring ----
