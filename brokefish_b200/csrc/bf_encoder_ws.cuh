@@ -1214,9 +1214,11 @@ __global__ void __launch_bounds__(640, 1) encoder_ws_kernel(const Params p) {
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     // The grid before this one may still be running.  Only the producer goes on without it: the first weights are
-    // nobody's output.  One-board tiles beside this call's own two-board ones start without it, since that grid lets
-    // them start only when what came before it has ended (the fence is for what that left in this SM's cache); they wait
-    // for it at their own end.
+    // nobody's output.  One-board tiles beside this call's own two-board ones start without waiting for that grid, and
+    // wait for it at their own end.  Their inputs may be outputs of the grid before it.  That one has ended: the two-board grid
+    // lets them start only after its own wait, so what it wrote is in L2; the fence drops what this SM's L1 may hold from
+    // before; and inputs are read by plain loads alone (an `__ldg` or a `const __restrict__` could be served or
+    // moved past the fence).
     if (p.after_waves) {
         __threadfence();
     } else if (warp != kProducerWarp || p.leaf_count != nullptr) {

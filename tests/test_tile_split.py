@@ -2,6 +2,7 @@
 host.  Every board is in one tile, of one launch, whatever the batch, the option and the way the length is known;
 both SMs of a pair have as many tiles; and no launch that has boards is left out."""
 import os
+import re
 import subprocess
 
 import pytest
@@ -61,3 +62,17 @@ def test_every_board_is_in_one_tile(wave, one, tmp_path):
     subprocess.run(["g++", "-std=c++17", "-w", str(src), "-o", str(exe)], check=True)
     out = subprocess.run([str(exe), str(wave), str(one)], capture_output=True, text=True)
     assert out.returncode == 0, out.stdout
+
+
+def test_inputs_are_read_by_plain_loads():
+    """One-board tiles beside two-board ones read what an earlier grid wrote behind a fence instead of a wait, which
+    loads from memory that is taken to be constant are not bound by: only the network's tables are read so."""
+    source = lambda name: re.sub(r"//.*", "", open(os.path.join(ROOT, "brokefish_b200", "csrc", name)).read())
+    text, rest = source("bf_encoder_ws.cuh"), source("bf_encoder.cu")
+    loads = re.findall(r"__ldg\((?:reinterpret_cast<[^>]*>\()?([^;]*?)\)", text)
+    assert len(loads) >= 8 and all(re.match(r"p\.tail \+|emb \+|[gb]4 \+", what) for what in loads), loads
+    assert re.findall(r"\* (?:emb|g4|b4) = (?:reinterpret_cast<[^>]*>\()?(p\.\w+)", text) == ["p.tail", "p.tail", "p.emb"]
+    assert "__restrict__" not in text + definition(rest, "struct Params") + definition(rest, "__device__ __forceinline__ void expand_board(")
+    assert "__ldg" not in definition(rest, "__device__ __forceinline__ void expand_board(")
+    kernel = definition(text, "__global__ void __launch_bounds__(640, 1) encoder_ws_kernel(")
+    assert kernel.index("__threadfence()") < kernel.index("p.leaf_count != nullptr) n_eval")
