@@ -2539,33 +2539,39 @@ cudaError_t pairs_at_a_time(int quant, int sm_count, int* wave) {
     return e;
 }
 
-// An evaluation on one- and two-board tiles: one launch, or two where a batch ends in one-board tiles or where only
-// the device knows a leaf list's length (`Tiles`).  The one-board tiles then start as SMs become free, without
-// waiting for the launch beside them, and wait for it when they are done: what comes after them in the
-// stream comes after both.
+// How an evaluation is launched on one- and two-board tiles: the CTAs of the launch of either, 0 where there is none.
+// Two launches where a batch ends in one-board tiles or where only the device knows a leaf list's length (`Tiles`).
 // `wave`: CTAs that run at a time (`pairs_at_a_time`).
-cudaError_t launch_tiles(bf::Params p, int wave, int one_board, cudaStream_t stream, bool early, int* launches) {
-    const int n = p.n, quant = static_cast<int>(p.quant);
-    const bool expand = p.prior != nullptr;
-    p.wave_ctas = wave;
-    p.one_most = one_board;
-    const int full = n / (2 * wave), rest = n - full * 2 * wave;
+struct TileLaunches {
+    int twos, ones;
+};
+TileLaunches tile_launches(int n, int wave, int one_board, bool list) {
+    const int rest = n % (2 * wave);
     const bool singles = n <= static_cast<long>(one_board) * wave;
-    const bool list = p.leaf_count != nullptr;
-    const bool twos = !singles, ones = singles || (one_board > 0 && (list || (rest > 0 && rest <= wave)));
+    const bool ones = singles || (one_board > 0 && (list || (rest > 0 && rest <= wave)));
     auto ctas = [&](int boards, int per) {
         const long pairs = (boards + 2L * per - 1) / (2 * per);
         return static_cast<int>(2 * pairs < wave ? 2 * pairs : wave);
     };
+    return {singles ? 0 : ctas(n, 2), !ones ? 0 : ctas(singles || list ? n : rest, 1)};
+}
+// Of two launches the one-board tiles' starts as SMs become free, without waiting for the launch beside it, and waits for
+// that when it is done: what comes after them in the stream comes after both.
+cudaError_t launch_tiles(bf::Params p, int wave, int one_board, cudaStream_t stream, bool early, int* launches) {
+    const int quant = static_cast<int>(p.quant);
+    const bool expand = p.prior != nullptr;
+    p.wave_ctas = wave;
+    p.one_most = one_board;
+    const TileLaunches made = tile_launches(p.n, wave, one_board, p.leaf_count != nullptr);
     cudaError_t e = cudaSuccess;
-    *launches = (twos ? 1 : 0) + (ones ? 1 : 0);
-    if (twos)
-        e = launch_early(small_tile_kernel(quant, expand, 2), ctas(n, 2), bf::ws::threads(expand, 2), bf::ws::kSmemRequest, 2, stream,
+    *launches = (made.twos != 0) + (made.ones != 0);
+    if (made.twos != 0)
+        e = launch_early(small_tile_kernel(quant, expand, 2), made.twos, bf::ws::threads(expand, 2), bf::ws::kSmemRequest, 2, stream,
                          early, p);
-    if (ones && e == cudaSuccess) {
-        p.after_waves = twos ? 1 : 0;
-        e = launch_early(small_tile_kernel(quant, expand, 1), ctas(singles || list ? n : rest, 1), bf::ws::threads(expand, 1),
-                         bf::ws::kSmemRequest, 2, stream, early || twos, p);
+    if (made.ones != 0 && e == cudaSuccess) {
+        p.after_waves = made.twos != 0;
+        e = launch_early(small_tile_kernel(quant, expand, 1), made.ones, bf::ws::threads(expand, 1), bf::ws::kSmemRequest, 2, stream,
+                         early || made.twos != 0, p);
     }
     return e;
 }
@@ -3152,19 +3158,10 @@ long long bf_launch_count(const bf_handle* h) { return h ? h->launches : 0; }
 
 double bf_host_link_gbps(const bf_handle* h) { return h ? h->d2h_gbps : 0.0; }
 
-// The tiles of evaluations whose SMs work by themselves, by the tiles of the busiest SM: what launches went by
-// before SMs worked in pairs, kept with its results for callers that size their batches by it.  Pairs of SMs take one- and
-// two-board tiles in every arithmetic (`launch_tiles`): four boards took an SM 272 us in fp16, a pair's two-board tile
-// takes 116.
 int bf_tile_boards(int quant, int n, int sm_count, int one_board) {
     if (n < 1 || sm_count < 1) return fail(BF_EINVAL, "n and sm_count must be positive");
-    if (n <= static_cast<long>(one_board) * sm_count) return 1;
-    if (quant != 0) return 2;
-    static const int t[3] = {129, 152, 272};
-    const long full = n / (2 * sm_count), rest = n - full * 2 * sm_count;
-    const long small = full * t[1] + (rest == 0 ? 0 : rest <= sm_count && one_board > 0 ? t[0] : t[1]);
-    const long four = static_cast<long>((n + 4L * sm_count - 1) / (4L * sm_count)) * t[2];
-    return small <= four ? 2 : 4;
+    (void)quant;                      // (the same tiles in every arithmetic)
+    return tile_launches(n, sm_count > 1 ? sm_count & ~1 : 2, one_board, false).twos != 0 ? 2 : 1;
 }
 
 int bf_host_aligned(const void* boards, const void* control, const void* legal, const void* policy, const void* promo,

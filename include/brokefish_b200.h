@@ -274,11 +274,9 @@ int bf_set_option(bf_handle* h, int option, int value);
  * first call): what the plan of the next call is chosen by.  No counterpart in the reference. */
 double bf_host_link_gbps(const bf_handle* h);
 
-/* How many positions (1, 2 or 4) the largest tiles of an evaluation of `n` positions would hold if each of a
- * GPU's `sm_count` SMs worked by itself under BF_OPT_ONE_BOARD `one_board`; `quant` is the blob's arithmetic
- * (0 fp16).  SMs work in pairs: a plain evaluation runs on one- and two-board tiles in every arithmetic, and
- * nothing goes by this rule any more; its results are kept.  No GPU is touched.  No counterpart in the
- * reference. */
+/* How many positions (1 or 2) the largest tiles of an evaluation of `n` positions hold, without re-injection, on a GPU
+ * whose `sm_count` SMs run the evaluator in pairs, under BF_OPT_ONE_BOARD `one_board`.  `quant`, the blob's
+ * arithmetic (0 fp16), makes no difference.  No GPU is touched.  No counterpart in the reference. */
 int bf_tile_boards(int quant, int n, int sm_count, int one_board);
 
 /* Whether the kernels can read and write host buffers at these addresses themselves (1) or the host

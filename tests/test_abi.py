@@ -94,22 +94,16 @@ def test_which_host_addresses_the_kernels_use_themselves():
 
 def test_which_tiles_an_evaluation_runs_on():
     """BF_OPT_ONE_BOARD is a promise: at most so many boards per SM run on one-board tiles, in every
-    arithmetic, and none do where it is off; above that only fp16 batches that fill them run on four-board
-    tiles, by the tiles of the busiest SM."""
+    arithmetic, and none do where it is off; above that two boards to a tile.  SMs run in pairs: an odd one
+    counts for nothing."""
     L = _native.lib()
-    sms = 148
-    for quant in (0, 1, 2, 3, 4):
-        for one in (0, 1, 2, 8):
-            for n in (1, sms, one * sms, one * sms + 1, 4096, 1 << 20):
-                got = L.bf_tile_boards(quant, n, sms, one)
-                if 0 < n <= one * sms:
-                    assert got == 1, (quant, one, n)
-                elif n == 0:
-                    assert got == -1
-                else:
-                    assert got in ((2, 4) if quant == 0 else (2,)), (quant, one, n)
-    form = lambda n, one=1: L.bf_tile_boards(0, n, sms, one)
-    assert form(2 * sms) == 2 and form(2 * sms + 1) == 4 == form(2 * sms + 1, 0)     # 152 us; 152 + 129 against 272
-    assert form(4 * sms) == 4 and form(4 * sms + 1) == 2                             # 272; 2 x 152 + 129 against 2 x 272
-    assert form(4 * sms + 1, 0) == 2 and form(5 * sms, 0) == 2                       # 3 x 152
-    assert form(1) == 1 and form(1, 0) == 2
+    for sms in (2, 147, 148):
+        pairs = sms & ~1
+        for quant in (0, 1, 2, 3, 4):
+            for one in (0, 1, 2, 8):
+                for n in (1, pairs, one * pairs, one * pairs + 1, 2 * sms, 4 * sms, 5 * sms, 4096, 1 << 20):
+                    got = L.bf_tile_boards(quant, n, sms, one)
+                    if n == 0:
+                        assert got == -1
+                    else:
+                        assert got == (1 if n <= one * pairs else 2), (quant, one, n)

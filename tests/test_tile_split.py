@@ -1,6 +1,6 @@
-"""How a batch is split into one- and two-board tiles, on the CPU: the kernels' own `Tiles`, compiled for the
-host.  Every board is in one tile, of one launch, whatever the batch, the option and the way the length is known;
-both SMs of a pair have as many tiles; and no launch that has boards is left out."""
+"""How a batch is split into one- and two-board tiles, on the CPU: the kernels' own `Tiles` and the host's
+`tile_launches`, compiled together.  Every board is in one tile, of one launch, whatever the batch, the option and the
+way the length is known; both SMs of a pair have as many tiles; and no launch that has boards is left out."""
 import os
 import re
 import subprocess
@@ -16,11 +16,7 @@ MAIN = r"""
 #include <vector>
 #define __device__
 TILES
-// boards per CTA and launch as `launch_tiles` sizes them
-static int ctas(int boards, int per, int wave) {
-    const long pairs = (boards + 2L * per - 1) / (2 * per);
-    return (int)(2 * pairs < wave ? 2 * pairs : wave);
-}
+RULE
 template <int NB> int take(int n, int wave, int grid, int one, std::vector<int>& seen) {
     int boards = 0;
     for (int cta = 0; cta < grid; ++cta) {
@@ -37,12 +33,10 @@ int main(int argc, char** argv) {
     for (int capacity : {1, 2, 3, wave - 1, wave, wave + 1, 2 * wave - 1, 2 * wave, 2 * wave + 1, 3 * wave, 3 * wave + 1, 4 * wave + 7, 9 * wave})
         for (int list = 0; list < 2; ++list)
             for (int n = list ? 0 : capacity; n <= capacity; n += list ? 1 + n / 7 : 1) {
-                const bool singles = capacity <= one * wave;
-                const int rest = capacity % (2 * wave);
-                const bool twos = !singles, ones = singles || (one > 0 && (list || (rest > 0 && rest <= wave)));
+                const TileLaunches made = tile_launches(capacity, wave, one, list);
                 std::vector<int> seen(n + 1);
-                const int in_twos = twos ? take<2>(n, wave, ctas(capacity, 2, wave), one, seen) : 0;
-                const int in_ones = ones ? take<1>(n, wave, ctas(singles || list ? capacity : rest, 1, wave), one, seen) : 0;
+                const int in_twos = take<2>(n, wave, made.twos, one, seen);
+                const int in_ones = take<1>(n, wave, made.ones, one, seen);
                 for (int i = 0; i < n; ++i)
                     if (seen[i] != 1) { std::printf("board %d of %d (capacity %d): in %d tiles\n", i, n, capacity, seen[i]); return 1; }
                 // the option's promise, and the two-board tiles' share
@@ -58,7 +52,9 @@ int main(int argc, char** argv) {
 def test_every_board_is_in_one_tile(wave, one, tmp_path):
     text = open(os.path.join(ROOT, "brokefish_b200", "csrc", "bf_encoder_ws.cuh")).read()
     src, exe = tmp_path / "tiles.cpp", tmp_path / "tiles"
-    src.write_text(MAIN.replace("TILES", definition(text, "struct Tiles")))
+    rule = open(os.path.join(ROOT, "brokefish_b200", "csrc", "bf_encoder.cu")).read()
+    rule = definition(rule, "struct TileLaunches") + "\n" + definition(rule, "TileLaunches tile_launches(")
+    src.write_text(MAIN.replace("TILES", definition(text, "struct Tiles")).replace("RULE", rule))
     subprocess.run(["g++", "-std=c++17", "-w", str(src), "-o", str(exe)], check=True)
     out = subprocess.run([str(exe), str(wave), str(one)], capture_output=True, text=True)
     assert out.returncode == 0, out.stdout
