@@ -72,22 +72,11 @@ enum { B_FULL = 0, B_EMPTY = 8, B_ACC = 16, B_PAR = 20, B_A = 22, B_H = 23, B_MA
 __device__ __forceinline__ uint32_t bar(uint32_t smem, int i) { return smem + SM_BAR + 8u * i; }
 
 // ---- what is different in a pair of SMs ----
-// These take the place of the functions of the same names for one SM in everything below: a product is the pair's,
-// its completion goes to the same barrier in both SMs, and an operand's or a weight stage's arrival to the first
-// SM's barrier, whose MMA warp issues the pair's products.  What crosses from SM to SM -- an operand's rows, a weight stage --
-// is written or copied into the writer's own shared memory and read by the product's asynchronous proxy: a writer's proxy fence,
-// the arrival's release and the MMA warp's acquire at cluster scope.
-__device__ __forceinline__ void umma_ws_i8(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-    umma_pair_i8(d, a, b, idesc, accumulate);
-}
-__device__ __forceinline__ void umma_ws_f16(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-    umma_pair_f16(d, a, b, idesc, accumulate);
-}
-__device__ __forceinline__ void umma_ws_f8(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-    umma_pair_f8(d, a, b, idesc, accumulate);
-}
-__device__ __forceinline__ void tc_commit(uint32_t bar) { tc_commit_pair(bar); }
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) { mbar_arrive_cluster(cluster_address(bar, 0)); }
+// A product is the pair's (`umma_pair_*`), its completion goes to the same barrier in both SMs (`tc_commit_pair`), and an
+// operand's or a weight stage's arrival to the first SM's barrier, whose MMA warp issues the pair's products.  What crosses
+// from SM to SM -- an operand's rows, a weight stage -- is written or copied into the writer's own shared memory and read by the
+// product's asynchronous proxy: a writer's proxy fence, the arrival's release and the MMA warp's acquire at cluster scope.
+__device__ __forceinline__ void mbar_arrive_first(uint32_t bar) { mbar_arrive_cluster(cluster_address(bar, 0)); }
 
 // Which boards a CTA evaluates, tile by tile.  A launch's tiles hold `NB` boards each.  At most `one_most` boards
 // per CTA: one-board tiles alone.  More: as many whole waves of two-board tiles as there are, then what is left, one board
@@ -182,7 +171,7 @@ __device__ __forceinline__ void publish(const Row& c, int b) {
     tc_fence_before();
     fence_proxy_async_smem();
     __syncwarp();
-    if (c.lane == 0) mbar_arrive(bar(c.smem, b));
+    if (c.lane == 0) mbar_arrive_first(bar(c.smem, b));
 }
 __device__ __forceinline__ float lds_f(uint32_t addr) {
     float v;
@@ -207,7 +196,7 @@ __device__ __forceinline__ void max_to(uint32_t addr, float v) {
 __device__ __forceinline__ void max_to(uint32_t addr, float v, const Row& c, int chunk) {
     max_to(addr, v);
     __syncwarp();
-    if (c.lane == 0) bfptx::mbar_arrive(bar(c.smem, B_MAX + chunk));
+    if (c.lane == 0) mbar_arrive(bar(c.smem, B_MAX + chunk));
 }
 // The chunk's maxima are all there.
 template <int NB>
@@ -815,7 +804,7 @@ __device__ __forceinline__ void heads(const Row& c, const Params& p, int board, 
             sts128(c.h + kStageAux + 512u * O::board(c) + 16u * lane, make_uint4(v[0], v[1], v[2], v[3]));
         }
         __syncwarp();
-        if (lane == 0) bfptx::mbar_arrive(bar(c.smem, B_STAGED));
+        if (lane == 0) mbar_arrive(bar(c.smem, B_STAGED));
     }
     if (hc < 64) {
         if (valid && p.policy != nullptr) {
@@ -889,7 +878,7 @@ __device__ __forceinline__ void expander(uint32_t smem, uint8_t* smem_gen, uint3
             expand_board(p, board, lane, true, word, ctl, moves, h + kStagePolicy + 4096u * which + 128u * lane, lane & 7,
                          h + kStageAux + 512u * which + 16u * lane, smem_gen + SM_LIST + kListBytes * which);
         __syncwarp();
-        if (lane == 0) bfptx::mbar_arrive(bar(smem, B_EXPANDED));
+        if (lane == 0) mbar_arrive(bar(smem, B_EXPANDED));
     }
 }
 
@@ -1119,12 +1108,12 @@ __device__ __forceinline__ void issue_unit(Issue& st, uint32_t d, uint32_t a_bas
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk) {
                 const uint32_t accumulate = (more || (s | kk) != 0) ? 1u : 0u;
-                if (kKind == kKindF16)     umma_ws_f16(d, ad + 2 * kk, bd + 2 * kk, idesc, accumulate);
-                else if (kKind == kKindF8) umma_ws_f8(d, ad + 2 * kk, bd + 2 * kk, idesc, accumulate);
-                else                       umma_ws_i8(d, ad + 2 * kk, bd + 2 * kk, idesc, accumulate);
+                if (kKind == kKindF16)     umma_pair_f16(d, ad + 2 * kk, bd + 2 * kk, idesc, accumulate);
+                else if (kKind == kKindF8) umma_pair_f8(d, ad + 2 * kk, bd + 2 * kk, idesc, accumulate);
+                else                       umma_pair_i8(d, ad + 2 * kk, bd + 2 * kk, idesc, accumulate);
             }
-            tc_commit(bar(st.smem, B_EMPTY + k));
-            if (s == slabs - 1 && done >= 0) tc_commit(bar(st.smem, B_ACC + done));
+            tc_commit_pair(bar(st.smem, B_EMPTY + k));
+            if (s == slabs - 1 && done >= 0) tc_commit_pair(bar(st.smem, B_ACC + done));
         }
         st.i++;
     }
@@ -1136,7 +1125,7 @@ __device__ __forceinline__ void relay(uint32_t smem, volatile int* abort_flag, u
     for (uint32_t i = 0; i < stages; ++i) {
         const uint32_t k = i % kStages;
         mbar_wait(bar(smem, B_FULL + k), (i / kStages) & 1u, abort_flag, kErrMmaWeights);
-        if (elect_one()) mbar_arrive(bar(smem, B_FULL + k));
+        if (elect_one()) mbar_arrive_first(bar(smem, B_FULL + k));
     }
 }
 __device__ __forceinline__ void issue_wait(const Issue& st, int b, uint32_t n) {

@@ -332,7 +332,8 @@ __device__ __forceinline__ void umma_f8(uint32_t d_tmem, uint64_t adesc, uint64_
 }
 // The weight-stationary forms: M = 32 or 64 rows, N = 64, 128 or 256, the product laid out over all
 // 128 lanes (M = 32: quadrant q has columns q N / 4 .. ; M = 64: rows 32 (q & 1) .., columns
-// (q >> 1) N / 2 ..).  Operands, descriptors and accumulators as above.
+// (q >> 1) N / 2 ..).  Operands, descriptors and accumulators as above.  Only the self test issues them: the evaluator's
+// products are those of a pair of SMs below, which lie in tensor memory as these of M = 64 do.
 __device__ __forceinline__ void umma_ws_i8(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                            uint32_t accumulate) {
     asm volatile(

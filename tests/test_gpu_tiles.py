@@ -63,8 +63,9 @@ def test_the_instrumented_kernel_gives_the_small_tiles_outputs(arithmetic, nets,
 @pytest.mark.parametrize("rows", [32, 64])
 @pytest.mark.parametrize("what", ["s8", "u8", "f16", "e4m3", "f16 heads"])
 def test_weight_stationary_products(what, rows):
-    """The small tiles' tensor-core products, read where the kernel reads them, against exact host products:
-    bytes over their full range, fp16 and e4m3 operands whose sums are all representable."""
+    """Products of one SM, which the self test alone issues -- those of 64 rows lie in tensor memory as the evaluator's
+    products of a pair of SMs do (test_gpu_pairs.py) --, against exact host products: bytes over their full range, fp16 and
+    e4m3 operands whose sums are all representable."""
     from brokefish_b200 import _native
     from brokefish_b200.nn.pack import sw128_image
     rng = np.random.default_rng(rows)

@@ -38,15 +38,15 @@ void say(const char* what, int b, int parity) { if (b >= B_ACC) std::printf("%s 
 void check(bool across, int b) { if (across != (b < B_EMPTY || (b >= B_A && b < B_MAX))) std::printf("scope %d 0\n", b); }
 bool mbar_wait(uint32_t b, uint32_t parity, volatile int*, int) { check(false, b); say("wait", b, parity); return true; }
 bool mbar_wait_cluster(uint32_t b, uint32_t parity, volatile int*, int) { check(true, b); say("wait", b, parity); return true; }
-void mbar_arrive(uint32_t b) { say("done", b, 0); }
-void tc_commit(uint32_t b) { say("done", b, 0); }
+void mbar_arrive_first(uint32_t b) { say("done", b, 0); }
+void tc_commit_pair(uint32_t b) { say("done", b, 0); }
 bool elect_one() { return true; }
 template <class... T> constexpr uint32_t umma_idesc(T...) { return 0; }
 template <int NB, class F> void each_piece(uint32_t, F&&) {}
 #define NOTHING(name) template <class... T> Any name(T&&...) { return Any(); }
 #define NOTHING_NB(name) template <int NB, class... T> Any name(T&&...) { return Any(); }
 NOTHING(__syncwarp) NOTHING(tc_fence_after) NOTHING(tc_fence_before) NOTHING(fence_proxy_async_smem)
-NOTHING(umma_ws_f16) NOTHING(umma_ws_f8) NOTHING(umma_ws_i8) NOTHING(named_bar_sync) NOTHING(pair_sync) NOTHING(lds_f) NOTHING(load_bias)
+NOTHING(umma_pair_f16) NOTHING(umma_pair_f8) NOTHING(umma_pair_i8) NOTHING(named_bar_sync) NOTHING(pair_sync) NOTHING(lds_f) NOTHING(load_bias)
 NOTHING(sts128) NOTHING(load_query) NOTHING(scores) NOTHING(softmax) NOTHING(weighted_values) NOTHING(store_outputs)
 NOTHING(max_to) NOTHING(scale_s8) NOTHING(scale_u8) NOTHING(scale_e4m3) NOTHING_NB(amax_h2) NOTHING_NB(board_sync)
 NOTHING_NB(store_operand16)
