@@ -2361,7 +2361,7 @@ void* mapped_host(const void* p) {
     return a.type == cudaMemoryTypeHost ? a.devicePointer : nullptr;
 }
 
-// A host call on a small batch whose buffers are all pinned, device-mapped and aligned runs as one launch on
+// A host call on a small batch whose buffers are all pinned, device-mapped and aligned runs on
 // them: no copies, one synchronisation.  B200, us through the Python API, copied / in place:
 //   logits, positions    1: 117/102   16: 118/109   64: 125/124   148: 141/152   296: 194/237
 //   edge lists           1: 112/104   148: 135/121   296: 172/156   592: 305/283

@@ -25,11 +25,11 @@
 // The arithmetic is the four-board kernel's, bit for bit (the order of every sum included).
 //
 // Measured on one B200, us, against tiles of one SM (M = 32 and 64 by `tcgen05.mma.ws`): a one-board tile
-// int8 85 (91), e4m3 91 (101), fp16 103 (129); a two-board tile 114 (127), 115 (130), 117 (152); batch 4096 1544
-// (1677), 1547 (1735), 1620 (1877, then on four-board tiles).  What bounds it: the row warps, four to a scheduler and all
-// in the same phase, at 61 % of the issue slots in int8; of a one-board tile's 18,900 cycles per layer a row warp waits 3,600
-// for products, of a two-board tile's 26,000 4,800.  In fp16 and e4m3 a loop of large batches also runs into
-// the 1000 W power cap (1.75 to 1.87 GHz; int8 stays at 890 W and 1.965 GHz).
+// int8 86 (91), e4m3 94 (101), fp16 105 to 110 (129); a two-board tile 116 (127), 117 (130), 121 to 126 (152); batch 4096 1560
+// (1677), 1576 (1735), 1764 (1877, then on four-board tiles; 1620 before the power cap).  What bounds it: the row warps, four to
+// a scheduler and all in the same phase, at 61 % of the issue slots in int8; of a one-board tile's 19,300 cycles per layer a
+// row warp waits 4,400 for products, of a two-board tile's 26,500 5,700.  In fp16 and e4m3 a loop of large batches also runs
+// into the 1000 W power cap (1.75 to 1.87 GHz; int8 stays at 890 W and 1.965 GHz).
 #pragma once
 
 namespace bf {
@@ -720,8 +720,8 @@ __device__ __forceinline__ void prenorm_means(const Row& c, uint32_t alive, cons
 // The three logits, in one warp, while the head product runs: lane & 3 is the quarter of the columns
 // (32 q .. + 31 and 128 + 32 q .. + 31), lane >> 2 the sum: of the means, of their squares, of
 // means x gamma x value row k (with it gamma x value row k), of beta x value row k.  Out of line: inlined, this
-// head's code slows the networks that do not have it (4096 positions, int8 1690 us against 1675, with edge
-// lists 1748 against 1727).
+// head's code slows the networks that do not have it (4096 positions on tiles of one SM, int8 1690 us against 1675, with
+// edge lists 1748 against 1727).
 template <int NB>
 __device__ __noinline__ void prenorm_logits(const Row& c, const Params& p, float (&logit)[3]) {
     const uint32_t means = c.smem + SM_LIST + kListBytes * Own<NB>::board(c);
@@ -851,10 +851,10 @@ __device__ __forceinline__ void heads(const Row& c, const Params& p, int board, 
 }
 
 // The fused expansion has two warps of its own, one per board of a tile: they make the legal words
-// while the layers run and expand while the next tile begins.  On row warps, between the head product and
-// the next tile: 4096 positions 1793 us with the words given, 1839 with the moves generated; here 1743 and
-// 1766.  Where the rows' first FFN of the next
-// tile would overwrite the staged logits they wait for B_EXPANDED.
+// while the layers run and expand while the next tile begins.  4096 positions on tiles of one SM: 1743 us with the words given
+// and 1766 with the moves generated, where row warps between the head product and the next tile took 1793 and 1839; by
+// pairs of SMs 1591 and 1595.  Where the rows' first FFN of the next tile would overwrite the staged logits they
+// wait for B_EXPANDED.
 template <int NB>
 __device__ __forceinline__ void expander(uint32_t smem, uint8_t* smem_gen, uint32_t h, volatile int* abort_flag, const Params& p,
                                          const Tiles<NB>& tiles, int which, int lane) {

@@ -58,7 +58,7 @@ __device__ __forceinline__ unsigned long long king_pattern(unsigned long long b)
 // One sliding piece along one line without loops or fills: on the line's squares other than the
 // piece's own, subtracting the piece's bit from the occupancy flips exactly the squares up to and
 // including the first occupied one above it; the same on the bit-reversed board gives the squares
-// below it.
+// below it (the method published as o^(o-2r) and, with a reversed board, as hyperbola quintessence).
 __device__ __forceinline__ unsigned long long line_attacks(unsigned long long s, unsigned long long occ,
                                                            unsigned long long line_ex) {
     const unsigned long long o = occ & line_ex;
@@ -471,7 +471,8 @@ __device__ __noinline__ bool board_moves_any(const unsigned* my, bool black, uns
 // ---- the faster form of the same, for boards whose pieces are in the slots they start in ----
 // What a slider sees along one line, looked up: the line's squares are folded into one byte (a rank, a
 // diagonal and an antidiagonal hold one square of each file, so the fold is two logical operations and a
-// multiplication), whose inner six bits pick the answer for the slider's file.  A file is folded by rank.
+// multiplication), whose inner six bits pick the answer for the slider's file.  A file is folded by rank.  (The method is
+// published as kindergarten bitboards.)
 // Row 64 of the tables by square, and rank 8 of `up`, are empty: a captured piece looks there.
 struct alignas(16) MoveTables {
     unsigned long long up[9 * 64];               // [rank][ranks 2-7 occupied]: squares of the a file

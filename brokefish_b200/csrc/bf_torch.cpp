@@ -79,7 +79,8 @@ T* ptr(const Tensor& t) {
 }
 void* stream_of(c10::Device d) { return c10::cuda::getCurrentCUDAStream(d.index()).stream(); }
 // An output on the inputs' device.  Straight from the allocator: through the dispatcher, `at::empty`, one takes 0.73 us
-// instead of 0.52, and a ply of games makes ten of them in 20 us.
+// instead of 0.52, and a ply of games makes ten of them in 20 us.  (So dispatch modes do not see it, and
+// `torch.utils.deterministic.fill_uninitialized_memory` does not fill it; the kernels write every element.)
 Tensor output(at::IntArrayRef size, at::ScalarType type, const Tensor& like) {
     return at::detail::empty_cuda(size, type, like.device(), std::nullopt);
 }

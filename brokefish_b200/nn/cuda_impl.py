@@ -312,7 +312,7 @@ class FusedEncoder:
 
     def forward_full(self, boards, control, rep, legal=None):
         """Boards to ``(policy_logits [n,32,64] fp16, promo [n,32,4] fp16, value [n] fp32)``
-        in one launch on the current stream.
+        in one launch or two on the current stream.
 
         ``policy_logits`` is raw unless ``legal`` (``[n,32]`` int64 legality words, bit s of
         word p set when p->s is legal) is given, in which case illegal entries are -inf.
@@ -325,7 +325,7 @@ class FusedEncoder:
         return self.policy_out, self.promo_out, self.value_out
 
     def forward_priors(self, boards, control, rep, legal, e_cap: int = 96, logits: bool = False):
-        """Evaluate and expand in one launch: ``(prior [n,e_cap] fp16, move [n,e_cap] int16,
+        """Evaluate and expand in the same launches: ``(prior [n,e_cap] fp16, move [n,e_cap] int16,
         nedges [n] int32, value [n] fp32)`` — the edges of each position's search node in
         canonical order with their priors, what the reference's search computes from the
         logits in ``Search._expand`` (brokefish/search/torch_impl.py:962-1033).  ``legal`` is

@@ -68,7 +68,7 @@ int bf_destroy(bf_handle* h);
 /* Number of layers / value rows / value mode recorded in the handle's blob. */
 int bf_info(const bf_handle* h, int* n_layers, int* n_value, int* vmode);
 
-/* Boards to logits, one launch.  Replaces `model_forward(..., debug_stage=0)`
+/* Boards to logits, in one launch or two (a batch may end in tiles of its own size).  Replaces `model_forward(..., debug_stage=0)`
  * (csrc/encoder.cu:1770-1876).
  *   boards  [n,32] u16 piece words      control [n] i16      rep [n] u8
  *   legal   [n,32] u64 or NULL: bit s of word p set <=> move p->s is legal; when given,
@@ -78,7 +78,7 @@ int bf_forward(bf_handle* h, const uint16_t* boards, const int16_t* control,
                const uint8_t* rep, const uint64_t* legal, int n, void* policy, void* promo,
                float* value, void* stream);
 
-/* Evaluate and expand in one launch: besides (optionally) the logits, write for every position
+/* Evaluate and expand in the same launches: besides (optionally) the logits, write for every position
  * the edges of its search node and their priors, which the reference's search derives in a
  * kernel of its own from the logits (`Search._expand`, brokefish/search/torch_impl.py:962-1033;
  * `expand_node`, csrc/search.cuh:593-798).  `legal` [n,32]: bit s of word p says the piece in
@@ -121,8 +121,8 @@ int bf_forward_leaves(bf_handle* h, const uint16_t* boards, const int16_t* contr
  * castling the king's two-square move, en passant a pawn's diagonal move to an empty square);
  * `in_check` [n] (may be NULL) for the side to move.  The engine contract of the reference's
  * `movegen` (brokefish/env/torch_impl.py:254-291; csrc/movegen.cuh): the input generator of the
- * evaluator's legality words and of the search's node masks.  One thread per board, one launch on
- * `stream`; needs no handle. */
+ * evaluator's legality words and of the search's node masks.  One launch on `stream`, by eight
+ * lanes per board up to 12,288 boards and by one thread per board above; needs no handle. */
 int bf_movegen(int device, const uint16_t* boards, const int16_t* control, int n, uint64_t* mask,
                unsigned char* in_check, void* stream);
 
@@ -234,7 +234,7 @@ int bf_forward_capture(bf_handle* h, const uint16_t* boards, const int16_t* cont
  * device, runs the evaluator as a few launches of shrinking size (the last one a single wave of
  * tiles), copies each launch's three outputs back on a second stream while the next launch
  * computes -- only the last wave's copy is exposed -- and synchronises.  A small batch in pinned,
- * device-mapped and aligned buffers (bf_host_aligned) runs as one launch that reads and writes them
+ * device-mapped and aligned buffers (bf_host_aligned) runs in launches that read and write them
  * in place; the buffers may start anywhere otherwise.
  * Device staging buffers are owned by the handle and grow to the largest `n` seen. */
 int bf_forward_host(bf_handle* h, const uint16_t* boards, const int16_t* control,
